@@ -69,16 +69,6 @@ omv_status guarded(F&& f)
     }
 }
 
-// PinholeCamera::stop (PinholeCamera.cpp:70-78): rgb / count, alpha 1
-__global__ void k_resolve(int64_t n, const double* sum, const uint32_t* count, float4* out)
-{
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double c = (double)count[i];
-    const double s = c < 0.5 ? 1.0 : 1.0 / c;
-    out[i] = make_float4((float)(sum[3 * i] * s), (float)(sum[3 * i + 1] * s), (float)(sum[3 * i + 2] * s), 1.0f);
-}
-
 struct DevTmp {
     void* p = nullptr;
     explicit DevTmp(size_t bytes) { OMV_CUDA(cudaMalloc(&p, bytes ? bytes : 16)); }
@@ -317,8 +307,9 @@ omv_status omv_render(omv_scene* scene, const omv_camera* camera, const omv_para
         omv::render_frame(*s.h, *camera, *params, s.sum, params->accumulate_variance ? s.sumsq : nullptr, s.count, st,
                           stats);
         if (image_rgba) {
-            k_resolve<<<(int)((npix + 255) / 256), 256, 0, st>>>(npix, s.sum, s.count, s.image);
-            OMV_CUDA(cudaGetLastError());
+            // PinholeCamera::stop (PinholeCamera.cpp:70-78): rgb / count, alpha 1
+            omv::develop_film(s.sum, s.count, camera->width, camera->height, 1.0f, 1.0f,
+                              reinterpret_cast<float*>(s.image), nullptr, nullptr, false, st);
             OMV_CUDA(cudaMemcpyAsync(image_rgba, s.image, sizeof(float4) * npix, cudaMemcpyDeviceToHost, st));
         }
         if (sum_rgb) OMV_CUDA(cudaMemcpyAsync(sum_rgb, s.sum, sizeof(double) * 3 * npix, cudaMemcpyDeviceToHost, st));

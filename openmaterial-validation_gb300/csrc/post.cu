@@ -9,7 +9,8 @@
 //               every channel clamped to [0, 1], alpha 1
 //   k_median3   SimpleDenoiserMedian<1> (Denoiser.h:24-64): per-channel median
 //               of the 3x3 window on pixels one away from every edge (alpha 1
-//               there), the border copied; a shared-memory tile per block
+//               there), the border copied; sorted row triples shared by the
+//               windows of a column
 //   k_median    the same for windows of 5x5 and 7x7
 //   k_rgba8     saveImage's conversion (main.cpp:92): unsigned char(255 f),
 //               rows optionally flipped (ImageSaver::flipVerticallyOnWrite)
@@ -65,24 +66,73 @@ __device__ __forceinline__ uchar4 to_u8x4(float4 p)
     return make_uchar4(to_u8(p.x), to_u8(p.y), to_u8(p.z), to_u8(p.w));
 }
 
-__global__ void k_develop(const double* __restrict__ sum, const uint32_t* __restrict__ count, int w, int h, float A,
-                          float gamma, float4* __restrict__ linear, float4* __restrict__ toned,
-                          uchar4* __restrict__ rgba8, int flip)
+// (float)(x * (1.0 / c)) of a film sum x (its 64 bits) by FP32 and integer
+// arithmetic, where (sh, sl) is 1 / c as a float-float: x is split into its
+// leading 24 bits h and the rest l, the product is p + e with p = h sh and e
+// its rounding error and the cross terms, within 2^-44 |p| of the exact value
+// (the FP64 expression is within 2^-51).  When adding 2^-42 |p| either way
+// gives the same float, that is the FP64 expression's value too; about one sum
+// in 2^17 lies closer to a rounding boundary, and false sends it, and
+// sums beyond 2^-70 .. 2^90, to the FP64 arithmetic.
+__device__ __forceinline__ bool scaled(unsigned long long x, float sh, float sl, float& out)
 {
-    const int64_t n = (int64_t)w * h;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double c = (double)count[i];
-        const double s = c < 0.5 ? 1.0 : __drcp_rn(c);  // 1.0 / c, the same correctly rounded bits
-        const float4 lin = make_float4((float)(sum[3 * i] * s), (float)(sum[3 * i + 1] * s),
-                                       (float)(sum[3 * i + 2] * s), 1.0f);
-        if (linear) linear[i] = lin;
-        if (!toned && !rgba8) continue;
-        const float4 t = gamma_correct(lin, A, gamma);
-        if (toned) toned[i] = t;
-        if (rgba8) {  // i < 2^31: a 32-bit division for the row
-            const int64_t y = (int64_t)((uint32_t)i / (uint32_t)w), x = i - y * w;
-            rgba8[flip ? (h - 1 - y) * (int64_t)w + x : i] = to_u8x4(t);
-        }
+    const uint32_t hi = (uint32_t)(x >> 32), lo = (uint32_t)x;
+    const uint32_t sign = hi & 0x80000000u, ex = (hi >> 20) & 0x7FFu;
+    if (((hi ^ sign) | lo) == 0u) {
+        out = __uint_as_float(sign);
+        return true;
+    }
+    if (ex - (1023u - 70u) > 160u) return false;
+    const uint32_t e32 = (ex - (1023u - 127u)) << 23;  // 2^(ex - 1023) as a float
+    const float h = __uint_as_float(e32 | ((hi & 0xFFFFFu) << 3) | (lo >> 29));
+    const float l = __fmul_rn((float)(lo & 0x1FFFFFFFu), __uint_as_float(e32 - (52u << 23)));
+    const float p = __fmul_rn(h, sh);
+    const float e = fmaf(l, sh, fmaf(h, sl, fmaf(h, sh, -p)));
+    const float tol = __fmul_rn(p, 0x1p-42f);
+    const float r0 = __fadd_rn(p, __fsub_rn(e, tol)), r1 = __fadd_rn(p, __fadd_rn(e, tol));
+    out = __uint_as_float(__float_as_uint(r0) | sign);
+    return r0 == r1;
+}
+
+// PinholeCamera::stop of one pixel: rgb / count as sum * (1.0 / count)
+static __device__ __noinline__ float4 normalised_fp64(const double* __restrict__ sum, uint32_t count)
+{
+    const double c = (double)count;
+    const double s = c < 0.5 ? 1.0 : __drcp_rn(c);  // 1.0 / c, the same correctly rounded bits
+    return make_float4((float)(sum[0] * s), (float)(sum[1] * s), (float)(sum[2] * s), 1.0f);
+}
+
+__device__ __forceinline__ float4 normalised(const double* __restrict__ sum, uint32_t count)
+{
+    const unsigned long long* q = reinterpret_cast<const unsigned long long*>(sum);
+    const unsigned long long x = q[0], y = q[1], z = q[2];
+    const float c = count == 0u ? 1.0f : (float)count;
+    const float sh = __fdiv_rn(1.0f, c);
+    const float sl = __fmul_rn(fmaf(-sh, c, 1.0f), sh);
+    float4 v;
+    v.w = 1.0f;
+    const bool ok = scaled(x, sh, sl, v.x) & scaled(y, sh, sl, v.y) & scaled(z, sh, sl, v.z);
+    return ok && count < (1u << 24) ? v : normalised_fp64(sum, count);  // the count is exact as a float
+}
+
+// Bound by HBM (28 B read, up to 36 B written per pixel) once the arithmetic
+// of the normalisation is off the FP64 pipe, which runs at about two lanes per
+// SM and cycle: 1920x1080 with all three outputs, 51.6 us with three FP64
+// multiplies, three conversions and the reciprocal per pixel, 27.3 so.
+__global__ void __launch_bounds__(256) k_develop(const double* __restrict__ sum, const uint32_t* __restrict__ count,
+                                                 int w, int h, float A, float gamma, float4* __restrict__ linear,
+                                                 float4* __restrict__ toned, uchar4* __restrict__ rgba8, int flip)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (int64_t)w * h) return;
+    const float4 lin = normalised(sum + 3 * i, count[i]);
+    if (linear) linear[i] = lin;
+    if (!toned && !rgba8) return;
+    const float4 t = gamma_correct(lin, A, gamma);
+    if (toned) toned[i] = t;
+    if (rgba8) {  // i < 2^31: a 32-bit division for the row
+        const int64_t y = (int64_t)((uint32_t)i / (uint32_t)w), x = i - y * w;
+        rgba8[flip ? (h - 1 - y) * (int64_t)w + x : i] = to_u8x4(t);
     }
 }
 
@@ -92,16 +142,29 @@ __global__ void k_tonemap(float4* __restrict__ img, int64_t n, float A, float ga
         img[i] = gamma_correct(img[i], A, gamma);
 }
 
-__global__ void k_rgba8(const float4* __restrict__ in, uchar4* __restrict__ out, int w, int h, int flip)
+// four pixels per thread, all loaded before the first is converted (one load
+// in flight per thread left it waiting for latency: 1920x1080 9.8 -> 8.4 us)
+constexpr int kRgbaPixels = 4;
+
+__global__ void __launch_bounds__(256) k_rgba8(const float4* __restrict__ in, uchar4* __restrict__ out, int w, int h,
+                                               int flip)
 {
     const int64_t n = (int64_t)w * h;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i0 = (int64_t)blockIdx.x * blockDim.x * kRgbaPixels + threadIdx.x;
+    float4 v[kRgbaPixels];
+#pragma unroll
+    for (int k = 0; k < kRgbaPixels; ++k) {
+        const int64_t i = i0 + k * blockDim.x;
+        if (i < n) v[k] = in[i];
+    }
+#pragma unroll
+    for (int k = 0; k < kRgbaPixels; ++k) {
+        const int64_t i = i0 + k * blockDim.x;
+        if (i >= n) return;
         const int64_t y = (int64_t)((uint32_t)i / (uint32_t)w), x = i - y * w;  // i < 2^31
-        out[flip ? (h - 1 - y) * (int64_t)w + x : i] = to_u8x4(in[i]);
+        out[flip ? (h - 1 - y) * (int64_t)w + x : i] = to_u8x4(v[k]);
     }
 }
-
-constexpr int kTileW = 32, kTileH = 8;
 
 __device__ __forceinline__ void order(float& a, float& b)
 {
@@ -125,39 +188,99 @@ __device__ __forceinline__ float median9(float p[9])
     return p[4];
 }
 
-// one 32x8 block of output pixels from a (32+2)x(8+2) tile in shared memory;
-// tile loads are clamped to the image, and only border pixels (which copy
-// their input) would see a clamped value
-__global__ void __launch_bounds__(kTileW* kTileH) k_median3(const float4* __restrict__ in, float4* __restrict__ out,
-                                                            int w, int h)
+__device__ __forceinline__ float med3(float a, float b, float c)
 {
-    __shared__ float4 tile[kTileH + 2][kTileW + 2];
-    const int x0 = blockIdx.x * kTileW - 1, y0 = blockIdx.y * kTileH - 1;
-    const int tid = threadIdx.y * kTileW + threadIdx.x;
-    for (int k = tid; k < (kTileW + 2) * (kTileH + 2); k += kTileW * kTileH) {
-        const int ty = k / (kTileW + 2), tx = k - ty * (kTileW + 2);
-        const int gx = min(max(x0 + tx, 0), w - 1), gy = min(max(y0 + ty, 0), h - 1);
-        tile[ty][tx] = in[(size_t)gy * w + gx];
-    }
-    __syncthreads();
-    const int x = blockIdx.x * kTileW + threadIdx.x, y = blockIdx.y * kTileH + threadIdx.y;
-    if (x >= w || y >= h) return;
-    const int cx = threadIdx.x + 1, cy = threadIdx.y + 1;
-    if (x < 1 || y < 1 || x >= w - 1 || y >= h - 1) {
-        out[(size_t)y * w + x] = tile[cy][cx];
-        return;
-    }
+    return fmaxf(fminf(a, b), fminf(fmaxf(a, b), c));
+}
+
+// the median of a pixel's window by the network above, for windows that may
+// hold a NaN (its result then depends on the order of the exchanges)
+static __device__ __noinline__ float4 median3_any(const float4* __restrict__ in, int w, int x, int y)
+{
     float r[9], g[9], b[9];
 #pragma unroll
     for (int dy = 0; dy < 3; ++dy)
 #pragma unroll
         for (int dx = 0; dx < 3; ++dx) {
-            const float4 p = tile[cy - 1 + dy][cx - 1 + dx];
+            const float4 p = in[(size_t)(y - 1 + dy) * w + (x - 1 + dx)];
             r[3 * dy + dx] = p.x;
             g[3 * dy + dx] = p.y;
             b[3 * dy + dx] = p.z;
         }
-    out[(size_t)y * w + x] = make_float4(median9(r), median9(g), median9(b), 1.0f);
+    return make_float4(median9(r), median9(g), median9(b), 1.0f);
+}
+
+// one channel of a row's three horizontal neighbours, sorted
+struct Sorted3 {
+    float lo, mid, hi;
+};
+__device__ __forceinline__ Sorted3 sort3(float a, float b, float c)
+{
+    return Sorted3{fminf(fminf(a, b), c), med3(a, b, c), fmaxf(fmaxf(a, b), c)};
+}
+// the median of nine from three sorted triples: the middle of the largest
+// minimum, the middle median and the smallest maximum
+__device__ __forceinline__ float median9(Sorted3 p, Sorted3 q, Sorted3 r)
+{
+    return med3(fmaxf(fmaxf(p.lo, q.lo), r.lo), med3(p.mid, q.mid, r.mid), fminf(fminf(p.hi, q.hi), r.hi));
+}
+
+struct MedianRow {
+    Sorted3 r, g, b;
+    float4 mid;   // the row's own pixel
+    bool plain;   // no NaN among the nine values (an infinity may clear it too)
+};
+__device__ __forceinline__ MedianRow median_row(const float4* __restrict__ row)
+{
+    const float4 a = row[-1], b = row[0], c = row[1];
+    MedianRow m;
+    m.r = sort3(a.x, b.x, c.x);
+    m.g = sort3(a.y, b.y, c.y);
+    m.b = sort3(a.z, b.z, c.z);
+    m.mid = b;
+    const float s = ((a.x + a.y + a.z) + (b.x + b.y + b.z)) + (c.x + c.y + c.z);
+    m.plain = s == s;
+    return m;
+}
+
+// 3x3 median.  A thread walks kMedRows rows of one column: each row's three
+// neighbours are loaded and sorted once and serve the three windows that
+// contain the row, about 17 min/max per channel and pixel where the
+// 19-exchange network of every pixel by itself takes 38.  Neighbouring lanes
+// read the same lines, so the loads need no shared tile.  1920x1080: 23.9 us
+// with a 34x10 tile and the full network per pixel (ALU bound), 20.2 so.
+constexpr int kMedRows = 4, kMedThreads = 128;
+
+__global__ void __launch_bounds__(kMedThreads) k_median3(const float4* __restrict__ in, float4* __restrict__ out,
+                                                         int w, int h)
+{
+    // one-dimensional grid (any width and height): column blocks, then row groups
+    const uint32_t cols = ((uint32_t)w + kMedThreads - 1) / kMedThreads, group = blockIdx.x / cols;
+    const int x = (int)((blockIdx.x - group * cols) * kMedThreads + threadIdx.x);
+    const int y0 = (int)group * kMedRows, y1 = min(y0 + kMedRows, h);
+    if (x >= w) return;
+    if (x == 0 || x == w - 1) {
+        for (int y = y0; y < y1; ++y) out[(size_t)y * w + x] = in[(size_t)y * w + x];
+        return;
+    }
+    MedianRow p = median_row(in + (size_t)max(y0 - 1, 0) * w + x);
+    MedianRow q = median_row(in + (size_t)y0 * w + x);
+#pragma unroll
+    for (int k = 0; k < kMedRows; ++k) {
+        const int y = y0 + k;
+        if (y >= y1) break;
+        const MedianRow r = median_row(in + (size_t)min(y + 1, h - 1) * w + x);
+        float4 o = q.mid;  // the border rows copy their input
+        if (y > 0 && y < h - 1) {
+            if (p.plain && q.plain && r.plain)
+                o = make_float4(median9(p.r, q.r, r.r), median9(p.g, q.g, r.g), median9(p.b, q.b, r.b), 1.0f);
+            else
+                o = median3_any(in, w, x, y);
+        }
+        out[(size_t)y * w + x] = o;
+        p = q;
+        q = r;
+    }
 }
 
 // the value with (n - 1) / 2 window elements before it in sorted order (ties
@@ -168,17 +291,78 @@ __device__ float select_median(const float* v)
     constexpr int target = (N - 1) / 2;
     for (int a = 0; a < N; ++a) {
         int before = 0;
-#pragma unroll
         for (int b = 0; b < N; ++b) before += (v[b] < v[a] || (v[b] == v[a] && b < a)) ? 1 : 0;
         if (before == target) return v[a];
     }
     return v[target];
 }
 
+// the median of a window that holds a NaN
 template <int H>
-__global__ void k_median(const float4* __restrict__ in, float4* __restrict__ out, int w, int h)
+__device__ __noinline__ float4 median_any(const float4* __restrict__ in, int w, int x, int y)
 {
     constexpr int S = 2 * H + 1;
+    float v[3][S * S];
+    for (int dy = 0; dy < S; ++dy)
+        for (int dx = 0; dx < S; ++dx) {
+            const float4 p = in[(size_t)(y - H + dy) * w + (x - H + dx)];
+            v[0][S * dy + dx] = p.x;
+            v[1][S * dy + dx] = p.y;
+            v[2][S * dy + dx] = p.z;
+        }
+    return make_float4(select_median<S * S>(v[0]), select_median<S * S>(v[1]), select_median<S * S>(v[2]), 1.0f);
+}
+
+// moves the smallest of p[0 .. K) to p[0] and the largest to p[K - 1]
+template <int K>
+__device__ __forceinline__ void extremes(float* p)
+{
+#pragma unroll
+    for (int i = 0; i < K / 2; ++i) order(p[i], p[K - 1 - i]);
+#pragma unroll
+    for (int i = 1; i < (K + 1) / 2; ++i) order(p[0], p[i]);
+#pragma unroll
+    for (int i = K / 2; i < K - 1; ++i) order(p[i], p[K - 1]);
+}
+
+// One step of the selection: with K values kept, the extremes go and the
+// window's element `at` comes in, until three are left.
+template <int H, int K>
+struct MedianStep {
+    static __device__ __forceinline__ void run(float* r, float* g, float* b, const float4* __restrict__ in, int w,
+                                               bool& plain)
+    {
+        constexpr int S = 2 * H + 1, N = S * S, at = N / 2 + 2 + (N / 2 + 2 - K);
+        extremes<K>(r);
+        extremes<K>(g);
+        extremes<K>(b);
+        const float4 p = in[(ptrdiff_t)(at / S - H) * w + (at % S - H)];
+        plain = plain && p.x == p.x && p.y == p.y && p.z == p.z;
+        r[0] = p.x;
+        g[0] = p.y;
+        b[0] = p.z;
+        MedianStep<H, K - 1>::run(r, g, b, in, w, plain);
+    }
+};
+template <int H>
+struct MedianStep<H, 3> {
+    static __device__ __forceinline__ void run(float* r, float* g, float* b, const float4* __restrict__, int, bool&)
+    {
+        extremes<3>(r);
+        extremes<3>(g);
+        extremes<3>(b);
+    }
+};
+
+// 5x5 and 7x7 medians by forgetful selection: of the first half of the window
+// and two more, neither the smallest nor the largest can be the median, so
+// both are dropped, one more element is taken in, and so on.  1920x1080, 5x5:
+// 673 us with a rank count of every element (N^2 comparisons per channel), 99
+// so; 7x7: 2736 and 364.
+template <int H>
+__global__ void __launch_bounds__(256) k_median(const float4* __restrict__ in, float4* __restrict__ out, int w, int h)
+{
+    constexpr int S = 2 * H + 1, N = S * S, K = N / 2 + 2;
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= w || y >= h) return;
     const size_t o = (size_t)y * w + x;
@@ -186,15 +370,18 @@ __global__ void k_median(const float4* __restrict__ in, float4* __restrict__ out
         out[o] = in[o];
         return;
     }
-    float r[S * S], g[S * S], b[S * S];
-    for (int dy = 0; dy < S; ++dy)
-        for (int dx = 0; dx < S; ++dx) {
-            const float4 p = in[(size_t)(y - H + dy) * w + (x - H + dx)];
-            r[S * dy + dx] = p.x;
-            g[S * dy + dx] = p.y;
-            b[S * dy + dx] = p.z;
-        }
-    out[o] = make_float4(select_median<S * S>(r), select_median<S * S>(g), select_median<S * S>(b), 1.0f);
+    float r[K], g[K], b[K];
+    bool plain = true;
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+        const float4 p = in[o + (ptrdiff_t)(i / S - H) * w + (i % S - H)];
+        plain = plain && p.x == p.x && p.y == p.y && p.z == p.z;
+        r[i] = p.x;
+        g[i] = p.y;
+        b[i] = p.z;
+    }
+    MedianStep<H, K>::run(r, g, b, in + o, w, plain);
+    out[o] = plain ? make_float4(r[1], g[1], b[1], 1.0f) : median_any<H>(in, w, x, y);
 }
 
 int stream_grid(int64_t n, int threads)
@@ -344,9 +531,9 @@ void develop_film(const double* d_sum, const uint32_t* d_count, int w, int h, fl
     check_image(w, h);
     if (!d_sum || !d_count) throw ArgError("develop: film sums and counts are required");
     const int64_t n = (int64_t)w * h;
-    k_develop<<<stream_grid(n, 256), 256, 0, st>>>(d_sum, d_count, w, h, A, gamma, reinterpret_cast<float4*>(d_linear),
-                                                  reinterpret_cast<float4*>(d_toned),
-                                                  reinterpret_cast<uchar4*>(d_rgba8), flip ? 1 : 0);
+    k_develop<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
+        d_sum, d_count, w, h, A, gamma, reinterpret_cast<float4*>(d_linear), reinterpret_cast<float4*>(d_toned),
+        reinterpret_cast<uchar4*>(d_rgba8), flip ? 1 : 0);
     OMV_CUDA(cudaGetLastError());
 }
 
@@ -367,8 +554,8 @@ void denoise_median(const float* d_in, float* d_out, int w, int h, int half, cud
     const auto* in = reinterpret_cast<const float4*>(d_in);
     auto* out = reinterpret_cast<float4*>(d_out);
     if (half == 1) {
-        const dim3 g((w + kTileW - 1) / kTileW, (h + kTileH - 1) / kTileH);
-        k_median3<<<g, dim3(kTileW, kTileH), 0, st>>>(in, out, w, h);
+        const int64_t blocks = ((int64_t)w + kMedThreads - 1) / kMedThreads * (((int64_t)h + kMedRows - 1) / kMedRows);
+        k_median3<<<(unsigned)blocks, kMedThreads, 0, st>>>(in, out, w, h);
     } else if (half == 2 || half == 3) {
         const dim3 b(16, 8), g((w + 15) / 16, (h + 7) / 8);
         if (half == 2)
@@ -386,8 +573,9 @@ void rgba8(const float* d_in, uint8_t* d_out, int w, int h, bool flip, cudaStrea
     check_image(w, h);
     if (!d_in || !d_out) throw ArgError("rgba8: image is NULL");
     const int64_t n = (int64_t)w * h;
-    k_rgba8<<<stream_grid(n, 256), 256, 0, st>>>(reinterpret_cast<const float4*>(d_in),
-                                                reinterpret_cast<uchar4*>(d_out), w, h, flip ? 1 : 0);
+    constexpr int64_t per = 256 * kRgbaPixels;
+    k_rgba8<<<(unsigned)((n + per - 1) / per), 256, 0, st>>>(reinterpret_cast<const float4*>(d_in),
+                                                            reinterpret_cast<uchar4*>(d_out), w, h, flip ? 1 : 0);
     OMV_CUDA(cudaGetLastError());
 }
 

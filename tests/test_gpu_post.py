@@ -59,6 +59,56 @@ def test_median_matches_oracle_on_ragged_sizes(post, oracle, half, shape):
     assert np.array_equal(y, oracle.median(img, half))
 
 
+@pytest.mark.parametrize("half", [1, 2, 3])
+@pytest.mark.parametrize("shape", [(1, 1), (2, 9), (3, 3), (5, 129), (9, 128), (130, 7)])
+def test_median_edges_and_infinities(post, oracle, half, shape):
+    """Row groups and column blocks cut short, windows that do not fit, infinite pixels: exact."""
+    torch, P = post
+    rng = np.random.default_rng(17 * half + shape[1])
+    img = rng.lognormal(0.0, 2.0, shape + (4,)).astype(np.float32)
+    img[rng.random(shape) < 0.05] = np.inf
+    y = _host(torch, P.SimpleDenoiserMedian(_dev(torch, img), half))
+    assert np.array_equal(y, oracle.median(img, half))
+
+
+def test_median3_of_windows_with_nan(post):
+    """A NaN in the window: the result of the 19-exchange network with IEEE minimum and maximum numbers."""
+    torch, P = post
+    rng = np.random.default_rng(3)
+    img = rng.uniform(0, 1, (23, 41, 4)).astype(np.float32)
+    img[rng.random((23, 41)) < 0.05] = np.nan
+    H, W = img.shape[:2]
+    p = [img[dy:H - 2 + dy, dx:W - 2 + dx, :3].copy() for dy in range(3) for dx in range(3)]
+    for a, b in [(1, 2), (4, 5), (7, 8), (0, 1), (3, 4), (6, 7), (1, 2), (4, 5), (7, 8), (0, 3), (5, 8), (4, 7), (3, 6),
+                 (1, 4), (2, 5), (4, 7), (4, 2), (6, 4), (4, 2)]:
+        p[a], p[b] = np.fmin(p[a], p[b]), np.fmax(p[a], p[b])
+    y = _host(torch, P.SimpleDenoiserMedian(_dev(torch, img), 1))
+    assert np.array_equal(y[1:-1, 1:-1, :3], p[4], equal_nan=True)
+
+
+@pytest.mark.parametrize("shape", [(1, 1), (3, 257), (512, 2048)])
+def test_develop_equals_the_fp64_expression(post, shape):
+    """(float)(sum * (1.0 / count)) bit for bit: counts up to 2^31, sums of any size and sign, zeros, infinities, and
+    sums whose quotient lies within an FP64 ulp or two of the middle between two floats."""
+    torch, P = post
+    rng = np.random.default_rng(shape[1])
+    count = rng.choice([0, 1, 3, 64, 1000, 2**24 - 1, 2**24 + 1, 2**31 - 1], shape).astype(np.int32)
+    count = np.where(rng.random(shape) < 0.5, rng.integers(1, 300, shape), count).astype(np.int32)
+    c = np.maximum(count, 1).astype(np.float64)[..., None]
+    s = rng.lognormal(0.0, 3.0, shape + (3,))
+    f = rng.lognormal(0.0, 3.0, shape + (3,)).astype(np.float32)
+    tie = (f.astype(np.float64) + np.nextafter(f, np.float32(np.inf)).astype(np.float64)) / 2 * c
+    tie = tie * (1.0 + rng.integers(-3, 4, tie.shape) * 2.0**-52)
+    s = np.where(rng.random(s.shape) < 0.3, tie, s)
+    s = np.where(rng.random(s.shape) < 0.1, -s, s)
+    special = np.array([0.0, -0.0, np.inf, 1e-310, 5e-324, 1e-44, 1e30, 1e37, 3e38, 1e300, 2.0**-70, 2.0**-71, 2.0**90, 2.0**91])
+    s = np.where(rng.random(s.shape) < 0.1, rng.choice(special, s.shape), s)
+    lin = _host(torch, P.develop(_dev(torch, s), _dev(torch, count), tonemapped=False, rgba8=False)["linear"])
+    with np.errstate(over="ignore"):
+        want = (s * np.where(count[..., None] < 1, 1.0, 1.0 / c)).astype(np.float32)
+    assert np.array_equal(lin[..., :3].view(np.uint32), want.view(np.uint32))
+
+
 def test_rgba8_matches_reference(post):
     torch, P = post
     g = golden("post")
