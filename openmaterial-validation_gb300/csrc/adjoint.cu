@@ -3,50 +3,149 @@
 // with respect to the material parameters, given the loss's derivative with
 // respect to every pixel (the adjoint image).
 //
-// One thread replays one path: it regenerates the light and camera subpaths
-// from the path's Philox keys (the same random numbers as the forward render),
-// traces their extension and shadow rays again, and keeps its few vertices
-// in registers and local memory only while the path is processed.  The path's
+// The replay regenerates every path's light and camera subpath from its Philox
+// keys (the same random numbers as the forward render) as a wavefront like the
+// renderer's, keeping each vertex's record (ray, hit, throughput, weight), and
+// then walks the records backwards, one launch per bounce.  The path's
 // estimate is a sum of products of per-vertex factors (BDPTRenderer.cpp:
 // 128-302 with weight 1); its derivative is taken with every sampled direction
 // held fixed, which for the GGX-sampled branches adds the score d log D / d
 // alpha of the half-vector density, so the result is an unbiased estimate of
 // the gradient of the expected image (luminance cutoffs are treated as fixed).
 // Two division-free backward recursions over the vertices give the factors'
-// adjoints.  Gradients are summed per thread, reduced per warp with shuffles,
-// per block in shared memory, and added to the output with one atomic per
-// block and parameter.
+// adjoints:
+//   camera  R_b = G_b + w_b R_{b+1}          (k_adj_camera_back)
+//   light   S_j = q_j + w_{j+1} S_{j+1}      (k_adj_light_back)
+// with G_b the vertex's visible connections and escape term, and q_j the
+// adjoint of light vertex j's radiance, both summed by k_adj_connect.
+//
+// Why a wavefront: the replay was one thread per path with all its vertices and
+// their derivatives in local memory (about 7 KB per thread); its warps waited
+// for their slowest path, traversal and derivative arithmetic shared 128
+// registers, and the records ran through L1 and L2 as local memory.  Split by
+// bounce, the traversal kernels are the renderer's, every launch's lanes do the
+// same work, and the derivatives, recomputed where the backward walk needs
+// them, never leave registers.  512x512, 32 spp, 100k triangles, 8 materials:
+// 103 ms before, 9.4 ms so.  Jobs of a batch share the waves: one step (forward
+// and replay) of an inverse fit of eight 128x128x16 scenes 29.1 -> 6.7 ms.
+//
+// Gradients: the lanes of a warp that meet the same material reduce by
+// shuffles into the warp's sums in shared memory, the block adds its totals to
+// FP64 accumulators, and one last launch adds those to the caller's buffers.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstring>
+#include <mutex>
+#include <vector>
 
 #include "dual.cuh"
 #include "scene.h"
 #include "shade.cuh"
+#include "wave.cuh"
 
 namespace omv {
 namespace {
 
 constexpr int kAdjThreads = 128;
 constexpr int kAdjMaxVerts = 16;      // per subpath
-constexpr int kAdjMaxMaterials = 16;  // materials with parameters
+constexpr int kAdjMaxMaterials = 16;  // materials with parameters, per scene
 constexpr int kSlots = OMV_MATERIAL_PARAMS;
+// gradient sums of one wave (jobs x materials x slots): each warp of a block
+// keeps all of them in shared memory, 4 x 4 KB
+constexpr int kAdjMaxKeys = 1024;
 
-struct AdjArgs {
+// Counter slots of a wave (reset per wave): queue sizes per bounce, then the
+// work counters of the tracing launches.
+constexpr int kAdjCtrLight = 0, kAdjCtrCam = 16, kAdjCtrConn = 32, kAdjCtrSeen = 48, kAdjCtrWork = 64,
+              kAdjCounters = 128;
+
+// One job of a wave: a scene of the handle, its camera, samples and materials,
+// the adjoint image and the gradient buffer.
+struct AdjJob {
+    omv_camera cam;
+    int64_t path_base;  // first path of the wave loop's concatenated paths
+    uint64_t seed;
+    const DevMaterial* mats;
+    const float* adj;   // W*H*3 adjoint image
+    float* grad;        // nmat * kSlots
+    FastDiv spp_div, width_div;
+    int32_t spp, sample_offset;
+    uint32_t tlas_root;
+    int32_t light_base, light_count;
+    float light_max;
+    uint32_t mat_base;  // first material of the scene (a scene of a group)
+    int32_t nmat;
+    int32_t key_base;   // first gradient sum
+    float inv_spp;
+};
+// a table's part that travels as a kernel parameter (a caller may capture the
+// call into a graph, where a copy from host memory would be read at replay)
+constexpr int kJobsPerPut = 12;
+struct AdjJobChunk {
+    AdjJob j[kJobsPerPut];
+};
+static_assert(sizeof(AdjJobChunk) <= 3800, "kernel parameters hold 4 KB");
+
+constexpr int kLenShift = 27;  // lmeta: 15 light vertices at most, 2^27 lights
+constexpr uint32_t kLightMask = (1u << kLenShift) - 1u;
+
+// Records of one wave of `cap` paths.  Camera records are kept in queue order
+// per bounce, light records by path.
+struct AdjWave {
     DevScene S;
     const uint32_t* items;
-    omv_camera cam;
-    uint64_t seed;
-    int64_t paths;
-    int32_t spp, sample_offset;
+    const AdjJob* jobs;
+    int32_t num_jobs, cap, wave_n, keys;
+    int64_t wave_base;
     int32_t cam_bounces, light_bounces, max_len, atten_mode;
     float light_scale, min_dist, cut;
-    const float* adj;  // W*H*3 adjoint image
-    float* grad;       // num_user_materials * kSlots
-    int32_t num_user_materials;
-    uint32_t mat_base;  // first material of the scene (a scene of a group)
+    uint32_t* ctr;
+    double* acc;         // gradient sums [keys]
+    uint32_t* path_job;  // job of each path (null for one job)
+    float4* suffix;      // R of the camera vertices processed so far
+    uint32_t* lmeta;     // light index | (light vertices on surfaces << kLenShift)
+    float4* ltp;         // light throughput, distance term
+    float4* lsuffix;     // w_{j+1} S_{j+1}
+    float4 *crq, *ctp, *cw, *cG;  // [bounce][cap]; crq: 2 per entry; ctp.w: the path went on
+    uint4* chit;
+    float4* lrq;         // [bounce][cap], 2 per entry
+    uint4* lhit;
+    float4 *lpos, *lrad, *lw, *lpre, *lq;  // [bounce][path]
+    float4* conn;        // connections of one bounce: light vertex and path, camera vertex and record
+    uint32_t* conn_v;    // their light vertex number
+    uint32_t* seen;      // the unoccluded ones
 };
+
+// ------------------------------------------------------------ paths ---
+// What a path needs of its job, and its pixel's derivative over the samples.
+struct AdjPath {
+    const AdjJob* J;
+    uint32_t pixel, sample;
+};
+__device__ __forceinline__ AdjPath adj_path(const AdjWave& A, int k)
+{
+    AdjPath p;
+    p.J = A.jobs + (A.path_job ? A.path_job[k] : 0u);
+    const int64_t local = A.wave_base + k - p.J->path_base;
+    const uint32_t spp = (uint32_t)p.J->spp;
+    if (local <= (int64_t)0xFFFFFFFFu) {
+        p.pixel = fast_div(p.J->spp_div, (uint32_t)local);
+        p.sample = (uint32_t)local - p.pixel * spp;
+    } else {
+        p.pixel = (uint32_t)(local / spp);
+        p.sample = (uint32_t)(local % spp);
+    }
+    p.sample += (uint32_t)p.J->sample_offset;
+    return p;
+}
+__device__ __forceinline__ V3 adj_delta(const AdjPath& p)
+{
+    const float* ad = p.J->adj + 3 * (size_t)p.pixel;
+    const float s = p.J->inv_spp;
+    return v3(ad[0] * s, ad[1] * s, ad[2] * s);
+}
+__device__ __forceinline__ bool is_zero(V3 a) { return a.x == 0.0f && a.y == 0.0f && a.z == 0.0f; }
 
 // derivatives of a vertex weight (or evaluation) with respect to the
 // material's local parameters: PBR r,g,b, alpha, metallic; OpenMATERIAL
@@ -123,335 +222,835 @@ __device__ __forceinline__ V3 eval_with_grad(const DevMaterial& M, const Surf& s
     return f;
 }
 
-// adds t to a gradient slot unless it is not finite: a degenerate path (an
-// infinite sample of the forward estimator) must not poison the sum
-__device__ __forceinline__ void add_finite(float& slot, float t)
-{
-    if (fabsf(t) <= kFltMax) slot += t;
-}
+// ------------------------------------------------- gradient sums ---
+// a term of a gradient unless it is not finite: a degenerate path (an infinite
+// sample of the forward estimator) must not poison the sum
+__device__ __forceinline__ float finite_or_zero(float t) { return fabsf(t) <= kFltMax ? t : 0.0f; }
 
-// adds sum_c a[c] * g.d[c][i] to the material's parameter slots (`mat`:
-// the material's number within the rendered scene)
-__device__ __forceinline__ void accumulate(float* acc, const DevMaterial& M, uint32_t mat, int nmat, V3 a,
+// A vertex's terms sum_c a[c] * g.d[c][i] for the parameter slots of its
+// material: `key` the first of six consecutive sums (-1: none).  PBR: slots
+// 0-4 (the sixth adds zero), OpenMATERIAL: slots 5-10.
+struct GradTerms {
+    int key;
+    float v[6];
+};
+__device__ __forceinline__ void no_terms(GradTerms& t)
+{
+    t.key = -1;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) t.v[i] = 0.0f;
+}
+__device__ __forceinline__ void grad_terms(GradTerms& t, const AdjJob& J, const DevMaterial& M, uint32_t mat, V3 a,
                                            const LocalGrad& g)
 {
-    if (mat >= (uint32_t)nmat) return;  // the missing material has no parameters
+    const uint32_t m = mat - J.mat_base;
+    if (m >= (uint32_t)J.nmat) return;  // the missing material has no parameters
     const float av[3] = {a.x, a.y, a.z};
-    float* o = acc + mat * kSlots;
     if (M.type == kMatPbr) {
+        t.key = J.key_base + (int)m * kSlots;
         const float rough = sqrtf(M.alpha);  // alpha = roughness^2
-        for (int c = 0; c < 3; ++c) {
-            add_finite(o[0], av[c] * g.d[c][0]);
-            add_finite(o[1], av[c] * g.d[c][1]);
-            add_finite(o[2], av[c] * g.d[c][2]);
-            add_finite(o[3], av[c] * g.d[c][3] * 2.0f * rough);
-            add_finite(o[4], av[c] * g.d[c][4]);
-        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int i = 0; i < 5; ++i)
+                t.v[i] += finite_or_zero(i == 3 ? av[c] * g.d[c][i] * 2.0f * rough : av[c] * g.d[c][i]);
     } else if (M.type == kMatOm) {
+        t.key = J.key_base + (int)m * kSlots + 5;
+#pragma unroll
         for (int c = 0; c < 3; ++c) {
-            add_finite(o[5 + c], av[c] * g.d[c][c]);
-            add_finite(o[8 + c], av[c] * g.d[c][3 + c]);
+            t.v[c] += finite_or_zero(av[c] * g.d[c][c]);
+            t.v[3 + c] += finite_or_zero(av[c] * g.d[c][3 + c]);
         }
     }
 }
 
-// BDPTRenderer::isConnected (BDPTRenderer.cpp:208-235)
-__device__ __forceinline__ bool connected(const DevScene& S, const uint32_t* items, V3 A, V3 B, TraceStack& st,
-                                          TraceCounters& tc)
+// Adds the lanes' terms to the warp's sums; every lane of the warp calls it.
+// The lanes of one material pair up and halve until its first lane holds their
+// total: at most five rounds for all materials at once, where a full reduction
+// per material in the warp takes up to eight times thirty shuffles (the replay
+// of 512x512x32: 9.54 ms so, 9.44 with pairs).
+__device__ __forceinline__ void add_terms(float* sums, GradTerms t)
 {
-    V3 dir = B - A;
-    const float len = sqrtf(dot(dir, dir));
-    const float safeD = 2.0f * kEpsAcc * kEps * max_abs(A, 1.0f);
-    if (len <= safeD) return true;
-    dir = v3(dir.x / len, dir.y / len, dir.z / len);
-    float tnear = safeD;
-    const float tfar = len + (0.1f * len > safeD ? 0.1f * len : safeD);
-    RayHit h;
-    if (!scene_intersect(S, items, A, dir, tnear, tfar, h, st, tc)) return true;
-    const Surf sp = surface_point(S, h.inst, h.prim, h.u, h.v, false);
-    const V3 dd = sp.pos - B;
-    const float sb = 10.0f * kEps * max_abs(B, 1.0f);
-    return dot(dd, dd) <= sb * sb;
+    const int lane = threadIdx.x & 31;
+    if (!__any_sync(0xFFFFFFFFu, t.key >= 0)) return;
+    const uint32_t same = __match_any_sync(0xFFFFFFFFu, t.key);
+    uint32_t rank = __popc(same & ((1u << lane) - 1u));
+    const bool first = rank == 0u;
+    uint32_t later = same & ~((2u << lane) - 1u);
+    while (__any_sync(0xFFFFFFFFu, later != 0u)) {
+        const int from = (__ffs(later) - 1) & 31;
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+            const float x = __shfl_sync(0xFFFFFFFFu, t.v[i], from);
+            if (later) t.v[i] += x;
+        }
+        later &= __ballot_sync(0xFFFFFFFFu, !(rank & 1u));
+        rank >>= 1;
+    }
+    if (first && t.key >= 0) {
+#pragma unroll
+        for (int i = 0; i < 6; ++i) sums[t.key + i] += t.v[i];
+    }
+    __syncwarp();
 }
 
-struct LightVert {
-    V3 pos, rad;   // connection end point and radiance (lv_pos, lv_rad)
-    V3 w, pre;     // sampled weight (brdf x ct) and the product before it (x Rad0 x att)
-    V3 q;          // adjoint of rad: sum over camera vertices of delta * tp * f * c
-    uint32_t mat;
-    LocalGrad g;   // d w / d params
-};
-struct CamVert {
-    V3 tp, w, G;   // throughput at the vertex, sampled weight, local contribution
-    uint32_t mat;
-    bool has_w;    // the path continued from this vertex
-    LocalGrad gw;  // d w / d params
-    LocalGrad gG;  // d G / d params (through the connection evaluations)
-};
-
-// 4 resident blocks of 128 (128 registers, some spilled): 0.109 s per
-// gradient of the 512x512x32 adjoint benchmark and 0.497 s per inverse-fit
-// step, against 0.111 / 0.509 at the natural 168 registers (3 blocks) and
-// 0.115 / 0.531 at 246 registers (2 blocks, no spills)
-__global__ void __launch_bounds__(kAdjThreads, 4) k_adjoint(AdjArgs A)
+// the warps' sums of a block: cleared before, added to the wave's after
+__device__ __forceinline__ float* clear_sums(float* shared, int keys)
 {
-    __shared__ uint2 sstack[kStackShared * kAdjThreads];
-    __shared__ float sgrad[kAdjMaxMaterials * kSlots];
+    for (int i = threadIdx.x; i < keys * (kAdjThreads / 32); i += kAdjThreads) shared[i] = 0.0f;
+    __syncthreads();
+    return shared + (threadIdx.x >> 5) * keys;
+}
+__device__ __forceinline__ void flush_sums(const float* shared, const AdjWave& A)
+{
+    __syncthreads();
+    for (int i = threadIdx.x; i < A.keys; i += kAdjThreads) {
+        float x = 0.0f;
+#pragma unroll
+        for (int w = 0; w < kAdjThreads / 32; ++w) x += shared[w * A.keys + i];
+        if (x != 0.0f) atomicAdd(A.acc + i, (double)x);
+    }
+}
+
+// ------------------------------------------------------------ setup ---
+__global__ void k_adj_put_jobs(AdjJobChunk c, AdjJob* table, int first, int n)
+{
+    const int i = threadIdx.x;
+    if (i < n) table[first + i] = c.j[i];
+}
+
+// job of every path of the wave (largest job whose first path <= g)
+__global__ void __launch_bounds__(kShadeThreads) k_adj_path_jobs(AdjWave A)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= A.wave_n) return;
+    const int64_t g = A.wave_base + k;
+    int lo = 0, hi = A.num_jobs - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (A.jobs[mid].path_base <= g)
+            lo = mid;
+        else
+            hi = mid - 1;
+    }
+    A.path_job[k] = (uint32_t)lo;
+}
+
+// Paths of pixels without a derivative add nothing: they are not queued.
+// (k_light_gen)
+__global__ void __launch_bounds__(kShadeThreads) k_adj_light_gen(AdjWave A)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    bool live = false;
+    V3 so = v3(0, 0, 0), R = v3(0, 0, 1);
+    if (k < A.wave_n) {
+        const AdjPath p = adj_path(A, k);
+        const AdjJob& J = *p.J;
+        if (!is_zero(adj_delta(p))) {
+            int li = J.light_base;
+            if (J.light_count > 1)
+                li += pick_light(A.S.light_cdf + J.light_base, J.light_count,
+                                 rng4(J.seed, p.pixel, p.sample, 0u, kStreamLight).u[0] * J.light_max);
+            A.lmeta[k] = (uint32_t)li;
+            A.lsuffix[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            live = A.light_bounces >= 1;
+            if (live) {
+                R = light_direction(J.seed, p.pixel, p.sample);
+                const float4 lp = __ldg(A.S.light_pos + li);
+                so = shifted_origin(v3(lp.x, lp.y, lp.z), R, 1.0f);
+            }
+        }
+    }
+    const uint32_t slot = warp_append(A.ctr + kAdjCtrLight, live);
+    if (live) {
+        A.lrq[2 * (size_t)slot] = make_float4(so.x, so.y, so.z, 0.0f);
+        A.lrq[2 * (size_t)slot + 1] = make_float4(R.x, R.y, R.z, __int_as_float(k));
+    }
+}
+
+// (k_camera_gen)
+__global__ void __launch_bounds__(kShadeThreads) k_adj_camera_gen(AdjWave A)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    bool live = false;
+    V3 so = v3(0, 0, 0), R = v3(0, 0, 1);
+    if (k < A.wave_n) {
+        const AdjPath p = adj_path(A, k);
+        live = !is_zero(adj_delta(p));
+        if (live) {
+            const AdjJob& J = *p.J;
+            const Rng4 r = rng4(J.seed, p.pixel, p.sample, 0u, kStreamCamera);
+            const uint32_t row = fast_div(J.width_div, p.pixel);
+            V3 O;
+            camera_ray(J.cam, (int)(p.pixel - row * (uint32_t)J.cam.width), (int)row, r.u[0], r.u[1], O, R);
+            so = shifted_origin(O, R, 1.0f);
+        }
+    }
+    const uint32_t slot = warp_append(A.ctr + kAdjCtrCam, live);
+    if (live) {
+        A.crq[2 * (size_t)slot] = make_float4(so.x, so.y, so.z, 0.0f);
+        A.crq[2 * (size_t)slot + 1] = make_float4(R.x, R.y, R.z, __int_as_float(k));
+    }
+}
+
+// ----------------------------------------------------------- tracing ---
+__device__ __forceinline__ uint32_t adj_root(const AdjWave& A, int k)
+{
+    return A.jobs[A.path_job ? A.path_job[k] : 0u].tlas_root;
+}
+
+__global__ void __launch_bounds__(kTraceThreads, kTraceMinBlocks)
+    k_adj_extend(AdjWave A, float4* rq, uint4* hits, const uint32_t* count, uint32_t* work)
+{
+    __shared__ uint2 sstack[kStackShared * kTraceThreads];
     TraceStack st;
     st.sh = sstack + threadIdx.x;
-    st.stride = kAdjThreads;
+    st.stride = kTraceThreads;
     st.overflow = 0;
     TraceCounters tc{0u, 0u};
-    for (int i = threadIdx.x; i < kAdjMaxMaterials * kSlots; i += blockDim.x) sgrad[i] = 0.0f;
-    __syncthreads();
-    const DevScene& S = A.S;
-    const int nmat = A.num_user_materials;
-    float acc[kAdjMaxMaterials * kSlots];
-#pragma unroll 1
-    for (int i = 0; i < kAdjMaxMaterials * kSlots; ++i) acc[i] = 0.0f;
-    LightVert L[kAdjMaxVerts];
-    CamVert Cv[kAdjMaxVerts];
-    const float inv_spp = 1.0f / (float)A.spp;
-    for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < A.paths;
-         g += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t pixel = (uint32_t)(g / A.spp);
-        const uint32_t sample = (uint32_t)(A.sample_offset + g % A.spp);
-        const float* ad = A.adj + 3 * (size_t)pixel;
-        const V3 delta = v3(ad[0] * inv_spp, ad[1] * inv_spp, ad[2] * inv_spp);
-        if (delta.x == 0.0f && delta.y == 0.0f && delta.z == 0.0f) continue;
-
-        // ---- light subpath (k_light_gen, k_extend, k_light_shade)
-        int nl = 0;  // light vertices on surfaces (lv[1..nl])
-        V3 l0pos = v3(0, 0, 0);
-        uint32_t li = 0;
-        if (S.num_lights > 0) {
-            const float d = rng4(A.seed, pixel, sample, 0u, kStreamLight).u[0] * S.light_max;
-            const int N = S.num_lights;
-            if (N > 1) {
-                if (d <= S.light_cdf[0])
-                    li = 0;
-                else if (d >= S.light_cdf[N - 2])
-                    li = N - 1;
-                else {
-                    int lo = 0, hi = N - 1;
-                    while (lo < hi) {
-                        int C = (lo + hi) / 2;
-                        if (d <= S.light_cdf[C])
-                            hi = C;
-                        else
-                            lo = C + 1;
-                    }
-                    li = (lo + hi) / 2;
-                }
-            }
-            V3 R = light_direction(A.seed, pixel, sample);  // as k_light_gen
-            const float4 lp = __ldg(S.light_pos + li);
-            const float4 I = __ldg(S.light_int + li);
-            l0pos = v3(lp.x, lp.y, lp.z);
-            const V3 rad0 = v3(I.x * A.light_scale, I.y * A.light_scale, I.z * A.light_scale);
-            V3 ltp = v3(1.0f, 1.0f, 1.0f);
-            float att = 1.0f;
-            V3 o = shifted_origin(l0pos, R, 1.0f);
-            float tn = 0.0f;
-            for (int b = 1; b <= A.light_bounces && b < kAdjMaxVerts; ++b) {
-                RayHit h;
-                if (!scene_intersect(S, A.items, o, R, tn, kFltMax, h, st, tc)) break;
-                const Surf sp = surface_point(S, h.inst, h.prim, h.u, h.v, true);
-                const DevMaterial M = S.mats[sp.mat];
-                const Rng4 u = rng4(A.seed, pixel, sample, kDimLightBounce + (uint32_t)b, kStreamLight);
-                V3 O;
-                LightVert& lv = L[b];
-                const V3 brdf = sample_with_grad(S, M, sp, R, false, u, O, lv.g);
-                const float ct = fabsf(dot(R, sp.nrm));
-                const V3 tp = v3(ltp.x * brdf.x * ct, ltp.y * brdf.y * ct, ltp.z * brdf.z * ct);
-                if (b == 1) {
-                    const V3 dd = sp.pos - l0pos;
-                    att = light_attenuation(A.atten_mode, A.min_dist, sqrtf(dot(dd, dd)), lp.w);
-                }
-                const V3 orad = v3(tp.x * rad0.x * att, tp.y * rad0.y * att, tp.z * rad0.z * att);
-                if (intensity(orad) < A.cut) break;
-                lv.pos = sp.pos;
-                lv.rad = orad;
-                lv.w = v3(brdf.x * ct, brdf.y * ct, brdf.z * ct);
-                lv.pre = v3(ltp.x * rad0.x * att, ltp.y * rad0.y * att, ltp.z * rad0.z * att);
-                lv.q = v3(0, 0, 0);
-                lv.mat = sp.mat;
-#pragma unroll
-                for (int c = 0; c < 3; ++c)
-#pragma unroll
-                    for (int i = 0; i < 6; ++i) lv.g.d[c][i] *= ct;
-                nl = b;
-                ltp = tp;
-                if (!(b < A.light_bounces && (tp.x != 0.0f || tp.y != 0.0f || tp.z != 0.0f))) break;
-                o = shifted_origin(sp.pos, O, 1.0f);
-                R = O;
-            }
-        }
-        const int lp_len = S.num_lights > 0 ? nl + 1 : 0;
-
-        // ---- camera subpath (k_camera_gen, k_extend, k_camera_shade, k_shadow)
-        int nc = 0;
-        {
-            const Rng4 r = rng4(A.seed, pixel, sample, 0u, kStreamCamera);
-            V3 O0, D;
-            camera_ray(A.cam, (int)(pixel % (uint32_t)A.cam.width), (int)(pixel / (uint32_t)A.cam.width), r.u[0],
-                       r.u[1], O0, D);
-            V3 o = shifted_origin(O0, D, 1.0f);
-            float tn = 0.0f;
-            V3 tp = v3(1.0f, 1.0f, 1.0f);
-            for (int b = 1; b <= A.cam_bounces && nc < kAdjMaxVerts; ++b) {
-                CamVert& cv = Cv[nc++];
-                cv.tp = tp;
-                cv.has_w = false;
-                cv.mat = 0xFFFFFFFFu;
-                cv.G = v3(0, 0, 0);
-                lg_zero(cv.gG);
-                RayHit h;
-                if (!scene_intersect(S, A.items, o, D, tn, kFltMax, h, st, tc)) {
-                    if (S.env.present && b <= A.max_len) cv.G = env_radiance(S.env, D);
-                    break;
-                }
-                const Surf sp = surface_point(S, h.inst, h.prim, h.u, h.v, true);
-                const DevMaterial M = S.mats[sp.mat];
-                cv.mat = sp.mat;
-                const Rng4 u = rng4(A.seed, pixel, sample, (uint32_t)b, kStreamCamera);
-                V3 Onext;
-                const V3 brdf = sample_with_grad(S, M, sp, D, true, u, Onext, cv.gw);
-                const float ct = fabsf(dot(Onext, sp.nrm));
-                const V3 outV = -D;
-                for (int li_v = 0; li_v < lp_len && li_v + b <= A.max_len; ++li_v) {
-                    const V3 lPos = li_v == 0 ? l0pos : L[li_v].pos;
-                    V3 lRad;
-                    const V3 LC = normalize(sp.pos - lPos);
-                    if (li_v == 0) {
-                        const float4 I = __ldg(S.light_int + li);
-                        const float4 Lp = __ldg(S.light_pos + li);
-                        const V3 dd = sp.pos - lPos;
-                        const float lsc = light_attenuation(A.atten_mode, A.min_dist, sqrtf(dot(dd, dd)), Lp.w);
-                        const float f = A.light_scale * lsc;
-                        lRad = v3(I.x * f, I.y * f, I.z * f);
-                    } else {
-                        lRad = L[li_v].rad;
-                    }
-                    const float c = fabsf(dot(LC, sp.nrm));
-                    V3 lc = v3(lRad.x * c * tp.x, lRad.y * c * tp.y, lRad.z * c * tp.z);
-                    if (intensity(lc) < A.cut) continue;
-                    LocalGrad ge;
-                    const V3 f = eval_with_grad(M, sp, LC, outV, ge) * c;
-                    lc = v3(f.x * tp.x * lRad.x, f.y * tp.y * lRad.y, f.z * tp.z * lRad.z);
-                    if (intensity(lc) < A.cut) continue;
-                    if (!connected(S, A.items, lPos, sp.pos, st, tc)) continue;
-                    cv.G = cv.G + mul(f, lRad);
-                    const float lr[3] = {lRad.x * c, lRad.y * c, lRad.z * c};
-#pragma unroll
-                    for (int cc = 0; cc < 3; ++cc)
-#pragma unroll
-                        for (int i = 0; i < 6; ++i) cv.gG.d[cc][i] += ge.d[cc][i] * lr[cc];
-                    if (li_v > 0) L[li_v].q = L[li_v].q + mul(mul(delta, tp), f);
-                }
-                const V3 tpn = v3(tp.x * brdf.x * ct, tp.y * brdf.y * ct, tp.z * brdf.z * ct);
-                cv.w = v3(brdf.x * ct, brdf.y * ct, brdf.z * ct);
-#pragma unroll
-                for (int cc = 0; cc < 3; ++cc)
-#pragma unroll
-                    for (int i = 0; i < 6; ++i) cv.gw.d[cc][i] *= ct;
-                if (!(b < A.cam_bounces && (tpn.x != 0.0f || tpn.y != 0.0f || tpn.z != 0.0f))) break;
-                cv.has_w = true;
-                tp = tpn;
-                o = shifted_origin(sp.pos, Onext, 1.0f);
-                D = Onext;
-            }
-        }
-
-        // ---- backward over the camera vertices: R = suffix radiance after a vertex
-        V3 Rs = v3(0, 0, 0);
-        for (int b = nc - 1; b >= 0; --b) {
-            const CamVert& cv = Cv[b];
-            if (cv.mat != 0xFFFFFFFFu) {
-                const DevMaterial M = S.mats[cv.mat];
-                // d/dparams of tp_b * (G_b + w_b * R_{b+1})
-                const V3 a = mul(delta, cv.tp);
-                accumulate(acc, M, cv.mat - A.mat_base, nmat, a, cv.gG);
-                if (cv.has_w) accumulate(acc, M, cv.mat - A.mat_base, nmat, mul(a, Rs), cv.gw);
-            }
-            Rs = cv.has_w ? cv.G + mul(cv.w, Rs) : cv.G;
-        }
-        // ---- backward over the light vertices: S = suffix of q through the weights
-        V3 Ss = v3(0, 0, 0);
-        for (int j = nl; j >= 1; --j) {
-            const LightVert& lv = L[j];
-            Ss = (j == nl) ? lv.q : lv.q + mul(L[j + 1].w, Ss);
-            accumulate(acc, S.mats[lv.mat], lv.mat - A.mat_base, nmat, mul(lv.pre, Ss), lv.g);
-        }
-    }
-    // ---- reduce: warp shuffles, block shared memory, one atomic per block and slot
-    const int lane = threadIdx.x & 31;
-    for (int i = 0; i < nmat * kSlots; ++i) {
-        float v = acc[i];
-        for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-        if (lane == 0 && v != 0.0f) atomicAdd(&sgrad[i], v);
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < nmat * kSlots; i += blockDim.x)
-        if (sgrad[i] != 0.0f) atomicAdd(&A.grad[i], sgrad[i]);
+    extend_rays(A.S, A.items, rq, hits, *count, work, st, tc, [&](int k) { return adj_root(A, k); });
 }
 
-}  // namespace
+// the connections of one camera bounce: the unoccluded ones are listed
+template <bool kMasked>
+__global__ void __launch_bounds__(kTraceThreads, kTraceMinBlocks)
+    k_adj_shadow(AdjWave A, const uint32_t* count, uint32_t* seen, uint32_t* work)
+{
+    __shared__ uint2 sstack[kStackShared * kTraceThreads];
+    TraceStack st;
+    st.sh = sstack + threadIdx.x;
+    st.stride = kTraceThreads;
+    st.overflow = 0;
+    TraceCounters tc{0u, 0u};
+    const uint32_t n = *count;
+    const int lane = threadIdx.x & 31;
+    while (true) {
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(work, 32u);
+        base = __shfl_sync(0xFFFFFFFFu, base, 0);
+        if (base >= n) break;
+        const uint32_t i = base + lane;
+        bool ok = false;
+        if (i < n) {
+            const float4 q0 = A.conn[2 * (size_t)i], q1 = A.conn[2 * (size_t)i + 1];
+            ok = is_connected<kMasked>(A.S, A.items, v3(q0.x, q0.y, q0.z), v3(q1.x, q1.y, q1.z), st, tc,
+                                       adj_root(A, __float_as_int(q0.w)));
+        }
+        const uint32_t slot = warp_append(seen, ok);
+        if (ok) A.seen[slot] = i;
+    }
+}
 
-void adjoint_frame(SceneHost& s, const omv_camera& cam, const omv_params& p, const float* d_adjoint, float* d_grad,
-                   cudaStream_t st, int part, const DevMaterial* mats)
+// ----------------------------------------------------------- forward ---
+// Light vertex b of every queued path (light_vertex, k_light_shade): the
+// connection end point, its weight and the product before it, the next ray.
+__global__ void __launch_bounds__(kShadeThreads, 4) k_adj_light(AdjWave A, int b)
+{
+    const DevScene& S = A.S;
+    const size_t off = (size_t)(b - 1) * A.cap;
+    const float4* rq = A.lrq + 2 * off;
+    const uint4* hits = A.lhit + off;
+    const uint32_t n = A.ctr[kAdjCtrLight + b - 1];
+    for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
+        const uint32_t i = i0 + threadIdx.x;
+        bool push = false;
+        V3 so = v3(0, 0, 0), O = v3(0, 0, 1);
+        float tnear = 0.0f;
+        int k = 0;
+        const uint4 h = i < n ? hits[i] : make_uint4(kInvalid, 0u, 0u, 0u);
+        if (h.x != kInvalid) {
+            const float4 ra = rq[2 * (size_t)i], rb = rq[2 * (size_t)i + 1];
+            k = __float_as_int(rb.w);
+            tnear = ra.w;
+            const AdjPath p = adj_path(A, k);
+            const AdjJob& J = *p.J;
+            const DevMaterial& M = J.mats[__ldg(&S.insts[h.x].material)];
+            const Surf sp = surface_point(S, h.x, h.y, __uint_as_float(h.z), __uint_as_float(h.w), true, &M);
+            const V3 R = v3(rb.x, rb.y, rb.z);
+            const Rng4 u = rng4(J.seed, p.pixel, p.sample, kDimLightBounce + (uint32_t)b, kStreamLight);
+            const V3 brdf = material_sample(S, M, sp, R, false, u, O);
+            const float ct = fabsf(dot(R, sp.nrm));
+            const uint32_t li = A.lmeta[k] & kLightMask;
+            const float4 I = __ldg(S.light_int + li);
+            const V3 rad0 = v3(I.x * A.light_scale, I.y * A.light_scale, I.z * A.light_scale);
+            V3 ltp = v3(1.0f, 1.0f, 1.0f);
+            float att;
+            if (b == 1) {
+                const float4 lp = __ldg(S.light_pos + li);
+                const V3 dd = sp.pos - v3(lp.x, lp.y, lp.z);
+                att = light_attenuation(A.atten_mode, A.min_dist, sqrtf(dot(dd, dd)), lp.w);
+            } else {
+                const float4 t = A.ltp[k];
+                ltp = v3(t.x, t.y, t.z);
+                att = t.w;
+            }
+            const V3 tp = v3(ltp.x * brdf.x * ct, ltp.y * brdf.y * ct, ltp.z * brdf.z * ct);
+            const V3 orad = v3(tp.x * rad0.x * att, tp.y * rad0.y * att, tp.z * rad0.z * att);
+            if (!(intensity(orad) < A.cut)) {
+                const size_t v = off + k;
+                A.lpos[v] = make_float4(sp.pos.x, sp.pos.y, sp.pos.z, 0.0f);
+                A.lrad[v] = make_float4(orad.x, orad.y, orad.z, 0.0f);
+                A.lw[v] = make_float4(brdf.x * ct, brdf.y * ct, brdf.z * ct, 0.0f);
+                A.lpre[v] = make_float4(ltp.x * rad0.x * att, ltp.y * rad0.y * att, ltp.z * rad0.z * att, 0.0f);
+                A.lq[v] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                A.lmeta[k] = li | ((uint32_t)b << kLenShift);
+                A.ltp[k] = make_float4(tp.x, tp.y, tp.z, att);
+                push = b < A.light_bounces && !is_zero(tp);
+                if (push) so = shifted_origin(sp.pos, O, 1.0f);
+            }
+        }
+        const uint32_t slot = warp_append(A.ctr + kAdjCtrLight + b, push);
+        if (push) {
+            float4* out = A.lrq + 2 * (off + A.cap + slot);
+            out[0] = make_float4(so.x, so.y, so.z, tnear);
+            out[1] = make_float4(O.x, O.y, O.z, __int_as_float(k));
+        }
+    }
+}
+
+// the radiance and direction cosine of the connection from light vertex v of
+// path k (position lPos, direction LC to the camera vertex)
+__device__ __forceinline__ V3 connection_radiance(const AdjWave& A, uint32_t li, int v, int k, V3 pos, V3 lPos)
+{
+    if (v > 0) {
+        const float4 r = A.lrad[(size_t)(v - 1) * A.cap + k];
+        return v3(r.x, r.y, r.z);
+    }
+    const float4 I = __ldg(A.S.light_int + li);
+    const V3 dd = pos - lPos;
+    const float f = A.light_scale * light_attenuation(A.atten_mode, A.min_dist, sqrtf(dot(dd, dd)),
+                                                      __ldg(A.S.light_pos + li).w);
+    return v3(I.x * f, I.y * f, I.z * f);
+}
+
+// Camera vertex b of every queued path (camera_vertex, k_camera_shade): its
+// record, its candidate connections and the next ray.
+__global__ void __launch_bounds__(kShadeThreads, 4) k_adj_camera(AdjWave A, int b)
+{
+    __shared__ BinScratch bins;
+    const DevScene& S = A.S;
+    const size_t off = (size_t)(b - 1) * A.cap;
+    const float4* rq = A.crq + 2 * off;
+    const uint32_t n = A.ctr[kAdjCtrCam + b - 1];
+    for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
+        const uint32_t i = i0 + threadIdx.x;
+        bool push = false;
+        V3 so = v3(0, 0, 0), O = v3(0, 0, 1), tpn = v3(0, 0, 0);
+        float tnear = 0.0f;
+        int k = 0;
+        if (i < n) {
+            const float4 ra = rq[2 * (size_t)i], rb = rq[2 * (size_t)i + 1];
+            const uint4 h = A.chit[off + i];
+            k = __float_as_int(rb.w);
+            tnear = ra.w;
+            const V3 in = v3(rb.x, rb.y, rb.z);
+            V3 G = v3(0.0f, 0.0f, 0.0f);
+            // the throughput: 1, or left by the previous bounce
+            const float4 tp4 = b == 1 ? make_float4(1.0f, 1.0f, 1.0f, 0.0f) : A.ctp[off + i];
+            const V3 tp = v3(tp4.x, tp4.y, tp4.z);
+            if (h.x == kInvalid) {
+                if (S.env.present && b <= A.max_len) G = env_radiance(S.env, in);
+            } else {
+                const AdjPath p = adj_path(A, k);
+                const AdjJob& J = *p.J;
+                const DevMaterial& M = J.mats[__ldg(&S.insts[h.x].material)];
+                const Surf sp = surface_point(S, h.x, h.y, __uint_as_float(h.z), __uint_as_float(h.w), true, &M);
+                const Rng4 u = rng4(J.seed, p.pixel, p.sample, (uint32_t)b, kStreamCamera);
+                const V3 brdf = material_sample(S, M, sp, in, true, u, O);
+                const float ct = fabsf(dot(O, sp.nrm));
+                if (J.light_count > 0) {
+                    const uint32_t meta = A.lmeta[k];
+                    const int lp_len = (int)(meta >> kLenShift) + 1;
+                    const uint32_t li = meta & kLightMask;
+                    for (int v = 0; v < lp_len && v + b <= A.max_len; ++v) {
+                        const float4 lp = v == 0 ? __ldg(S.light_pos + li) : A.lpos[(size_t)(v - 1) * A.cap + k];
+                        const V3 lPos = v3(lp.x, lp.y, lp.z);
+                        const V3 LC = normalize(sp.pos - lPos);
+                        const V3 lRad = connection_radiance(A, li, v, k, sp.pos, lPos);
+                        const float c = fabsf(dot(LC, sp.nrm));
+                        V3 lc = v3(lRad.x * c * tp.x, lRad.y * c * tp.y, lRad.z * c * tp.z);
+                        if (intensity(lc) < A.cut) continue;
+                        const V3 f = material_eval(M, sp, LC, -in) * c;
+                        lc = v3(f.x * tp.x * lRad.x, f.y * tp.y * lRad.y, f.z * tp.z * lRad.z);
+                        if (intensity(lc) < A.cut) continue;
+                        const uint32_t q = coalesced_append(A.ctr + kAdjCtrConn + b - 1);
+                        A.conn[2 * (size_t)q] = make_float4(lPos.x, lPos.y, lPos.z, __int_as_float(k));
+                        A.conn[2 * (size_t)q + 1] = make_float4(sp.pos.x, sp.pos.y, sp.pos.z, __uint_as_float(i));
+                        A.conn_v[q] = (uint32_t)v;
+                    }
+                }
+                tpn = v3(tp.x * brdf.x * ct, tp.y * brdf.y * ct, tp.z * brdf.z * ct);
+                A.cw[off + i] = make_float4(brdf.x * ct, brdf.y * ct, brdf.z * ct, 0.0f);
+                push = b < A.cam_bounces && !is_zero(tpn);
+                if (push) so = shifted_origin(sp.pos, O, 1.0f);
+            }
+            A.ctp[off + i] = make_float4(tp.x, tp.y, tp.z, push ? 1.0f : 0.0f);
+            A.cG[off + i] = make_float4(G.x, G.y, G.z, 0.0f);
+        }
+        const uint32_t slot = block_append_binned(A.ctr + kAdjCtrCam + b, push, direction_bin(O), bins);
+        if (push) {
+            const size_t e = off + A.cap + slot;
+            A.crq[2 * e] = make_float4(so.x, so.y, so.z, tnear);
+            A.crq[2 * e + 1] = make_float4(O.x, O.y, O.z, __int_as_float(k));
+            A.ctp[e] = make_float4(tpn.x, tpn.y, tpn.z, 0.0f);
+        }
+    }
+}
+
+// ---------------------------------------------------------- backward ---
+// Every unoccluded connection of camera bounce b: its term of the vertex's G
+// and of the light vertex's q, and its derivatives.
+__global__ void __launch_bounds__(kAdjThreads) k_adj_connect(AdjWave A, int b)
+{
+    extern __shared__ float shared_sums[];
+    const uint32_t n = A.ctr[kAdjCtrSeen + b - 1];
+    if (blockIdx.x * kAdjThreads >= n) return;
+    float* sums = clear_sums(shared_sums, A.keys);
+    const DevScene& S = A.S;
+    const size_t off = (size_t)(b - 1) * A.cap;
+    for (uint32_t i0 = blockIdx.x * kAdjThreads; i0 < n; i0 += gridDim.x * kAdjThreads) {
+        const uint32_t s = i0 + threadIdx.x;
+        GradTerms t;
+        no_terms(t);
+        if (s < n) {
+            const uint32_t q = A.seen[s];
+            const float4 q0 = A.conn[2 * (size_t)q], q1 = A.conn[2 * (size_t)q + 1];
+            const int v = (int)A.conn_v[q], k = __float_as_int(q0.w);
+            const size_t e = off + __float_as_uint(q1.w);
+            const uint4 h = A.chit[e];
+            const float4 rb = A.crq[2 * e + 1], tp4 = A.ctp[e];
+            const V3 lPos = v3(q0.x, q0.y, q0.z), tp = v3(tp4.x, tp4.y, tp4.z);
+            const AdjPath p = adj_path(A, k);
+            const AdjJob& J = *p.J;
+            const uint32_t mat = __ldg(&S.insts[h.x].material);
+            const DevMaterial& M = J.mats[mat];
+            const Surf sp = surface_point(S, h.x, h.y, __uint_as_float(h.z), __uint_as_float(h.w), true, &M);
+            const V3 LC = normalize(sp.pos - lPos);
+            const V3 lRad = connection_radiance(A, A.lmeta[k] & kLightMask, v, k, sp.pos, lPos);
+            const float c = fabsf(dot(LC, sp.nrm));
+            LocalGrad g;
+            const V3 f = eval_with_grad(M, sp, LC, -v3(rb.x, rb.y, rb.z), g) * c;
+            const V3 delta = adj_delta(p);
+            const V3 a = mul(delta, tp);
+            grad_terms(t, J, M, mat, mul(a, v3(lRad.x * c, lRad.y * c, lRad.z * c)), g);
+            const V3 G = mul(f, lRad);
+            float* pg = &A.cG[e].x;
+            atomicAdd(pg, G.x);
+            atomicAdd(pg + 1, G.y);
+            atomicAdd(pg + 2, G.z);
+            if (v > 0) {
+                const V3 dq = mul(a, f);
+                float* pq = &A.lq[(size_t)(v - 1) * A.cap + k].x;
+                atomicAdd(pq, dq.x);
+                atomicAdd(pq + 1, dq.y);
+                atomicAdd(pq + 2, dq.z);
+            }
+        }
+        add_terms(sums, t);
+    }
+    flush_sums(shared_sums, A);
+}
+
+// Camera vertices of bounce b, last bounce first: the derivative of the sampled
+// weight against the suffix radiance, then the suffix through the vertex.
+__global__ void __launch_bounds__(kAdjThreads) k_adj_camera_back(AdjWave A, int b)
+{
+    extern __shared__ float shared_sums[];
+    const uint32_t n = A.ctr[kAdjCtrCam + b - 1];
+    if (blockIdx.x * kAdjThreads >= n) return;
+    float* sums = clear_sums(shared_sums, A.keys);
+    const DevScene& S = A.S;
+    const size_t off = (size_t)(b - 1) * A.cap;
+    for (uint32_t i0 = blockIdx.x * kAdjThreads; i0 < n; i0 += gridDim.x * kAdjThreads) {
+        const uint32_t i = i0 + threadIdx.x;
+        GradTerms t;
+        no_terms(t);
+        if (i < n) {
+            const float4 tp4 = A.ctp[off + i], G4 = A.cG[off + i];
+            const float4 rb = A.crq[2 * (off + i) + 1];
+            const int k = __float_as_int(rb.w);
+            V3 R = v3(G4.x, G4.y, G4.z);
+            if (tp4.w != 0.0f) {  // the path went on
+                const float4 s4 = A.suffix[k], w4 = A.cw[off + i];
+                const V3 Rs = v3(s4.x, s4.y, s4.z);
+                const AdjPath p = adj_path(A, k);
+                const V3 a = mul(mul(adj_delta(p), v3(tp4.x, tp4.y, tp4.z)), Rs);
+                if (!is_zero(a)) {
+                    const AdjJob& J = *p.J;
+                    const uint4 h = A.chit[off + i];
+                    const uint32_t mat = __ldg(&S.insts[h.x].material);
+                    const DevMaterial& M = J.mats[mat];
+                    const Surf sp = surface_point(S, h.x, h.y, __uint_as_float(h.z), __uint_as_float(h.w), true, &M);
+                    const Rng4 u = rng4(J.seed, p.pixel, p.sample, (uint32_t)b, kStreamCamera);
+                    V3 O;
+                    LocalGrad g;
+                    sample_with_grad(S, M, sp, v3(rb.x, rb.y, rb.z), true, u, O, g);
+                    const float ct = fabsf(dot(O, sp.nrm));
+#pragma unroll
+                    for (int c = 0; c < 3; ++c)
+#pragma unroll
+                        for (int j = 0; j < 6; ++j) g.d[c][j] *= ct;
+                    grad_terms(t, J, M, mat, a, g);
+                }
+                R = R + mul(v3(w4.x, w4.y, w4.z), Rs);
+            }
+            A.suffix[k] = make_float4(R.x, R.y, R.z, 0.0f);
+        }
+        add_terms(sums, t);
+    }
+    flush_sums(shared_sums, A);
+}
+
+// Light vertices of bounce b, last bounce first.
+__global__ void __launch_bounds__(kAdjThreads) k_adj_light_back(AdjWave A, int b)
+{
+    extern __shared__ float shared_sums[];
+    const uint32_t n = A.ctr[kAdjCtrLight + b - 1];
+    if (blockIdx.x * kAdjThreads >= n) return;
+    float* sums = clear_sums(shared_sums, A.keys);
+    const DevScene& S = A.S;
+    const size_t off = (size_t)(b - 1) * A.cap;
+    for (uint32_t i0 = blockIdx.x * kAdjThreads; i0 < n; i0 += gridDim.x * kAdjThreads) {
+        const uint32_t i = i0 + threadIdx.x;
+        GradTerms t;
+        no_terms(t);
+        const uint4 h = i < n ? A.lhit[off + i] : make_uint4(kInvalid, 0u, 0u, 0u);
+        if (h.x != kInvalid) {
+            const float4 rb = A.lrq[2 * (off + i) + 1];
+            const int k = __float_as_int(rb.w);
+            if ((int)(A.lmeta[k] >> kLenShift) >= b) {  // the vertex was kept (its radiance passed the cutoff)
+                const size_t v = off + k;
+                const float4 q4 = A.lq[v], s4 = A.lsuffix[k], pre = A.lpre[v], w4 = A.lw[v];
+                const V3 Ss = v3(q4.x + s4.x, q4.y + s4.y, q4.z + s4.z);
+                A.lsuffix[k] = make_float4(w4.x * Ss.x, w4.y * Ss.y, w4.z * Ss.z, 0.0f);
+                const V3 a = mul(v3(pre.x, pre.y, pre.z), Ss);
+                if (!is_zero(a)) {
+                    const AdjPath p = adj_path(A, k);
+                    const AdjJob& J = *p.J;
+                    const uint32_t mat = __ldg(&S.insts[h.x].material);
+                    const DevMaterial& M = J.mats[mat];
+                    const Surf sp = surface_point(S, h.x, h.y, __uint_as_float(h.z), __uint_as_float(h.w), true, &M);
+                    const Rng4 u = rng4(J.seed, p.pixel, p.sample, kDimLightBounce + (uint32_t)b, kStreamLight);
+                    const V3 R = v3(rb.x, rb.y, rb.z);
+                    V3 O;
+                    LocalGrad g;
+                    sample_with_grad(S, M, sp, R, false, u, O, g);
+                    const float ct = fabsf(dot(R, sp.nrm));
+#pragma unroll
+                    for (int c = 0; c < 3; ++c)
+#pragma unroll
+                        for (int j = 0; j < 6; ++j) g.d[c][j] *= ct;
+                    grad_terms(t, J, M, mat, a, g);
+                }
+            }
+        }
+        add_terms(sums, t);
+    }
+    flush_sums(shared_sums, A);
+}
+
+// the wave loop's sums to the callers' buffers (which may be shared by jobs)
+__global__ void k_adj_out(AdjWave A)
+{
+    for (int j = 0; j < A.num_jobs; ++j) {
+        const AdjJob& J = A.jobs[j];
+        for (int i = threadIdx.x; i < J.nmat * kSlots; i += blockDim.x) {
+            const float x = (float)A.acc[J.key_base + i];
+            if (x != 0.0f) atomicAdd(J.grad + i, x);
+        }
+    }
+}
+
+// -------------------------------------------------------------- host ---
+// Byte offsets of a wave's arrays in one block (each on a 256-byte boundary).
+struct AdjLayout {
+    size_t ctr, acc, jobs, path_job, suffix, lmeta, ltp, lsuffix, crq, ctp, cw, cG, chit, lrq, lhit, lpos, lrad, lw,
+        lpre, lq, conn, conn_v, seen, bytes;
+};
+AdjLayout adj_layout(int64_t cap, int njobs, int B, int L, bool lights)
+{
+    const size_t W = (size_t)cap, cb = (size_t)std::max(B, 1), lb = lights ? (size_t)std::max(L, 1) : 0;
+    const size_t lw = lights ? W : 0, slots = lights ? (size_t)L + 1 : 0;
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        const size_t o = off;
+        off += (bytes + 255) & ~(size_t)255;
+        return o;
+    };
+    AdjLayout l;
+    l.ctr = take(kAdjCounters * 4);
+    l.acc = take(kAdjMaxKeys * 8);
+    l.jobs = take(sizeof(AdjJob) * (size_t)njobs);
+    l.path_job = take(njobs > 1 ? W * 4 : 0);
+    l.suffix = take(W * 16);
+    l.lmeta = take(lw * 4);
+    l.ltp = take(lw * 16);
+    l.lsuffix = take(lw * 16);
+    l.crq = take(cb * W * 32);
+    l.ctp = take(cb * W * 16);
+    l.cw = take(cb * W * 16);
+    l.cG = take(cb * W * 16);
+    l.chit = take(cb * W * 16);
+    l.lrq = take(lb * W * 32);
+    l.lhit = take(lb * W * 16);
+    l.lpos = take(lb * W * 16);
+    l.lrad = take(lb * W * 16);
+    l.lw = take(lb * W * 16);
+    l.lpre = take(lb * W * 16);
+    l.lq = take(lb * W * 16);
+    l.conn = take(slots * W * 32);
+    l.conn_v = take(slots * W * 4);
+    l.seen = take(slots * W * 4);
+    l.bytes = off;
+    return l;
+}
+void carve_wave(AdjWave& A, char* b, const AdjLayout& l, int njobs)
+{
+    A.ctr = (uint32_t*)(b + l.ctr);
+    A.acc = (double*)(b + l.acc);
+    A.jobs = (const AdjJob*)(b + l.jobs);
+    A.path_job = njobs > 1 ? (uint32_t*)(b + l.path_job) : nullptr;
+    A.suffix = (float4*)(b + l.suffix);
+    A.lmeta = (uint32_t*)(b + l.lmeta);
+    A.ltp = (float4*)(b + l.ltp);
+    A.lsuffix = (float4*)(b + l.lsuffix);
+    A.crq = (float4*)(b + l.crq);
+    A.ctp = (float4*)(b + l.ctp);
+    A.cw = (float4*)(b + l.cw);
+    A.cG = (float4*)(b + l.cG);
+    A.chit = (uint4*)(b + l.chit);
+    A.lrq = (float4*)(b + l.lrq);
+    A.lhit = (uint4*)(b + l.lhit);
+    A.lpos = (float4*)(b + l.lpos);
+    A.lrad = (float4*)(b + l.lrad);
+    A.lw = (float4*)(b + l.lw);
+    A.lpre = (float4*)(b + l.lpre);
+    A.lq = (float4*)(b + l.lq);
+    A.conn = (float4*)(b + l.conn);
+    A.conn_v = (uint32_t*)(b + l.conn_v);
+    A.seen = (uint32_t*)(b + l.seen);
+}
+
+// Records of one wave: up to 8 GiB, and at most half of the free memory.  Every
+// further wave pays the latency of the last, nearly empty bounces again: a
+// 512x512x32 replay with 6 bounces (14 GB of records) takes two waves, 0.34 ms
+// more than one wave of 16 GiB would (gradient step 17.05 against 16.71 ms).
+constexpr size_t kAdjBudget = (size_t)8 << 30;
+constexpr int64_t kAdjMinCap = 1 << 14;  // tried at least, whatever memory is free
+
+// Where a wave's records live while its launches are in flight: the scene's own
+// block, used by one call after another (a call on another stream waits for
+// the last one's event), or, when the caller captures the stream into a graph,
+// memory that the graph allocates and frees.
+struct AdjWorkspace {
+    SceneHost& s;
+    cudaStream_t st;
+    bool captured;
+    void* base = nullptr;
+    int64_t cap = 0;
+    AdjWorkspace(SceneHost& s_, cudaStream_t st_, int64_t total, int njobs, int B, int L, bool lights)
+        : s(s_), st(st_), captured(false)
+    {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        // (a legacy-stream query while another thread captures is an error: not captured)
+        if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) (void)cudaGetLastError();
+        captured = cs == cudaStreamCaptureStatusActive;
+        auto need = [&](int64_t c) { return adj_layout(c, njobs, B, L, lights).bytes; };
+        const size_t per = std::max<size_t>(1, (need(1 << 20) - need(0)) >> 20);
+        const int64_t most = std::min<int64_t>(total, (int64_t)1 << 30);
+        cap = std::max<int64_t>(1, std::min<int64_t>(most, (int64_t)(kAdjBudget / per)));
+        if (!captured && s.adj_scratch && s.adj_bytes >= need(cap)) {
+            base = s.adj_scratch;
+        } else {
+            size_t free_b = 0, total_b = 0;
+            OMV_CUDA(cudaMemGetInfo(&free_b, &total_b));
+            const size_t own = captured ? 0 : s.adj_bytes;
+            const int64_t fit = (int64_t)(std::min(kAdjBudget, (free_b + own) / 2) / per);
+            cap = std::min(cap, std::max<int64_t>(std::min(most, kAdjMinCap), fit));
+            if (captured) {
+                OMV_CUDA(cudaMallocAsync(&base, need(cap), st));
+            } else if (s.adj_scratch && s.adj_bytes >= need(cap)) {
+                base = s.adj_scratch;
+            } else {
+                if (s.adj_scratch) {
+                    OMV_CUDA(cudaEventSynchronize(s.adj_done));
+                    cudaFree(s.adj_scratch);
+                    s.adj_scratch = nullptr;
+                    s.adj_bytes = 0;
+                }
+                OMV_CUDA(cudaMalloc(&base, need(cap)));
+                s.adj_scratch = base;
+                s.adj_bytes = need(cap);
+            }
+        }
+        if (!captured) {
+            if (!s.adj_done)
+                OMV_CUDA(cudaEventCreateWithFlags(&s.adj_done, cudaEventDisableTiming));
+            else
+                OMV_CUDA(cudaStreamWaitEvent(st, s.adj_done, 0));
+        }
+    }
+    ~AdjWorkspace()
+    {
+        if (captured)
+            cudaFreeAsync(base, st);
+        else
+            cudaEventRecord(s.adj_done, st);
+    }
+    AdjWorkspace(const AdjWorkspace&) = delete;
+    AdjWorkspace& operator=(const AdjWorkspace&) = delete;
+};
+
+inline unsigned blocks_for(int64_t n, int t) { return (unsigned)std::max<int64_t>(1, (n + t - 1) / t); }
+
+template <typename K>
+int resident_grid(K kernel, int threads, size_t smem, int sms)
+{
+    int occ = 0;
+    OMV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem));
+    return std::max(1, occ) * sms;
+}
+
+// the checked device form of one job
+AdjJob make_job(const SceneHost& s, const omv_camera& cam, const omv_params& p, int32_t spp, int32_t sample_offset,
+                uint64_t seed, const float* d_adjoint, float* d_grad, int part, const DevMaterial* mats)
 {
     if (part < 0 || part >= (int)s.parts.size()) throw ArgError("adjoint scene (part) out of range");
     const ScenePart& P = s.parts[part];
     if (cam.width <= 0 || cam.height <= 0) throw ArgError("camera resolution must be positive");
-    if (p.samples_per_pixel <= 0) throw ArgError("the adjoint needs at least one sample per pixel");
+    if (spp <= 0) throw ArgError("the adjoint needs at least one sample per pixel");
     if (p.camera_bounces < 0 || p.light_bounces < 0) throw ArgError("negative bounce count");
     if (p.camera_bounces >= kAdjMaxVerts || p.light_bounces >= kAdjMaxVerts)
         throw ArgError("the adjoint supports at most 15 camera and 15 light bounces");
-    const int nmat = P.mat_count;
-    if (nmat > kAdjMaxMaterials) throw ArgError("the adjoint supports at most 16 materials per scene");
+    if (P.mat_count > kAdjMaxMaterials) throw ArgError("the adjoint supports at most 16 materials per scene");
     if (!d_adjoint || !d_grad) throw ArgError("adjoint image and gradient buffers are required");
     if (p.estimator != OMV_ESTIMATOR_REFERENCE) throw ArgError("the adjoint replays the reference estimator only");
     for (const DevMaterial& m : s.h_mats)
         if (m.type == kMatPbr && (m.textured || m.emissive_on))
             throw ArgError("the adjoint differentiates untextured materials only");
-    AdjArgs A;
+    AdjJob J{};
+    J.cam = cam;
+    J.seed = seed;
+    J.mats = mats ? mats : s.dev.mats;
+    J.adj = d_adjoint;
+    J.grad = d_grad;
+    J.spp = spp;
+    J.sample_offset = sample_offset;
+    J.spp_div = make_fastdiv((uint32_t)spp);
+    J.width_div = make_fastdiv((uint32_t)cam.width);
+    J.inv_spp = 1.0f / (float)spp;
+    J.tlas_root = P.tlas_root;
+    J.light_base = P.light_base;
+    J.light_count = P.light_count;
+    J.light_max = P.light_max;
+    J.mat_base = (uint32_t)P.mat_base;
+    J.nmat = P.mat_count;
+    return J;
+}
+
+// The replay of jobs [0, n) as one sequence of waves.
+void run_adjoint(SceneHost& s, std::vector<AdjJob>& jobs, const omv_params& p, cudaStream_t st)
+{
+    int64_t total = 0;
+    int keys = 0;
+    bool lights = false;
+    for (AdjJob& J : jobs) {
+        J.path_base = total;
+        J.key_base = keys;
+        total += (int64_t)J.cam.width * J.cam.height * J.spp;
+        keys += J.nmat * kSlots;
+        lights = lights || J.light_count > 0;
+    }
+    if (keys == 0 || p.camera_bounces == 0) return;  // no parameter, or no vertex to differentiate
+    bool masked = false;
+    for (const DevMaterial& m : s.h_mats) masked = masked || m.masked != 0;
+    const int nj = (int)jobs.size(), B = p.camera_bounces, L = p.light_bounces;
+    std::lock_guard<std::mutex> lock(s.adj_mutex);
+    AdjWorkspace ws(s, st, total, nj, B, L, lights);
+    AdjWave A{};
+    const AdjLayout lay = adj_layout(ws.cap, nj, B, L, lights);
+    carve_wave(A, static_cast<char*>(ws.base), lay, nj);
     A.S = s.dev;
-    // the scene of the group: its top-level tree, its lights, the job's materials
-    A.S.tlas_root = P.tlas_root;
-    A.S.light_pos += P.light_base;
-    A.S.light_int += P.light_base;
-    A.S.light_cdf += P.light_base;
-    A.S.num_lights = P.light_count;
-    A.S.light_max = P.light_max;
-    if (mats) A.S.mats = mats;
-    A.mat_base = (uint32_t)P.mat_base;
     A.items = s.tlas_items;
-    A.cam = cam;
-    A.seed = p.seed;
-    A.paths = (int64_t)cam.width * cam.height * p.samples_per_pixel;
-    A.spp = p.samples_per_pixel;
-    A.sample_offset = p.sample_offset;
-    A.cam_bounces = p.camera_bounces;
-    A.light_bounces = p.light_bounces;
+    A.num_jobs = nj;
+    A.cap = (int32_t)ws.cap;
+    A.keys = keys;
+    A.cam_bounces = B;
+    A.light_bounces = L;
     A.max_len = p.max_path_length;
     A.atten_mode = p.light_distance_attenuation;
     A.light_scale = p.light_scale;
     A.min_dist = p.light_min_distance;
     A.cut = p.ray_cut_value;
-    A.adj = d_adjoint;
-    A.grad = d_grad;
-    A.num_user_materials = nmat;
-    int occ = 0;
-    OMV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_adjoint, kAdjThreads, 0));
-    const int64_t want = (A.paths + kAdjThreads - 1) / kAdjThreads;
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)std::max(1, occ) * s.num_sms * 4));
-    k_adjoint<<<grid, kAdjThreads, 0, st>>>(A);
+    for (int f = 0; f < nj; f += kJobsPerPut) {
+        AdjJobChunk c;
+        const int m = std::min(kJobsPerPut, nj - f);
+        for (int i = 0; i < m; ++i) c.j[i] = jobs[f + i];
+        k_adj_put_jobs<<<1, 32, 0, st>>>(c, const_cast<AdjJob*>(A.jobs), f, m);
+    }
+    OMV_CUDA(cudaMemsetAsync(A.acc, 0, sizeof(double) * keys, st));
+    const size_t smem = sizeof(float) * (size_t)keys * (kAdjThreads / 32);
+    const int trace_grid = resident_grid(k_adj_extend, kTraceThreads, 0, s.num_sms);
+    const int light_grid = resident_grid(k_adj_light, kShadeThreads, 0, s.num_sms);
+    const int camera_grid = resident_grid(k_adj_camera, kShadeThreads, 0, s.num_sms);
+    const int connect_grid = resident_grid(k_adj_connect, kAdjThreads, smem, s.num_sms);
+    const int back_grid = resident_grid(k_adj_camera_back, kAdjThreads, smem, s.num_sms);
+    const int lback_grid = resident_grid(k_adj_light_back, kAdjThreads, smem, s.num_sms);
+    for (int64_t wb = 0; wb < total; wb += ws.cap) {
+        A.wave_base = wb;
+        A.wave_n = (int32_t)std::min<int64_t>(ws.cap, total - wb);
+        OMV_CUDA(cudaMemsetAsync(A.ctr, 0, kAdjCounters * 4, st));
+        uint32_t* work = A.ctr + kAdjCtrWork;
+        const unsigned gen = blocks_for(A.wave_n, kShadeThreads);
+        if (A.path_job) k_adj_path_jobs<<<gen, kShadeThreads, 0, st>>>(A);
+        if (lights) {
+            k_adj_light_gen<<<gen, kShadeThreads, 0, st>>>(A);
+            for (int b = 1; b <= L; ++b) {
+                const size_t off = (size_t)(b - 1) * A.cap;
+                k_adj_extend<<<trace_grid, kTraceThreads, 0, st>>>(A, A.lrq + 2 * off, A.lhit + off,
+                                                                   A.ctr + kAdjCtrLight + b - 1, work++);
+                k_adj_light<<<light_grid, kShadeThreads, 0, st>>>(A, b);
+            }
+        }
+        k_adj_camera_gen<<<gen, kShadeThreads, 0, st>>>(A);
+        for (int b = 1; b <= B; ++b) {
+            const size_t off = (size_t)(b - 1) * A.cap;
+            k_adj_extend<<<trace_grid, kTraceThreads, 0, st>>>(A, A.crq + 2 * off, A.chit + off,
+                                                               A.ctr + kAdjCtrCam + b - 1, work++);
+            k_adj_camera<<<camera_grid, kShadeThreads, 0, st>>>(A, b);
+            if (lights) {
+                uint32_t* seen = A.ctr + kAdjCtrSeen + b - 1;
+                const uint32_t* count = A.ctr + kAdjCtrConn + b - 1;
+                if (masked)
+                    k_adj_shadow<true><<<trace_grid, kTraceThreads, 0, st>>>(A, count, seen, work++);
+                else
+                    k_adj_shadow<false><<<trace_grid, kTraceThreads, 0, st>>>(A, count, seen, work++);
+                k_adj_connect<<<connect_grid, kAdjThreads, smem, st>>>(A, b);
+            }
+        }
+        for (int b = B; b >= 1; --b) k_adj_camera_back<<<back_grid, kAdjThreads, smem, st>>>(A, b);
+        if (lights)
+            for (int b = L; b >= 1; --b) k_adj_light_back<<<lback_grid, kAdjThreads, smem, st>>>(A, b);
+        OMV_CUDA(cudaGetLastError());
+    }
+    k_adj_out<<<1, 256, 0, st>>>(A);
     OMV_CUDA(cudaGetLastError());
+}
+
+}  // namespace
+
+void adjoint_frame(SceneHost& s, const omv_camera& cam, const omv_params& p, const float* d_adjoint, float* d_grad,
+                   cudaStream_t st)
+{
+    std::vector<AdjJob> jobs{
+        make_job(s, cam, p, p.samples_per_pixel, p.sample_offset, p.seed, d_adjoint, d_grad, 0, nullptr)};
+    run_adjoint(s, jobs, p, st);
 }
 
 void adjoint_batch(SceneHost& s, int n, const omv_adjoint_job* jobs, const omv_params& p, cudaStream_t st)
 {
+    std::vector<AdjJob> all;
+    all.reserve(n);
     for (int i = 0; i < n; ++i) {  // checked before anything is enqueued
         const omv_job& j = jobs[i].job;
         if (j.material_set < -1 || j.material_set >= s.num_mat_sets)
@@ -460,15 +1059,19 @@ void adjoint_batch(SceneHost& s, int n, const omv_adjoint_job* jobs, const omv_p
         if (j.samples_per_pixel <= 0 || j.camera.width <= 0 || j.camera.height <= 0)
             throw ArgError("adjoint job without samples or pixels");
         if (!jobs[i].d_adjoint_rgb || !jobs[i].d_grad) throw ArgError("adjoint job without adjoint image or gradient");
-    }
-    for (int i = 0; i < n; ++i) {
-        const omv_job& j = jobs[i].job;
-        omv_params q = p;
-        q.samples_per_pixel = j.samples_per_pixel;
-        q.sample_offset = j.sample_offset;
-        q.seed = j.seed;
         const DevMaterial* mats = j.material_set < 0 ? nullptr : s.mat_sets + (size_t)j.material_set * s.num_materials;
-        adjoint_frame(s, j.camera, q, jobs[i].d_adjoint_rgb, jobs[i].d_grad, st, j.part, mats);
+        all.push_back(make_job(s, j.camera, p, j.samples_per_pixel, j.sample_offset, j.seed, jobs[i].d_adjoint_rgb,
+                               jobs[i].d_grad, j.part, mats));
+    }
+    // as many jobs per sequence of waves as the gradient sums have room for
+    for (size_t i = 0; i < all.size();) {
+        std::vector<AdjJob> group;
+        int keys = 0;
+        while (i < all.size() && (group.empty() || keys + all[i].nmat * kSlots <= kAdjMaxKeys)) {
+            keys += all[i].nmat * kSlots;
+            group.push_back(all[i++]);
+        }
+        run_adjoint(s, group, p, st);
     }
 }
 

@@ -19,7 +19,6 @@
 // (ballot + popc); the tracing kernels are persistent and fetch 32 rays per
 // warp from an atomic work counter.  Random numbers are Philox4x32-10 keyed by
 // (pixel, sample, vertex) so any partition of the work gives the same image.
-#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 
@@ -32,20 +31,11 @@
 
 #include "omv_device.cuh"
 #include "scene.h"
-#include "trace.cuh"
-#include "shade.cuh"
+#include "wave.cuh"
 
 namespace omv {
 
 namespace {
-
-constexpr int kTraceThreads = 128;
-// 6 resident blocks of the trace kernels per SM (80 registers, a few spilled
-// stack words): more warps in flight for the latency-bound traversal than the
-// 5 blocks its unconstrained 96 registers allow (measured 3.18 -> 3.06 ms per
-// extension launch on the 1920x1080x64 frame; 7 and 8 blocks spill more)
-constexpr int kTraceMinBlocks = 6;
-constexpr int kShadeThreads = 256;
 
 // counter slots within RenderScratch::ctr (reset per wave)
 constexpr int kCtrLight = 0;     // + bounce (0..light_bounces)
@@ -78,18 +68,6 @@ constexpr uint32_t kTailPaths = 1u << 18;
 constexpr int kCtrTailWorkCam = 510;
 constexpr int kCtrTailDone = 511;
 
-__device__ __forceinline__ uint32_t warp_append(uint32_t* counter, bool want)
-{
-    const uint32_t m = __ballot_sync(0xFFFFFFFFu, want);
-    if (!m) return 0;
-    const int lane = threadIdx.x & 31;
-    const int leader = __ffs(m) - 1;
-    uint32_t base = 0;
-    if (lane == leader) base = atomicAdd(counter, (uint32_t)__popc(m));
-    base = __shfl_sync(0xFFFFFFFFu, base, leader);
-    return base + __popc(m & ((1u << lane) - 1u));
-}
-
 // NVTX range for profilers (a wave, a stage, a bounce); free without a tool attached
 struct NvtxRange {
     explicit NvtxRange(const char* name) { nvtxRangePushA(name); }
@@ -101,98 +79,6 @@ constexpr const char* kBounceNames[] = {"bounce 0",  "bounce 1",  "bounce 2",  "
                                         "bounce 6",  "bounce 7",  "bounce 8",  "bounce 9",  "bounce 10", "bounce 11",
                                         "bounce 12", "bounce 13", "bounce 14", "bounce 15", "bounce > 15"};
 inline const char* bounce_name(int b) { return kBounceNames[b < 16 ? b : 16]; }
-
-// Opportunistic warp aggregation (for appends inside divergent code): the
-// threads of a warp that arrive together take consecutive slots with one atomic.
-__device__ __forceinline__ uint32_t coalesced_append(uint32_t* counter)
-{
-    namespace cg = cooperative_groups;
-    const cg::coalesced_group g = cg::coalesced_threads();
-    uint32_t base = 0;
-    if (g.thread_rank() == 0) base = atomicAdd(counter, (uint32_t)g.size());
-    return g.shfl(base, 0) + (uint32_t)g.thread_rank();
-}
-
-// Direction bin of a ray: the cube face its direction points to (dominant
-// axis and sign) and the quadrant on that face, 24 bins.
-constexpr int kDirBins = 24;
-__device__ __forceinline__ uint32_t direction_bin(V3 d)
-{
-    const float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
-    uint32_t f;
-    float u, v;
-    if (ax >= ay && ax >= az) {
-        f = d.x < 0.0f ? 1u : 0u;
-        u = d.y;
-        v = d.z;
-    } else if (ay >= az) {
-        f = d.y < 0.0f ? 3u : 2u;
-        u = d.z;
-        v = d.x;
-    } else {
-        f = d.z < 0.0f ? 5u : 4u;
-        u = d.x;
-        v = d.y;
-    }
-    return 4u * f + (u < 0.0f ? 2u : 0u) + (v < 0.0f ? 1u : 0u);
-}
-
-struct BinScratch {
-    uint32_t count[kDirBins];
-    uint32_t base;
-};
-
-// Block-wide append to a queue with the block's entries grouped by bin, so
-// that the warps tracing the queue get rays of similar direction from nearby
-// pixels.  One atomic per block; every thread of the block must call it.
-__device__ __forceinline__ uint32_t block_append_binned(uint32_t* counter, bool want, uint32_t bin, BinScratch& sh)
-{
-    if (threadIdx.x < kDirBins) sh.count[threadIdx.x] = 0;
-    __syncthreads();
-    const uint32_t rank = want ? atomicAdd(&sh.count[bin], 1u) : 0u;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        // exclusive scan of the bin counts in the first warp; lane 31 reserves
-        const uint32_t c = threadIdx.x < kDirBins ? sh.count[threadIdx.x] : 0u;
-        uint32_t x = c;
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-            if ((int)threadIdx.x >= o) x += y;
-        }
-        if (threadIdx.x < kDirBins) sh.count[threadIdx.x] = x - c;
-        if (threadIdx.x == 31) sh.base = x ? atomicAdd(counter, x) : 0u;
-    }
-    __syncthreads();
-    const uint32_t slot = sh.base + sh.count[bin] + rank;
-    __syncthreads();  // the scratch is reused by the next call
-    return slot;
-}
-
-// Division of 32-bit unsigned integers by a divisor fixed for a frame, by one
-// multiply-high, a subtraction and two shifts (Granlund & Montgomery,
-// "Division by invariant integers using multiplication", PLDI 1994, 4.1):
-// exact for every numerator and every divisor >= 1, where the hardware has
-// no integer divide.
-struct FastDiv {
-    uint32_t d, m;
-    int s1, s2;
-};
-inline FastDiv make_fastdiv(uint32_t d)
-{
-    int l = 0;
-    while (l < 32 && (1ull << l) < d) ++l;
-    FastDiv f;
-    f.d = d;
-    f.m = (uint32_t)(((((1ull << l) - d) << 32) / d) + 1);
-    f.s1 = l < 1 ? l : 1;
-    f.s2 = l > 1 ? l - 1 : 0;
-    return f;
-}
-__device__ __forceinline__ uint32_t fast_div(const FastDiv& f, uint32_t n)
-{
-    const uint32_t t1 = __umulhi(f.m, n);
-    return (t1 + ((n - t1) >> f.s1)) >> f.s2;
-}
 
 struct WaveArgs {
     DevScene S;
@@ -321,26 +207,9 @@ __global__ void __launch_bounds__(kShadeThreads) k_light_gen(WaveArgs A)
             lmax = J.light_max;
         }
         const float* cdf = S.light_cdf + lbase;
-        // DistanceRandom::getValue (DistanceRandom.h:98-115); one light: no draw
+        // one light: no draw
         int li = 0;
-        if (N > 1) {
-            const float d = rng4(c.seed, pixel, sample, 0u, kStreamLight).u[0] * lmax;
-            if (d <= cdf[0])
-                li = 0;
-            else if (d >= cdf[N - 2])
-                li = N - 1;
-            else {
-                int L = 0, Rr = N - 1;
-                while (L < Rr) {
-                    int C = (L + Rr) / 2;
-                    if (d <= cdf[C])
-                        Rr = C;
-                    else
-                        L = C + 1;
-                }
-                li = (L + Rr) / 2;
-            }
-        }
+        if (N > 1) li = pick_light(cdf, N, rng4(c.seed, pixel, sample, 0u, kStreamLight).u[0] * lmax);
         li += lbase;
         R = light_direction(c.seed, pixel, sample);  // RandomSampler::uniformSphere
         const float4 lp = __ldg(S.light_pos + li);
@@ -361,10 +230,7 @@ __global__ void __launch_bounds__(kShadeThreads) k_light_gen(WaveArgs A)
 }
 
 // ------------------------------------------------------------ extend ---
-// Persistent closest-hit over one ray queue (count at *count): a warp takes 32
-// consecutive rays and the next 32 when all are done (camera rays: the 32
-// samples of one pixel stay together).  Replacing finished rays lane by lane
-// (Aila & Laine 2009) was measured slower on every bounce.
+// Persistent closest hit over one ray queue (count at *count).
 // `jobs` (batches over a group of scenes, else null): the top-level tree of
 // the path's scene (the path index travels in the ray's last word)
 __device__ __forceinline__ uint32_t path_root(const DevJob* jobs, const uint32_t* path_job, int k)
@@ -385,27 +251,7 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceMinBlocks) k_extend(DevSc
     TraceCounters tc{0u, 0u};
     const uint32_t n = *count;
     const int lane = threadIdx.x & 31;
-    while (true) {
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(work, 32u);
-        base = __shfl_sync(0xFFFFFFFFu, base, 0);
-        if (base >= n) break;
-        const uint32_t i = base + lane;
-        if (i < n) {
-            float4 a = rq[2 * (size_t)i], b = rq[2 * (size_t)i + 1];
-            V3 o = v3(a.x, a.y, a.z), d = v3(b.x, b.y, b.z);
-            float tnear = a.w;
-            RayHit h;
-            uint4 out;
-            if (scene_intersect(S, items, o, d, tnear, kFltMax, h, st, tc,
-                                path_root(jobs, path_job, __float_as_int(b.w))))
-                out = make_uint4(h.inst, h.prim, __float_as_uint(h.u), __float_as_uint(h.v));
-            else
-                out = make_uint4(kInvalid, kInvalid, 0u, 0u);
-            hits[i] = out;
-            if (tnear != a.w) rq[2 * (size_t)i].w = tnear;
-        }
-    }
+    extend_rays(S, items, rq, hits, n, work, st, tc, [&](int k) { return path_root(jobs, path_job, k); });
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&stats[stat_kind], (unsigned long long)n);
     uint32_t nodes = tc.nodes, tris = tc.tris;
     for (int o = 16; o; o >>= 1) {
@@ -705,49 +551,6 @@ __global__ void __launch_bounds__(kShadeThreads, kMis ? 3 : 4) k_camera_shade(Wa
 }
 
 // ------------------------------------------------------------ shadow ---
-// BDPTRenderer::isConnected (BDPTRenderer.cpp:208-235): whether vertex A sees
-// vertex B.  Without alpha-masked materials the closest-hit query stops at a
-// hit well short of B, which already decides "not connected".
-template <bool kMasked>
-__device__ __forceinline__ bool is_connected(const DevScene& S, const uint32_t* items, V3 A, V3 B, TraceStack& st,
-                                             TraceCounters& tc, uint32_t root)
-{
-    bool connected = true;
-    V3 dir = B - A;
-    const float len = sqrtf(dot(dir, dir));
-    float maxsz = max_abs(A, 1.0f);
-    float safeD = 2.0f * kEpsAcc * kEps * maxsz;
-    if (!(len <= safeD)) {
-        dir = v3(dir.x / len, dir.y / len, dir.z / len);
-        float tnear = safeD;
-        const float tfar = len + (0.1f * len > safeD ? 0.1f * len : safeD);
-        const float sb = 10.0f * kEps * max_abs(B, 1.0f);
-        RayHit h;
-        bool hit;
-        if (kMasked) {
-            hit = scene_intersect(S, items, A, dir, tnear, tfar, h, st, tc, root);
-        } else {
-            // any hit this far short of B is farther than sb from it (the
-            // margin is ~800 ulps of the coordinates, far above the error of
-            // the hit's surface position), so it decides: not connected,
-            // whichever hit is the closest.  Hits near B get the exact test.
-            const float margin = 1.0e-4f * fmaxf(maxsz, max_abs(B, 1.0f)) + 2.0f * sb;
-            hit = trace_closest_or_below(S, items, A, dir, tnear, tfar, len - margin, h, st, tc, root);
-            if (hit && h.t < len - margin) {
-                hit = false;
-                connected = false;
-            }
-        }
-        if (hit) {
-            const Surf sp = surface_point(S, h.inst, h.prim, h.u, h.v, false);
-            const V3 dd = sp.pos - B;
-            const float sd = dot(dd, dd);
-            connected = sd <= sb * sb;
-        }
-    }
-    return connected;
-}
-
 // whether the environment ray (shifted origin so, direction w, the path's
 // tnear) escapes: no hit at all
 template <bool kMasked>

@@ -219,6 +219,8 @@ SceneHost::~SceneHost()
     if (stream) cudaStreamSynchronize(stream);
     for (void* p : allocs) cudaFree(p);
     if (scratch.base) cudaFree(scratch.base);
+    if (adj_scratch) cudaFree(adj_scratch);
+    if (adj_done) cudaEventDestroy(adj_done);
     if (mat_sets) cudaFree(mat_sets);
     if (d_jobs) cudaFree(d_jobs);
     if (batch_graph) cudaGraphExecDestroy(batch_graph);

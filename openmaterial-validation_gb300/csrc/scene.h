@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -127,6 +128,10 @@ struct SceneHost {
     int64_t batch_wave_paths = 0;            // autotuned wave size for batches (0: automatic)
     int batch_shade_threads = 0;             // autotuned threads per shading block for batches (0: 256)
     std::vector<ScenePart> parts;            // the scenes of a group (one for a single scene)
+    std::mutex adj_mutex;                    // one adjoint call at a time enqueues
+    void* adj_scratch = nullptr;             // records of an adjoint wave
+    size_t adj_bytes = 0;
+    cudaEvent_t adj_done = nullptr;          // the last use of adj_scratch
 
     ~SceneHost();
     void* alloc(size_t bytes);
@@ -167,7 +172,7 @@ void ensure_env_sampler(SceneHost& s);
 void set_scene_materials(SceneHost& s, int num, const omv_material_desc* descs);
 // path-replay gradient of an image loss with respect to the material parameters
 void adjoint_frame(SceneHost& s, const omv_camera& cam, const omv_params& p, const float* d_adjoint, float* d_grad,
-                   cudaStream_t st, int part = 0, const DevMaterial* mats = nullptr);
+                   cudaStream_t st);
 // the adjoint of every job of a list (each job's scene, material set, camera and samples)
 void adjoint_batch(SceneHost& s, int n, const omv_adjoint_job* jobs, const omv_params& p, cudaStream_t st);
 

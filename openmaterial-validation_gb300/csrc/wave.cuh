@@ -1,0 +1,220 @@
+// Building blocks of the wavefront pipelines (the renderer's and the
+// path-replay adjoint's): queue appends, division by frame constants, the
+// light pick, the closest-hit loop over a ray queue and the connection test.
+#pragma once
+
+#include <cooperative_groups.h>
+#include <cuda_runtime.h>
+
+#include "omv_device.cuh"
+#include "shade.cuh"
+#include "trace.cuh"
+
+namespace omv {
+
+constexpr int kTraceThreads = 128;
+// 6 resident blocks of the trace kernels per SM (80 registers, a few spilled
+// stack words): more warps in flight for the latency-bound traversal than the
+// 5 blocks its unconstrained 96 registers allow (measured 3.18 -> 3.06 ms per
+// extension launch on the 1920x1080x64 frame; 7 and 8 blocks spill more)
+constexpr int kTraceMinBlocks = 6;
+constexpr int kShadeThreads = 256;
+
+__device__ __forceinline__ uint32_t warp_append(uint32_t* counter, bool want)
+{
+    const uint32_t m = __ballot_sync(0xFFFFFFFFu, want);
+    if (!m) return 0;
+    const int lane = threadIdx.x & 31;
+    const int leader = __ffs(m) - 1;
+    uint32_t base = 0;
+    if (lane == leader) base = atomicAdd(counter, (uint32_t)__popc(m));
+    base = __shfl_sync(0xFFFFFFFFu, base, leader);
+    return base + __popc(m & ((1u << lane) - 1u));
+}
+
+// Opportunistic warp aggregation (for appends inside divergent code): the
+// threads of a warp that arrive together take consecutive slots with one atomic.
+__device__ __forceinline__ uint32_t coalesced_append(uint32_t* counter)
+{
+    namespace cg = cooperative_groups;
+    const cg::coalesced_group g = cg::coalesced_threads();
+    uint32_t base = 0;
+    if (g.thread_rank() == 0) base = atomicAdd(counter, (uint32_t)g.size());
+    return g.shfl(base, 0) + (uint32_t)g.thread_rank();
+}
+
+// Direction bin of a ray: the cube face its direction points to (dominant
+// axis and sign) and the quadrant on that face, 24 bins.
+constexpr int kDirBins = 24;
+__device__ __forceinline__ uint32_t direction_bin(V3 d)
+{
+    const float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
+    uint32_t f;
+    float u, v;
+    if (ax >= ay && ax >= az) {
+        f = d.x < 0.0f ? 1u : 0u;
+        u = d.y;
+        v = d.z;
+    } else if (ay >= az) {
+        f = d.y < 0.0f ? 3u : 2u;
+        u = d.z;
+        v = d.x;
+    } else {
+        f = d.z < 0.0f ? 5u : 4u;
+        u = d.x;
+        v = d.y;
+    }
+    return 4u * f + (u < 0.0f ? 2u : 0u) + (v < 0.0f ? 1u : 0u);
+}
+
+struct BinScratch {
+    uint32_t count[kDirBins];
+    uint32_t base;
+};
+
+// Block-wide append to a queue with the block's entries grouped by bin, so
+// that the warps tracing the queue get rays of similar direction from nearby
+// pixels.  One atomic per block; every thread of the block must call it.
+__device__ __forceinline__ uint32_t block_append_binned(uint32_t* counter, bool want, uint32_t bin, BinScratch& sh)
+{
+    if (threadIdx.x < kDirBins) sh.count[threadIdx.x] = 0;
+    __syncthreads();
+    const uint32_t rank = want ? atomicAdd(&sh.count[bin], 1u) : 0u;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        // exclusive scan of the bin counts in the first warp; lane 31 reserves
+        const uint32_t c = threadIdx.x < kDirBins ? sh.count[threadIdx.x] : 0u;
+        uint32_t x = c;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+            if ((int)threadIdx.x >= o) x += y;
+        }
+        if (threadIdx.x < kDirBins) sh.count[threadIdx.x] = x - c;
+        if (threadIdx.x == 31) sh.base = x ? atomicAdd(counter, x) : 0u;
+    }
+    __syncthreads();
+    const uint32_t slot = sh.base + sh.count[bin] + rank;
+    __syncthreads();  // the scratch is reused by the next call
+    return slot;
+}
+
+// Division of 32-bit unsigned integers by a divisor fixed for a frame, by one
+// multiply-high, a subtraction and two shifts (Granlund & Montgomery,
+// "Division by invariant integers using multiplication", PLDI 1994, 4.1):
+// exact for every numerator and every divisor >= 1, where the hardware has
+// no integer divide.
+struct FastDiv {
+    uint32_t d, m;
+    int s1, s2;
+};
+inline FastDiv make_fastdiv(uint32_t d)
+{
+    int l = 0;
+    while (l < 32 && (1ull << l) < d) ++l;
+    FastDiv f;
+    f.d = d;
+    f.m = (uint32_t)(((((1ull << l) - d) << 32) / d) + 1);
+    f.s1 = l < 1 ? l : 1;
+    f.s2 = l > 1 ? l - 1 : 0;
+    return f;
+}
+__device__ __forceinline__ uint32_t fast_div(const FastDiv& f, uint32_t n)
+{
+    const uint32_t t1 = __umulhi(f.m, n);
+    return (t1 + ((n - t1) >> f.s1)) >> f.s2;
+}
+
+// DistanceRandom::getValue (DistanceRandom.h:98-115): the light of a draw d
+// from the power CDF of n > 1 lights
+__device__ __forceinline__ int pick_light(const float* cdf, int n, float d)
+{
+    if (d <= cdf[0]) return 0;
+    if (d >= cdf[n - 2]) return n - 1;
+    int L = 0, R = n - 1;
+    while (L < R) {
+        const int C = (L + R) / 2;
+        if (d <= cdf[C])
+            R = C;
+        else
+            L = C + 1;
+    }
+    return (L + R) / 2;
+}
+
+// Persistent closest hit over the n rays of a queue (*work counts the rays
+// taken): a warp takes 32 consecutive rays and the next 32 when all are done
+// (camera rays: the 32 samples of one pixel stay together).  Replacing
+// finished rays lane by lane (Aila & Laine 2009) was measured slower on every
+// bounce.  root(k): the top-level tree of path k's scene (k travels in the
+// ray's last word).
+template <typename Root>
+__device__ __forceinline__ void extend_rays(const DevScene& S, const uint32_t* items, float4* rq, uint4* hits,
+                                            uint32_t n, uint32_t* work, TraceStack& st, TraceCounters& tc, Root root)
+{
+    const int lane = threadIdx.x & 31;
+    while (true) {
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(work, 32u);
+        base = __shfl_sync(0xFFFFFFFFu, base, 0);
+        if (base >= n) break;
+        const uint32_t i = base + lane;
+        if (i < n) {
+            float4 a = rq[2 * (size_t)i], b = rq[2 * (size_t)i + 1];
+            V3 o = v3(a.x, a.y, a.z), d = v3(b.x, b.y, b.z);
+            float tnear = a.w;
+            RayHit h;
+            uint4 out;
+            if (scene_intersect(S, items, o, d, tnear, kFltMax, h, st, tc, root(__float_as_int(b.w))))
+                out = make_uint4(h.inst, h.prim, __float_as_uint(h.u), __float_as_uint(h.v));
+            else
+                out = make_uint4(kInvalid, kInvalid, 0u, 0u);
+            hits[i] = out;
+            if (tnear != a.w) rq[2 * (size_t)i].w = tnear;
+        }
+    }
+}
+
+// BDPTRenderer::isConnected (BDPTRenderer.cpp:208-235): whether vertex A sees
+// vertex B.  Without alpha-masked materials the closest-hit query stops at a
+// hit well short of B, which already decides "not connected".
+template <bool kMasked>
+__device__ __forceinline__ bool is_connected(const DevScene& S, const uint32_t* items, V3 A, V3 B, TraceStack& st,
+                                             TraceCounters& tc, uint32_t root)
+{
+    bool connected = true;
+    V3 dir = B - A;
+    const float len = sqrtf(dot(dir, dir));
+    float maxsz = max_abs(A, 1.0f);
+    float safeD = 2.0f * kEpsAcc * kEps * maxsz;
+    if (!(len <= safeD)) {
+        dir = v3(dir.x / len, dir.y / len, dir.z / len);
+        float tnear = safeD;
+        const float tfar = len + (0.1f * len > safeD ? 0.1f * len : safeD);
+        const float sb = 10.0f * kEps * max_abs(B, 1.0f);
+        RayHit h;
+        bool hit;
+        if (kMasked) {
+            hit = scene_intersect(S, items, A, dir, tnear, tfar, h, st, tc, root);
+        } else {
+            // any hit this far short of B is farther than sb from it (the
+            // margin is ~800 ulps of the coordinates, far above the error of
+            // the hit's surface position), so it decides: not connected,
+            // whichever hit is the closest.  Hits near B get the exact test.
+            const float margin = 1.0e-4f * fmaxf(maxsz, max_abs(B, 1.0f)) + 2.0f * sb;
+            hit = trace_closest_or_below(S, items, A, dir, tnear, tfar, len - margin, h, st, tc, root);
+            if (hit && h.t < len - margin) {
+                hit = false;
+                connected = false;
+            }
+        }
+        if (hit) {
+            const Surf sp = surface_point(S, h.inst, h.prim, h.u, h.v, false);
+            const V3 dd = sp.pos - B;
+            const float sd = dot(dd, dd);
+            connected = sd <= sb * sb;
+        }
+    }
+    return connected;
+}
+
+}  // namespace omv
