@@ -26,8 +26,8 @@
 // bounce, the traversal kernels are the renderer's, every launch's lanes do the
 // same work, and the derivatives, recomputed where the backward walk needs
 // them, never leave registers.  512x512, 32 spp, 100k triangles, 8 materials:
-// 103 ms before, 9.4 ms so.  Jobs of a batch share the waves: one step (forward
-// and replay) of an inverse fit of eight 128x128x16 scenes 29.1 -> 6.7 ms.
+// 103 ms before, 7.7 ms so.  Jobs of a batch share the waves: one step (forward
+// and replay) of an inverse fit of eight 128x128x16 scenes 29.1 -> 6.0 ms.
 //
 // Gradients: the lanes of a warp that meet the same material reduce by
 // shuffles into the warp's sums in shared memory, the block adds its totals to
@@ -147,81 +147,6 @@ __device__ __forceinline__ V3 adj_delta(const AdjPath& p)
 }
 __device__ __forceinline__ bool is_zero(V3 a) { return a.x == 0.0f && a.y == 0.0f && a.z == 0.0f; }
 
-// derivatives of a vertex weight (or evaluation) with respect to the
-// material's local parameters: PBR r,g,b, alpha, metallic; OpenMATERIAL
-// n r,g,b, k r,g,b
-struct LocalGrad {
-    float d[3][6];
-};
-__device__ __forceinline__ void lg_zero(LocalGrad& g)
-{
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-#pragma unroll
-        for (int i = 0; i < 6; ++i) g.d[c][i] = 0.0f;
-}
-
-// material_sample's weight and its local derivatives (direction fixed)
-__device__ __forceinline__ V3 sample_with_grad(const DevScene& S, const DevMaterial& M, const Surf& sp, V3 in, bool inv,
-                                               const Rng4& u, V3& out, LocalGrad& g)
-{
-    lg_zero(g);
-    SampleInfo info;
-    const V3 w = material_sample(S, M, sp, in, inv, u, out, &info);
-    if (M.type == kMatPbr) {
-        if (info.kind < 0) return w;
-        const PbrDual m = pbr_dual(M.color, M.alpha, M.metal);
-        Dual<5> dw[3];
-        d_bsdf_evaluate(in, out, info.N, m, info.kind, info.H, info.p, dw);
-        const float score = info.kind != 0 ? ggx_log_pdf_dalpha(fabsf(dot(info.N, info.H)), M.alpha) : 0.0f;
-        const float wv[3] = {w.x, w.y, w.z};
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-#pragma unroll
-            for (int i = 0; i < 5; ++i) g.d[c][i] = dw[c].d[i];
-            g.d[c][3] += wv[c] * score;
-        }
-    } else if (M.type == kMatOm && M.om_valid) {
-        const float cth = dot(out, sp.nrm);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const Dual<2> r = d_om_channel(M.om_n[c], M.om_k[c], cth);
-            g.d[c][c] = r.d[0];
-            g.d[c][3 + c] = r.d[1];
-        }
-    }
-    return w;
-}
-
-// material_eval and its local derivatives
-__device__ __forceinline__ V3 eval_with_grad(const DevMaterial& M, const Surf& sp, V3 in, V3 out, LocalGrad& g)
-{
-    lg_zero(g);
-    const V3 f = material_eval(M, sp, in, out);
-    if (M.type == kMatPbr) {
-        V3 N = sp.nrm;
-        if (dot(in, N) > 0.0f && M.transmissive) N = -N;
-        const PbrDual m = pbr_dual(M.color, M.alpha, M.metal);
-        Dual<5> df[3];
-        d_bsdf_eval_direct(in, out, N, m, df);
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-#pragma unroll
-            for (int i = 0; i < 5; ++i) g.d[c][i] = df[c].d[i];
-    } else if (M.type == kMatOm && M.om_valid) {
-        const float cth = -dot(in, sp.nrm);
-        if (!(fabsf(dot(out, sp.nrm) - cth) > 1e-6f)) {
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const Dual<2> r = d_om_channel(M.om_n[c], M.om_k[c], cth);
-                g.d[c][c] = r.d[0];
-                g.d[c][3 + c] = r.d[1];
-            }
-        }
-    }
-    return f;
-}
-
 // ------------------------------------------------- gradient sums ---
 // a term of a gradient unless it is not finite: a degenerate path (an infinite
 // sample of the forward estimator) must not poison the sum
@@ -240,28 +165,93 @@ __device__ __forceinline__ void no_terms(GradTerms& t)
 #pragma unroll
     for (int i = 0; i < 6; ++i) t.v[i] = 0.0f;
 }
-__device__ __forceinline__ void grad_terms(GradTerms& t, const AdjJob& J, const DevMaterial& M, uint32_t mat, V3 a,
-                                           const LocalGrad& g)
+__device__ __forceinline__ float channel(V3 a, int c) { return c == 0 ? a.x : c == 1 ? a.y : a.z; }
+
+// key of the material's sums; false for the missing material, which has no
+// parameters
+__device__ __forceinline__ bool terms_key(GradTerms& t, const AdjJob& J, const DevMaterial& M, uint32_t mat)
 {
     const uint32_t m = mat - J.mat_base;
-    if (m >= (uint32_t)J.nmat) return;  // the missing material has no parameters
-    const float av[3] = {a.x, a.y, a.z};
+    if (m >= (uint32_t)J.nmat || M.type == kMatMissing) return false;
+    t.key = J.key_base + (int)m * kSlots + (M.type == kMatOm ? 5 : 0);
+    return true;
+}
+// a channel's terms: its adjoint a times its derivatives
+__device__ __forceinline__ void pbr_terms(GradTerms& t, int c, float a, float rough, Dual<3> f)
+{
+    const float col = finite_or_zero(a * f.d[0]);
+    t.v[0] += c == 0 ? col : 0.0f;
+    t.v[1] += c == 1 ? col : 0.0f;
+    t.v[2] += c == 2 ? col : 0.0f;
+    t.v[3] += finite_or_zero(a * f.d[1] * 2.0f * rough);  // alpha = roughness^2
+    t.v[4] += finite_or_zero(a * f.d[2]);
+}
+__device__ __forceinline__ void om_terms(GradTerms& t, int c, float a, Dual<2> f)
+{
+    const float n = finite_or_zero(a * f.d[0]), k = finite_or_zero(a * f.d[1]);
+    t.v[0] += c == 0 ? n : 0.0f;
+    t.v[1] += c == 1 ? n : 0.0f;
+    t.v[2] += c == 2 ? n : 0.0f;
+    t.v[3] += c == 0 ? k : 0.0f;
+    t.v[4] += c == 1 ? k : 0.0f;
+    t.v[5] += c == 2 ? k : 0.0f;
+}
+
+// The terms of a sampled weight (material_sample times the cosine of `out` or,
+// for a light vertex, of `in`; directions fixed) against its adjoint a.
+__device__ __forceinline__ void sample_terms(GradTerms& t, const AdjJob& J, const DevScene& S, const DevMaterial& M,
+                                             const Surf& sp, uint32_t mat, V3 in, bool light, const Rng4& u, V3 a)
+{
+    SampleInfo info;
+    V3 out;
+    const V3 w = material_sample(S, M, sp, in, !light, u, out, &info);
+    const float ct = fabsf(dot(light ? in : out, sp.nrm));
     if (M.type == kMatPbr) {
-        t.key = J.key_base + (int)m * kSlots;
-        const float rough = sqrtf(M.alpha);  // alpha = roughness^2
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-#pragma unroll
-            for (int i = 0; i < 5; ++i)
-                t.v[i] += finite_or_zero(i == 3 ? av[c] * g.d[c][i] * 2.0f * rough : av[c] * g.d[c][i]);
-    } else if (M.type == kMatOm) {
-        t.key = J.key_base + (int)m * kSlots + 5;
-#pragma unroll
+        if (info.kind < 0 || !terms_key(t, J, M, mat)) return;
+        const float alpha = M.alpha, metal = M.metal, rough = sqrtf(alpha);
+        const DualEvaluate e = d_bsdf_evaluate(in, out, info.N, alpha, info.kind, info.H, info.p);
+        const float score = info.kind != 0 ? ggx_log_pdf_dalpha(fabsf(dot(info.N, info.H)), alpha) : 0.0f;
+#pragma unroll 1
         for (int c = 0; c < 3; ++c) {
-            t.v[c] += finite_or_zero(av[c] * g.d[c][c]);
-            t.v[3 + c] += finite_or_zero(av[c] * g.d[c][3 + c]);
+            Dual<3> f = d_evaluate_channel(e, M.color[c], metal);
+            f.d[1] += channel(w, c) * score;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) f.d[i] *= ct;
+            pbr_terms(t, c, channel(a, c), rough, f);
+        }
+    } else if (M.type == kMatOm && M.om_valid) {
+        if (!terms_key(t, J, M, mat)) return;
+        const float cth = dot(out, sp.nrm);
+#pragma unroll 1
+        for (int c = 0; c < 3; ++c) {
+            Dual<2> f = d_om_channel(M.om_n[c], M.om_k[c], cth);
+            f.d[0] *= ct;
+            f.d[1] *= ct;
+            om_terms(t, c, channel(a, c), f);
         }
     }
+}
+
+// material_eval, and its terms against its adjoint a
+__device__ __forceinline__ V3 eval_terms(GradTerms& t, const AdjJob& J, const DevMaterial& M, const Surf& sp,
+                                         uint32_t mat, V3 in, V3 out, V3 a)
+{
+    const V3 f = material_eval(M, sp, in, out);
+    if (M.type == kMatPbr) {
+        if (!terms_key(t, J, M, mat)) return f;
+        V3 N = sp.nrm;
+        if (dot(in, N) > 0.0f && M.transmissive) N = -N;
+        const float alpha = M.alpha, metal = M.metal, rough = sqrtf(alpha);
+        const DualDirect e = d_bsdf_eval_direct(in, out, N, alpha);
+#pragma unroll 1
+        for (int c = 0; c < 3; ++c) pbr_terms(t, c, channel(a, c), rough, d_direct_channel(e, M.color[c], metal));
+    } else if (M.type == kMatOm && M.om_valid) {
+        const float cth = -dot(in, sp.nrm);
+        if (fabsf(dot(out, sp.nrm) - cth) > 1e-6f || !terms_key(t, J, M, mat)) return f;
+#pragma unroll 1
+        for (int c = 0; c < 3; ++c) om_terms(t, c, channel(a, c), d_om_channel(M.om_n[c], M.om_k[c], cth));
+    }
+    return f;
 }
 
 // Adds the lanes' terms to the warp's sums; every lane of the warp calls it.
@@ -628,11 +618,10 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_connect(AdjWave A, int b)
             const V3 LC = normalize(sp.pos - lPos);
             const V3 lRad = connection_radiance(A, A.lmeta[k] & kLightMask, v, k, sp.pos, lPos);
             const float c = fabsf(dot(LC, sp.nrm));
-            LocalGrad g;
-            const V3 f = eval_with_grad(M, sp, LC, -v3(rb.x, rb.y, rb.z), g) * c;
-            const V3 delta = adj_delta(p);
-            const V3 a = mul(delta, tp);
-            grad_terms(t, J, M, mat, mul(a, v3(lRad.x * c, lRad.y * c, lRad.z * c)), g);
+            const V3 a = mul(adj_delta(p), tp);
+            const V3 f = eval_terms(t, J, M, sp, mat, LC, -v3(rb.x, rb.y, rb.z),
+                                    mul(a, v3(lRad.x * c, lRad.y * c, lRad.z * c))) *
+                         c;
             const V3 G = mul(f, lRad);
             float* pg = &A.cG[e].x;
             atomicAdd(pg, G.x);
@@ -682,15 +671,7 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_camera_back(AdjWave A, int 
                     const DevMaterial& M = J.mats[mat];
                     const Surf sp = surface_point(S, h.x, h.y, __uint_as_float(h.z), __uint_as_float(h.w), true, &M);
                     const Rng4 u = rng4(J.seed, p.pixel, p.sample, (uint32_t)b, kStreamCamera);
-                    V3 O;
-                    LocalGrad g;
-                    sample_with_grad(S, M, sp, v3(rb.x, rb.y, rb.z), true, u, O, g);
-                    const float ct = fabsf(dot(O, sp.nrm));
-#pragma unroll
-                    for (int c = 0; c < 3; ++c)
-#pragma unroll
-                        for (int j = 0; j < 6; ++j) g.d[c][j] *= ct;
-                    grad_terms(t, J, M, mat, a, g);
+                    sample_terms(t, J, S, M, sp, mat, v3(rb.x, rb.y, rb.z), false, u, a);
                 }
                 R = R + mul(v3(w4.x, w4.y, w4.z), Rs);
             }
@@ -731,16 +712,7 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_light_back(AdjWave A, int b
                     const DevMaterial& M = J.mats[mat];
                     const Surf sp = surface_point(S, h.x, h.y, __uint_as_float(h.z), __uint_as_float(h.w), true, &M);
                     const Rng4 u = rng4(J.seed, p.pixel, p.sample, kDimLightBounce + (uint32_t)b, kStreamLight);
-                    const V3 R = v3(rb.x, rb.y, rb.z);
-                    V3 O;
-                    LocalGrad g;
-                    sample_with_grad(S, M, sp, R, false, u, O, g);
-                    const float ct = fabsf(dot(R, sp.nrm));
-#pragma unroll
-                    for (int c = 0; c < 3; ++c)
-#pragma unroll
-                        for (int j = 0; j < 6; ++j) g.d[c][j] *= ct;
-                    grad_terms(t, J, M, mat, a, g);
+                    sample_terms(t, J, S, M, sp, mat, v3(rb.x, rb.y, rb.z), true, u, a);
                 }
             }
         }

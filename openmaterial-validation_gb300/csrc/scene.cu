@@ -820,7 +820,9 @@ __global__ void k_hook_sample(int64_t n, const float* in, float* out)
     d.eta = x[15];
     d.transmissive = x[16] != 0.0f;
     V3 O;
-    V3 w = bsdf_sample_indirect(d, x[17], x[18], x[19], O);
+    float sphi, cphi;
+    azimuth(x[18], sphi, cphi);
+    V3 w = bsdf_sample_indirect(d, x[17], sphi, cphi, x[19], O);
     float* o = out + 6 * i;
     o[0] = O.x;
     o[1] = O.y;

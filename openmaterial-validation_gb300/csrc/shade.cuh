@@ -36,7 +36,9 @@ __device__ __forceinline__ TexHit tex_hit(const Surf& sp)
 
 // BitmapTexture::getPixCoords + texture(u, v, fvec4) (BitmapTexture.cpp:73-125):
 // bilinear over the four wrapped neighbours, texels scaled by 1/255
-__device__ __forceinline__ float4 tex_sample(const DevScene& S, int t, float u, float v)
+// One copy of the code per kernel (see bsdf_evaluate): up to five lookups per
+// vertex share it.
+static __device__ __noinline__ float4 tex_sample(const DevScene& S, int t, float u, float v)
 {
     const DevTexture T = S.textures[t];
     if (!T.present) return make_float4(0.5f, 0.5f, 0.5f, 1.0f);
@@ -50,7 +52,10 @@ __device__ __forceinline__ float4 tex_sample(const DevScene& S, int t, float u, 
     const int iu = (int)u, iv = (int)v;
     const float kui = u - (float)iu, kvi = v - (float)iv;
     const float ku = 1.0f - kui, kv = 1.0f - kvi;
-    const int l = iu % W, r = (iu + 1) % W, b = iv % H, tp = (iv + 1) % H;
+    // u and v are in [0, 1 + half a texel) here (0 for NaN coordinates), so iu is
+    // in [0, W] and iv in [0, H]: the remainders by conditional subtractions
+    const int l = iu >= W ? iu - W : iu, b = iv >= H ? iv - H : iv;
+    const int r = l + 1 >= W ? 0 : l + 1, tp = b + 1 >= H ? 0 : b + 1;
     const uchar4* px = S.texels + T.offset;
     const uchar4 c0 = __ldg(px + b * W + l), c1 = __ldg(px + b * W + r);
     const uchar4 c2 = __ldg(px + tp * W + l), c3 = __ldg(px + tp * W + r);
@@ -262,38 +267,51 @@ __device__ __forceinline__ V3 face_normal(const DevScene& S, const Surf& sp)
     return normalize(m33(nm, cross(e1, e2)));
 }
 
+// the BsdfIn material_sample builds for a PBR vertex
+__device__ __forceinline__ BsdfIn pbr_bsdf_in(const DevMaterial& M, const PbrParams& P, const Surf& sp, V3 in)
+{
+    BsdfIn d;
+    d.I = in;
+    d.N = sp.nrm;
+    d.T = sp.tan;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) d.color[i] = P.color[i];
+    d.metal = P.metal;
+    d.alpha = P.alpha;
+    d.eta = M.eta;
+    d.transmissive = P.transmissive;
+    return d;
+}
+
+// the OpenMATERIAL Fresnel term of the three channels (one copy of its code)
+__device__ __forceinline__ V3 om_rgb(const DevMaterial& M, float c)
+{
+    return v3(om_channel(M.om_n[0], M.om_k[0], c), om_channel(M.om_n[1], M.om_k[1], c),
+              om_channel(M.om_n[2], M.om_k[2], c));
+}
+
 // RenderMaterial::getRayAndBrdf of each material kind; u = the vertex's
 // uniforms, P = the vertex's PBR values (pbr_params)
 __device__ __forceinline__ V3 material_sample(const DevScene& S, const DevMaterial& M, const PbrParams& P,
                                               const Surf& sp, V3 in, bool inv, const Rng4& u, V3& out,
                                               SampleInfo* info = nullptr)
 {
-    if (M.type == kMatPbr) {  // PhysicallyBasedMaterial::getRayAndBrdf (:248-291)
-        BsdfIn d;
-        d.I = in;
-        d.N = sp.nrm;
-        d.T = sp.tan;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) d.color[i] = P.color[i];
-        d.metal = P.metal;
-        d.alpha = P.alpha;
-        d.eta = M.eta;
-        d.transmissive = P.transmissive;
-        return bsdf_sample_indirect(d, u.u[0], u.u[1], u.u[2], out, info);
-    }
     if (M.type == kMatOm) {  // OpenMaterial::defineNextDirection + getRayAndBrdf (:72-93, :165-232)
         out = reflect3(in, sp.nrm);
         V3 tfn = face_normal(S, sp);
         float corr = dot(out, tfn);
         if (corr < 0.1f) out = normalize(tfn * (0.1f - corr) + out);
         if (!M.om_valid) return v3(0.0f, 0.0f, 0.0f);
-        float c = dot(out, sp.nrm);
-        return v3(om_channel(M.om_n[0], M.om_k[0], c), om_channel(M.om_n[1], M.om_k[1], c),
-                  om_channel(M.om_n[2], M.om_k[2], c));
+        return om_rgb(M, dot(out, sp.nrm));
     }
-    // missing material: DiffuseColorMaterial (uniform hemisphere, brdf = albedo)
-    out = to_basis(sp.tan, sp.bin, sp.nrm, uniform_hemisphere(u.u[0], u.u[1]));
     (void)inv;
+    const bool pbr = M.type == kMatPbr;
+    float sphi, cphi;
+    azimuth(pbr ? u.u[1] : u.u[0], sphi, cphi);
+    if (pbr)  // PhysicallyBasedMaterial::getRayAndBrdf (:248-291)
+        return bsdf_sample_indirect(pbr_bsdf_in(M, P, sp, in), u.u[0], sphi, cphi, u.u[2], out, info);
+    // missing material: DiffuseColorMaterial (uniform hemisphere, brdf = albedo)
+    out = to_basis(sp.tan, sp.bin, sp.nrm, uniform_hemisphere(sphi, cphi, u.u[1]));
     return v3(M.color[0], M.color[1], M.color[2]);
 }
 
@@ -309,26 +327,9 @@ __device__ __forceinline__ V3 material_eval(const DevMaterial& M, const PbrParam
         if (!M.om_valid) return v3(0.0f, 0.0f, 0.0f);
         float c = -dot(in, sp.nrm);
         if (fabsf(dot(out, sp.nrm) - c) > 1e-6f) return v3(0.0f, 0.0f, 0.0f);
-        return v3(om_channel(M.om_n[0], M.om_k[0], c), om_channel(M.om_n[1], M.om_k[1], c),
-                  om_channel(M.om_n[2], M.om_k[2], c));
+        return om_rgb(M, c);
     }
     return v3(M.color[0], M.color[1], M.color[2]);
-}
-
-// the BsdfIn material_sample builds for a PBR vertex
-__device__ __forceinline__ BsdfIn pbr_bsdf_in(const DevMaterial& M, const PbrParams& P, const Surf& sp, V3 in)
-{
-    BsdfIn d;
-    d.I = in;
-    d.N = sp.nrm;
-    d.T = sp.tan;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) d.color[i] = P.color[i];
-    d.metal = P.metal;
-    d.alpha = P.alpha;
-    d.eta = M.eta;
-    d.transmissive = P.transmissive;
-    return d;
 }
 
 // the same without textures (the material's constants)
