@@ -390,7 +390,7 @@ __device__ __forceinline__ uint32_t adj_root(const AdjWave& A, int k)
 }
 
 __global__ void __launch_bounds__(kTraceThreads, kTraceMinBlocks)
-    k_adj_extend(AdjWave A, float4* rq, uint4* hits, const uint32_t* count, uint32_t* work)
+    k_adj_extend(const __grid_constant__ AdjWave A, float4* rq, uint4* hits, const uint32_t* count, uint32_t* work)
 {
     __shared__ uint2 sstack[kStackShared * kTraceThreads];
     TraceStack st;
@@ -398,13 +398,43 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceMinBlocks)
     st.stride = kTraceThreads;
     st.overflow = 0;
     TraceCounters tc{0u, 0u};
-    extend_rays(A.S, A.items, rq, hits, *count, work, st, tc, [&](int k) { return adj_root(A, k); });
+    const AdjJob* jobs = A.jobs;
+    const uint32_t* path_job = A.path_job;
+    auto root = [=](int k) { return jobs[path_job ? path_job[k] : 0u].tlas_root; };
+    const uint32_t n = *count;
+    if (n <= kCoopRays)
+        extend_rays_coop(A.S, A.items, rq, hits, n, work, sstack, root);
+    else
+        extend_rays(A.S, A.items, rq, hits, n, work, st, tc, root);
+}
+
+// k_adj_shadow's loop for short queues, eight lanes per connection
+template <bool kMasked>
+__device__ __noinline__ void adj_shadow_coop(const AdjWave& A, uint32_t n, uint32_t* seen, uint32_t* work, uint2* stacks)
+{
+    CoopGroup g = coop_group(stacks);
+    TraceCounters tc{0u, 0u};
+    TraceStack unused;
+    RayShares shares = ray_shares(work, 32u / kCoopLanes);
+    uint32_t base;
+    while (next_share(shares, n, base)) {
+        const uint32_t i = base + (uint32_t)g.index;
+        bool ok = false;
+        if (i < n) {
+            const float4 q0 = A.conn[2 * (size_t)i], q1 = A.conn[2 * (size_t)i + 1];
+            ok = is_connected<kMasked>(A.S, A.items, v3(q0.x, q0.y, q0.z), v3(q1.x, q1.y, q1.z), unused, tc,
+                                       adj_root(A, __float_as_int(q0.w)), &g) &&
+                 g.sub == 0;
+        }
+        const uint32_t slot = warp_append(seen, ok);
+        if (ok) A.seen[slot] = i;
+    }
 }
 
 // the connections of one camera bounce: the unoccluded ones are listed
 template <bool kMasked>
 __global__ void __launch_bounds__(kTraceThreads, kTraceMinBlocks)
-    k_adj_shadow(AdjWave A, const uint32_t* count, uint32_t* seen, uint32_t* work)
+    k_adj_shadow(const __grid_constant__ AdjWave A, const uint32_t* count, uint32_t* seen, uint32_t* work)
 {
     __shared__ uint2 sstack[kStackShared * kTraceThreads];
     TraceStack st;
@@ -414,11 +444,13 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceMinBlocks)
     TraceCounters tc{0u, 0u};
     const uint32_t n = *count;
     const int lane = threadIdx.x & 31;
-    while (true) {
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(work, 32u);
-        base = __shfl_sync(0xFFFFFFFFu, base, 0);
-        if (base >= n) break;
+    if (n <= kCoopRays) {
+        adj_shadow_coop<kMasked>(A, n, seen, work, sstack);
+        return;
+    }
+    RayShares shares = ray_shares(work, 32u);
+    uint32_t base;
+    while (next_share(shares, n, base)) {
         const uint32_t i = base + lane;
         bool ok = false;
         if (i < n) {

@@ -60,10 +60,16 @@ enum {
 // shadow-ray kernel (measured: the 256x256x16 C1 frame 1.72 instead of 1.30
 // ms, the 1920x1080x64 one 48.4 instead of 47.1, the 256-job sweep one job
 // per call 94.5 instead of 103.1 jobs/s), and so did the light subpaths'
-// analogue.  On the benchmark frame: 38.40 instead of 38.67 ms (at most 2^17
-// paths: the same; 2^19 or 2^20, which start the tail at bounce 4: 39.0).
+// analogue.  At most 2^15 paths (a 960x540x16 MIS frame 3190 us; 2^13: 3215,
+// 2^18: 3455, no tail kernel 3280 with an empty launch's 5 us): more are traced
+// faster by the wavefront, whose short queues take eight lanes per ray, and
+// fewer cost a launch pair per bounce (the 1920x1080x64 sky frame 21.83 ms,
+// 21.90 at 2^13).  A wave of at most 2^18 paths goes to the tail at its third
+// bounce whatever is alive (160x90x16: 648-652 us either way; the tail kernel
+// is then the only launch with work).
 constexpr int kTailMin = 3;
-constexpr uint32_t kTailPaths = 1u << 18;
+constexpr uint32_t kTailPaths = 1u << 15;
+constexpr int32_t kTailWave = 1 << 18;
 // counter slots of the tail kernel (beyond the per-bounce ranges)
 constexpr int kCtrTailWorkCam = 510;
 constexpr int kCtrTailDone = 511;
@@ -238,7 +244,7 @@ __device__ __forceinline__ uint32_t path_root(const DevJob* jobs, const uint32_t
     return jobs ? jobs[path_job[k]].tlas_root : kInvalid;
 }
 
-__global__ void __launch_bounds__(kTraceThreads, kTraceMinBlocks) k_extend(DevScene S, const uint32_t* items, float4* rq, uint4* hits,
+__global__ void __launch_bounds__(kTraceThreads, kTraceMinBlocks) k_extend(const __grid_constant__ DevScene S, const uint32_t* items, float4* rq, uint4* hits,
                                                           const uint32_t* count, uint32_t* work,
                                                           unsigned long long* stats, int stat_kind,
                                                           const DevJob* jobs, const uint32_t* path_job)
@@ -251,7 +257,14 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceMinBlocks) k_extend(DevSc
     TraceCounters tc{0u, 0u};
     const uint32_t n = *count;
     const int lane = threadIdx.x & 31;
-    extend_rays(S, items, rq, hits, n, work, st, tc, [&](int k) { return path_root(jobs, path_job, k); });
+    auto root = [=](int k) { return path_root(jobs, path_job, k); };
+    if (n <= kCoopRays) {
+        const CoopCounts c = extend_rays_coop(S, items, rq, hits, n, work, sstack, root);
+        tc = c.tc;
+        st.overflow = c.overflow;
+    } else {
+        extend_rays(S, items, rq, hits, n, work, st, tc, root);
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&stats[stat_kind], (unsigned long long)n);
     uint32_t nodes = tc.nodes, tris = tc.tris;
     for (int o = 16; o; o >>= 1) {
@@ -555,11 +568,47 @@ __global__ void __launch_bounds__(kShadeThreads, kMis ? 3 : 4) k_camera_shade(Wa
 // tnear) escapes: no hit at all
 template <bool kMasked>
 __device__ __forceinline__ bool env_escapes(const DevScene& S, const uint32_t* items, V3 so, V3 w, float tnear,
-                                            TraceStack& st, TraceCounters& tc, uint32_t root)
+                                            TraceStack& st, TraceCounters& tc, uint32_t root, CoopGroup* g = nullptr)
 {
     RayHit h;
+    if (g) {
+        const float inf = __int_as_float(0x7F800000);
+        return kMasked ? !coop_intersect(S, items, so, w, tnear, kFltMax, h, g->st, tc, root, g->mask, g->sub)
+                       : !coop_trace<true>(S, items, so, w, tnear, kFltMax, inf, h, g->st, tc, root, g->mask, g->sub);
+    }
     return kMasked ? !scene_intersect(S, items, so, w, tnear, kFltMax, h, st, tc, root)
                    : !trace_any(S, items, so, w, tnear, kFltMax, st, tc, root);
+}
+
+// k_shadow's loop for short queues, eight lanes per ray
+template <bool kEnv, bool kMasked>
+__device__ __noinline__ CoopCounts shadow_coop(const DevScene& S, const uint32_t* items, const float4* sq, uint32_t n,
+                                               uint32_t* work, float4* rad, uint2* stacks, const DevJob* jobs,
+                                               const uint32_t* path_job)
+{
+    CoopGroup g = coop_group(stacks);
+    TraceCounters tc{0u, 0u};
+    TraceStack unused;
+    RayShares shares = ray_shares(work, 32u / kCoopLanes);
+    uint32_t base;
+    while (next_share(shares, n, base)) {
+        const uint32_t i = base + (uint32_t)g.index;
+        if (i < n) {
+            const float4 q0 = sq[3 * (size_t)i], q1 = sq[3 * (size_t)i + 1], q2 = sq[3 * (size_t)i + 2];
+            const V3 A = v3(q0.x, q0.y, q0.z), B = v3(q1.x, q1.y, q1.z);
+            const int k = __float_as_int(q0.w);
+            const uint32_t root = path_root(jobs, path_job, k);
+            const bool connected = kEnv ? env_escapes<kMasked>(S, items, A, B, q1.w, unused, tc, root, &g)
+                                        : is_connected<kMasked>(S, items, A, B, unused, tc, root, &g);
+            if (connected && g.sub == 0) {
+                atomicAdd(&rad[k].x, q2.x);
+                atomicAdd(&rad[k].y, q2.y);
+                atomicAdd(&rad[k].z, q2.z);
+            }
+        }
+        __syncwarp();
+    }
+    return CoopCounts{tc, g.st.overflow};
 }
 
 // kEnv = false: the vertex connections (records: end points A, B and the
@@ -569,7 +618,7 @@ __device__ __forceinline__ bool env_escapes(const DevScene& S, const uint32_t* i
 // all.  Without alpha-masked materials that is an any-hit query; with them
 // sceneIntersect's closest hit and retries decide, as in k_extend.
 template <bool kEnv, bool kMasked>
-__global__ void __launch_bounds__(kTraceThreads, kTraceMinBlocks) k_shadow(DevScene S, const uint32_t* items, const float4* sq,
+__global__ void __launch_bounds__(kTraceThreads, kTraceMinBlocks) k_shadow(const __grid_constant__ DevScene S, const uint32_t* items, const float4* sq,
                                                           const uint32_t* count, uint32_t* work, float4* rad,
                                                           unsigned long long* stats, const DevJob* jobs,
                                                           const uint32_t* path_job)
@@ -582,24 +631,27 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceMinBlocks) k_shadow(DevSc
     TraceCounters tc{0u, 0u};
     const uint32_t n = *count;
     const int lane = threadIdx.x & 31;
-    while (true) {
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(work, 32u);
-        base = __shfl_sync(0xFFFFFFFFu, base, 0);
-        if (base >= n) break;
+    if (n <= kCoopRays) {
+        const CoopCounts c = shadow_coop<kEnv, kMasked>(S, items, sq, n, work, rad, sstack, jobs, path_job);
+        tc = c.tc;
+        st.overflow = c.overflow;
+    }
+    RayShares shares = ray_shares(work, 32u);
+    uint32_t base;
+    while (n > kCoopRays && next_share(shares, n, base)) {
         const uint32_t i = base + lane;
         if (i < n) {
-        const float4 q0 = sq[3 * (size_t)i], q1 = sq[3 * (size_t)i + 1], q2 = sq[3 * (size_t)i + 2];
-        const V3 A = v3(q0.x, q0.y, q0.z), B = v3(q1.x, q1.y, q1.z);
-        const int k = __float_as_int(q0.w);
-        const uint32_t root = path_root(jobs, path_job, k);
-        const bool connected = kEnv ? env_escapes<kMasked>(S, items, A, B, q1.w, st, tc, root)
-                                    : is_connected<kMasked>(S, items, A, B, st, tc, root);
-        if (connected) {
-            atomicAdd(&rad[k].x, q2.x);
-            atomicAdd(&rad[k].y, q2.y);
-            atomicAdd(&rad[k].z, q2.z);
-        }
+            const float4 q0 = sq[3 * (size_t)i], q1 = sq[3 * (size_t)i + 1], q2 = sq[3 * (size_t)i + 2];
+            const V3 A = v3(q0.x, q0.y, q0.z), B = v3(q1.x, q1.y, q1.z);
+            const int k = __float_as_int(q0.w);
+            const uint32_t root = path_root(jobs, path_job, k);
+            const bool connected = kEnv ? env_escapes<kMasked>(S, items, A, B, q1.w, st, tc, root)
+                                        : is_connected<kMasked>(S, items, A, B, st, tc, root);
+            if (connected) {
+                atomicAdd(&rad[k].x, q2.x);
+                atomicAdd(&rad[k].y, q2.y);
+                atomicAdd(&rad[k].z, q2.z);
+            }
         }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&stats[kStatShadow], (unsigned long long)n);
@@ -674,13 +726,11 @@ __global__ void __launch_bounds__(kTraceThreads, 4) k_camera_tail(WaveArgs A, in
     uint32_t rays = 0, tests = 0;
     const DevScene& S = A.S;
     const uint32_t n = A.R.ctr[kCtrCam + b0];
-    if (n == 0u || n > kTailPaths) return;  // the same decision in every block
+    if (n == 0u || (n > kTailPaths && A.wave_n > kTailWave)) return;  // the same decision in every block
     const int lane = threadIdx.x & 31;
-    while (true) {
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(work, 32u);
-        base = __shfl_sync(0xFFFFFFFFu, base, 0);
-        if (base >= n) break;
+    RayShares shares = ray_shares(work, 32u);
+    uint32_t base;
+    while (next_share(shares, n, base)) {
         const uint32_t i = base + lane;
         if (i < n) {
             float4 ra = rq_in[2 * (size_t)i], rb = rq_in[2 * (size_t)i + 1];

@@ -403,4 +403,20 @@ __device__ __forceinline__ bool scene_intersect(const DevScene& S, const uint32_
     return false;
 }
 
+// scene_intersect with eight lanes per ray (coop_trace)
+__device__ __forceinline__ bool coop_intersect(const DevScene& S, const uint32_t* items, V3 o, V3 d, float& tnear,
+                                               float tfar, RayHit& h, CoopStack& st, TraceCounters& tc, uint32_t root,
+                                               uint32_t mask, int sub)
+{
+    const float t1 = tfar;
+    for (int itr = 0; itr < kMaskedTries; ++itr) {
+        if (!coop_trace<false>(S, items, o, d, tnear, tfar, 0.0f, h, st, tc, root, mask, sub)) return false;
+        if (!hit_masked(S, h)) return true;
+        tnear = masked_retry_tnear(o, d, h.t);
+        tfar = t1;
+        if (tfar <= tnear) return false;
+    }
+    return false;
+}
+
 }  // namespace omv

@@ -438,4 +438,184 @@ __device__ __forceinline__ bool trace_closest(const DevScene& S, const uint32_t*
     return trace_end(T, hit);
 }
 
+// ------------------------------------------------ one ray per eight lanes ---
+// The same traversal with a ray's eight lanes sharing each step: lane s tests
+// child slot s of the node and the triangles of its leaf, and the group keeps
+// one stack in shared memory.  A step is then a short chain (load, one box,
+// one or two triangles, a reduction) instead of eight boxes and all leaf
+// triangles in a row, and four rays per warp diverge less than thirty-two: a
+// queue too short to fill the GPU with one ray per thread is bound by that
+// chain.  The hits are the same (boxes are conservative, and a hit is chosen
+// by (t, instance, primitive) in any order of tests).
+constexpr int kCoopLanes = 8;
+
+struct CoopStack {
+    uint2* sh;  // the group's first entry
+    int sp;
+    int overflow;
+};
+
+// kStop as in trace_step: over as soon as a hit below stop_below is taken.
+// Every lane of the group calls it with the same ray; `mask` holds the group's
+// lanes, `sub` is the lane's number in it.
+template <bool kStop>
+__device__ __forceinline__ bool coop_trace(const DevScene& S, const uint32_t* __restrict__ tlas_items, V3 o, V3 d,
+                                           float tnear, float tfar, float stop_below, RayHit& hit, CoopStack& st,
+                                           TraceCounters& tc, uint32_t root, uint32_t mask, int sub)
+{
+    if (!(tnear <= tfar) || S.num_instances == 0) return false;
+    Shear rs;
+    if (!shear_setup(d, rs)) return false;
+    const V3 idw = v3(box_rcp(d.x), box_rcp(d.y), box_rcp(d.z));
+    V3 ro = o, rid = idw;
+    float best_t = tfar, bu = 0.0f, bv = 0.0f;
+    uint32_t best_inst = kInvalid, best_prim = kInvalid, cur_inst = 0;
+    int blas_base = 0;
+    bool in_blas = false;
+    if (sub == 0) st.sh[0] = make_uint2(root == kInvalid ? S.tlas_root : root, __float_as_uint(tnear));
+    st.sp = 1;
+    __syncwarp(mask);
+    for (uint32_t guard = 0; st.sp > 0; ++guard) {
+        if (guard > (1u << 22)) {  // a malformed tree can never spin a warp forever
+            st.overflow = 1;
+            break;
+        }
+        if (in_blas && st.sp == blas_base) {
+            in_blas = false;
+            ro = o;
+            rid = idw;
+        }
+        const uint2 e = st.sh[--st.sp];
+        __syncwarp(mask);  // read by all before a push overwrites it
+        if (__uint_as_float(e.y) > best_t) continue;
+        if (e.x & kInstTag) {
+            const uint32_t ii = e.x & ~kInstTag;
+            const DevInstance* I = S.insts + ii;
+            float m[12];
+#pragma unroll
+            for (int k = 0; k < 12; ++k) m[k] = __ldg(&I->inv[k]);
+            V3 rd;
+            to_object(m, o, d, ro, rd);
+            const V3 r = v3(box_rcp(rd.x), box_rcp(rd.y), box_rcp(rd.z));
+            if (!object_box_hit(__ldg(&I->olo), __ldg(&I->ohi), ro, r, tnear, best_t) || !shear_setup(rd, rs)) {
+                ro = o;
+                continue;
+            }
+            rid = r;
+            in_blas = true;
+            blas_base = st.sp;
+            cur_inst = ii;
+            if (sub == 0) st.sh[st.sp] = make_uint2(__ldg(&I->blas_root), e.y);
+            ++st.sp;
+            __syncwarp(mask);
+            continue;
+        }
+        if (sub == 0) ++tc.nodes;
+        const uint4* N = S.nodes + 8 * (size_t)e.x;
+        const uint4 w0 = __ldg(N + 0), w1 = __ldg(N + 1);
+        const uint16_t* P = reinterpret_cast<const uint16_t*>(N + 2) + sub;  // lower planes x, y, z, then upper
+        const bool fx = rid.x >= 0.0f, fy = rid.y >= 0.0f, fz = rid.z >= 0.0f;
+        const uint32_t nx = __ldg(P + (fx ? 0 : 24)), hx = __ldg(P + (fx ? 24 : 0));
+        const uint32_t ny = __ldg(P + (fy ? 8 : 32)), hy = __ldg(P + (fy ? 32 : 8));
+        const uint32_t nz = __ldg(P + (fz ? 16 : 40)), hz = __ldg(P + (fz ? 40 : 16));
+        const uint32_t exps = w0.w;
+        const float sx = __uint_as_float(((exps & 0xFFu) + 15u) << 23);
+        const float sy = __uint_as_float((((exps >> 8) & 0xFFu) + 15u) << 23);
+        const float sz = __uint_as_float((((exps >> 16) & 0xFFu) + 15u) << 23);
+        const float ax = sx * rid.x, ay = sy * rid.y, az = sz * rid.z;
+        const float bx = (__uint_as_float(w0.x) - ro.x) * rid.x, by = (__uint_as_float(w0.y) - ro.y) * rid.y,
+                    bz = (__uint_as_float(w0.z) - ro.z) * rid.z;
+        auto plane = [](uint32_t q) { return __uint_as_float(0x3F000000u | (q << 8)); };  // qplane
+        const float tin = fmaxf(fmaxf(fmaxf(fmaf(plane(nx), ax, plane_offset<true>(bx, ax)),
+                                            fmaf(plane(ny), ay, plane_offset<true>(by, ay))),
+                                      fmaf(plane(nz), az, plane_offset<true>(bz, az))) *
+                                    0.99999952f,
+                                tnear);
+        const float tout = fminf(fminf(fminf(fmaf(plane(hx), ax, plane_offset<false>(bx, ax)),
+                                             fmaf(plane(hy), ay, plane_offset<false>(by, ay))),
+                                       fmaf(plane(hz), az, plane_offset<false>(bz, az))) *
+                                     1.00000048f,
+                                 best_t);
+        const uint32_t meta = ((sub < 4 ? w1.z : w1.w) >> (8 * (sub & 3))) & 0xFFu;
+        const bool internal = (exps >> (24 + sub)) & 1u;
+        const bool in = (internal || meta != 0u) && tin <= tout;
+        const bool leaf = in && !internal && in_blas;
+        if (__any_sync(mask, leaf)) {
+            float t = best_t, u = 0.0f, v = 0.0f;
+            uint32_t prim = kInvalid;
+            if (leaf) {
+                const uint32_t cnt = meta >> 5;
+                const float4* Tp = S.tris + 3 * (size_t)(w1.y + (meta & 31u));
+                for (uint32_t k = 0; k < cnt; ++k, Tp += 3) {
+                    const float4 a = __ldg(Tp), b = __ldg(Tp + 1), c = __ldg(Tp + 2);
+                    ++tc.tris;
+                    float tt, uu, vv;
+                    if (tri_hit(rs, ro, a, b, c, tnear, t, tt, uu, vv)) {
+                        const uint32_t pr = __float_as_uint(a.w);
+                        if (prim == kInvalid || tt < t || (tt == t && pr < prim)) {
+                            t = tt;
+                            u = uu;
+                            v = vv;
+                            prim = pr;
+                        }
+                    }
+                }
+            }
+            // the group's closest (lowest primitive on equal t)
+#pragma unroll
+            for (int x = 1; x < kCoopLanes; x <<= 1) {
+                const float t2 = __shfl_xor_sync(mask, t, x), u2 = __shfl_xor_sync(mask, u, x),
+                            v2 = __shfl_xor_sync(mask, v, x);
+                const uint32_t p2 = __shfl_xor_sync(mask, prim, x);
+                if (p2 != kInvalid && (prim == kInvalid || t2 < t || (t2 == t && p2 < prim))) {
+                    t = t2;
+                    u = u2;
+                    v = v2;
+                    prim = p2;
+                }
+            }
+            if (prim != kInvalid &&
+                (best_inst == kInvalid || t < best_t ||
+                 (t == best_t && (cur_inst < best_inst || (cur_inst == best_inst && prim < best_prim))))) {
+                best_t = t;
+                bu = u;
+                bv = v;
+                best_inst = cur_inst;
+                best_prim = prim;
+                if (kStop && t < stop_below) break;
+            }
+        }
+        // children pushed far to near: a lane's place is the number of nearer ones
+        const uint32_t key = (__float_as_uint(fmaxf(tin, 0.0f)) & ~7u) | (uint32_t)sub;
+        const float te = __uint_as_float(key & ~7u);
+        const bool push = in && !leaf && te <= best_t;
+        const uint32_t pushers = __ballot_sync(mask, push) & mask;
+        if (pushers) {
+            const int cnt = __popc(pushers);
+            const uint32_t mine = push ? key : 0xFFFFFFFFu;
+            int nearer = 0;
+#pragma unroll
+            for (int x = 1; x < kCoopLanes; ++x) nearer += __shfl_xor_sync(mask, mine, x) < mine ? 1 : 0;
+            const int at = st.sp + cnt - 1 - nearer;
+            if (push) {
+                if (at < kStackTotal)
+                    st.sh[at] = make_uint2(internal ? w1.x + meta : kInstTag | __ldg(tlas_items + w1.y + (meta & 31u)),
+                                           __float_as_uint(te));
+                else
+                    st.overflow = 1;
+            }
+            st.sp = min(st.sp + cnt, kStackTotal);
+            __syncwarp(mask);
+        }
+    }
+    __syncwarp(mask);
+    if (best_inst == kInvalid) return false;
+    hit.inst = best_inst;
+    hit.prim = best_prim;
+    hit.t = best_t;
+    hit.u = bu;
+    hit.v = bv;
+    return true;
+}
+
 }  // namespace omv

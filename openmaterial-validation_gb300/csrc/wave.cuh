@@ -141,22 +141,76 @@ __device__ __forceinline__ int pick_light(const float* cdf, int n, float d)
     return (L + R) / 2;
 }
 
-// Persistent closest hit over the n rays of a queue (*work counts the rays
-// taken): a warp takes 32 consecutive rays and the next 32 when all are done
+// The rays of a persistent tracing launch: warp w of the grid starts with the
+// w-th share of `take` rays and draws further shares from an atomic counter, so
+// that a launch with less than a share per warp (or an empty one: 5.1 us with an
+// atomic per warp, 2.8 so) makes no atomic at all.
+struct RayShares {
+    uint32_t* work;
+    uint32_t take, rest, mine;
+    bool begun;
+};
+__device__ __forceinline__ RayShares ray_shares(uint32_t* work, uint32_t take)
+{
+    const uint32_t warps = blockDim.x >> 5, w = blockIdx.x * warps + (threadIdx.x >> 5);
+    return RayShares{work, take, gridDim.x * warps * take, w * take, false};
+}
+// first ray of the warp's next share; false when none is left
+__device__ __forceinline__ bool next_share(RayShares& s, uint32_t n, uint32_t& base)
+{
+    if (!s.begun) {
+        s.begun = true;
+        base = s.mine;
+        return base < n;
+    }
+    if (s.rest >= n) return false;  // the first shares covered the queue
+    uint32_t x = 0;
+    if ((threadIdx.x & 31) == 0) x = atomicAdd(s.work, s.take);
+    base = s.rest + __shfl_sync(0xFFFFFFFFu, x, 0);
+    return base < n;
+}
+
+// Queues of at most this many rays are traced with eight lanes per ray
+// (coop_trace), longer ones with one ray per thread: a 256x256x16 point-light
+// frame 1121 us with the line at 2^15 (1119 at 2^16, 1142 at 2^14, 1155 at
+// 2^17; 1245 without the eight-lane path), a 64x64x1 one 532 (728), an
+// eight-scene inverse-fit step 5.78 ms (5.78, 5.91, 5.94; 5.99).
+constexpr uint32_t kCoopRays = 1u << 15;
+static_assert(kStackShared * kTraceThreads >= kStackTotal * (kTraceThreads / kCoopLanes),
+              "the groups of a block share its stacks' memory");
+
+// The eight-lane groups of a warp and their part of the block's stack memory.
+struct CoopGroup {
+    uint32_t mask;
+    int sub, index;  // lane in the group, group in the warp
+    CoopStack st;
+};
+__device__ __forceinline__ CoopGroup coop_group(uint2* stacks)
+{
+    CoopGroup g;
+    const int lane = threadIdx.x & 31;
+    g.sub = lane & (kCoopLanes - 1);
+    g.index = lane / kCoopLanes;
+    g.mask = ((1u << kCoopLanes) - 1u) << (g.index * kCoopLanes);
+    g.st.sh = stacks + (threadIdx.x / kCoopLanes) * kStackTotal;
+    g.st.sp = 0;
+    g.st.overflow = 0;
+    return g;
+}
+
+// Persistent closest hit over the n rays of a queue: a warp takes 32 consecutive rays and the next 32 when all are done
 // (camera rays: the 32 samples of one pixel stay together).  Replacing
 // finished rays lane by lane (Aila & Laine 2009) was measured slower on every
 // bounce.  root(k): the top-level tree of path k's scene (k travels in the
-// ray's last word).
+// ray's last word).  Short queues: four rays per warp.
 template <typename Root>
 __device__ __forceinline__ void extend_rays(const DevScene& S, const uint32_t* items, float4* rq, uint4* hits,
                                             uint32_t n, uint32_t* work, TraceStack& st, TraceCounters& tc, Root root)
 {
     const int lane = threadIdx.x & 31;
-    while (true) {
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(work, 32u);
-        base = __shfl_sync(0xFFFFFFFFu, base, 0);
-        if (base >= n) break;
+    RayShares shares = ray_shares(work, 32u);
+    uint32_t base;
+    while (next_share(shares, n, base)) {
         const uint32_t i = base + lane;
         if (i < n) {
             float4 a = rq[2 * (size_t)i], b = rq[2 * (size_t)i + 1];
@@ -174,12 +228,48 @@ __device__ __forceinline__ void extend_rays(const DevScene& S, const uint32_t* i
     }
 }
 
+// what a call on the eight-lane path counted
+struct CoopCounts {
+    TraceCounters tc;
+    int overflow;
+};
+
+// extend_rays for short queues, four rays per warp.  Out of line, so that its
+// registers do not weigh on the one-thread path of the same kernel.
+template <typename Root>
+__device__ __noinline__ CoopCounts extend_rays_coop(const DevScene& S, const uint32_t* items, float4* rq, uint4* hits,
+                                                    uint32_t n, uint32_t* work, uint2* stacks, Root root)
+{
+    CoopGroup g = coop_group(stacks);
+    TraceCounters tc{0u, 0u};
+    RayShares shares = ray_shares(work, 32u / kCoopLanes);
+    uint32_t base;
+    while (next_share(shares, n, base)) {
+        const uint32_t i = base + (uint32_t)g.index;
+        if (i < n) {
+            const float4 a = rq[2 * (size_t)i], b = rq[2 * (size_t)i + 1];
+            float tnear = a.w;
+            RayHit h;
+            const bool hit = coop_intersect(S, items, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), tnear, kFltMax, h, g.st, tc,
+                                            root(__float_as_int(b.w)), g.mask, g.sub);
+            if (g.sub == 0) {
+                hits[i] = hit ? make_uint4(h.inst, h.prim, __float_as_uint(h.u), __float_as_uint(h.v))
+                              : make_uint4(kInvalid, kInvalid, 0u, 0u);
+                if (tnear != a.w) rq[2 * (size_t)i].w = tnear;
+            }
+        }
+        __syncwarp();
+    }
+    return CoopCounts{tc, g.st.overflow};
+}
+
 // BDPTRenderer::isConnected (BDPTRenderer.cpp:208-235): whether vertex A sees
 // vertex B.  Without alpha-masked materials the closest-hit query stops at a
-// hit well short of B, which already decides "not connected".
+// hit well short of B, which already decides "not connected".  With a group
+// `g`, its eight lanes test one connection together.
 template <bool kMasked>
 __device__ __forceinline__ bool is_connected(const DevScene& S, const uint32_t* items, V3 A, V3 B, TraceStack& st,
-                                             TraceCounters& tc, uint32_t root)
+                                             TraceCounters& tc, uint32_t root, CoopGroup* g = nullptr)
 {
     bool connected = true;
     V3 dir = B - A;
@@ -194,14 +284,16 @@ __device__ __forceinline__ bool is_connected(const DevScene& S, const uint32_t* 
         RayHit h;
         bool hit;
         if (kMasked) {
-            hit = scene_intersect(S, items, A, dir, tnear, tfar, h, st, tc, root);
+            hit = g ? coop_intersect(S, items, A, dir, tnear, tfar, h, g->st, tc, root, g->mask, g->sub)
+                    : scene_intersect(S, items, A, dir, tnear, tfar, h, st, tc, root);
         } else {
             // any hit this far short of B is farther than sb from it (the
             // margin is ~800 ulps of the coordinates, far above the error of
             // the hit's surface position), so it decides: not connected,
             // whichever hit is the closest.  Hits near B get the exact test.
             const float margin = 1.0e-4f * fmaxf(maxsz, max_abs(B, 1.0f)) + 2.0f * sb;
-            hit = trace_closest_or_below(S, items, A, dir, tnear, tfar, len - margin, h, st, tc, root);
+            hit = g ? coop_trace<true>(S, items, A, dir, tnear, tfar, len - margin, h, g->st, tc, root, g->mask, g->sub)
+                    : trace_closest_or_below(S, items, A, dir, tnear, tfar, len - margin, h, st, tc, root);
             if (hit && h.t < len - margin) {
                 hit = false;
                 connected = false;
