@@ -415,9 +415,8 @@ __device__ __noinline__ void adj_shadow_coop(const AdjWave& A, uint32_t n, uint3
     CoopGroup g = coop_group(stacks);
     TraceCounters tc{0u, 0u};
     TraceStack unused;
-    RayShares shares = ray_shares(work, 32u / kCoopLanes);
-    uint32_t base;
-    while (next_share(shares, n, base)) {
+    for (RayShares s = ray_shares(32u / kCoopLanes, n); s.next < n; next_step(s, 32u / kCoopLanes, n, work)) {
+        const uint32_t base = s.next;
         const uint32_t i = base + (uint32_t)g.index;
         bool ok = false;
         if (i < n) {
@@ -448,9 +447,8 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceMinBlocks)
         adj_shadow_coop<kMasked>(A, n, seen, work, sstack);
         return;
     }
-    RayShares shares = ray_shares(work, 32u);
-    uint32_t base;
-    while (next_share(shares, n, base)) {
+    for (RayShares s = ray_shares(32u, n); s.next < n; next_step(s, 32u, n, work)) {
+        const uint32_t base = s.next;
         const uint32_t i = base + lane;
         bool ok = false;
         if (i < n) {

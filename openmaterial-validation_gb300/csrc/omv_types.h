@@ -149,6 +149,12 @@ struct DevScene {
     const float2* uv1;           // TEXCOORD_1 per vertex (TEXCOORD_0 is in verts), or null
 };
 
+// division by an invariant (wave.cuh)
+struct FastDiv {
+    uint32_t d, m;
+    int s1, s2;
+};
+
 // hit record of a closest-hit query
 struct alignas(16) HitRec {
     uint32_t inst;  // kInvalid on a miss

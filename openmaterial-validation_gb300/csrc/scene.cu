@@ -220,6 +220,7 @@ SceneHost::~SceneHost()
     for (void* p : allocs) cudaFree(p);
     if (scratch.base) cudaFree(scratch.base);
     if (adj_scratch) cudaFree(adj_scratch);
+    if (tiles) cudaFree(tiles);
     if (adj_done) cudaEventDestroy(adj_done);
     if (mat_sets) cudaFree(mat_sets);
     if (d_jobs) cudaFree(d_jobs);

@@ -63,6 +63,13 @@ struct RenderScratch {
 
 constexpr int kMaxCounters = 512;
 
+// Tiles of a frame: 2^lx x 2^ly pixels each (beam.cuh).
+struct TileGrid {
+    int32_t lx, ly;
+    uint32_t per_row;  // tiles in a row
+};
+struct TileList;
+
 // One job of a batch render (device copy): its camera, samples, seed and
 // material table, its film, and where its paths and pixels start in the
 // batch's concatenated path and pixel ranges.
@@ -82,6 +89,7 @@ struct DevJob {
     int32_t light_base;       // the scene's lights: [light_base, light_base + light_count)
     int32_t light_count;
     float light_max;          // their total power (the light-pick CDF's last value)
+    FastDiv spp_div, width_div;  // by spp and by cam.width
 };
 
 // One scene of a group (omv_scene_create_group) within the group's arrays:
@@ -128,6 +136,8 @@ struct SceneHost {
     int64_t batch_wave_paths = 0;            // autotuned wave size for batches (0: automatic)
     int batch_shade_threads = 0;             // autotuned threads per shading block for batches (0: 256)
     std::vector<ScenePart> parts;            // the scenes of a group (one for a single scene)
+    TileList* tiles = nullptr;               // start nodes of the first camera bounce (beam.cuh)
+    int64_t tiles_cap = 0;
     std::mutex adj_mutex;                    // one adjoint call at a time enqueues
     void* adj_scratch = nullptr;             // records of an adjoint wave
     size_t adj_bytes = 0;

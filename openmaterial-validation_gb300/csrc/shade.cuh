@@ -403,6 +403,19 @@ __device__ __forceinline__ bool scene_intersect(const DevScene& S, const uint32_
     return false;
 }
 
+// scene_intersect of a camera ray from its tile's start nodes
+__device__ __forceinline__ bool tile_intersect(const DevScene& S, const uint32_t* items, V3 o, V3 d, float& tnear,
+                                               RayHit& h, TraceStack& st, TraceCounters& tc, const TileList* tile)
+{
+    for (int itr = 0; itr < kMaskedTries; ++itr) {
+        if (!trace_closest_tile(S, items, o, d, tnear, kFltMax, h, st, tc, tile)) return false;
+        if (!hit_masked(S, h)) return true;
+        tnear = masked_retry_tnear(o, d, h.t);
+        if (kFltMax <= tnear) return false;
+    }
+    return false;
+}
+
 // scene_intersect with eight lanes per ray (coop_trace)
 __device__ __forceinline__ bool coop_intersect(const DevScene& S, const uint32_t* items, V3 o, V3 d, float& tnear,
                                                float tfar, RayHit& h, CoopStack& st, TraceCounters& tc, uint32_t root,

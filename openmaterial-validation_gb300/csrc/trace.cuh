@@ -19,6 +19,9 @@ namespace omv {
 constexpr int kStackShared = 16;  // entries per thread kept in shared memory
 constexpr int kStackTotal = 64;   // further entries spill to local memory
 constexpr uint32_t kInstTag = 0x80000000u;
+constexpr uint32_t kRunTag = 0x40000000u;  // with kInstTag: a run of a tile's start nodes (beam.cuh)
+
+struct TileList;
 
 struct TraceStack {
     uint2* sh;  // this thread's first shared entry; entry i at sh[i * stride]
@@ -214,6 +217,17 @@ struct TraceCounters {
     uint32_t tris;
 };
 
+// a tile list as the traversal reads it (beam.cuh)
+__device__ __forceinline__ uint4 tile_run(const TileList* t, uint32_t i)
+{
+    return __ldg(reinterpret_cast<const uint4*>(t) + 1 + i);
+}
+__device__ __forceinline__ void push_tile_node(const TileList* t, uint32_t i, TraceStack& st)
+{
+    const uint2 n = __ldg(reinterpret_cast<const uint2*>(t) + 2 + 2 * 8 + i);
+    st.push(n.x, __uint_as_float(n.y));
+}
+
 // Traversal state of one ray: trace_begin, then trace_step until it returns
 // false, then trace_end (trace_closest runs the three in a row).  Keeping the
 // state in one struct and one stack entry per step also compiles to a faster
@@ -255,10 +269,12 @@ __device__ __forceinline__ bool trace_begin(const DevScene& S, V3 o, V3 d, float
 
 // Processes one stack entry (an instance or a node); false when the traversal is
 // over.  kStop: also over as soon as a hit with t < stop_below is taken (an
-// occlusion query stops at any hit: stop_below = infinity).
-template <bool kStop = false>
+// occlusion query stops at any hit: stop_below = infinity).  kRuns: the stack
+// may hold runs of the tile's start nodes.
+template <bool kStop = false, bool kRuns = false>
 __device__ __forceinline__ bool trace_step(const DevScene& S, const uint32_t* __restrict__ tlas_items, TraceState& T,
-                                          TraceStack& st, TraceCounters& tc, float stop_below = 0.0f)
+                                          TraceStack& st, TraceCounters& tc, float stop_below = 0.0f,
+                                          const TileList* __restrict__ tile = nullptr)
 {
     if (T.guard++ > (1u << 22)) {  // a malformed tree can never spin a warp forever
         st.overflow = 1;
@@ -273,7 +289,18 @@ __device__ __forceinline__ bool trace_step(const DevScene& S, const uint32_t* __
     const uint2 e = st.pop();
     if (__uint_as_float(e.y) > T.best_t) return true;
     if (e.x & kInstTag) {
-        const uint32_t ii = e.x & ~kInstTag;
+        uint32_t ii = e.x & ~kInstTag;
+        uint32_t first = 0, last = 0;
+        if (kRuns && (ii & kRunTag)) {
+            const uint4 r = tile_run(tile, ii & ~kRunTag);
+            ii = r.x;
+            first = r.y;
+            last = r.y + r.z;
+            if (ii == kInvalid) {  // nodes of the top-level tree
+                for (uint32_t k = last; k > first; --k) push_tile_node(tile, k - 1u, st);
+                return true;
+            }
+        }
         const DevInstance* I = S.insts + ii;
         float m[12];
 #pragma unroll
@@ -291,6 +318,10 @@ __device__ __forceinline__ bool trace_step(const DevScene& S, const uint32_t* __
         T.in_blas = true;
         T.blas_base = st.sp;
         T.cur_inst = ii;
+        if (kRuns && last > first) {
+            for (uint32_t k = last; k > first; --k) push_tile_node(tile, k - 1u, st);
+            return true;
+        }
         st.push(__ldg(&I->blas_root), __uint_as_float(e.y));
         return true;
     }
@@ -434,6 +465,22 @@ __device__ __forceinline__ bool trace_closest(const DevScene& S, const uint32_t*
     TraceState T;
     if (!trace_begin(S, o, d, tnear, tfar, T, st, root)) return false;
     while (trace_step(S, tlas_items, T, st, tc)) {
+    }
+    return trace_end(T, hit);
+}
+
+// Closest hit of a camera ray, from its tile's start nodes.
+__device__ __forceinline__ bool trace_closest_tile(const DevScene& S, const uint32_t* __restrict__ tlas_items, V3 o,
+                                                   V3 d, float tnear, float tfar, RayHit& hit, TraceStack& st,
+                                                   TraceCounters& tc, const TileList* __restrict__ tile)
+{
+    const uint32_t runs = __ldg(reinterpret_cast<const uint32_t*>(tile));
+    if (runs == 0u) return false;
+    TraceState T;
+    if (!trace_begin(S, o, d, tnear, tfar, T, st, 0u)) return false;
+    st.sp = 0;
+    for (uint32_t k = runs; k > 0; --k) st.push(kInstTag | kRunTag | (k - 1u), __uint_as_float(tile_run(tile, k - 1u).w));
+    while (trace_step<false, true>(S, tlas_items, T, st, tc, 0.0f, tile)) {
     }
     return trace_end(T, hit);
 }

@@ -103,10 +103,6 @@ __device__ __forceinline__ uint32_t block_append_binned(uint32_t* counter, bool 
 // "Division by invariant integers using multiplication", PLDI 1994, 4.1):
 // exact for every numerator and every divisor >= 1, where the hardware has
 // no integer divide.
-struct FastDiv {
-    uint32_t d, m;
-    int s1, s2;
-};
 inline FastDiv make_fastdiv(uint32_t d)
 {
     int l = 0;
@@ -141,33 +137,49 @@ __device__ __forceinline__ int pick_light(const float* cdf, int n, float d)
     return (L + R) / 2;
 }
 
-// The rays of a persistent tracing launch: warp w of the grid starts with the
-// w-th share of `take` rays and draws further shares from an atomic counter, so
-// that a launch with less than a share per warp (or an empty one: 5.1 us with an
-// atomic per warp, 2.8 so) makes no atomic at all.
+// The rays of a persistent tracing launch, in shares that its warps draw from
+// an atomic counter: kBigShare steps of `take` rays while many are left, single
+// steps for the last kSmallRays (large shares there leave some warps with much
+// more work than others: from 2^22 on, an 8.4M-ray launch 0.53 -> 0.71 ms).  The
+// counter is one address, which takes about one atomic per nanosecond: a draw
+// per 32 rays bounds a launch at 24 G rays/s, and the first bounce of the
+// 1920x1080x64 sky frame took 5.5 ms from its tile lists with it, 2.3 so.
+// Warp w starts with share w, so a launch with at most a share per warp makes
+// no atomic at all (empty: 5.1 -> 2.8 us).
+constexpr uint32_t kBigShare = 8, kSmallRays = 1u << 23;
+// Only the next ray's number lives across a step: a share of several steps ends
+// at a multiple of its size.
 struct RayShares {
-    uint32_t* work;
-    uint32_t take, rest, mine;
-    bool begun;
+    uint32_t next;
 };
-__device__ __forceinline__ RayShares ray_shares(uint32_t* work, uint32_t take)
+__device__ __forceinline__ uint32_t share_start(uint32_t j, uint32_t take, uint32_t n)
 {
-    const uint32_t warps = blockDim.x >> 5, w = blockIdx.x * warps + (threadIdx.x >> 5);
-    return RayShares{work, take, gridDim.x * warps * take, w * take, false};
+    const uint32_t span = kBigShare * take, big = n > kSmallRays ? (n - kSmallRays) / span : 0u;
+    if (j < big) return j * span;
+    const uint64_t at = (uint64_t)big * span + (uint64_t)(j - big) * take;
+    return at < n ? (uint32_t)at : 0xFFFFFFFFu;
 }
-// first ray of the warp's next share; false when none is left
-__device__ __forceinline__ bool next_share(RayShares& s, uint32_t n, uint32_t& base)
+__device__ __forceinline__ RayShares ray_shares(uint32_t take, uint32_t n)
 {
-    if (!s.begun) {
-        s.begun = true;
-        base = s.mine;
-        return base < n;
+    return RayShares{share_start(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), take, n)};
+}
+// after a step: the warp's next one
+__device__ __forceinline__ void next_step(RayShares& s, uint32_t take, uint32_t n, uint32_t* work)
+{
+    const uint32_t span = kBigShare * take, at = s.next + take;
+    const uint32_t big_end = n > kSmallRays ? (n - kSmallRays) / span * span : 0u;
+    if (at <= big_end && at % span != 0u) {
+        s.next = at;
+        return;
     }
-    if (s.rest >= n) return false;  // the first shares covered the queue
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    if (big_end == 0u && (uint64_t)warps * take >= n) {  // all shares were first shares
+        s.next = 0xFFFFFFFFu;
+        return;
+    }
     uint32_t x = 0;
-    if ((threadIdx.x & 31) == 0) x = atomicAdd(s.work, s.take);
-    base = s.rest + __shfl_sync(0xFFFFFFFFu, x, 0);
-    return base < n;
+    if ((threadIdx.x & 31) == 0) x = atomicAdd(work, 1u);
+    s.next = share_start(warps + __shfl_sync(0xFFFFFFFFu, x, 0), take, n);
 }
 
 // Queues of at most this many rays are traced with eight lanes per ray
@@ -208,9 +220,8 @@ __device__ __forceinline__ void extend_rays(const DevScene& S, const uint32_t* i
                                             uint32_t n, uint32_t* work, TraceStack& st, TraceCounters& tc, Root root)
 {
     const int lane = threadIdx.x & 31;
-    RayShares shares = ray_shares(work, 32u);
-    uint32_t base;
-    while (next_share(shares, n, base)) {
+    for (RayShares s = ray_shares(32u, n); s.next < n; next_step(s, 32u, n, work)) {
+        const uint32_t base = s.next;
         const uint32_t i = base + lane;
         if (i < n) {
             float4 a = rq[2 * (size_t)i], b = rq[2 * (size_t)i + 1];
@@ -242,9 +253,8 @@ __device__ __noinline__ CoopCounts extend_rays_coop(const DevScene& S, const uin
 {
     CoopGroup g = coop_group(stacks);
     TraceCounters tc{0u, 0u};
-    RayShares shares = ray_shares(work, 32u / kCoopLanes);
-    uint32_t base;
-    while (next_share(shares, n, base)) {
+    for (RayShares s = ray_shares(32u / kCoopLanes, n); s.next < n; next_step(s, 32u / kCoopLanes, n, work)) {
+        const uint32_t base = s.next;
         const uint32_t i = base + (uint32_t)g.index;
         if (i < n) {
             const float4 a = rq[2 * (size_t)i], b = rq[2 * (size_t)i + 1];
