@@ -26,6 +26,7 @@
 #include <cfloat>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -1201,7 +1202,7 @@ uint32_t batch_global_pixel(const std::vector<DevJob>& jobs, int64_t g)
 // created: no frame or kernel timing, and `stats` must be null.
 void run_waves(SceneHost& s, RenderScratch& R, const FramePlan& P, const omv_camera& cam, const omv_params& p,
                double* d_sum, double* d_sumsq, uint32_t* d_count, cudaStream_t st, omv_stats* stats, bool events,
-               const BatchPlan* batch = nullptr)
+               const BatchPlan* batch = nullptr, const std::function<void()>* while_running = nullptr)
 {
     const int64_t total = P.total, npix = P.npix, cap = P.cap;
     const bool lights = P.lights;
@@ -1384,6 +1385,7 @@ void run_waves(SceneHost& s, RenderScratch& R, const FramePlan& P, const omv_cam
         return;
     }
     OMV_CUDA(cudaEventRecord(e1, st));
+    if (while_running) (*while_running)();  // host work beside the frame
     if (stats) {
         unsigned long long h[16];
         OMV_CUDA(cudaMemcpyAsync(h, R.stats, sizeof(h), cudaMemcpyDeviceToHost, st));
@@ -1475,10 +1477,14 @@ static bool ensure_tiles(SceneHost& s, int64_t n)
 constexpr size_t kWaveScratchBudget = (size_t)32 << 30;
 
 void render_frame(SceneHost& s, const omv_camera& cam, const omv_params& p, double* d_sum, double* d_sumsq,
-                  uint32_t* d_count, cudaStream_t st, omv_stats* stats)
+                  uint32_t* d_count, cudaStream_t st, omv_stats* stats, const std::function<void()>* while_running)
 {
     FramePlan P = plan_frame(s, cam, p, 1);
-    if (p.wave_paths <= 0) {
+    const RenderScratch& R = s.scratch;
+    if (p.wave_paths <= 0 && P.total > 0 && R.wave_cap >= P.total && R.light_slots >= P.light_slots &&
+        R.shadow_slots >= P.shadow_slots) {
+        P.cap = P.total;  // the scratch holds the whole frame: no need to ask what memory is free
+    } else if (p.wave_paths <= 0) {
         size_t free_b = 0, total_b = 0;
         OMV_CUDA(cudaMemGetInfo(&free_b, &total_b));
         const size_t budget = std::min(kWaveScratchBudget, (free_b + s.scratch.bytes) / 2);
@@ -1491,7 +1497,7 @@ void render_frame(SceneHost& s, const omv_camera& cam, const omv_params& p, doub
         const int64_t n = tile_count(P.tiles, cam);
         if (n <= kTileMaxCount && ensure_tiles(s, n)) P.num_tiles = (uint32_t)n;
     }
-    run_waves(s, s.scratch, P, cam, p, d_sum, d_sumsq, d_count, st, stats, true);
+    run_waves(s, s.scratch, P, cam, p, d_sum, d_sumsq, d_count, st, stats, true, nullptr, while_running);
 }
 
 // ------------------------------------------------------------- batches ---

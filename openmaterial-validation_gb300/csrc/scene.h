@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <functional>
 #include <mutex>
 #include <stdexcept>
 #include <string>
@@ -162,8 +163,10 @@ SceneHost* scene_create(const omv_scene_desc& desc, int device, const std::vecto
 // top-level tree per scene; batch jobs pick their scene
 SceneHost* scene_create_group(int num, const omv_scene_desc* descs, int device);
 
+// while_running: host work to do once everything is enqueued
 void render_frame(SceneHost& s, const omv_camera& cam, const omv_params& p, double* d_sum, double* d_sumsq,
-                  uint32_t* d_count, cudaStream_t st, omv_stats* stats);
+                  uint32_t* d_count, cudaStream_t st, omv_stats* stats,
+                  const std::function<void()>* while_running = nullptr);
 DevMaterial material_from_desc(const omv_material_desc& md, int num_textures);
 DevMaterial missing_material();
 // material sets for batch jobs: num_sets x (scene materials without the missing one)
