@@ -1005,13 +1005,17 @@ void run_adjoint(SceneHost& s, std::vector<AdjJob>& jobs, const omv_params& p, c
         uint32_t* work = A.ctr + kAdjCtrWork;
         const unsigned gen = blocks_for(A.wave_n, kShadeThreads);
         if (A.path_job) k_adj_path_jobs<<<gen, kShadeThreads, 0, st>>>(A);
+        // beside the main stream: the light subpaths beside the camera rays' first
+        // hits, then each bounce's connections beside the next bounce's hits
+        const cudaStream_t side = lights ? s.adj_side.stream : st;
         if (lights) {
-            k_adj_light_gen<<<gen, kShadeThreads, 0, st>>>(A);
+            fork_side(s.adj_side, st);
+            k_adj_light_gen<<<gen, kShadeThreads, 0, side>>>(A);
             for (int b = 1; b <= L; ++b) {
                 const size_t off = (size_t)(b - 1) * A.cap;
-                k_adj_extend<<<trace_grid, kTraceThreads, 0, st>>>(A, A.lrq + 2 * off, A.lhit + off,
-                                                                   A.ctr + kAdjCtrLight + b - 1, work++);
-                k_adj_light<<<light_grid, kShadeThreads, 0, st>>>(A, b);
+                k_adj_extend<<<trace_grid, kTraceThreads, 0, side>>>(A, A.lrq + 2 * off, A.lhit + off,
+                                                                     A.ctr + kAdjCtrLight + b - 1, work++);
+                k_adj_light<<<light_grid, kShadeThreads, 0, side>>>(A, b);
             }
         }
         k_adj_camera_gen<<<gen, kShadeThreads, 0, st>>>(A);
@@ -1019,17 +1023,20 @@ void run_adjoint(SceneHost& s, std::vector<AdjJob>& jobs, const omv_params& p, c
             const size_t off = (size_t)(b - 1) * A.cap;
             k_adj_extend<<<trace_grid, kTraceThreads, 0, st>>>(A, A.crq + 2 * off, A.chit + off,
                                                                A.ctr + kAdjCtrCam + b - 1, work++);
+            if (lights) join_side(s.adj_side, st);
             k_adj_camera<<<camera_grid, kShadeThreads, 0, st>>>(A, b);
             if (lights) {
                 uint32_t* seen = A.ctr + kAdjCtrSeen + b - 1;
                 const uint32_t* count = A.ctr + kAdjCtrConn + b - 1;
+                fork_side(s.adj_side, st);
                 if (masked)
-                    k_adj_shadow<true><<<trace_grid, kTraceThreads, 0, st>>>(A, count, seen, work++);
+                    k_adj_shadow<true><<<trace_grid, kTraceThreads, 0, side>>>(A, count, seen, work++);
                 else
-                    k_adj_shadow<false><<<trace_grid, kTraceThreads, 0, st>>>(A, count, seen, work++);
-                k_adj_connect<<<connect_grid, kAdjThreads, smem, st>>>(A, b);
+                    k_adj_shadow<false><<<trace_grid, kTraceThreads, 0, side>>>(A, count, seen, work++);
+                k_adj_connect<<<connect_grid, kAdjThreads, smem, side>>>(A, b);
             }
         }
+        if (lights) join_side(s.adj_side, st);
         for (int b = B; b >= 1; --b) k_adj_camera_back<<<back_grid, kAdjThreads, smem, st>>>(A, b);
         if (lights)
             for (int b = L; b >= 1; --b) k_adj_light_back<<<lback_grid, kAdjThreads, smem, st>>>(A, b);

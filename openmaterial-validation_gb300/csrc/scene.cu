@@ -329,14 +329,22 @@ SceneHost::~SceneHost()
 {
     if (device >= 0) cudaSetDevice(device);
     if (stream) cudaStreamSynchronize(stream);
+    if (side.stream) cudaStreamSynchronize(side.stream);
+    if (adj_side.stream) cudaStreamSynchronize(adj_side.stream);
     for (void* p : allocs) cudaFree(p);
     if (scratch.base) cudaFree(scratch.base);
     if (adj_scratch) cudaFree(adj_scratch);
     if (tiles) cudaFree(tiles);
+    if (light_queue) cudaFree(light_queue);
     if (adj_done) cudaEventDestroy(adj_done);
     if (mat_sets) cudaFree(mat_sets);
     if (d_jobs) cudaFree(d_jobs);
     if (batch_graph) cudaGraphExecDestroy(batch_graph);
+    for (const Side& x : {side, adj_side}) {
+        if (x.fork) cudaEventDestroy(x.fork);
+        if (x.join) cudaEventDestroy(x.join);
+        if (x.stream) cudaStreamDestroy(x.stream);
+    }
     if (fork_ev) cudaEventDestroy(fork_ev);
     if (join_ev) cudaEventDestroy(join_ev);
     if (stream) cudaStreamDestroy(stream);
@@ -564,6 +572,11 @@ SceneHost* scene_create(const omv_scene_desc& d, int device, const std::vector<i
     std::unique_ptr<SceneHost> s(new SceneHost);
     s->device = device;
     OMV_CUDA(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
+    for (SceneHost::Side* x : {&s->side, &s->adj_side}) {
+        OMV_CUDA(cudaStreamCreateWithFlags(&x->stream, cudaStreamNonBlocking));
+        OMV_CUDA(cudaEventCreateWithFlags(&x->fork, cudaEventDisableTiming));
+        OMV_CUDA(cudaEventCreateWithFlags(&x->join, cudaEventDisableTiming));
+    }
     OMV_CUDA(cudaDeviceGetAttribute(&s->num_sms, cudaDevAttrMultiProcessorCount, device));
 
     // ---- materials (+ the missing material, RenderScene.cpp:62-68)

@@ -132,11 +132,18 @@ struct SceneHost {
     DevJob* d_jobs = nullptr;                // batch job table
     size_t jobs_cap = 0;
     cudaGraphExec_t batch_graph = nullptr;   // captured batch render, replayed for an identical job list
+    // work beside a call's main stream: a frame's (or batch's), an adjoint's
+    struct Side {
+        cudaStream_t stream = nullptr;
+        cudaEvent_t fork = nullptr, join = nullptr;
+    } side, adj_side;
     cudaEvent_t fork_ev = nullptr, join_ev = nullptr;  // order `stream` after / before a caller's default stream
     std::vector<unsigned char> batch_key;    // what batch_graph was captured for
     int64_t batch_wave_paths = 0;            // autotuned wave size for batches (0: automatic)
     int batch_shade_threads = 0;             // autotuned threads per shading block for batches (0: 256)
     std::vector<ScenePart> parts;            // the scenes of a group (one for a single scene)
+    void* light_queue = nullptr;             // the light subpaths' own queues (small frames)
+    int64_t light_queue_cap = 0;
     TileList* tiles = nullptr;               // start nodes of the first camera bounce (beam.cuh)
     int64_t tiles_cap = 0;
     std::mutex adj_mutex;                    // one adjoint call at a time enqueues
@@ -154,6 +161,18 @@ struct SceneHost {
         return p;
     }
 };
+
+// orders the side stream after what `st` holds so far, and `st` after the side's
+inline void fork_side(const SceneHost::Side& x, cudaStream_t st)
+{
+    OMV_CUDA(cudaEventRecord(x.fork, st));
+    OMV_CUDA(cudaStreamWaitEvent(x.stream, x.fork, 0));
+}
+inline void join_side(const SceneHost::Side& x, cudaStream_t st)
+{
+    OMV_CUDA(cudaEventRecord(x.join, x.stream));
+    OMV_CUDA(cudaStreamWaitEvent(st, x.join, 0));
+}
 
 // `parts` (optional): the scenes a merged description holds (instances of
 // scene p have inst_part[i] == p; light and material ranges per scene)
