@@ -996,35 +996,55 @@ __global__ void k_ids(DevScene S, const uint32_t* items, omv_camera cam, const f
     out[p] = o;
 }
 
-__global__ void k_trace_rays(DevScene S, const uint32_t* items, int64_t n, const float* rays, omv_hit* out)
+// Closest hits of a caller's rays (8 floats each).  A block's 128 rays stay
+// with its threads (a grid as large as the rays); up to 2^15 rays, eight lanes
+// share a ray, as in extend_rays.
+__device__ __forceinline__ void store_hit(const DevScene& S, bool hit, const RayHit& h, omv_hit* out)
+{
+    uint4 a = make_uint4(kInvalid, kInvalid, kInvalid, kInvalid);
+    float t = 0.0f, u = 0.0f, v = 0.0f;
+    if (hit) {
+        const DevInstance* I = S.insts + h.inst;
+        a = make_uint4(h.inst, __ldg(&I->mesh), h.prim, __ldg(&I->material));
+        t = h.t;
+        u = h.u;
+        v = h.v;
+    }
+    uint4* o = reinterpret_cast<uint4*>(out);
+    o[0] = a;
+    o[1] = make_uint4(__float_as_uint(t), __float_as_uint(u), __float_as_uint(v), 0u);
+}
+__global__ void __launch_bounds__(kTraceThreads, kTraceMinBlocks)
+    k_trace_rays(const __grid_constant__ DevScene S, const uint32_t* items, int64_t n, const float* rays, omv_hit* out)
 {
     __shared__ uint2 sstack[kStackShared * kTraceThreads];
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
     TraceStack st;
     st.sh = sstack + threadIdx.x;
     st.stride = kTraceThreads;
     st.overflow = 0;
     TraceCounters tc{0u, 0u};
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float* r = rays + 8 * i;
-    float tnear = r[3];
+    const float4 a = reinterpret_cast<const float4*>(rays)[2 * i], b = reinterpret_cast<const float4*>(rays)[2 * i + 1];
+    float tnear = a.w;
     RayHit h;
-    omv_hit o;
-    if (scene_intersect(S, items, v3(r[0], r[1], r[2]), v3(r[4], r[5], r[6]), tnear, r[7], h, st, tc)) {
-        const DevInstance* I = S.insts + h.inst;
-        o.inst = h.inst;
-        o.geom = I->mesh;
-        o.prim = h.prim;
-        o.material = I->material;
-        o.t = h.t;
-        o.u = h.u;
-        o.v = h.v;
-    } else {
-        o.inst = o.geom = o.prim = o.material = kInvalid;
-        o.t = o.u = o.v = 0.0f;
-    }
-    o.pad = 0;
-    out[i] = o;
+    const bool hit = scene_intersect(S, items, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), tnear, b.w, h, st, tc);
+    store_hit(S, hit, h, out + i);
+}
+__global__ void __launch_bounds__(kTraceThreads, kTraceMinBlocks)
+    k_trace_rays_coop(const __grid_constant__ DevScene S, const uint32_t* items, int64_t n, const float* rays, omv_hit* out)
+{
+    __shared__ uint2 sstack[kStackShared * kTraceThreads];
+    CoopGroup g = coop_group(sstack);
+    TraceCounters tc{0u, 0u};
+    const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kCoopLanes;
+    if (i >= n) return;  // whole groups
+    const float4 a = reinterpret_cast<const float4*>(rays)[2 * i], b = reinterpret_cast<const float4*>(rays)[2 * i + 1];
+    float tnear = a.w;
+    RayHit h;
+    const bool hit =
+        coop_intersect(S, items, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), tnear, b.w, h, g.st, tc, kInvalid, g.mask, g.sub);
+    if (g.sub == 0) store_hit(S, hit, h, out + i);
 }
 
 __global__ void k_env(DevEnv env, int64_t n, const float* dirs, float* rgb)
@@ -1884,7 +1904,11 @@ void render_ids(SceneHost& s, const omv_camera& cam, const float* d_jitter, uint
 void trace_rays(SceneHost& s, int64_t n, const float* d_rays, omv_hit* d_hits, cudaStream_t st)
 {
     if (n <= 0) return;
-    k_trace_rays<<<grid_for(n, kTraceThreads), kTraceThreads, 0, st>>>(s.dev, s.tlas_items, n, d_rays, d_hits);
+    if (n <= (int64_t)kCoopRays)
+        k_trace_rays_coop<<<grid_for(n * kCoopLanes, kTraceThreads), kTraceThreads, 0, st>>>(s.dev, s.tlas_items, n, d_rays,
+                                                                                           d_hits);
+    else
+        k_trace_rays<<<grid_for(n, kTraceThreads), kTraceThreads, 0, st>>>(s.dev, s.tlas_items, n, d_rays, d_hits);
     OMV_CUDA(cudaGetLastError());
 }
 

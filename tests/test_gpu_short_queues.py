@@ -54,3 +54,25 @@ def test_masked_sky_scene(gpu, scenes):
         a, _ = _render(gpu, rs, sc, estimator=estimator)
         b, _ = _render(gpu, rs, sc, estimator=estimator, wave_paths=2048)
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [1, 3, 129, 32768])
+def test_traced_rays_do_not_depend_on_the_queue_length(gpu, scenes, n):
+    """A few rays alone (eight lanes each) and among 33000 (one thread each): negative tnear, short and empty intervals,
+    zero, axis-parallel and non-finite directions, masked materials."""
+    sc = scenes.scene_textured(8, 8, 1)
+    rng = np.random.default_rng(n)
+    rs = gpu.RenderScene(sc)
+    rays = np.zeros((33_000, 8), np.float32)
+    rays[:, 0:3] = rng.uniform(-3, 3, (len(rays), 3)) + [0, 0, -4]
+    rays[:, 4:7] = rng.normal(size=(len(rays), 3))
+    rays[:, 7] = rng.choice([3e38, 2.0, 0.5], len(rays))
+    rays[:, 3] = rng.choice([0.0, 0.0, 1.0, -2.0], len(rays))
+    rays[rng.random(len(rays)) < 0.1, 4] = 0.0
+    rays[rng.random(len(rays)) < 0.05, 5:7] = 0.0
+    rays[::97, 4:7] = 0.0
+    rays[1::211, 5] = np.nan
+    rays[2::211, 6] = np.inf
+    whole, alone = rs.trace(rays), rs.trace(rays[:n])
+    assert (whole["inst"] != 0xFFFFFFFF).sum() > 5000
+    assert np.array_equal(whole[:n].view(np.uint32), alone.view(np.uint32))
