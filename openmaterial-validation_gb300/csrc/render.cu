@@ -28,6 +28,7 @@
 #include <cstring>
 #include <functional>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "beam.cuh"
@@ -591,43 +592,60 @@ __device__ __forceinline__ bool camera_vertex(const WaveArgs& A, int b, int k, f
 // kMis: the MIS estimator's environment connections (a separate instantiation,
 // so the reference estimator's kernel carries none of their registers).  Four
 // resident blocks of 256 (64 registers, 28 B of spills) hide more of the
-// vertex-gather latency than three (72 registers): 37.9 vs 38.5 ms per frame.
-// The MIS instantiation keeps three (it would spill 140 B at four).
-template <bool kMis>
-__global__ void __launch_bounds__(kShadeThreads, kMis ? 3 : 4) k_camera_shade(WaveArgs A, int b, const float4* rq_in,
+// vertex-gather latency than three (72 registers): 37.9 vs 38.5 ms per frame;
+// the MIS instantiation too, for all its spills (a 960x540x16 frame 3010 -> 2970
+// us).
+// kStaged: the next rays are grouped over windows of several steps (StagedRays)
+// instead of one step (block_append_binned).
+template <bool kMis, bool kStaged>
+__global__ void __launch_bounds__(kShadeThreads, 4) k_camera_shade(WaveArgs A, int b, const float4* rq_in,
                                                                  float4* rq_out)
 {
-    __shared__ BinScratch bins;
+    static_assert(!(kMis && kStaged), "environment rays are appended step by step");
+    __shared__ typename std::conditional<kStaged, StagedRays, BinScratch>::type group;
     const uint32_t n = A.R.ctr[kCtrCam + b];
-    for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
-        const uint32_t i = i0 + threadIdx.x;
-        bool push = false;
-        V3 so = v3(0, 0, 0), O = v3(0, 0, 1);
-        float tnear = 0.0f;
-        int k = 0;
-        EnvRay er;
-        er.push = false;
-        er.w = v3(0.0f, 0.0f, 1.0f);
-        if (i < n) {
-            const float4 ra = rq_in[2 * (size_t)i], rb = rq_in[2 * (size_t)i + 1];
-            k = __float_as_int(rb.w);
-            QueueSink qs;
-            push = camera_vertex<kMis>(A, b, k, ra, rb, A.R.hits[i], so, O, tnear, er, qs);
-        }
-        const uint32_t slot = block_append_binned(&A.R.ctr[kCtrCam + b + 1], push, direction_bin(O), bins);
-        if (push) {
-            rq_out[2 * (size_t)slot] = make_float4(so.x, so.y, so.z, tnear);
-            rq_out[2 * (size_t)slot + 1] = make_float4(O.x, O.y, O.z, __int_as_float(k));
-        }
-        if (kMis) {  // environment rays grouped by direction like the next-bounce rays
-            const uint32_t es = block_append_binned(&A.R.ctr[kCtrEnv + b], er.push, direction_bin(er.w), bins);
-            if (er.push) {
-                float4* q = A.env_q + 3 * (size_t)es;
-                q[0] = make_float4(er.so.x, er.so.y, er.so.z, __int_as_float(k));
-                q[1] = make_float4(er.w.x, er.w.y, er.w.z, er.tnear);
-                q[2] = make_float4(er.c.x, er.c.y, er.c.z, 0.0f);
+    // up to kStageSteps steps per window while every block has kStageWindows windows
+    const uint32_t steps =
+        kStaged ? min(max(n / (kStageWindows * gridDim.x * blockDim.x), 1u), (uint32_t)kStageSteps) : 1u;
+    const uint32_t window = steps * blockDim.x;
+    for (uint32_t w = blockIdx.x * window; w < n; w += gridDim.x * window) {
+        if constexpr (kStaged) staged_begin(group);
+        for (uint32_t i0 = w; i0 < w + window; i0 += blockDim.x) {
+            const uint32_t i = i0 + threadIdx.x;
+            bool push = false;
+            V3 so = v3(0, 0, 0), O = v3(0, 0, 1);
+            float tnear = 0.0f;
+            int k = 0;
+            EnvRay er;
+            er.push = false;
+            er.w = v3(0.0f, 0.0f, 1.0f);
+            if (i < n) {
+                const float4 ra = rq_in[2 * (size_t)i], rb = rq_in[2 * (size_t)i + 1];
+                k = __float_as_int(rb.w);
+                QueueSink qs;
+                push = camera_vertex<kMis>(A, b, k, ra, rb, A.R.hits[i], so, O, tnear, er, qs);
+            }
+            const float4 na = make_float4(so.x, so.y, so.z, tnear), nb = make_float4(O.x, O.y, O.z, __int_as_float(k));
+            if constexpr (kStaged) {
+                staged_add(group, push, na, nb);
+            } else {
+                const uint32_t slot = block_append_binned(&A.R.ctr[kCtrCam + b + 1], push, direction_bin(O), group);
+                if (push) {
+                    rq_out[2 * (size_t)slot] = na;
+                    rq_out[2 * (size_t)slot + 1] = nb;
+                }
+                if (kMis) {  // environment rays grouped by direction like the next-bounce rays
+                    const uint32_t es = block_append_binned(&A.R.ctr[kCtrEnv + b], er.push, direction_bin(er.w), group);
+                    if (er.push) {
+                        float4* q = A.env_q + 3 * (size_t)es;
+                        q[0] = make_float4(er.so.x, er.so.y, er.so.z, __int_as_float(k));
+                        q[1] = make_float4(er.w.x, er.w.y, er.w.z, er.tnear);
+                        q[2] = make_float4(er.c.x, er.c.y, er.c.z, 0.0f);
+                    }
+                }
             }
         }
+        if constexpr (kStaged) staged_append(group, &A.R.ctr[kCtrCam + b + 1], rq_out);
     }
 }
 
@@ -1221,6 +1239,13 @@ uint32_t batch_global_pixel(const std::vector<DevJob>& jobs, int64_t g)
 // rays (64x64x1 401 -> 382 us, 256x256x16 997 -> 955); larger ones keep the GPU busy by themselves, and the queues'
 // 80 bytes per path are better spent on fewer waves.
 constexpr int64_t kBesideLightPaths = 1 << 22;
+// Waves of at least this many paths of one frame group their rays over windows
+// of several shading steps: the 1920x1080x64 point-light frame 38.85 -> 37.65 ms
+// (its second bounce 5.2 -> 4.3 ms), the sky frame 17.0 -> 16.83.  Where a block
+// has few windows, or its window spans much of the image, the shared memory and
+// the coarser steps cost more (1280x720x32: even; a 641x479x17 frame 3.96 ->
+// 3.99 ms, 16 batched jobs 19.13 -> 19.30).
+constexpr int64_t kStagedPaths = 1 << 25;
 void light_queues(RenderScratch& R, void* base, int64_t paths)
 {
     float4* q = static_cast<float4*>(base);
@@ -1274,7 +1299,7 @@ void run_waves(SceneHost& s, RenderScratch& R, const FramePlan& P, const omv_cam
     // threads per block of the shading-side kernels: 256, or a batch's
     // autotuned choice (a multiple of 32 up to 256)
     const int sth = batch && s.batch_shade_threads > 0 ? s.batch_shade_threads : kShadeThreads;
-    OMV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, mis ? k_camera_shade<true> : k_camera_shade<false>,
+    OMV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, mis ? k_camera_shade<true, false> : k_camera_shade<false, false>,
                                                            sth, 0));
     const int trace_grid = std::max(1, occ_t) * s.num_sms;
     int occ_tail = 0;
@@ -1283,6 +1308,7 @@ void run_waves(SceneHost& s, RenderScratch& R, const FramePlan& P, const omv_cam
     // a batch over a group of scenes: every ray starts at its own scene's top-level tree
     const DevJob* gjobs = batch && s.parts.size() > 1 ? batch->d_jobs : nullptr;
     const int shade_grid = std::max(1, occ_s) * s.num_sms;
+    const bool staged = !batch && !mis && cap >= kStagedPaths;
     int64_t launches = 0;
     // optional per-launch events around the closest-hit kernels
     std::vector<cudaEvent_t> ext_ev, sh_ev, tail_ev;
@@ -1399,9 +1425,11 @@ void run_waves(SceneHost& s, RenderScratch& R, const FramePlan& P, const omv_cam
                 if (time_kernels) timed(ext_ev);
                 join();
                 if (mis)
-                    k_camera_shade<true><<<shade_grid, sth, 0, st>>>(A, b, in, out);
+                    k_camera_shade<true, false><<<shade_grid, sth, 0, st>>>(A, b, in, out);
+                else if (staged)
+                    k_camera_shade<false, true><<<shade_grid, sth, 0, st>>>(A, b, in, out);
                 else
-                    k_camera_shade<false><<<shade_grid, sth, 0, st>>>(A, b, in, out);
+                    k_camera_shade<false, false><<<shade_grid, sth, 0, st>>>(A, b, in, out);
                 launches += 2;
                 fork();
                 if (lights) {
@@ -1837,7 +1865,7 @@ void load_wave_kernels()
     OMV_CUDA(cudaFuncGetAttributes(&a, k_light_gen));
     OMV_CUDA(cudaFuncGetAttributes(&a, k_extend));
     OMV_CUDA(cudaFuncGetAttributes(&a, k_light_shade));
-    OMV_CUDA(cudaFuncGetAttributes(&a, k_camera_shade<false>));
+    OMV_CUDA(cudaFuncGetAttributes(&a, k_camera_shade<false, false>));
     OMV_CUDA(cudaFuncGetAttributes(&a, k_shadow<false, false>));
     OMV_CUDA(cudaFuncGetAttributes(&a, k_shadow<false, true>));
     OMV_CUDA(cudaFuncGetAttributes(&a, k_camera_tail<false, false>));

@@ -98,6 +98,70 @@ __device__ __forceinline__ uint32_t block_append_binned(uint32_t* counter, bool 
     return slot;
 }
 
+// The next rays of a block's window of kStageSteps steps, kept in shared memory
+// and then appended to the queue grouped by direction: four times the rays of
+// block_append_binned per group, and its barriers once per window instead of
+// once per step (32 KB per block; kStagedPaths says where it pays).
+constexpr int kStageSteps = 4;
+constexpr uint32_t kStageWindows = 8;
+struct StagedRays {
+    float4 ray[2 * kStageSteps * kShadeThreads];
+    uint32_t count[32];  // per bin, then the bin's start
+    uint32_t n, base;
+};
+// every thread of the block calls the three; staged_add by whole warps
+__device__ __forceinline__ void staged_begin(StagedRays& s)
+{
+    if (threadIdx.x < 32) s.count[threadIdx.x] = 0;
+    if (threadIdx.x == 0) s.n = 0;
+    __syncthreads();
+}
+__device__ __forceinline__ void staged_add(StagedRays& s, bool want, float4 a, float4 b)
+{
+    const uint32_t at = warp_append(&s.n, want);
+    if (want) {
+        s.ray[2 * at] = a;
+        s.ray[2 * at + 1] = b;
+    }
+}
+__device__ __forceinline__ void staged_append(StagedRays& s, uint32_t* counter, float4* queue)
+{
+    __syncthreads();
+    const uint32_t n = s.n;
+    uint32_t bin[kStageSteps], rank[kStageSteps];
+#pragma unroll
+    for (int j = 0; j < kStageSteps; ++j) {
+        const uint32_t t = j * blockDim.x + threadIdx.x;
+        if (t < n) {
+            const float4 d = s.ray[2 * t + 1];
+            bin[j] = direction_bin(v3(d.x, d.y, d.z));
+            rank[j] = atomicAdd(&s.count[bin[j]], 1u);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const uint32_t c = s.count[threadIdx.x];
+        uint32_t x = c;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+            if ((int)threadIdx.x >= o) x += y;
+        }
+        s.count[threadIdx.x] = x - c;
+        if (threadIdx.x == 31) s.base = x ? atomicAdd(counter, x) : 0u;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kStageSteps; ++j) {
+        const uint32_t t = j * blockDim.x + threadIdx.x;
+        if (t < n) {
+            float4* q = queue + 2 * ((size_t)s.base + s.count[bin[j]] + rank[j]);
+            q[0] = s.ray[2 * t];
+            q[1] = s.ray[2 * t + 1];
+        }
+    }
+    __syncthreads();  // the window's rays are read before the next one's come
+}
+
 // Division of 32-bit unsigned integers by a divisor fixed for a frame, by one
 // multiply-high, a subtraction and two shifts (Granlund & Montgomery,
 // "Division by invariant integers using multiplication", PLDI 1994, 4.1):

@@ -33,6 +33,16 @@ def test_unlit_film_does_not_depend_on_the_queue_length(gpu, scenes, estimator, 
     assert np.array_equal(ca, cb) and np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("size", [(1024, 512, 64), (1023, 517, 65)])
+def test_rays_grouped_over_several_shading_steps(gpu, scenes, size):
+    """One wave of 2^25 paths or more groups its rays over windows of several steps, waves of 2^22 step by step."""
+    sc = scenes.scene_c2(*size, tri_scale=0.02, sky_size=(128, 64))
+    rs = gpu.RenderScene(sc)
+    a, ca = _render(gpu, rs, sc)
+    b, cb = _render(gpu, rs, sc, wave_paths=size[2] << 16)
+    assert np.array_equal(ca, cb) and np.array_equal(a, b)
+
+
 @pytest.mark.parametrize("name", ["c1", "mixed", "textured"])
 def test_lit_film_does_not_depend_on_the_queue_length(gpu, scenes, name):
     """Conductors, transmission, blended and texture-masked materials (retries past masked hits)."""
