@@ -985,18 +985,29 @@ __device__ __forceinline__ Box empty_box()
     return b;
 }
 
-// a child range: a leaf reference (~position), or a new internal node and its task
-__device__ __forceinline__ int sah_child(int first, int last, int parent, uint32_t* node_counter, SahTask* next_large,
-                                         uint32_t* n_large, SahTask* next_small, uint32_t* n_small)
+// Task lists of the next level by size: more than kSweepMaxDev items, more than
+// kTinyMax, and the rest.
+constexpr int kTinyMax = 8;
+struct SahLists {
+    SahTask* list[3];  // large, small, tiny
+    uint32_t* count;   // of each
+};
+__device__ __forceinline__ int sah_class(int cnt) { return cnt > kSweepMaxDev ? 0 : cnt > kTinyMax ? 1 : 2; }
+
+// A subtree of m items has m - 1 nodes: the node of a range whose subtree starts
+// at number `node` has its left subtree at node + 1 and its right one behind it,
+// so no counter is needed (with one, and a queue entry per node, two atomics on
+// one address per node, about a nanosecond each, took most of a build).
+__device__ __forceinline__ int sah_left_node(const SahTask& t) { return t.node + 1; }
+__device__ __forceinline__ int sah_right_node(const SahTask& t, int split) { return t.node + (split - t.first + 1); }
+
+// a child range of a large task: a leaf reference (~position), or its node and a task
+__device__ __forceinline__ int sah_child(int first, int last, int node, int parent, const SahLists& next)
 {
     if (first == last) return ~first;
-    const int id = (int)atomicAdd(node_counter, 1u);
-    const SahTask t{first, last, id, parent};
-    if (last - first + 1 > kSweepMaxDev)
-        next_large[atomicAdd(n_large, 1u)] = t;
-    else
-        next_small[atomicAdd(n_small, 1u)] = t;
-    return id;
+    const int c = sah_class(last - first + 1);
+    next.list[c][atomicAdd(next.count + c, 1u)] = SahTask{first, last, node, parent};
+    return node;
 }
 
 __device__ __forceinline__ int sah_bin(float c2, float cmin, float scale)
@@ -1006,9 +1017,7 @@ __device__ __forceinline__ int sah_bin(float c2, float cmin, float scale)
 
 __global__ void __launch_bounds__(kSahLargeThreads) k_sah_large(const SahTask* __restrict__ tasks,
                                                                 const Box* __restrict__ item_boxes, uint32_t* order,
-                                                                uint32_t* tmp, Node2* nodes, uint32_t* node_counter,
-                                                                SahTask* next_large, uint32_t* n_large,
-                                                                SahTask* next_small, uint32_t* n_small)
+                                                                uint32_t* tmp, Node2* nodes, SahLists next)
 {
     constexpr int NW = kSahLargeThreads / 32;
     __shared__ uint32_t sbox[6], scen[6];
@@ -1208,20 +1217,21 @@ __global__ void __launch_bounds__(kSahLargeThreads) k_sah_large(const SahTask* _
             nd.box.lo[k] = ord2f(sbox[k]);
             nd.box.hi[k] = ord2f(sbox[3 + k]);
         }
-        nd.left = sah_child(t.first, split, t.node, node_counter, next_large, n_large, next_small, n_small);
-        nd.right = sah_child(split + 1, t.last, t.node, node_counter, next_large, n_large, next_small, n_small);
+        nd.left = sah_child(t.first, split, sah_left_node(t), t.node, next);
+        nd.right = sah_child(split + 1, t.last, sah_right_node(t, split), t.node, next);
         nodes[t.node] = nd;
     }
 }
 
-// warp-wide bitonic sort of one 64-bit key per lane, ascending
-__device__ __forceinline__ uint64_t warp_sort64(uint64_t key)
+// bitonic sort of one 64-bit key per lane over groups of G lanes, ascending
+template <int G>
+__device__ __forceinline__ uint64_t group_sort64(uint64_t key)
 {
-    const int lane = threadIdx.x & 31;
-    for (int k = 2; k <= 32; k <<= 1)
+    const int lane = threadIdx.x & (G - 1);
+    for (int k = 2; k <= G; k <<= 1)
         for (int j = k >> 1; j > 0; j >>= 1) {
-            const uint32_t lo = __shfl_xor_sync(0xFFFFFFFFu, (uint32_t)key, j);
-            const uint32_t hi = __shfl_xor_sync(0xFFFFFFFFu, (uint32_t)(key >> 32), j);
+            const uint32_t lo = __shfl_xor_sync(0xFFFFFFFFu, (uint32_t)key, j, G);
+            const uint32_t hi = __shfl_xor_sync(0xFFFFFFFFu, (uint32_t)(key >> 32), j, G);
             const uint64_t other = ((uint64_t)hi << 32) | lo;
             const bool up = (lane & k) == 0;
             const bool lower = (lane & j) == 0;
@@ -1231,64 +1241,76 @@ __device__ __forceinline__ uint64_t warp_sort64(uint64_t key)
     return key;
 }
 
-// ranges of 2..kSweepMaxDev items: one warp each, full sweep on every axis
-__global__ void k_sah_small(int ntasks, const SahTask* __restrict__ tasks, const Box* __restrict__ item_boxes,
-                            uint32_t* order, Node2* nodes, uint32_t* node_counter, SahTask* next_large,
-                            uint32_t* n_large, SahTask* next_small, uint32_t* n_small)
+template <int G>
+__device__ __forceinline__ Box group_box(const Box& b, int src)
 {
-    const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (w >= ntasks) return;  // whole warps leave together
-    const int lane = threadIdx.x & 31;
-    const SahTask t = tasks[w];
+    Box r;
+    for (int k = 0; k < 3; ++k) {
+        r.lo[k] = __shfl_sync(0xFFFFFFFFu, b.lo[k], src, G);
+        r.hi[k] = __shfl_sync(0xFFFFFFFFu, b.hi[k], src, G);
+    }
+    return r;
+}
+
+// Ranges of 2..G items: G lanes each, full sweep on every axis.  Ranges of up to
+// kTinyMax items, most of a tree's nodes, take eight lanes, four to a warp, with
+// the shorter sorts and scans; a child of two items becomes a node at once; the
+// warp's tasks are queued with one atomic.  A 1M-triangle forest: 2.1 ms of
+// these launches with a warp per range, an atomic per node and one per task, 0.46 ms so.
+template <int G>
+__global__ void __launch_bounds__(128) k_sah_small(int ntasks, const SahTask* __restrict__ tasks,
+                                                   const Box* __restrict__ item_boxes, uint32_t* order, Node2* nodes,
+                                                   SahLists next)
+{
+    const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) / G);
+    const bool live = w < ntasks;
+    if (!__any_sync(0xFFFFFFFFu, live)) return;  // whole warps leave together
+    const int lane = threadIdx.x & (G - 1);
+    const SahTask t = live ? tasks[w] : SahTask{0, -1, 0, 0};
     const int cnt = t.last - t.first + 1;
     const bool valid = lane < cnt;
     const uint32_t item = valid ? order[t.first + lane] : 0u;
     const Box b = valid ? item_boxes[item] : empty_box();
     // node box
     Box nb = b;
-    for (int o = 16; o; o >>= 1)
+    for (int o = G / 2; o; o >>= 1)
         for (int k = 0; k < 3; ++k) {
-            nb.lo[k] = fminf(nb.lo[k], __shfl_xor_sync(0xFFFFFFFFu, nb.lo[k], o));
-            nb.hi[k] = fmaxf(nb.hi[k], __shfl_xor_sync(0xFFFFFFFFu, nb.hi[k], o));
+            nb.lo[k] = fminf(nb.lo[k], __shfl_xor_sync(0xFFFFFFFFu, nb.lo[k], o, G));
+            nb.hi[k] = fmaxf(nb.hi[k], __shfl_xor_sync(0xFFFFFFFFu, nb.hi[k], o, G));
         }
     float best = 3.0e38f;
-    int best_axis = -1, best_k = 0;
+    int best_axis = -1, best_k = 0, best_src = lane;
     for (int a = 0; a < 3; ++a) {
         // stable order along the axis: key = (doubled centroid, position)
         const uint64_t key = valid ? (((uint64_t)f2ord(b.lo[a] + b.hi[a]) << 32) | (uint32_t)lane) : ~0ull;
-        const uint64_t sk = warp_sort64(key);
-        const int src = (int)(sk & 31u);
-        Box sb;
-        for (int k = 0; k < 3; ++k) {
-            sb.lo[k] = __shfl_sync(0xFFFFFFFFu, b.lo[k], src);
-            sb.hi[k] = __shfl_sync(0xFFFFFFFFu, b.hi[k], src);
-        }
+        const int src = (int)(group_sort64<G>(key) & (uint64_t)(G - 1));
+        Box sb = group_box<G>(b, src);
         if (lane >= cnt) sb = empty_box();
         Box pre = sb, suf = sb;
-        for (int o = 1; o < 32; o <<= 1) {
+        for (int o = 1; o < G; o <<= 1) {
             Box x, y;
             for (int k = 0; k < 3; ++k) {
-                x.lo[k] = __shfl_up_sync(0xFFFFFFFFu, pre.lo[k], o);
-                x.hi[k] = __shfl_up_sync(0xFFFFFFFFu, pre.hi[k], o);
-                y.lo[k] = __shfl_down_sync(0xFFFFFFFFu, suf.lo[k], o);
-                y.hi[k] = __shfl_down_sync(0xFFFFFFFFu, suf.hi[k], o);
+                x.lo[k] = __shfl_up_sync(0xFFFFFFFFu, pre.lo[k], o, G);
+                x.hi[k] = __shfl_up_sync(0xFFFFFFFFu, pre.hi[k], o, G);
+                y.lo[k] = __shfl_down_sync(0xFFFFFFFFu, suf.lo[k], o, G);
+                y.hi[k] = __shfl_down_sync(0xFFFFFFFFu, suf.hi[k], o, G);
             }
             if (lane >= o) pre = box_union(x, pre);
-            if (lane + o < 32) suf = box_union(suf, y);
+            if (lane + o < G) suf = box_union(suf, y);
         }
         Box r;
         for (int k = 0; k < 3; ++k) {
-            r.lo[k] = __shfl_down_sync(0xFFFFFFFFu, suf.lo[k], 1);
-            r.hi[k] = __shfl_down_sync(0xFFFFFFFFu, suf.hi[k], 1);
+            r.lo[k] = __shfl_down_sync(0xFFFFFFFFu, suf.lo[k], 1, G);
+            r.hi[k] = __shfl_down_sync(0xFFFFFFFFu, suf.hi[k], 1, G);
         }
         float cost = 3.4e38f;
         if (lane < cnt - 1)
             cost = half_area(pre) * (float)(lane + 1) + half_area(r) * (float)(cnt - 1 - lane);
         float mc = cost;
         int mk = lane;
-        for (int o = 16; o; o >>= 1) {
-            const float oc = __shfl_xor_sync(0xFFFFFFFFu, mc, o);
-            const int ok_ = __shfl_xor_sync(0xFFFFFFFFu, mk, o);
+        for (int o = G / 2; o; o >>= 1) {
+            const float oc = __shfl_xor_sync(0xFFFFFFFFu, mc, o, G);
+            const int ok_ = __shfl_xor_sync(0xFFFFFFFFu, mk, o, G);
             if (oc < mc || (oc == mc && ok_ < mk)) {
                 mc = oc;
                 mk = ok_;
@@ -1298,27 +1320,64 @@ __global__ void k_sah_small(int ntasks, const SahTask* __restrict__ tasks, const
             best = mc;
             best_axis = a;
             best_k = mk;
+            best_src = src;
         }
     }
-    int split;
-    if (best_axis >= 0) {
-        const uint64_t key = valid ? (((uint64_t)f2ord(b.lo[best_axis] + b.hi[best_axis]) << 32) | (uint32_t)lane)
-                                   : ~0ull;
-        const uint64_t sk = warp_sort64(key);
-        const uint32_t it = __shfl_sync(0xFFFFFFFFu, item, (int)(sk & 31u));
-        if (valid) order[t.first + lane] = it;
-        split = t.first + best_k;
-    } else {
-        split = t.first + cnt / 2 - 1;
+    // without a best axis (boxes too large for an area) the halves of the range as it stands
+    const int left = best_axis >= 0 ? best_k + 1 : cnt / 2;
+    const uint32_t it = __shfl_sync(0xFFFFFFFFu, item, best_src, G);
+    const Box sb = group_box<G>(b, best_src);
+    if (valid) order[t.first + lane] = it;
+    __syncwarp();  // a pair's lead may write two of these again
+    const int split = t.first + left - 1;
+    const int child_node[2] = {sah_left_node(t), sah_right_node(t, split)};
+    int ref[2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        const int p0 = c == 0 ? 0 : left, m = c == 0 ? left : cnt - left;  // the child's positions in the range
+        const int first = t.first + p0;
+        ref[c] = m == 1 ? ~first : child_node[c];
+        // a pair: its node, in order of the centroids along x
+        const uint32_t i0 = __shfl_sync(0xFFFFFFFFu, it, p0 & (G - 1), G);
+        const uint32_t i1 = __shfl_sync(0xFFFFFFFFu, it, (p0 + 1) & (G - 1), G);
+        const Box b0 = group_box<G>(sb, p0 & (G - 1)), b1 = group_box<G>(sb, (p0 + 1) & (G - 1));
+        const bool lead = live && lane == 0;
+        if (lead && m == 2) {
+            if (b1.lo[0] + b1.hi[0] < b0.lo[0] + b0.hi[0]) {
+                order[first] = i1;
+                order[first + 1] = i0;
+            }
+            Node2 nd;
+            nd.first = first;
+            nd.last = first + 1;
+            nd.parent = t.node;
+            nd.box = box_union(b0, b1);
+            nd.left = ~first;
+            nd.right = ~(first + 1);
+            nodes[child_node[c]] = nd;
+        }
+        const bool want = lead && m > 2;
+        const int cls = sah_class(m);
+#pragma unroll
+        for (int x = 1; x < 3; ++x) {
+            const uint32_t mask = __ballot_sync(0xFFFFFFFFu, want && cls == x);
+            if (!mask) continue;
+            uint32_t base = 0;
+            if ((int)(threadIdx.x & 31) == __ffs(mask) - 1) base = atomicAdd(next.count + x, (uint32_t)__popc(mask));
+            base = __shfl_sync(0xFFFFFFFFu, base, __ffs(mask) - 1);
+            if (want && cls == x)
+                next.list[x][base + __popc(mask & ((1u << (threadIdx.x & 31)) - 1u))] =
+                    SahTask{first, first + m - 1, child_node[c], t.node};
+        }
     }
-    if (lane == 0) {
+    if (live && lane == 0) {
         Node2 nd;
         nd.first = t.first;
         nd.last = t.last;
         nd.parent = t.parent;
         nd.box = nb;
-        nd.left = sah_child(t.first, split, t.node, node_counter, next_large, n_large, next_small, n_small);
-        nd.right = sah_child(split + 1, t.last, t.node, node_counter, next_large, n_large, next_small, n_small);
+        nd.left = ref[0];
+        nd.right = ref[1];
         nodes[t.node] = nd;
     }
 }
@@ -1629,9 +1688,19 @@ static void sah_forest(int n, const std::vector<uint32_t>& seg_base, const Box* 
     const int nseg = (int)seg_base.size();
     f.alloc(n);
     k_iota<<<blocks(n, 256), 256, 0, st>>>(n, f.vals);
-    DBuf<uint32_t> tmp(n), ctr(3);  // nodes, large tasks, small tasks
-    DBuf<SahTask> la(n), lb(n), sa(n), sb(n);
-    std::vector<SahTask> large, small;
+    DBuf<uint32_t> tmp(n), ctr(3);
+    // two sets of lists (a level's tasks and the next one's): at most one task per
+    // two items, a large one per kSweepMaxDev + 1
+    const size_t most[3] = {(size_t)n / (kSweepMaxDev + 1) + 1, (size_t)n / (kTinyMax + 1) + 1, (size_t)n / 2 + 1};
+    DBuf<SahTask> tasks(2 * (most[0] + most[1] + most[2]));
+    SahTask* set[2][3];
+    size_t at = 0;
+    for (auto& lists : set)
+        for (int c = 0; c < 3; ++c) {
+            lists[c] = tasks.p + at;
+            at += most[c];
+        }
+    std::vector<SahTask> first_tasks[3];
     std::vector<int> roots(nseg);
     int next_id = 0;
     for (int s = 0; s < nseg; ++s) {
@@ -1640,33 +1709,34 @@ static void sah_forest(int n, const std::vector<uint32_t>& seg_base, const Box* 
             roots[s] = ~first;
             continue;
         }
-        const SahTask t{first, last, next_id, -2 - s};
-        roots[s] = next_id++;
-        (last - first + 1 > kSweepMaxDev ? large : small).push_back(t);
+        roots[s] = next_id;
+        const int cnt = last - first + 1;
+        first_tasks[cnt > kSweepMaxDev ? 0 : cnt > kTinyMax ? 1 : 2].push_back(SahTask{first, last, next_id, -2 - s});
+        next_id += cnt - 1;
     }
-    uint32_t h[3] = {(uint32_t)next_id, (uint32_t)large.size(), (uint32_t)small.size()};
-    if (!large.empty())
-        OMV_CK(cudaMemcpyAsync(la.p, large.data(), sizeof(SahTask) * large.size(), cudaMemcpyHostToDevice, st));
-    if (!small.empty())
-        OMV_CK(cudaMemcpyAsync(sa.p, small.data(), sizeof(SahTask) * small.size(), cudaMemcpyHostToDevice, st));
-    OMV_CK(cudaMemcpyAsync(ctr.p, h, sizeof(h), cudaMemcpyHostToDevice, st));
-    SahTask *cl = la.p, *nl = lb.p, *cs = sa.p, *ns = sb.p;
-    for (int level = 0; h[1] + h[2] > 0; ++level) {
+    uint32_t h[3];
+    for (int c = 0; c < 3; ++c) {
+        h[c] = (uint32_t)first_tasks[c].size();
+        if (h[c])
+            OMV_CK(cudaMemcpyAsync(set[0][c], first_tasks[c].data(), sizeof(SahTask) * h[c], cudaMemcpyHostToDevice, st));
+    }
+    for (int level = 0; h[0] + h[1] + h[2] > 0; ++level) {
         if (level > 4096) throw std::runtime_error("device SAH build did not terminate");
-        const int nlarge = (int)h[1], nsmall = (int)h[2];
-        OMV_CK(cudaMemsetAsync(ctr.p + 1, 0, 2 * sizeof(uint32_t), st));
-        if (nlarge)
-            k_sah_large<<<nlarge, kSahLargeThreads, 0, st>>>(cl, item_boxes, f.vals, tmp.p, f.nodes, ctr.p, nl,
-                                                             ctr.p + 1, ns, ctr.p + 2);
-        if (nsmall)
-            k_sah_small<<<blocks((size_t)nsmall * 32, 128), 128, 0, st>>>(nsmall, cs, item_boxes, f.vals, f.nodes,
-                                                                          ctr.p, nl, ctr.p + 1, ns, ctr.p + 2);
+        SahTask** cur = set[level & 1];
+        SahTask** nxt = set[(level + 1) & 1];
+        const SahLists next{{nxt[0], nxt[1], nxt[2]}, ctr.p};
+        OMV_CK(cudaMemsetAsync(ctr.p, 0, 3 * sizeof(uint32_t), st));
+        if (h[0])
+            k_sah_large<<<(int)h[0], kSahLargeThreads, 0, st>>>(cur[0], item_boxes, f.vals, tmp.p, f.nodes, next);
+        if (h[1])
+            k_sah_small<32><<<blocks((size_t)h[1] * 32, 128), 128, 0, st>>>((int)h[1], cur[1], item_boxes, f.vals,
+                                                                           f.nodes, next);
+        if (h[2])
+            k_sah_small<kTinyMax><<<blocks((size_t)h[2] * kTinyMax, 128), 128, 0, st>>>((int)h[2], cur[2], item_boxes,
+                                                                                     f.vals, f.nodes, next);
         OMV_CK(cudaGetLastError());
         OMV_CK(cudaMemcpyAsync(h, ctr.p, sizeof(h), cudaMemcpyDeviceToHost, st));
         OMV_CK(cudaStreamSynchronize(st));
-        if ((int)h[0] > std::max(1, n - nseg)) throw std::runtime_error("device SAH build: node capacity exceeded");
-        std::swap(cl, nl);
-        std::swap(cs, ns);
     }
     f.roots = roots;
 }
