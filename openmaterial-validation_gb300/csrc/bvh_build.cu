@@ -969,7 +969,6 @@ __global__ void k_ploc_nodes(int ni, const int2* child, const Box* node_box, con
 // placement pass.
 constexpr int kSahBinsDev = 32;
 constexpr int kSweepMaxDev = 32;
-constexpr int kSahLargeThreads = 256;
 
 struct SahTask {
     int first, last, node, parent;
@@ -985,14 +984,21 @@ __device__ __forceinline__ Box empty_box()
     return b;
 }
 
-// Task lists of the next level by size: more than kSweepMaxDev items, more than
-// kTinyMax, and the rest.
-constexpr int kTinyMax = 8;
+// Task lists of the next level by size: classes 0..2 for k_sah_large with blocks
+// of 1024, 256 and 128 threads, 3 and 4 for k_sah_small with a warp and with
+// eight lanes.  With one size of block (256) a 1M-triangle forest's first
+// levels, few ranges of 16k items, and the last ones, thousands of 50 items,
+// took most of k_sah_large's 1.06 ms: 0.83 ms so.
+constexpr int kHugeMin = 2048, kMidMax = 256, kTinyMax = 8;
+constexpr int kSahClasses = 5, kSahSmall = 3;
 struct SahLists {
-    SahTask* list[3];  // large, small, tiny
-    uint32_t* count;   // of each
+    SahTask* list[kSahClasses];
+    uint32_t* count;  // of each
 };
-__device__ __forceinline__ int sah_class(int cnt) { return cnt > kSweepMaxDev ? 0 : cnt > kTinyMax ? 1 : 2; }
+__host__ __device__ __forceinline__ int sah_class(int cnt)
+{
+    return cnt >= kHugeMin ? 0 : cnt > kMidMax ? 1 : cnt > kSweepMaxDev ? 2 : cnt > kTinyMax ? 3 : 4;
+}
 
 // A subtree of m items has m - 1 nodes: the node of a range whose subtree starts
 // at number `node` has its left subtree at node + 1 and its right one behind it,
@@ -1015,11 +1021,11 @@ __device__ __forceinline__ int sah_bin(float c2, float cmin, float scale)
     return (int)fminf((float)(kSahBinsDev - 1), (c2 - cmin) * scale);
 }
 
-__global__ void __launch_bounds__(kSahLargeThreads) k_sah_large(const SahTask* __restrict__ tasks,
-                                                                const Box* __restrict__ item_boxes, uint32_t* order,
-                                                                uint32_t* tmp, Node2* nodes, SahLists next)
+template <int NT>
+__global__ void __launch_bounds__(NT) k_sah_large(const SahTask* __restrict__ tasks, const Box* __restrict__ item_boxes,
+                                                  uint32_t* order, uint32_t* tmp, Node2* nodes, SahLists next)
 {
-    constexpr int NW = kSahLargeThreads / 32;
+    constexpr int NW = NT / 32;
     __shared__ uint32_t sbox[6], scen[6];
     __shared__ uint32_t bcnt[3][kSahBinsDev];
     __shared__ uint32_t bbox[3][kSahBinsDev][6];
@@ -1359,7 +1365,7 @@ __global__ void __launch_bounds__(128) k_sah_small(int ntasks, const SahTask* __
         const bool want = lead && m > 2;
         const int cls = sah_class(m);
 #pragma unroll
-        for (int x = 1; x < 3; ++x) {
+        for (int x = kSahSmall; x < kSahClasses; ++x) {
             const uint32_t mask = __ballot_sync(0xFFFFFFFFu, want && cls == x);
             if (!mask) continue;
             uint32_t base = 0;
@@ -1688,19 +1694,21 @@ static void sah_forest(int n, const std::vector<uint32_t>& seg_base, const Box* 
     const int nseg = (int)seg_base.size();
     f.alloc(n);
     k_iota<<<blocks(n, 256), 256, 0, st>>>(n, f.vals);
-    DBuf<uint32_t> tmp(n), ctr(3);
+    DBuf<uint32_t> tmp(n), ctr(kSahClasses);
     // two sets of lists (a level's tasks and the next one's): at most one task per
-    // two items, a large one per kSweepMaxDev + 1
-    const size_t most[3] = {(size_t)n / (kSweepMaxDev + 1) + 1, (size_t)n / (kTinyMax + 1) + 1, (size_t)n / 2 + 1};
-    DBuf<SahTask> tasks(2 * (most[0] + most[1] + most[2]));
-    SahTask* set[2][3];
+    // `fewest` items of its class
+    constexpr int kFewest[kSahClasses] = {kHugeMin, kMidMax + 1, kSweepMaxDev + 1, kTinyMax + 1, 2};
+    size_t total = 0;
+    for (int fewest : kFewest) total += (size_t)(n / fewest + 1);
+    DBuf<SahTask> tasks(2 * total);
+    SahTask* set[2][kSahClasses];
     size_t at = 0;
     for (auto& lists : set)
-        for (int c = 0; c < 3; ++c) {
+        for (int c = 0; c < kSahClasses; ++c) {
             lists[c] = tasks.p + at;
-            at += most[c];
+            at += (size_t)(n / kFewest[c] + 1);
         }
-    std::vector<SahTask> first_tasks[3];
+    std::vector<SahTask> first_tasks[kSahClasses];
     std::vector<int> roots(nseg);
     int next_id = 0;
     for (int s = 0; s < nseg; ++s) {
@@ -1711,32 +1719,38 @@ static void sah_forest(int n, const std::vector<uint32_t>& seg_base, const Box* 
         }
         roots[s] = next_id;
         const int cnt = last - first + 1;
-        first_tasks[cnt > kSweepMaxDev ? 0 : cnt > kTinyMax ? 1 : 2].push_back(SahTask{first, last, next_id, -2 - s});
+        first_tasks[sah_class(cnt)].push_back(SahTask{first, last, next_id, -2 - s});
         next_id += cnt - 1;
     }
-    uint32_t h[3];
-    for (int c = 0; c < 3; ++c) {
+    uint32_t h[kSahClasses];
+    bool more = false;
+    for (int c = 0; c < kSahClasses; ++c) {
+        more = more || !first_tasks[c].empty();
         h[c] = (uint32_t)first_tasks[c].size();
         if (h[c])
             OMV_CK(cudaMemcpyAsync(set[0][c], first_tasks[c].data(), sizeof(SahTask) * h[c], cudaMemcpyHostToDevice, st));
     }
-    for (int level = 0; h[0] + h[1] + h[2] > 0; ++level) {
+    for (int level = 0; more; ++level) {
         if (level > 4096) throw std::runtime_error("device SAH build did not terminate");
         SahTask** cur = set[level & 1];
-        SahTask** nxt = set[(level + 1) & 1];
-        const SahLists next{{nxt[0], nxt[1], nxt[2]}, ctr.p};
-        OMV_CK(cudaMemsetAsync(ctr.p, 0, 3 * sizeof(uint32_t), st));
-        if (h[0])
-            k_sah_large<<<(int)h[0], kSahLargeThreads, 0, st>>>(cur[0], item_boxes, f.vals, tmp.p, f.nodes, next);
-        if (h[1])
-            k_sah_small<32><<<blocks((size_t)h[1] * 32, 128), 128, 0, st>>>((int)h[1], cur[1], item_boxes, f.vals,
+        SahLists next;
+        std::copy(set[(level + 1) & 1], set[(level + 1) & 1] + kSahClasses, next.list);
+        next.count = ctr.p;
+        OMV_CK(cudaMemsetAsync(ctr.p, 0, sizeof(h), st));
+        if (h[0]) k_sah_large<1024><<<(int)h[0], 1024, 0, st>>>(cur[0], item_boxes, f.vals, tmp.p, f.nodes, next);
+        if (h[1]) k_sah_large<256><<<(int)h[1], 256, 0, st>>>(cur[1], item_boxes, f.vals, tmp.p, f.nodes, next);
+        if (h[2]) k_sah_large<128><<<(int)h[2], 128, 0, st>>>(cur[2], item_boxes, f.vals, tmp.p, f.nodes, next);
+        if (h[3])
+            k_sah_small<32><<<blocks((size_t)h[3] * 32, 128), 128, 0, st>>>((int)h[3], cur[3], item_boxes, f.vals,
                                                                            f.nodes, next);
-        if (h[2])
-            k_sah_small<kTinyMax><<<blocks((size_t)h[2] * kTinyMax, 128), 128, 0, st>>>((int)h[2], cur[2], item_boxes,
+        if (h[4])
+            k_sah_small<kTinyMax><<<blocks((size_t)h[4] * kTinyMax, 128), 128, 0, st>>>((int)h[4], cur[4], item_boxes,
                                                                                      f.vals, f.nodes, next);
         OMV_CK(cudaGetLastError());
         OMV_CK(cudaMemcpyAsync(h, ctr.p, sizeof(h), cudaMemcpyDeviceToHost, st));
         OMV_CK(cudaStreamSynchronize(st));
+        more = false;
+        for (uint32_t c : h) more = more || c > 0;
     }
     f.roots = roots;
 }

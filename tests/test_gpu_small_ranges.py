@@ -1,6 +1,7 @@
 """The SAH build gives ranges of up to 8 triangles eight lanes each, of up to 32
-a warp, and longer ones a block, and makes nodes of pairs with their parents:
-hits of meshes at those sizes are the oracle's, bit for bit."""
+a warp, and longer ones blocks of 128, 256 (from 257) and 1024 threads (from
+2048), and makes nodes of pairs with their parents: hits of meshes at those
+sizes are the oracle's, bit for bit."""
 import dataclasses
 
 import numpy as np
@@ -9,12 +10,17 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
+SHORT = [2, 3, 4, 7, 8, 9, 10, 16, 31, 32, 33, 34, 63, 65, 257]
+LONG = [256, 258, 2047, 2048, 2049, 6007]
+
+
+@pytest.mark.parametrize("sizes", [SHORT, LONG], ids=["short", "long"])
 @pytest.mark.parametrize("kind", ["random", "equal", "line", "huge"])
-def test_mesh_sizes_at_the_edges_of_the_classes(gpu, oracle, scenes, kind):
+def test_mesh_sizes_at_the_edges_of_the_classes(gpu, oracle, scenes, kind, sizes):
     rng = np.random.default_rng(31)
     base = scenes.scene_mixed(8, 8, 1)
     meshes, insts = [], []
-    for k, nt in enumerate([2, 3, 4, 7, 8, 9, 10, 16, 31, 32, 33, 34, 63, 65, 257]):
+    for k, nt in enumerate(sizes):
         v = rng.normal(size=(nt, 3, 3)).astype(np.float32) * np.float32(0.3)
         if kind == "equal":   # every split costs the same
             v[:] = v[:1]
