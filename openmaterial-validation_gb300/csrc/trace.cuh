@@ -328,8 +328,16 @@ __device__ __forceinline__ bool trace_step(const DevScene& S, const uint32_t* __
     ++tc.nodes;
     const uint4* N = S.nodes + 8 * (size_t)e.x;
     const uint4 w0 = __ldg(N + 0), w1 = __ldg(N + 1);
-    const uint4 qlx = __ldg(N + 2), qly = __ldg(N + 3), qlz = __ldg(N + 4);
-    const uint4 qhx = __ldg(N + 5), qhy = __ldg(N + 6), qhz = __ldg(N + 7);
+    // entry and exit planes per axis from the ray direction: for a child with
+    // qlo <= qhi these are exactly min() and max() of the two slab distances.
+    // Chosen by address: the ALU pipe is the busiest (56%), and 24 selects of
+    // loaded words and their registers cost more than six addresses
+    // (1920x1080x64 frames 37.64 -> 36.81 and 16.79 -> 16.46 ms, spills of
+    // k_extend 120 -> 88 bytes; fused two-wide multiply-adds instead of the 48
+    // single ones: 1-2% slower, for their registers).
+    const int ox = T.rid.x >= 0.0f ? 0 : 3, oy = T.rid.y >= 0.0f ? 0 : 3, oz = T.rid.z >= 0.0f ? 0 : 3;
+    const uint4 nx = __ldg(N + (2 + ox)), ny = __ldg(N + (3 + oy)), nz = __ldg(N + (4 + oz));
+    const uint4 fx = __ldg(N + (5 - ox)), fy = __ldg(N + (6 - oy)), fz = __ldg(N + (7 - oz));
     const float px = __uint_as_float(w0.x), py = __uint_as_float(w0.y), pz = __uint_as_float(w0.z);
     const uint32_t exps = w0.w;
     const uint32_t imask = exps >> 24;
@@ -344,11 +352,6 @@ __device__ __forceinline__ bool trace_step(const DevScene& S, const uint32_t* __
     const float bnx = plane_offset<true>(bx, ax), bfx = plane_offset<false>(bx, ax);
     const float bny = plane_offset<true>(by, ay), bfy = plane_offset<false>(by, ay);
     const float bnz = plane_offset<true>(bz, az), bfz = plane_offset<false>(bz, az);
-    // entry and exit planes per axis from the ray direction: for a child with
-    // qlo <= qhi these are exactly min() and max() of the two slab distances
-    const uint4 nx = rid.x >= 0.0f ? qlx : qhx, fx = rid.x >= 0.0f ? qhx : qlx;
-    const uint4 ny = rid.y >= 0.0f ? qly : qhy, fy = rid.y >= 0.0f ? qhy : qly;
-    const uint4 nz = rid.z >= 0.0f ? qlz : qhz, fz = rid.z >= 0.0f ? qhz : qlz;
     const float lim = T.best_t, tnear = T.tnear;
     uint32_t key[8];
     uint32_t leafmask = 0;
@@ -411,11 +414,9 @@ __device__ __forceinline__ bool trace_step(const DevScene& S, const uint32_t* __
         const float te = __uint_as_float(k & ~7u);
         if (te > T.best_t) continue;
         const uint32_t s = k & 7u;
-        const uint32_t meta = ((s < 4 ? meta_lo : meta_hi) >> (8 * (s & 3))) & 0xFFu;
-        if ((imask >> s) & 1u)
-            st.push(child_base + meta, te);
-        else
-            st.push(kInstTag | __ldg(tlas_items + prim_base + (meta & 31u)), te);
+        const uint32_t meta = __byte_perm(meta_lo, meta_hi, s) & 0xFFu;
+        const uint32_t ref = (imask >> s) & 1u ? child_base + meta : kInstTag | __ldg(tlas_items + prim_base + (meta & 31u));
+        st.push(ref, te);
     }
     return true;
 }
