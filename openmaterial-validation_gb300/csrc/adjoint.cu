@@ -25,9 +25,10 @@
 // registers, and the records ran through L1 and L2 as local memory.  Split by
 // bounce, the traversal kernels are the renderer's, every launch's lanes do the
 // same work, and the derivatives, recomputed where the backward walk needs
-// them, never leave registers.  512x512, 32 spp, 100k triangles, 8 materials:
-// 103 ms before, 7.7 ms so.  Jobs of a batch share the waves: one step (forward
-// and replay) of an inverse fit of eight 128x128x16 scenes 29.1 -> 6.0 ms.
+// them, never leave registers.  One gradient (forward and replay) of 512x512,
+// 32 spp, 100k triangles, 8 materials: 111 ms before, 13.1 ms so.  Jobs of a
+// batch share the waves: one step of an inverse fit of eight 128x128x16 scenes
+// 28.5 -> 5.1 ms.
 //
 // Gradients: the lanes of a warp that meet the same material reduce by
 // shuffles into the warp's sums in shared memory, the block adds its totals to

@@ -2,7 +2,8 @@
 // BDPTRenderer::render -> renderRow -> computePaths (BDPTRenderer.cpp:237-393).
 //
 // A frame of W*H*spp paths is processed in waves of up to `wave_cap` paths.
-// Per wave (all launches on one stream, queue sizes stay on the device):
+// Per wave (queue sizes stay on the device; what does not depend on one another
+// runs beside it on a second stream, joined by events):
 //   light stage  (only with point lights)
 //     k_light_gen       light pick + uniformSphere emission (tryComputeLightPath)
 //     k_extend          closest hit of every queued ray
@@ -16,8 +17,8 @@
 //     k_shadow          isConnected (closest hit + end-point test), add
 //   k_film              per-path radiance into the FP64 film (PinholeCamera::hit)
 // Queues are SoA-packed float4 records appended with warp-aggregated atomics
-// (ballot + popc); the tracing kernels are persistent and fetch 32 rays per
-// warp from an atomic work counter.  Random numbers are Philox4x32-10 keyed by
+// (ballot + popc); the tracing kernels are persistent and take shares of the
+// queue from an atomic work counter.  Random numbers are Philox4x32-10 keyed by
 // (pixel, sample, vertex) so any partition of the work gives the same image.
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
@@ -1183,7 +1184,7 @@ int64_t tile_count(const TileGrid& g, const omv_camera& cam)
 // frames lose (300x200x20 of 50k triangles 1.50 -> 1.54 ms), and so do batches,
 // whose jobs are small: a tile then spans much of the tree, and its rays visit
 // start nodes that they would not meet (16 jobs of 128 to 512 pixels a side 19.30
-// -> 19.57 ms).  Beyond 2^21 tiles (576 MB of lists) rays start at the root.
+// -> 19.57 ms).  Beyond 2^21 tiles (570 MB of lists) rays start at the root.
 constexpr int64_t kTileMinPaths = 1 << 22, kTileMaxCount = 1 << 21;
 
 // the MIS estimator (environment connections) runs when asked for and the
