@@ -232,14 +232,18 @@ __device__ __forceinline__ void push_tile_node(const TileList* t, uint32_t i, Tr
 // false, then trace_end (trace_closest runs the three in a row).  Keeping the
 // state in one struct and one stack entry per step also compiles to a faster
 // loop than the single-function form (38.5 vs 38.9 ms per benchmark frame).
+// What other fields tell has no flag of its own: at 80 registers every word of
+// state is a spill (k_extend 88 -> 60 bytes, frames 1% faster).
 struct TraceState {
     V3 o, d, idw;      // world ray and box reciprocal
     V3 ro, rid;        // the ray in the current space (world or instance object space)
     Shear rs;          // shear of the current space's direction
     float tnear, best_t, bu, bv;
     uint32_t best_inst, best_prim, cur_inst, guard;
-    int blas_base;     // stack depth at which the current instance's tree started
-    bool in_blas, found;
+    int blas_base;     // stack depth at which the current instance's tree started, -1 outside one
+
+    __device__ __forceinline__ bool in_blas() const { return blas_base >= 0; }
+    __device__ __forceinline__ bool found() const { return best_prim != kInvalid; }
 };
 
 // false when the ray cannot hit anything (empty interval, zero or non-finite direction)
@@ -259,9 +263,7 @@ __device__ __forceinline__ bool trace_begin(const DevScene& S, V3 o, V3 d, float
     T.best_inst = T.best_prim = kInvalid;
     T.cur_inst = 0;
     T.guard = 0;
-    T.blas_base = 0;
-    T.in_blas = false;
-    T.found = false;
+    T.blas_base = -1;
     st.sp = 0;
     st.push(root == kInvalid ? S.tlas_root : root, tnear);  // root: one scene of a group
     return true;
@@ -280,8 +282,8 @@ __device__ __forceinline__ bool trace_step(const DevScene& S, const uint32_t* __
         st.overflow = 1;
         return false;
     }
-    if (T.in_blas && st.sp == T.blas_base) {
-        T.in_blas = false;
+    if (st.sp == T.blas_base) {
+        T.blas_base = -1;
         T.ro = T.o;
         T.rid = T.idw;
     }
@@ -315,7 +317,6 @@ __device__ __forceinline__ bool trace_step(const DevScene& S, const uint32_t* __
             return true;
         }
         T.rid = rid;
-        T.in_blas = true;
         T.blas_base = st.sp;
         T.cur_inst = ii;
         if (kRuns && last > first) {
@@ -367,7 +368,7 @@ __device__ __forceinline__ bool trace_step(const DevScene& S, const uint32_t* __
         const float tout = fminf(fminf(fminf(tfx, tfy), tfz) * 1.00000048f, lim);
         key[s] = 0xFFFFFFFFu;
         if (valid && tin <= tout) {
-            if (!internal && T.in_blas)
+            if (!internal && T.in_blas())
                 leafmask |= 1u << s;
             else  // entry distance rounded down to 8 ulp | slot
                 key[s] = (__float_as_uint(fmaxf(tin, 0.0f)) & ~7u) | (uint32_t)s;
@@ -385,11 +386,10 @@ __device__ __forceinline__ bool trace_step(const DevScene& S, const uint32_t* __
             float t, u, v;
             if (tri_hit(T.rs, T.ro, a, b, c, tnear, T.best_t, t, u, v)) {
                 const uint32_t prim = __float_as_uint(a.w);
-                const bool take = !T.found || t < T.best_t ||
+                const bool take = !T.found() || t < T.best_t ||
                                   (t == T.best_t && (T.cur_inst < T.best_inst ||
                                                      (T.cur_inst == T.best_inst && prim < T.best_prim)));
                 if (take) {
-                    T.found = true;
                     T.best_t = t;
                     T.bu = u;
                     T.bv = v;
@@ -423,7 +423,7 @@ __device__ __forceinline__ bool trace_step(const DevScene& S, const uint32_t* __
 
 __device__ __forceinline__ bool trace_end(const TraceState& T, RayHit& hit)
 {
-    if (!T.found) return false;
+    if (!T.found()) return false;
     hit.inst = T.best_inst;
     hit.prim = T.best_prim;
     hit.t = T.best_t;
@@ -442,7 +442,7 @@ __device__ __forceinline__ bool trace_any(const DevScene& S, const uint32_t* __r
     if (!trace_begin(S, o, d, tnear, tfar, T, st, root)) return false;
     while (trace_step<true>(S, tlas_items, T, st, tc, __int_as_float(0x7F800000))) {
     }
-    return T.found;
+    return T.found();
 }
 
 // Closest hit, except that the traversal stops at the first hit found with
