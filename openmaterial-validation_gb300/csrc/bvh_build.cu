@@ -963,8 +963,8 @@ __global__ void k_ploc_nodes(int ni, const int2* child, const Box* node_box, con
 // centroid bins per axis (one block per range: bounds, binning in shared
 // memory, one warp scans the bins, a stable block-wide partition), smaller
 // ranges at the best position of a full sweep over the items sorted along
-// each axis (one warp per range: bitonic sort, prefix and suffix box
-// unions).  Every range of a level is processed in the same launch, across
+// each axis (a warp or eight lanes per range: bitonic sort, prefix and suffix
+// box unions).  Every range of a level is processed in the same launch, across
 // all meshes; a range's items stay contiguous, so node ranges need no
 // placement pass.
 constexpr int kSahBinsDev = 32;
