@@ -1084,55 +1084,15 @@ inline int grid_for(int64_t n, int t) { return (int)std::max<int64_t>(1, (n + t 
 
 namespace {
 
-// Byte offsets of one wave's arrays inside a single scratch block (each array
-// starts on a 256-byte boundary).
-struct ScratchLayout {
-    size_t tp, rad, ltp, lrad, lmeta, lvp, lvr, rq0, rq1, hits, pjob, sq, ctr, stats, bytes;
-};
-
-ScratchLayout scratch_layout(int64_t wave_cap, int light_slots, int shadow_slots)
+void carve_scratch(RenderScratch& R, void* base, int64_t wave_cap, int64_t queue_cap, int light_slots,
+                   int shadow_slots)
 {
-    const size_t W = (size_t)wave_cap;
-    size_t off = 0;
-    auto take = [&](size_t bytes) {
-        size_t o = off;
-        off += (bytes + 255) & ~(size_t)255;
-        return o;
-    };
-    ScratchLayout L;
-    L.tp = take(W * 16);
-    L.rad = take(W * 16);
-    L.ltp = take(W * 16);
-    L.lrad = take(W * 16);
-    L.lmeta = take(W * 4);
-    L.lvp = take((size_t)light_slots * W * 16);
-    L.lvr = take((size_t)light_slots * W * 16);
-    L.rq0 = take(W * 32);
-    L.rq1 = take(W * 32);
-    L.hits = take(W * 16);
-    L.pjob = take(W * 4);
-    L.sq = take((size_t)shadow_slots * W * 48 + 48);
-    L.ctr = take(kMaxCounters * 4);
-    L.stats = take(16 * 8);
-    L.bytes = off;
-    return L;
-}
-
-// Scratch bytes of one path: tp rad ltp lrad (16 B each), lmeta 4, light
-// vertices 32 per slot, two ray-queue entries 64, hit 16, batch job 4, shadow
-// entries 48 per slot (each array is further rounded up to 256 bytes).
-size_t path_scratch_bytes(int light_slots, int shadow_slots)
-{
-    return 68 + 32 * (size_t)light_slots + 84 + 48 * (size_t)shadow_slots;
-}
-
-void carve_scratch(RenderScratch& R, void* base, int64_t wave_cap, int light_slots, int shadow_slots)
-{
-    const ScratchLayout L = scratch_layout(wave_cap, light_slots, shadow_slots);
+    const ScratchLayout L = scratch_layout(wave_cap, queue_cap, light_slots, shadow_slots);
     char* b = static_cast<char*>(base);
     R.base = base;
     R.bytes = L.bytes;
     R.wave_cap = wave_cap;
+    R.queue_cap = queue_cap;
     R.light_slots = light_slots;
     R.shadow_slots = shadow_slots;
     R.tp = (float4*)(b + L.tp);
@@ -1236,10 +1196,6 @@ uint32_t batch_global_pixel(const std::vector<DevJob>& jobs, int64_t g)
     return jobs[lo].pixel_base + (uint32_t)((g - jobs[lo].path_base) / jobs[lo].spp);
 }
 
-// Waves of at most this many paths run their light subpaths beside the camera
-// rays (64x64x1 401 -> 382 us, 256x256x16 997 -> 955); larger ones keep the GPU busy by themselves, and the queues'
-// 80 bytes per path are better spent on fewer waves.
-constexpr int64_t kBesideLightPaths = 1 << 22;
 // Waves of at least this many paths of one frame group their rays over windows
 // of several shading steps: the 1920x1080x64 point-light frame 38.85 -> 37.65 ms
 // (its second bounce 5.2 -> 4.3 ms), the sky frame 17.0 -> 16.83.  Where a block
@@ -1247,13 +1203,6 @@ constexpr int64_t kBesideLightPaths = 1 << 22;
 // the coarser steps cost more (1280x720x32: even; a 641x479x17 frame 3.96 ->
 // 3.99 ms, 16 batched jobs 19.13 -> 19.30).
 constexpr int64_t kStagedPaths = 1 << 25;
-void light_queues(RenderScratch& R, void* base, int64_t paths)
-{
-    float4* q = static_cast<float4*>(base);
-    R.rq[0] = q;
-    R.rq[1] = q + 2 * paths;
-    R.hits = reinterpret_cast<uint4*>(q + 4 * paths);
-}
 
 // The wave loop of one frame (or, with `batch`, of all jobs of a batch) on
 // scratch R (at least P.cap paths).  With `events` false no CUDA event is
@@ -1374,8 +1323,11 @@ void run_waves(SceneHost& s, RenderScratch& R, const FramePlan& P, const omv_cam
             const NvtxRange light_range("omv light subpaths");
             WaveArgs AL = A;
             cudaStream_t light_st = st;
-            if (beside && s.light_queue && A.wave_n <= kBesideLightPaths) {  // beside the camera rays and their first hits
-                light_queues(AL.R, s.light_queue, s.light_queue_cap);
+            const int64_t own = beside ? light_queue_first(A.wave_n, R.queue_cap) : 0;
+            if (own > 0) {  // queues of their own: beside the camera rays and their first hits
+                AL.R.rq[0] += 2 * own;
+                AL.R.rq[1] += 2 * own;
+                AL.R.hits += own;
                 light_st = s.side.stream;
                 fork();
             }
@@ -1539,8 +1491,15 @@ static void ensure_scratch(SceneHost& s, int64_t wave_cap, int light_slots, int 
         }
     }
     void* base = nullptr;
-    OMV_CUDA(cudaMalloc(&base, scratch_layout(wave_cap, light_slots, shadow_slots).bytes));
-    carve_scratch(R, base, wave_cap, light_slots, shadow_slots);
+    int64_t queue_cap = queue_entries(wave_cap, s.num_lights > 0);
+    if (queue_cap > wave_cap &&
+        cudaMalloc(&base, scratch_layout(wave_cap, queue_cap, light_slots, shadow_slots).bytes) != cudaSuccess) {
+        (void)cudaGetLastError();  // the light subpaths go without queues of their own
+        base = nullptr;
+        queue_cap = wave_cap;
+    }
+    if (!base) OMV_CUDA(cudaMalloc(&base, scratch_layout(wave_cap, queue_cap, light_slots, shadow_slots).bytes));
+    carve_scratch(R, base, wave_cap, queue_cap, light_slots, shadow_slots);
 }
 
 // Room for n tile lists; false (no tiles) when the memory is not there.
@@ -1560,31 +1519,6 @@ static bool ensure_tiles(SceneHost& s, int64_t n)
     }
     s.tiles_cap = n;
     return true;
-}
-
-// Queues of the light subpaths' own (two ray queues and the hits), so that they
-// can run beside the camera rays; a frame goes without when the memory is not
-// there.
-static void ensure_light_queue(SceneHost& s, int64_t paths)
-{
-    if (s.light_queue_cap >= paths) return;
-    if (s.light_queue) {
-        OMV_CUDA(cudaDeviceSynchronize());  // the last frame may be on any stream
-        cudaFree(s.light_queue);
-        s.light_queue = nullptr;
-        s.light_queue_cap = 0;
-        if (s.batch_graph) {  // it refers to the old queues
-            cudaGraphExecDestroy(s.batch_graph);
-            s.batch_graph = nullptr;
-            s.batch_key.clear();
-        }
-    }
-    if (cudaMalloc(&s.light_queue, 80 * (size_t)paths) != cudaSuccess) {
-        (void)cudaGetLastError();
-        s.light_queue = nullptr;
-        return;
-    }
-    s.light_queue_cap = paths;
 }
 
 // Default wave scratch: up to 32 GiB (and at most half of the free device
@@ -1608,7 +1542,6 @@ void render_frame(SceneHost& s, const omv_camera& cam, const omv_params& p, doub
         P.cap = std::max<int64_t>(1, std::min<int64_t>({fit, std::max<int64_t>(P.total, 1), (int64_t)0x7FFFFFFF}));
     }
     ensure_scratch(s, P.cap, P.light_slots, P.shadow_slots);
-    if (P.lights && P.cap <= kBesideLightPaths) ensure_light_queue(s, P.cap);
     if (P.total >= kTileMinPaths && p.camera_bounces > 0) {
         P.tiles = tile_grid(cam, p.samples_per_pixel);
         const int64_t n = tile_count(P.tiles, cam);
@@ -1728,7 +1661,6 @@ void render_batch(SceneHost& s, int n, const omv_job* jobs, const omv_params& p,
     const FramePlan P = batch_frame_plan(s, B, p, s.batch_wave_paths);
     if (mis_on(s, p)) ensure_env_sampler(s);  // allocates: never inside a graph capture
     ensure_scratch(s, P.cap, P.light_slots, P.shadow_slots);
-    if (P.lights && P.cap <= kBesideLightPaths) ensure_light_queue(s, P.cap);
     upload_jobs(s, B, st);
     const BatchPlan plan{s.d_jobs, &B.jobs, B.min_spp};
     omv_camera cam0 = B.jobs[0].cam;
@@ -1893,7 +1825,7 @@ int64_t static_wave_limit(int light_slots, int shadow_slots)
     const size_t per_path = path_scratch_bytes(light_slots, shadow_slots);
     const size_t fixed = 48 + kMaxCounters * 4 + 16 * 8 + 14 * 256;
     int64_t cap = (int64_t)((OMV_STATIC_SCRATCH_BYTES - fixed) / per_path) & ~(int64_t)31;
-    while (cap > 0 && scratch_layout(cap, light_slots, shadow_slots).bytes > OMV_STATIC_SCRATCH_BYTES) cap -= 32;
+    while (cap > 0 && scratch_layout(cap, cap, light_slots, shadow_slots).bytes > OMV_STATIC_SCRATCH_BYTES) cap -= 32;
     return cap;
 }
 
@@ -1907,7 +1839,7 @@ void render_frame_static(SceneHost& s, const omv_camera& cam, const omv_params& 
     FramePlan P = plan_frame(s, cam, p, 1);
     const int64_t limit = static_wave_limit(P.light_slots, P.shadow_slots);
     if (p.wave_paths > 0) {
-        const size_t need = scratch_layout(P.cap, P.light_slots, P.shadow_slots).bytes;
+        const size_t need = scratch_layout(P.cap, P.cap, P.light_slots, P.shadow_slots).bytes;
         if (need > OMV_STATIC_SCRATCH_BYTES)
             throw ArgError("wave_paths " + std::to_string(p.wave_paths) + " needs " + std::to_string(need) +
                            " bytes of scratch; the static scratch holds " +
@@ -1917,7 +1849,7 @@ void render_frame_static(SceneHost& s, const omv_camera& cam, const omv_params& 
         P.cap = std::min<int64_t>(limit, std::max<int64_t>(P.total, 1));
     }
     RenderScratch R;
-    carve_scratch(R, static_scratch_address(), P.cap, P.light_slots, P.shadow_slots);
+    carve_scratch(R, static_scratch_address(), P.cap, P.cap, P.light_slots, P.shadow_slots);
     run_waves(s, R, P, cam, p, d_sum, d_sumsq, d_count, st, nullptr, false, false);
 }
 

@@ -335,7 +335,6 @@ SceneHost::~SceneHost()
     if (scratch.base) cudaFree(scratch.base);
     if (adj_scratch) cudaFree(adj_scratch);
     if (tiles) cudaFree(tiles);
-    if (light_queue) cudaFree(light_queue);
     if (adj_done) cudaEventDestroy(adj_done);
     if (mat_sets) cudaFree(mat_sets);
     if (d_jobs) cudaFree(d_jobs);

@@ -13,6 +13,7 @@
 
 #include "../../include/omv.h"
 #include "omv_types.h"
+#include "wave_layout.h"
 
 // A failed call throws; the runtime's non-sticky error state is cleared so
 // that the next call on the handle starts clean (an allocation that does not
@@ -43,6 +44,7 @@ struct ArgError : std::runtime_error {
 // reusable per-scene device work space of the wavefront renderer
 struct RenderScratch {
     int64_t wave_cap = 0;
+    int64_t queue_cap = 0;  // entries of rq and hits (wave_layout.h)
     int light_slots = 0;
     int shadow_slots = 0;
     void* base = nullptr;  // one allocation, carved into the arrays below
@@ -54,15 +56,13 @@ struct RenderScratch {
     uint32_t* lmeta = nullptr;   // light index | (light vertex count << 16)
     float4* lv_pos = nullptr;    // [light_slots][wave_cap]
     float4* lv_rad = nullptr;    // [light_slots][wave_cap]
-    float4* rq[2] = {nullptr, nullptr};  // ray queues: 2 float4 per entry
-    uint4* hits = nullptr;       // per queue entry
+    float4* rq[2] = {nullptr, nullptr};  // [queue_cap] ray queues: 2 float4 per entry
+    uint4* hits = nullptr;       // [queue_cap] per queue entry
     uint32_t* path_job = nullptr;  // batch: job of each path
     float4* sq = nullptr;        // shadow queue: 3 float4 per entry
     uint32_t* ctr = nullptr;     // per-wave queue and work counters
     unsigned long long* stats = nullptr;  // cumulative ray counters
 };
-
-constexpr int kMaxCounters = 512;
 
 // Tiles of a frame: 2^lx x 2^ly pixels each (beam.cuh).
 struct TileGrid {
@@ -142,8 +142,6 @@ struct SceneHost {
     int64_t batch_wave_paths = 0;            // autotuned wave size for batches (0: automatic)
     int batch_shade_threads = 0;             // autotuned threads per shading block for batches (0: 256)
     std::vector<ScenePart> parts;            // the scenes of a group (one for a single scene)
-    void* light_queue = nullptr;             // the light subpaths' own queues (small frames)
-    int64_t light_queue_cap = 0;
     TileList* tiles = nullptr;               // start nodes of the first camera bounce (beam.cuh)
     int64_t tiles_cap = 0;
     std::mutex adj_mutex;                    // one adjoint call at a time enqueues
