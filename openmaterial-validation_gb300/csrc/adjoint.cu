@@ -999,6 +999,16 @@ void run_adjoint(SceneHost& s, std::vector<AdjJob>& jobs, const omv_params& p, c
     const int connect_grid = resident_grid(k_adj_connect, kAdjThreads, smem, s.num_sms);
     const int back_grid = resident_grid(k_adj_camera_back, kAdjThreads, smem, s.num_sms);
     const int lback_grid = resident_grid(k_adj_light_back, kAdjThreads, smem, s.num_sms);
+    // beside the main stream: the light subpaths beside the camera rays' first
+    // hits, then each bounce's connections beside the next bounce's hits
+    const SceneHost::Side* beside = lights ? side_of(s.adj_side, st) : nullptr;
+    const cudaStream_t side = beside ? beside->stream : st;
+    auto fork = [&] {
+        if (beside) fork_side(*beside, st);
+    };
+    auto join = [&] {
+        if (beside) join_side(*beside, st);
+    };
     for (int64_t wb = 0; wb < total; wb += ws.cap) {
         A.wave_base = wb;
         A.wave_n = (int32_t)std::min<int64_t>(ws.cap, total - wb);
@@ -1006,11 +1016,8 @@ void run_adjoint(SceneHost& s, std::vector<AdjJob>& jobs, const omv_params& p, c
         uint32_t* work = A.ctr + kAdjCtrWork;
         const unsigned gen = blocks_for(A.wave_n, kShadeThreads);
         if (A.path_job) k_adj_path_jobs<<<gen, kShadeThreads, 0, st>>>(A);
-        // beside the main stream: the light subpaths beside the camera rays' first
-        // hits, then each bounce's connections beside the next bounce's hits
-        const cudaStream_t side = lights ? s.adj_side.stream : st;
         if (lights) {
-            fork_side(s.adj_side, st);
+            fork();
             k_adj_light_gen<<<gen, kShadeThreads, 0, side>>>(A);
             for (int b = 1; b <= L; ++b) {
                 const size_t off = (size_t)(b - 1) * A.cap;
@@ -1024,12 +1031,12 @@ void run_adjoint(SceneHost& s, std::vector<AdjJob>& jobs, const omv_params& p, c
             const size_t off = (size_t)(b - 1) * A.cap;
             k_adj_extend<<<trace_grid, kTraceThreads, 0, st>>>(A, A.crq + 2 * off, A.chit + off,
                                                                A.ctr + kAdjCtrCam + b - 1, work++);
-            if (lights) join_side(s.adj_side, st);
+            join();
             k_adj_camera<<<camera_grid, kShadeThreads, 0, st>>>(A, b);
             if (lights) {
                 uint32_t* seen = A.ctr + kAdjCtrSeen + b - 1;
                 const uint32_t* count = A.ctr + kAdjCtrConn + b - 1;
-                fork_side(s.adj_side, st);
+                fork();
                 if (masked)
                     k_adj_shadow<true><<<trace_grid, kTraceThreads, 0, side>>>(A, count, seen, work++);
                 else
@@ -1037,7 +1044,7 @@ void run_adjoint(SceneHost& s, std::vector<AdjJob>& jobs, const omv_params& p, c
                 k_adj_connect<<<connect_grid, kAdjThreads, smem, side>>>(A, b);
             }
         }
-        if (lights) join_side(s.adj_side, st);
+        join();
         for (int b = B; b >= 1; --b) k_adj_camera_back<<<back_grid, kAdjThreads, smem, st>>>(A, b);
         if (lights)
             for (int b = L; b >= 1; --b) k_adj_light_back<<<lback_grid, kAdjThreads, smem, st>>>(A, b);

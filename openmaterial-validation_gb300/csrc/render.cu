@@ -1277,16 +1277,17 @@ void run_waves(SceneHost& s, RenderScratch& R, const FramePlan& P, const omv_cam
     // other's ends (a 64x64x1 point-light frame 507 -> 403 us, 256x256x16 1075 ->
     // 996, 1920x1080x64 39.15 -> 38.94 ms).  Kernels that are timed one by one run
     // alone.
-    const bool beside = overlap && !time_kernels && (lights || mis);
-    const cudaStream_t shadow_st = beside ? s.side.stream : st;
+    const SceneHost::Side* side = overlap && !time_kernels && (lights || mis) ? side_of(s.side, st) : nullptr;
+    const bool beside = side != nullptr;
+    const cudaStream_t shadow_st = beside ? side->stream : st;
     bool forked = false;
     auto fork = [&] {
         if (!beside) return;
-        fork_side(s.side, st);
+        fork_side(*side, st);
         forked = true;
     };
     auto join = [&] {
-        if (forked) join_side(s.side, st);
+        if (forked) join_side(*side, st);
         forked = false;
     };
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -1328,7 +1329,7 @@ void run_waves(SceneHost& s, RenderScratch& R, const FramePlan& P, const omv_cam
                 AL.R.rq[0] += 2 * own;
                 AL.R.rq[1] += 2 * own;
                 AL.R.hits += own;
-                light_st = s.side.stream;
+                light_st = side->stream;
                 fork();
             }
             k_light_gen<<<grid_for(A.wave_n, sth), sth, 0, light_st>>>(AL);

@@ -325,12 +325,52 @@ const float kRgbWl[3] = {6.50000004e-07f, 5.10000007e-07f, 4.40000008e-07f};
 
 }  // namespace
 
+// the capture that a stream takes part in (false: none; also for a legacy stream
+// that another thread's capture forbids to ask)
+static bool capture_of(cudaStream_t st, unsigned long long& id)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamGetCaptureInfo(st, &status, &id) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return status != cudaStreamCaptureStatusNone;
+}
+
+void SceneHost::Side::make()
+{
+    if (!fork) OMV_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+    if (!join) OMV_CUDA(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
+    if (!stream) OMV_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+}
+
+// While it lives, this thread may make calls that an open capture forbids (they
+// take no part in it).
+struct OutsideCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    OutsideCapture() { OMV_CUDA(cudaThreadExchangeStreamCaptureMode(&mode)); }
+    ~OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    OutsideCapture(const OutsideCapture&) = delete;
+    OutsideCapture& operator=(const OutsideCapture&) = delete;
+};
+
+const SceneHost::Side* side_of(SceneHost::Side (&sides)[2], cudaStream_t st)
+{
+    unsigned long long id = 0, other = 0;
+    if (!capture_of(st, id)) return &sides[0];
+    if (!sides[1].stream) {
+        const OutsideCapture outside;
+        sides[1].make();
+    }
+    return !capture_of(sides[1].stream, other) || other == id ? &sides[1] : nullptr;
+}
+
 SceneHost::~SceneHost()
 {
     if (device >= 0) cudaSetDevice(device);
     if (stream) cudaStreamSynchronize(stream);
-    if (side.stream) cudaStreamSynchronize(side.stream);
-    if (adj_side.stream) cudaStreamSynchronize(adj_side.stream);
+    for (const Side& x : {side[0], side[1], adj_side[0], adj_side[1]})
+        if (x.stream) cudaStreamSynchronize(x.stream);
     for (void* p : allocs) cudaFree(p);
     if (scratch.base) cudaFree(scratch.base);
     if (adj_scratch) cudaFree(adj_scratch);
@@ -339,7 +379,7 @@ SceneHost::~SceneHost()
     if (mat_sets) cudaFree(mat_sets);
     if (d_jobs) cudaFree(d_jobs);
     if (batch_graph) cudaGraphExecDestroy(batch_graph);
-    for (const Side& x : {side, adj_side}) {
+    for (const Side& x : {side[0], side[1], adj_side[0], adj_side[1]}) {
         if (x.fork) cudaEventDestroy(x.fork);
         if (x.join) cudaEventDestroy(x.join);
         if (x.stream) cudaStreamDestroy(x.stream);
@@ -571,11 +611,8 @@ SceneHost* scene_create(const omv_scene_desc& d, int device, const std::vector<i
     std::unique_ptr<SceneHost> s(new SceneHost);
     s->device = device;
     OMV_CUDA(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
-    for (SceneHost::Side* x : {&s->side, &s->adj_side}) {
-        OMV_CUDA(cudaStreamCreateWithFlags(&x->stream, cudaStreamNonBlocking));
-        OMV_CUDA(cudaEventCreateWithFlags(&x->fork, cudaEventDisableTiming));
-        OMV_CUDA(cudaEventCreateWithFlags(&x->join, cudaEventDisableTiming));
-    }
+    s->side[0].make();
+    s->adj_side[0].make();
     OMV_CUDA(cudaDeviceGetAttribute(&s->num_sms, cudaDevAttrMultiProcessorCount, device));
 
     // ---- materials (+ the missing material, RenderScene.cpp:62-68)

@@ -132,11 +132,13 @@ struct SceneHost {
     DevJob* d_jobs = nullptr;                // batch job table
     size_t jobs_cap = 0;
     cudaGraphExec_t batch_graph = nullptr;   // captured batch render, replayed for an identical job list
-    // work beside a call's main stream: a frame's (or batch's), an adjoint's
+    // work beside a call's main stream: a frame's (or batch's), an adjoint's; the
+    // second of each for calls that are captured into a graph (side_of)
     struct Side {
         cudaStream_t stream = nullptr;
         cudaEvent_t fork = nullptr, join = nullptr;
-    } side, adj_side;
+        void make();
+    } side[2], adj_side[2];
     cudaEvent_t fork_ev = nullptr, join_ev = nullptr;  // order `stream` after / before a caller's default stream
     std::vector<unsigned char> batch_key;    // what batch_graph was captured for
     int64_t batch_wave_paths = 0;            // autotuned wave size for batches (0: automatic)
@@ -160,6 +162,11 @@ struct SceneHost {
     }
 };
 
+// The side stream that a call on `st` may fork.  A stream that is forked from a
+// captured one belongs to that capture until it ends, so direct calls and
+// captured ones have a side each, and a second capture that is open at the same time has
+// none (null): its work runs in line.
+const SceneHost::Side* side_of(SceneHost::Side (&sides)[2], cudaStream_t st);
 // orders the side stream after what `st` holds so far, and `st` after the side's
 inline void fork_side(const SceneHost::Side& x, cudaStream_t st)
 {

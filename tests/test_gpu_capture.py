@@ -1,0 +1,174 @@
+"""Frames and gradients captured into CUDA graphs, in every capture mode, while
+other calls on the same handle go on: a captured call neither needs memory that
+a capture may not allocate, nor shares streams or buffers with calls outside
+it.  Films of lit scenes agree up to the order of the FP32 additions to a path's
+radiance (5e-6), gradients up to the order of their sums (1e-4, as in
+test_gpu_adjoint_waves.py)."""
+import ctypes as C
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+MODES = {"global": 0, "thread_local": 1, "relaxed": 2}
+
+
+@pytest.fixture(scope="module")
+def torch(gpu):
+    return pytest.importorskip("torch")
+
+
+class Graph:
+    """A graph captured from a stream, and its instances (driver API)."""
+
+    def __init__(self, torch, mode):
+        self.cu = C.CDLL("libcuda.so.1")
+        self.stream = torch.cuda.Stream()
+        self.s = C.c_void_p(self.stream.cuda_stream)
+        self.graph, self.execs = C.c_void_p(), []
+        self.mode, self.capturing = MODES[mode], False
+
+    def _ok(self, r):
+        assert r == 0, f"CUDA driver error {r}"
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *error):
+        if self.capturing:
+            self.cu.cuStreamEndCapture(self.s, C.byref(self.graph))
+            self.capturing = False
+        self.destroy()
+
+    def begin(self):
+        self._ok(self.cu.cuStreamBeginCapture_v2(self.s, self.mode))
+        self.capturing = True
+
+    def end(self):
+        self.capturing = False
+        self._ok(self.cu.cuStreamEndCapture(self.s, C.byref(self.graph)))
+
+    def instantiate(self):
+        e = C.c_void_p()
+        self._ok(self.cu.cuGraphInstantiateWithFlags(C.byref(e), self.graph, C.c_uint64(0)))
+        self.execs.append(e)
+        return e
+
+    def launch(self, e):
+        self._ok(self.cu.cuGraphLaunch(e, self.s))
+
+    def destroy(self):
+        for e in self.execs:
+            self._ok(self.cu.cuGraphExecDestroy(e))
+        if self.graph:
+            self._ok(self.cu.cuGraphDestroy(self.graph))
+        self.execs, self.graph = [], C.c_void_p()
+
+
+class Frame:
+    """omv_render_device of a scene with point lights into a film of its own per call."""
+
+    rtol = 5e-6
+
+    def __init__(self, gpu, scenes, torch, w=96, h=64, spp=8):
+        self.gpu, self.torch = gpu, torch
+        self.sc = scenes.scene_c1(w, h, spp)
+        self.rs = gpu.RenderScene(self.sc)
+        self.size(w, h, spp)
+
+    def size(self, w, h, spp):
+        cam = self.gpu.PinholeCamera.from_spec(self.sc.camera)
+        cam.width, cam.height = w, h
+        cam.adjust_to_resolution()
+        cam.set_y_fov(45.0)
+        self.cam = cam.to_c()
+        self.prm = self.gpu.RendererParameters.for_scene(self.sc, samplesPerPixel=spp, seed=5).to_c()
+
+    def buffers(self):
+        return (self.torch.zeros((self.cam.height, self.cam.width, 3), dtype=self.torch.float64, device="cuda"),
+                self.torch.zeros((self.cam.height, self.cam.width), dtype=self.torch.int32, device="cuda"))
+
+    def call(self, stream, out):
+        self.gpu.check(self.gpu.lib().omv_render_device(self.rs.handle, C.byref(self.cam), C.byref(self.prm),
+                                                        C.c_void_p(out[0].data_ptr()), None, C.c_void_p(out[1].data_ptr()),
+                                                        C.c_void_p(stream.cuda_stream), None))
+
+    def check(self, out, want, times):
+        assert int(out[1].min()) == int(out[1].max()) == times * self.prm.samples_per_pixel
+        assert float((out[0] - times * want[0]).abs().max()) <= self.rtol * times * float(want[0].abs().max())
+
+
+class Gradient:
+    """omv_adjoint of a scene with point lights."""
+
+    rtol = 1e-4
+
+    def __init__(self, gpu, scenes, torch, side=48, spp=32):
+        self.gpu, self.torch = gpu, torch
+        self.sc = scenes.scene_materials(side, side, 1, tris=4_000, n_materials=4, bounces=4, seed=3)
+        self.rs = gpu.RenderScene(self.sc)
+        self.cam = gpu.PinholeCamera.from_spec(self.sc.camera).to_c()
+        self.prm = gpu.RendererParameters.for_scene(self.sc, samplesPerPixel=spp, seed=11).to_c()
+        self.adj = torch.rand((side, side, 3), device="cuda", generator=torch.Generator(device="cuda").manual_seed(5)) - 0.3
+
+    def buffers(self):
+        return (self.torch.zeros((len(self.sc.materials), 11), device="cuda"),)
+
+    def call(self, stream, out):
+        self.gpu.check(self.gpu.lib().omv_adjoint(self.rs.handle, C.byref(self.cam), C.byref(self.prm),
+                                                  C.c_void_p(self.adj.data_ptr()), C.c_void_p(out[0].data_ptr()),
+                                                  C.c_void_p(stream.cuda_stream)))
+
+    def check(self, out, want, times):
+        scale = float(want[0].abs().max())
+        assert scale > 0
+        assert float((out[0] - times * want[0]).abs().max()) <= self.rtol * times * scale
+
+
+def _want(torch, work):
+    out = work.buffers()
+    work.call(torch.cuda.current_stream(), out)
+    torch.cuda.synchronize()
+    return out
+
+
+@pytest.mark.parametrize("work", [Frame, Gradient])
+def test_direct_calls_while_a_stream_is_captured(gpu, scenes, torch, work):
+    """Another stream's calls before the capture ends run at once and leave it alone."""
+    w = work(gpu, scenes, torch)
+    want, direct, inside = _want(torch, w), w.buffers(), w.buffers()
+    other = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with Graph(torch, "relaxed") as g:
+        g.begin()
+        w.call(g.stream, inside)
+        w.call(other, direct)
+        other.synchronize()
+        w.call(g.stream, inside)  # and on in the capture
+        w.call(other, direct)
+        other.synchronize()
+        g.end()
+        w.check(direct, want, 2)
+        g.launch(g.instantiate())
+        torch.cuda.synchronize()
+        w.check(inside, want, 2)
+
+
+@pytest.mark.parametrize("work", [Frame, Gradient])
+def test_two_streams_captured_at_once(gpu, scenes, torch, work):
+    w = work(gpu, scenes, torch)
+    want, a, b = _want(torch, w), w.buffers(), w.buffers()
+    torch.cuda.synchronize()
+    with Graph(torch, "relaxed") as ga, Graph(torch, "relaxed") as gb:
+        ga.begin()
+        w.call(ga.stream, a)
+        gb.begin()
+        w.call(gb.stream, b)
+        w.call(ga.stream, a)
+        ga.end()
+        w.call(gb.stream, b)
+        gb.end()
+        for g in (ga, gb):
+            g.launch(g.instantiate())
+            torch.cuda.synchronize()
+        w.check(a, want, 2)
+        w.check(b, want, 2)
