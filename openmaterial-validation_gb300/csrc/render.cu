@@ -1117,7 +1117,8 @@ struct FramePlan {
     int light_slots, shadow_slots;
     bool lights;
     TileGrid tiles{};        // of the frame's camera
-    uint32_t num_tiles = 0;  // 0: no tile lists
+    uint32_t num_tiles = 0;
+    TileList* tile_lists = nullptr;  // null: none
 };
 
 // Tiles of a camera: about kTileRays rays each (1024: the same within 1%), so
@@ -1243,7 +1244,7 @@ void run_waves(SceneHost& s, RenderScratch& R, const FramePlan& P, const omv_cam
     A.path_job = R.path_job;
     A.tiles = P.tiles;
     A.num_tiles = P.num_tiles;
-    A.tile_lists = P.num_tiles ? s.tiles : nullptr;
+    A.tile_lists = P.tile_lists;
     int occ_t = 0, occ_s = 0;
     OMV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_t, k_extend, kTraceThreads, 0));
     // threads per block of the shading-side kernels: 256, or a batch's
@@ -1503,23 +1504,18 @@ static void ensure_scratch(SceneHost& s, int64_t wave_cap, int light_slots, int 
     carve_scratch(R, base, wave_cap, queue_cap, light_slots, shadow_slots);
 }
 
-// Room for n tile lists; false (no tiles) when the memory is not there.
-static bool ensure_tiles(SceneHost& s, int64_t n)
+// Room for the n tile lists of a frame on `st`, in `block` or, for a captured
+// frame, its graph's.  Null (no tiles) when the memory is not there.
+static TileList* tile_room(SceneHost& s, int64_t n, cudaStream_t st, WorkBlock& block)
 {
-    if (s.tiles_cap >= n) return true;
-    if (s.tiles) {
-        OMV_CUDA(cudaDeviceSynchronize());  // the last frame may be on any stream
-        cudaFree(s.tiles);
-        s.tiles = nullptr;
-        s.tiles_cap = 0;
+    const size_t bytes = sizeof(TileList) * (size_t)n;
+    try {
+        if (is_captured(st)) return static_cast<TileList*>(graph_block(s, st, bytes));
+        block.take(work_pool(s), bytes, bytes, st);
+        return static_cast<TileList*>(block.p);
+    } catch (const DeviceOutOfMemory&) {
+        return nullptr;
     }
-    if (cudaMalloc(&s.tiles, sizeof(TileList) * (size_t)n) != cudaSuccess) {
-        (void)cudaGetLastError();
-        s.tiles = nullptr;
-        return false;
-    }
-    s.tiles_cap = n;
-    return true;
 }
 
 // Default wave scratch: up to 32 GiB (and at most half of the free device
@@ -1543,10 +1539,14 @@ void render_frame(SceneHost& s, const omv_camera& cam, const omv_params& p, doub
         P.cap = std::max<int64_t>(1, std::min<int64_t>({fit, std::max<int64_t>(P.total, 1), (int64_t)0x7FFFFFFF}));
     }
     ensure_scratch(s, P.cap, P.light_slots, P.shadow_slots);
+    WorkBlock tiles;
     if (P.total >= kTileMinPaths && p.camera_bounces > 0) {
         P.tiles = tile_grid(cam, p.samples_per_pixel);
         const int64_t n = tile_count(P.tiles, cam);
-        if (n <= kTileMaxCount && ensure_tiles(s, n)) P.num_tiles = (uint32_t)n;
+        if (n <= kTileMaxCount) {
+            P.tile_lists = tile_room(s, n, st, tiles);
+            P.num_tiles = (uint32_t)n;
+        }
     }
     run_waves(s, s.scratch, P, cam, p, d_sum, d_sumsq, d_count, st, stats, true, true, nullptr, while_running);
 }

@@ -12,7 +12,9 @@
 #include <cmath>
 #include <cstring>
 #include <exception>
+#include <map>
 #include <memory>
+#include <mutex>
 #include <system_error>
 #include <thread>
 #include <vector>
@@ -327,14 +329,20 @@ const float kRgbWl[3] = {6.50000004e-07f, 5.10000007e-07f, 4.40000008e-07f};
 
 // the capture that a stream takes part in (false: none; also for a legacy stream
 // that another thread's capture forbids to ask)
-static bool capture_of(cudaStream_t st, unsigned long long& id)
+static bool capture_of(cudaStream_t st, unsigned long long& id, cudaGraph_t* graph = nullptr)
 {
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-    if (cudaStreamGetCaptureInfo(st, &status, &id) != cudaSuccess) {
+    if (cudaStreamGetCaptureInfo(st, &status, &id, graph) != cudaSuccess) {
         (void)cudaGetLastError();
         return false;
     }
     return status != cudaStreamCaptureStatusNone;
+}
+
+bool is_captured(cudaStream_t st)
+{
+    unsigned long long id = 0;
+    return capture_of(st, id);
 }
 
 void SceneHost::Side::make()
@@ -365,6 +373,133 @@ const SceneHost::Side* side_of(SceneHost::Side (&sides)[2], cudaStream_t st)
     return !capture_of(sides[1].stream, other) || other == id ? &sides[1] : nullptr;
 }
 
+WorkPool::WorkPool(int device)
+{
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.handleTypes = cudaMemHandleTypeNone;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    OMV_CUDA(cudaMemPoolCreate(&pool_, &props));
+}
+WorkPool::~WorkPool() { cudaMemPoolDestroy(pool_); }
+
+void* WorkPool::take(size_t bytes, size_t keep, cudaStream_t st)
+{
+    {
+        const std::lock_guard<std::mutex> lock(mutex_);
+        if (keep > keep_) {
+            uint64_t v = keep;
+            OMV_CUDA(cudaMemPoolSetAttribute(pool_, cudaMemPoolAttrReleaseThreshold, &v));
+            keep_ = keep;
+        }
+    }
+    void* p = nullptr;
+    cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, pool_, st);
+    if (e == cudaErrorMemoryAllocation) {  // idle blocks of other sizes go first
+        (void)cudaGetLastError();
+        cudaMemPoolTrimTo(pool_, 0);
+        e = cudaMallocFromPoolAsync(&p, bytes, pool_, st);
+    }
+    OMV_CUDA(e);
+    return p;
+}
+
+// a number of the current context (a device reset makes a new one)
+static unsigned long long context_id()
+{
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+    unsigned long long id = 0;
+    if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &fn, 12000, cudaEnableDefault, &found) == cudaSuccess &&
+        found == cudaDriverEntryPointSuccess)
+        reinterpret_cast<int (*)(void*, unsigned long long*)>(fn)(nullptr, &id);
+    else
+        (void)cudaGetLastError();
+    return id;
+}
+
+WorkPool& work_pool(SceneHost& s)
+{
+    std::call_once(s.pool_once, [&] {
+        static std::mutex mutex;
+        static auto& pools = *new std::map<std::pair<int, unsigned long long>, std::weak_ptr<WorkPool>>;
+        const OutsideCapture outside;
+        const std::lock_guard<std::mutex> lock(mutex);
+        std::weak_ptr<WorkPool>& known = pools[{s.device, context_id()}];
+        s.pool = known.lock();
+        if (!s.pool) {
+            s.pool = std::make_shared<WorkPool>(s.device);
+            known = s.pool;
+        }
+    });
+    return *s.pool;
+}
+
+namespace {
+
+// a graph's claim on a block; the callback runs when the last of the graph and its
+// instances is gone, on a thread that may make no CUDA call
+struct GraphClaim {
+    std::shared_ptr<GraphMemory> memory;
+    void* p;
+};
+void CUDART_CB end_claim(void* arg)
+{
+    const std::unique_ptr<GraphClaim> claim(static_cast<GraphClaim*>(arg));
+    const std::lock_guard<std::mutex> lock(claim->memory->mutex);
+    for (GraphMemory::Block& b : claim->memory->blocks)
+        if (b.p == claim->p) b.used = false;
+}
+
+// an unclaimed block of at least `bytes`, or a new one in place of all that no graph claims
+void* take_block(GraphMemory& m, size_t bytes)
+{
+    const std::lock_guard<std::mutex> lock(m.mutex);
+    GraphMemory::Block* best = nullptr;
+    for (GraphMemory::Block& b : m.blocks)
+        if (!b.used && b.bytes >= bytes && (!best || b.bytes < best->bytes)) best = &b;
+    if (!best) {
+        size_t kept = 0;
+        for (const GraphMemory::Block& b : m.blocks) {
+            if (b.used)
+                m.blocks[kept++] = b;
+            else
+                cudaFree(b.p);
+        }
+        m.blocks.resize(kept);
+        m.blocks.reserve(kept + 1);
+        void* p = nullptr;
+        OMV_CUDA(cudaMalloc(&p, bytes));
+        m.blocks.push_back(GraphMemory::Block{p, bytes, false});
+        best = &m.blocks.back();
+    }
+    best->used = true;
+    return best->p;
+}
+
+}  // namespace
+
+void* graph_block(SceneHost& s, cudaStream_t st, size_t bytes)
+{
+    const OutsideCapture outside;
+    unsigned long long id = 0;
+    cudaGraph_t graph = nullptr;
+    if (!capture_of(st, id, &graph) || !graph) throw CudaError("the stream is not being captured");
+    std::unique_ptr<GraphClaim> claim(new GraphClaim{s.graph_memory, nullptr});
+    claim->p = take_block(*s.graph_memory, bytes);
+    void* const p = claim->p;
+    cudaUserObject_t object = nullptr;
+    const cudaError_t e = cudaUserObjectCreate(&object, claim.get(), end_claim, 1, cudaUserObjectNoDestructorSync);
+    if (e != cudaSuccess) end_claim(claim.release());
+    OMV_CUDA(e);
+    claim.release();
+    const cudaError_t r = cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove);
+    if (r != cudaSuccess) cudaUserObjectRelease(object, 1);
+    OMV_CUDA(r);
+    return p;
+}
+
 SceneHost::~SceneHost()
 {
     if (device >= 0) cudaSetDevice(device);
@@ -374,7 +509,11 @@ SceneHost::~SceneHost()
     for (void* p : allocs) cudaFree(p);
     if (scratch.base) cudaFree(scratch.base);
     if (adj_scratch) cudaFree(adj_scratch);
-    if (tiles) cudaFree(tiles);
+    {
+        const std::lock_guard<std::mutex> lock(graph_memory->mutex);
+        for (const GraphMemory::Block& b : graph_memory->blocks) cudaFree(b.p);
+        graph_memory->blocks.clear();
+    }
     if (adj_done) cudaEventDestroy(adj_done);
     if (mat_sets) cudaFree(mat_sets);
     if (d_jobs) cudaFree(d_jobs);

@@ -6,6 +6,7 @@
 
 #include <cstdint>
 #include <functional>
+#include <memory>
 #include <mutex>
 #include <stdexcept>
 #include <string>
@@ -69,7 +70,6 @@ struct TileGrid {
     int32_t lx, ly;
     uint32_t per_row;  // tiles in a row
 };
-struct TileList;
 
 // One job of a batch render (device copy): its camera, samples, seed and
 // material table, its film, and where its paths and pixels start in the
@@ -101,6 +101,58 @@ struct ScenePart {
     int32_t light_base = 0, light_count = 0;
     float light_max = 0.0f;
     int32_t mat_base = 0, mat_count = 0;  // without the shared missing material
+};
+
+// Stream-ordered device memory for what one call needs besides the wave scratch,
+// shared by all handles of a context: no handle keeps such memory of its own, a
+// call makes no allocation that an open capture forbids and waits for no other
+// stream.  It keeps as much as its calls have asked to find again (keep_ is the
+// largest of them) and goes back when the context's last handle is destroyed.
+class WorkPool {
+public:
+    explicit WorkPool(int device);
+    ~WorkPool();
+    WorkPool(const WorkPool&) = delete;
+    WorkPool& operator=(const WorkPool&) = delete;
+    // `bytes` for work on `st`; up to `keep` bytes stay in the pool afterwards
+    // (DeviceOutOfMemory when there is no room)
+    void* take(size_t bytes, size_t keep, cudaStream_t st);
+
+private:
+    cudaMemPool_t pool_ = nullptr;
+    std::mutex mutex_;
+    size_t keep_ = 0;
+};
+// a block of the pool, given back behind the stream's work
+struct WorkBlock {
+    cudaStream_t st = nullptr;
+    void* p = nullptr;
+    WorkBlock() = default;
+    ~WorkBlock()
+    {
+        if (p) cudaFreeAsync(p, st);
+    }
+    WorkBlock(const WorkBlock&) = delete;
+    WorkBlock& operator=(const WorkBlock&) = delete;
+    void take(WorkPool& pool, size_t bytes, size_t keep, cudaStream_t stream)
+    {
+        p = pool.take(bytes, keep, stream);
+        st = stream;
+    }
+};
+
+// Device memory of captured calls: a block belongs to the graph that a call was
+// captured into until the graph and its instances are gone, and then to the next
+// capture that it fits.  A replay may run beside any other call, so captured calls
+// use no buffer of the handle that another call may use or replace.
+struct GraphMemory {
+    struct Block {
+        void* p;
+        size_t bytes;
+        bool used;
+    };
+    std::mutex mutex;
+    std::vector<Block> blocks;
 };
 
 struct SceneHost {
@@ -144,8 +196,9 @@ struct SceneHost {
     int64_t batch_wave_paths = 0;            // autotuned wave size for batches (0: automatic)
     int batch_shade_threads = 0;             // autotuned threads per shading block for batches (0: 256)
     std::vector<ScenePart> parts;            // the scenes of a group (one for a single scene)
-    TileList* tiles = nullptr;               // start nodes of the first camera bounce (beam.cuh)
-    int64_t tiles_cap = 0;
+    std::once_flag pool_once;
+    std::shared_ptr<WorkPool> pool;          // work_pool
+    std::shared_ptr<GraphMemory> graph_memory = std::make_shared<GraphMemory>();
     std::mutex adj_mutex;                    // one adjoint call at a time enqueues
     void* adj_scratch = nullptr;             // records of an adjoint wave
     size_t adj_bytes = 0;
@@ -167,6 +220,13 @@ struct SceneHost {
 // captured ones have a side each, and a second capture that is open at the same time has
 // none (null): its work runs in line.
 const SceneHost::Side* side_of(SceneHost::Side (&sides)[2], cudaStream_t st);
+// the pool of the handle's context
+WorkPool& work_pool(SceneHost& s);
+// whether `st` is being captured into a graph
+bool is_captured(cudaStream_t st);
+// a block of at least `bytes` for the call that is being captured on `st`
+// (DeviceOutOfMemory when there is none)
+void* graph_block(SceneHost& s, cudaStream_t st, size_t bytes);
 // orders the side stream after what `st` holds so far, and `st` after the side's
 inline void fork_side(const SceneHost::Side& x, cudaStream_t st)
 {

@@ -172,3 +172,71 @@ def test_two_streams_captured_at_once(gpu, scenes, torch, work):
             torch.cuda.synchronize()
         w.check(a, want, 2)
         w.check(b, want, 2)
+
+
+# 2^22 paths each, so that one scratch serves all three: 8192 tiles of 512 pixels, 8192 and 131072
+MANY_TILES = [(2048, 2048, 1), (65536, 64, 1), (4194304, 1, 1)]
+
+
+@pytest.mark.parametrize("mode", MODES)
+def test_captured_frame_with_more_tiles_than_any_before(gpu, scenes, torch, mode):
+    w = Frame(gpu, scenes, torch, *MANY_TILES[0])
+    _want(torch, w)
+    w.size(*MANY_TILES[2])
+    out = w.buffers()
+    torch.cuda.synchronize()
+    with Graph(torch, mode) as g:
+        g.begin()
+        w.call(g.stream, out)
+        g.end()
+        e0, e1 = g.instantiate(), g.instantiate()
+        for e in (e0, e1):
+            g.launch(e)
+        torch.cuda.synchronize()
+        w.check(out, _want(torch, w), 2)
+
+
+def test_direct_frames_of_more_tiles_between_replays(gpu, scenes, torch):
+    """A captured frame's tile lists are its graph's: direct frames with more tiles, before the capture ends and between
+    replays, change nothing."""
+    w = Frame(gpu, scenes, torch, *MANY_TILES[0])
+    want, out = _want(torch, w), w.buffers()
+    other = torch.cuda.Stream()
+    w.size(*MANY_TILES[2])
+    more = w.buffers()
+    w.size(*MANY_TILES[0])
+    torch.cuda.synchronize()
+    with Graph(torch, "relaxed") as g:
+        g.begin()
+        w.call(g.stream, out)
+        w.size(*MANY_TILES[2])
+        w.call(other, more)
+        other.synchronize()
+        g.end()
+        e = g.instantiate()
+        for _ in range(2):
+            g.launch(e)
+            w.call(g.stream, more)
+        torch.cuda.synchronize()
+        w.check(more, _want(torch, w), 3)
+        w.size(*MANY_TILES[0])
+        w.check(out, want, 2)
+
+
+def test_captures_one_after_another_use_the_same_memory(gpu, scenes, torch):
+    """Blocks of graphs that are gone serve the next captures: 64 graphs of frames with 36 MB of tile lists each leave
+    less than three blocks behind."""
+    w = Frame(gpu, scenes, torch, *MANY_TILES[2])
+    out = w.buffers()
+    _want(torch, w)
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    for _ in range(64):
+        with Graph(torch, "thread_local") as g:
+            g.begin()
+            w.call(g.stream, out)
+            g.end()
+            g.launch(g.instantiate())
+            torch.cuda.synchronize()
+    assert free0 - torch.cuda.mem_get_info()[0] < 3 * 36 * 2**20
+    w.check(out, _want(torch, w), 64)
