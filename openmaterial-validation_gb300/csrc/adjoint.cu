@@ -843,35 +843,35 @@ constexpr int64_t kAdjMinCap = 1 << 14;  // tried at least, whatever memory is f
 
 // Where a wave's records live while its launches are in flight: the scene's own
 // block, used by one call after another (a call on another stream waits for
-// the last one's event), or, when the caller captures the stream into a graph,
-// memory that the graph allocates and frees.
+// the last one's event), or, when the caller captures the stream into a graph, a
+// block of that graph, used by one call of the capture and by one replay of any
+// instance after another (the graph waits for and records an external event).
 struct AdjWorkspace {
     SceneHost& s;
     cudaStream_t st;
-    bool captured;
+    GraphMemory::Block* captured = nullptr;
     void* base = nullptr;
     int64_t cap = 0;
     AdjWorkspace(SceneHost& s_, cudaStream_t st_, int64_t total, int njobs, int B, int L, bool lights)
-        : s(s_), st(st_), captured(false)
+        : s(s_), st(st_)
     {
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        // (a legacy-stream query while another thread captures is an error: not captured)
-        if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) (void)cudaGetLastError();
-        captured = cs == cudaStreamCaptureStatusActive;
+        const bool capturing = is_captured(st);
         auto need = [&](int64_t c) { return adj_layout(c, njobs, B, L, lights).bytes; };
         const size_t per = std::max<size_t>(1, (need(1 << 20) - need(0)) >> 20);
         const int64_t most = std::min<int64_t>(total, (int64_t)1 << 30);
         cap = std::max<int64_t>(1, std::min<int64_t>(most, (int64_t)(kAdjBudget / per)));
-        if (!captured && s.adj_scratch && s.adj_bytes >= need(cap)) {
+        if (!capturing && s.adj_scratch && s.adj_bytes >= need(cap)) {
             base = s.adj_scratch;
         } else {
+            const OutsideCapture outside;
             size_t free_b = 0, total_b = 0;
             OMV_CUDA(cudaMemGetInfo(&free_b, &total_b));
-            const size_t own = captured ? 0 : s.adj_bytes;
+            const size_t own = capturing ? 0 : s.adj_bytes;
             const int64_t fit = (int64_t)(std::min(kAdjBudget, (free_b + own) / 2) / per);
             cap = std::min(cap, std::max<int64_t>(std::min(most, kAdjMinCap), fit));
-            if (captured) {
-                OMV_CUDA(cudaMallocAsync(&base, need(cap), st));
+            if (capturing) {
+                captured = &graph_block(s, st, need(cap), GraphMemory::kRecords);
+                base = captured->p;
             } else if (s.adj_scratch && s.adj_bytes >= need(cap)) {
                 base = s.adj_scratch;
             } else {
@@ -886,7 +886,10 @@ struct AdjWorkspace {
                 s.adj_bytes = need(cap);
             }
         }
-        if (!captured) {
+        if (captured) {
+            if (!captured->fresh) OMV_CUDA(cudaStreamWaitEvent(st, captured->call, 0));
+            OMV_CUDA(cudaStreamWaitEvent(st, captured->instance, cudaEventWaitExternal));
+        } else {
             if (!s.adj_done)
                 OMV_CUDA(cudaEventCreateWithFlags(&s.adj_done, cudaEventDisableTiming));
             else
@@ -895,10 +898,12 @@ struct AdjWorkspace {
     }
     ~AdjWorkspace()
     {
-        if (captured)
-            cudaFreeAsync(base, st);
-        else
+        if (captured) {
+            cudaEventRecord(captured->call, st);
+            cudaEventRecordWithFlags(captured->instance, st, cudaEventRecordExternal);
+        } else {
             cudaEventRecord(s.adj_done, st);
+        }
     }
     AdjWorkspace(const AdjWorkspace&) = delete;
     AdjWorkspace& operator=(const AdjWorkspace&) = delete;

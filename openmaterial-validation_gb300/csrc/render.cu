@@ -1510,7 +1510,7 @@ static TileList* tile_room(SceneHost& s, int64_t n, cudaStream_t st, WorkBlock& 
 {
     const size_t bytes = sizeof(TileList) * (size_t)n;
     try {
-        if (is_captured(st)) return static_cast<TileList*>(graph_block(s, st, bytes));
+        if (is_captured(st)) return static_cast<TileList*>(graph_block(s, st, bytes, GraphMemory::kTiles).p);
         block.take(work_pool(s), bytes, bytes, st);
         return static_cast<TileList*>(block.p);
     } catch (const DeviceOutOfMemory&) {

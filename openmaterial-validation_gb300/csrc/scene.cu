@@ -352,16 +352,6 @@ void SceneHost::Side::make()
     if (!stream) OMV_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
 }
 
-// While it lives, this thread may make calls that an open capture forbids (they
-// take no part in it).
-struct OutsideCapture {
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    OutsideCapture() { OMV_CUDA(cudaThreadExchangeStreamCaptureMode(&mode)); }
-    ~OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-    OutsideCapture(const OutsideCapture&) = delete;
-    OutsideCapture& operator=(const OutsideCapture&) = delete;
-};
-
 const SceneHost::Side* side_of(SceneHost::Side (&sides)[2], cudaStream_t st)
 {
     unsigned long long id = 0, other = 0;
@@ -449,55 +439,80 @@ void CUDART_CB end_claim(void* arg)
     const std::unique_ptr<GraphClaim> claim(static_cast<GraphClaim*>(arg));
     const std::lock_guard<std::mutex> lock(claim->memory->mutex);
     for (GraphMemory::Block& b : claim->memory->blocks)
-        if (b.p == claim->p) b.used = false;
+        if (b.p == claim->p) {
+            b.used = false;
+            b.capture = 0;
+        }
+}
+
+void free_block(const GraphMemory::Block& b)
+{
+    cudaFree(b.p);
+    if (b.used) return;  // a graph still holds the events
+    if (b.call) cudaEventDestroy(b.call);
+    if (b.instance) cudaEventDestroy(b.instance);
 }
 
 // an unclaimed block of at least `bytes`, or a new one in place of all that no graph claims
-void* take_block(GraphMemory& m, size_t bytes)
+GraphMemory::Block& take_block(GraphMemory& m, size_t bytes, GraphMemory::Kind kind)
 {
-    const std::lock_guard<std::mutex> lock(m.mutex);
     GraphMemory::Block* best = nullptr;
     for (GraphMemory::Block& b : m.blocks)
-        if (!b.used && b.bytes >= bytes && (!best || b.bytes < best->bytes)) best = &b;
-    if (!best) {
-        size_t kept = 0;
-        for (const GraphMemory::Block& b : m.blocks) {
-            if (b.used)
-                m.blocks[kept++] = b;
-            else
-                cudaFree(b.p);
+        if (!b.used && b.kind == kind && b.bytes >= bytes && (!best || b.bytes < best->bytes)) best = &b;
+    if (best) return *best;
+    for (auto b = m.blocks.begin(); b != m.blocks.end();) {
+        if (!b->used) {
+            free_block(*b);
+            b = m.blocks.erase(b);
+        } else {
+            ++b;
         }
-        m.blocks.resize(kept);
-        m.blocks.reserve(kept + 1);
-        void* p = nullptr;
-        OMV_CUDA(cudaMalloc(&p, bytes));
-        m.blocks.push_back(GraphMemory::Block{p, bytes, false});
-        best = &m.blocks.back();
     }
-    best->used = true;
-    return best->p;
+    GraphMemory::Block b;
+    b.kind = kind;
+    b.bytes = bytes;
+    try {
+        if (kind == GraphMemory::kRecords) {
+            OMV_CUDA(cudaEventCreateWithFlags(&b.call, cudaEventDisableTiming));
+            OMV_CUDA(cudaEventCreateWithFlags(&b.instance, cudaEventDisableTiming));
+        }
+        OMV_CUDA(cudaMalloc(&b.p, bytes));
+        m.blocks.push_back(b);
+    } catch (...) {
+        free_block(b);
+        throw;
+    }
+    return m.blocks.back();
 }
 
 }  // namespace
 
-void* graph_block(SceneHost& s, cudaStream_t st, size_t bytes)
+GraphMemory::Block& graph_block(SceneHost& s, cudaStream_t st, size_t bytes, GraphMemory::Kind kind)
 {
     const OutsideCapture outside;
     unsigned long long id = 0;
     cudaGraph_t graph = nullptr;
     if (!capture_of(st, id, &graph) || !graph) throw CudaError("the stream is not being captured");
-    std::unique_ptr<GraphClaim> claim(new GraphClaim{s.graph_memory, nullptr});
-    claim->p = take_block(*s.graph_memory, bytes);
-    void* const p = claim->p;
+    GraphMemory& m = *s.graph_memory;
+    std::unique_lock<std::mutex> lock(m.mutex);
+    for (GraphMemory::Block& b : m.blocks)
+        if (b.used && b.capture == id && b.kind == kind && b.bytes >= bytes) {
+            b.fresh = false;
+            return b;
+        }
+    GraphMemory::Block& b = take_block(m, bytes, kind);
+    std::unique_ptr<GraphClaim> claim(new GraphClaim{s.graph_memory, b.p});
     cudaUserObject_t object = nullptr;
-    const cudaError_t e = cudaUserObjectCreate(&object, claim.get(), end_claim, 1, cudaUserObjectNoDestructorSync);
-    if (e != cudaSuccess) end_claim(claim.release());
-    OMV_CUDA(e);
+    OMV_CUDA(cudaUserObjectCreate(&object, claim.get(), end_claim, 1, cudaUserObjectNoDestructorSync));
     claim.release();
-    const cudaError_t r = cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove);
-    if (r != cudaSuccess) cudaUserObjectRelease(object, 1);
-    OMV_CUDA(r);
-    return p;
+    b.used = true;
+    b.capture = id;
+    b.fresh = true;
+    lock.unlock();
+    const cudaError_t e = cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove);
+    if (e != cudaSuccess) cudaUserObjectRelease(object, 1);  // ends the claim
+    OMV_CUDA(e);
+    return b;
 }
 
 SceneHost::~SceneHost()
@@ -511,7 +526,7 @@ SceneHost::~SceneHost()
     if (adj_scratch) cudaFree(adj_scratch);
     {
         const std::lock_guard<std::mutex> lock(graph_memory->mutex);
-        for (const GraphMemory::Block& b : graph_memory->blocks) cudaFree(b.p);
+        for (const GraphMemory::Block& b : graph_memory->blocks) free_block(b);
         graph_memory->blocks.clear();
     }
     if (adj_done) cudaEventDestroy(adj_done);

@@ -6,6 +6,7 @@
 
 #include <cstdint>
 #include <functional>
+#include <list>
 #include <memory>
 #include <mutex>
 #include <stdexcept>
@@ -141,18 +142,25 @@ struct WorkBlock {
     }
 };
 
-// Device memory of captured calls: a block belongs to the graph that a call was
+// Device memory of captured calls: a block belongs to the graph that calls were
 // captured into until the graph and its instances are gone, and then to the next
 // capture that it fits.  A replay may run beside any other call, so captured calls
-// use no buffer of the handle that another call may use or replace.
+// use no buffer of the handle that another call may use or replace.  The calls of
+// one capture share a block of their kind.
 struct GraphMemory {
+    enum Kind { kTiles, kRecords };
     struct Block {
-        void* p;
-        size_t bytes;
-        bool used;
+        void* p = nullptr;
+        size_t bytes = 0;
+        bool used = false;
+        Kind kind = kTiles;
+        unsigned long long capture = 0;
+        bool fresh = false;               // no earlier call of the capture uses it
+        cudaEvent_t call = nullptr;       // kRecords: the last call of the capture
+        cudaEvent_t instance = nullptr;   // kRecords: the last replay (an external event of the graph)
     };
     std::mutex mutex;
-    std::vector<Block> blocks;
+    std::list<Block> blocks;
 };
 
 struct SceneHost {
@@ -220,13 +228,23 @@ struct SceneHost {
 // captured ones have a side each, and a second capture that is open at the same time has
 // none (null): its work runs in line.
 const SceneHost::Side* side_of(SceneHost::Side (&sides)[2], cudaStream_t st);
+// While it lives, this thread may make calls that an open capture forbids (they
+// take no part in it).
+struct OutsideCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    OutsideCapture() { OMV_CUDA(cudaThreadExchangeStreamCaptureMode(&mode)); }
+    ~OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    OutsideCapture(const OutsideCapture&) = delete;
+    OutsideCapture& operator=(const OutsideCapture&) = delete;
+};
+
 // the pool of the handle's context
 WorkPool& work_pool(SceneHost& s);
 // whether `st` is being captured into a graph
 bool is_captured(cudaStream_t st);
 // a block of at least `bytes` for the call that is being captured on `st`
 // (DeviceOutOfMemory when there is none)
-void* graph_block(SceneHost& s, cudaStream_t st, size_t bytes);
+GraphMemory::Block& graph_block(SceneHost& s, cudaStream_t st, size_t bytes, GraphMemory::Kind kind);
 // orders the side stream after what `st` holds so far, and `st` after the side's
 inline void fork_side(const SceneHost::Side& x, cudaStream_t st)
 {

@@ -240,3 +240,71 @@ def test_captures_one_after_another_use_the_same_memory(gpu, scenes, torch):
             torch.cuda.synchronize()
     assert free0 - torch.cuda.mem_get_info()[0] < 3 * 36 * 2**20
     w.check(out, _want(torch, w), 64)
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("work", [Frame, Gradient])
+def test_two_instances_of_a_graph(gpu, scenes, torch, work, mode):
+    """A captured call has no memory nodes: its graph is instantiated twice, in every capture mode."""
+    w = work(gpu, scenes, torch)
+    want, out, direct = _want(torch, w), w.buffers(), w.buffers()
+    torch.cuda.synchronize()
+    with Graph(torch, mode) as g:
+        g.begin()
+        w.call(g.stream, out)
+        g.end()
+        e0, e1 = g.instantiate(), g.instantiate()
+        for e in (e0, e1, e0):
+            g.launch(e)
+        torch.cuda.synchronize()
+        w.call(g.stream, direct)
+        g.launch(e1)
+        torch.cuda.synchronize()
+        w.check(out, want, 4)
+        w.check(direct, want, 1)
+
+
+def test_instances_and_direct_gradients_on_their_own_streams(gpu, scenes, torch):
+    """A graph of three gradients, two of them on branches side by side, as two instances on two streams with direct
+    calls on a third, none waiting for another: each has its records to itself while it runs."""
+    w = Gradient(gpu, scenes, torch, side=64, spp=64)
+    want, out, direct = _want(torch, w), w.buffers(), w.buffers()
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    branch, fork, join = torch.cuda.Stream(), torch.cuda.Event(), torch.cuda.Event()
+    torch.cuda.synchronize()
+    with Graph(torch, "relaxed") as g:
+        g.begin()
+        w.call(g.stream, out)
+        fork.record(g.stream)
+        branch.wait_event(fork)
+        w.call(branch, out)
+        join.record(branch)
+        w.call(g.stream, out)
+        g.stream.wait_event(join)
+        g.end()
+        execs = [g.instantiate(), g.instantiate()]
+        for _ in range(20):
+            for e, st in zip(execs, streams):
+                g._ok(g.cu.cuGraphLaunch(e, C.c_void_p(st.cuda_stream)))
+            w.call(streams[2], direct)
+        torch.cuda.synchronize()
+        w.check(out, want, 120)
+        w.check(direct, want, 20)
+
+
+def test_gradients_of_one_capture_share_their_records(gpu, scenes, torch):
+    """Graphs of 16 gradients of 1.2 GB of records each, one graph after another, leave less than 3 GiB behind."""
+    w = Gradient(gpu, scenes, torch, side=128, spp=64)
+    want, out = _want(torch, w), w.buffers()
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    for _ in range(8):
+        with Graph(torch, "thread_local") as g:
+            g.begin()
+            for _ in range(16):
+                w.call(g.stream, out)
+            g.end()
+            g.launch(g.instantiate())
+            torch.cuda.synchronize()
+    assert free0 - torch.cuda.mem_get_info()[0] < 3 * 2**30
+    w.check(out, want, 128)
