@@ -870,7 +870,7 @@ struct AdjWorkspace {
             const int64_t fit = (int64_t)(std::min(kAdjBudget, (free_b + own) / 2) / per);
             cap = std::min(cap, std::max<int64_t>(std::min(most, kAdjMinCap), fit));
             if (capturing) {
-                captured = &graph_block(s, st, need(cap), GraphMemory::kRecords);
+                captured = &graph_block(s, st, need(cap));
                 base = captured->p;
             } else if (s.adj_scratch && s.adj_bytes >= need(cap)) {
                 base = s.adj_scratch;

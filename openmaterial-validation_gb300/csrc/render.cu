@@ -112,8 +112,8 @@ struct WaveArgs {
     float light_scale, min_dist, cut;
     FastDiv spp_div, width_div;  // by spp and by cam.width (one frame)
     TileGrid tiles;              // of the frame's camera
-    TileList* tile_lists;        // start nodes of the first camera bounce (null: none)
-    uint32_t num_tiles;
+    TileList* tile_lists;        // by tile of the frame: start nodes of the wave's first camera bounce (null: none)
+    uint32_t first_tile, num_tiles;  // the wave's tiles
     RenderScratch R;
 };
 
@@ -308,8 +308,8 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceMinBlocks) k_extend(const
 __global__ void __launch_bounds__(kTileThreads) k_tiles(WaveArgs A)
 {
     __shared__ TileEntry entries[kTileThreads / 32][kTileNodes];
-    const uint32_t t = (blockIdx.x * kTileThreads + threadIdx.x) >> 5;
-    if (t >= A.num_tiles) return;
+    const uint32_t i = (blockIdx.x * kTileThreads + threadIdx.x) >> 5, t = A.first_tile + i;
+    if (i >= A.num_tiles) return;
     const uint32_t row = t / A.tiles.per_row, col = t - row * A.tiles.per_row;
     const int x = (int)(col << A.tiles.lx), y = (int)(row << A.tiles.ly);
     tile_list(A.S, A.items, A.cam, A.S.tlas_root, x, min(x + (1 << A.tiles.lx), A.cam.width), y,
@@ -1085,9 +1085,9 @@ inline int grid_for(int64_t n, int t) { return (int)std::max<int64_t>(1, (n + t 
 namespace {
 
 void carve_scratch(RenderScratch& R, void* base, int64_t wave_cap, int64_t queue_cap, int light_slots,
-                   int shadow_slots)
+                   int shadow_slots, size_t tile_bytes = 0)
 {
-    const ScratchLayout L = scratch_layout(wave_cap, queue_cap, light_slots, shadow_slots);
+    const ScratchLayout L = scratch_layout(wave_cap, queue_cap, light_slots, shadow_slots, tile_bytes);
     char* b = static_cast<char*>(base);
     R.base = base;
     R.bytes = L.bytes;
@@ -1109,6 +1109,8 @@ void carve_scratch(RenderScratch& R, void* base, int64_t wave_cap, int64_t queue
     R.sq = (float4*)(b + L.sq);
     R.ctr = (uint32_t*)(b + L.ctr);
     R.stats = (unsigned long long*)(b + L.stats);
+    R.tiles = b + L.tiles;
+    R.tile_bytes = tile_bytes;
 }
 
 // Validated sizes of one frame: paths, wave capacity and vertex slots.
@@ -1116,9 +1118,8 @@ struct FramePlan {
     int64_t npix, total, cap;
     int light_slots, shadow_slots;
     bool lights;
-    TileGrid tiles{};        // of the frame's camera
-    uint32_t num_tiles = 0;
-    TileList* tile_lists = nullptr;  // null: none
+    TileGrid tiles{};         // of the frame's camera
+    uint32_t num_tiles = 0;   // 0: no tile lists
 };
 
 // Tiles of a camera: about kTileRays rays each (1024: the same within 1%), so
@@ -1205,6 +1206,32 @@ uint32_t batch_global_pixel(const std::vector<DevJob>& jobs, int64_t g)
 // 3.99 ms, 16 batched jobs 19.13 -> 19.30).
 constexpr int64_t kStagedPaths = 1 << 25;
 
+// The tile lists that the wave at hand makes (0: none) and reads.  They are no memory
+// of their own that a frame would have to ask for: the scratch has room for all
+// lists of the frame of several waves that it was made for, and its first wave
+// makes them; other frames make the lists of a wave's own tiles, where its
+// first camera shading will queue connections (48 bytes per path and more; a list has
+// 272 and serves 512 paths, of a one-pixel-wide frame at least 16).  The launch
+// takes about 20 us, in each of 64 waves of 2^17 paths 5% of the frame.
+void wave_tiles(WaveArgs& A, const FramePlan& P, const RenderScratch& R)
+{
+    A.first_tile = A.num_tiles = 0;
+    if (P.num_tiles == 0) return;
+    if (sizeof(TileList) * (size_t)P.num_tiles <= R.tile_bytes) {
+        A.tile_lists = static_cast<TileList*>(R.tiles);
+        if (A.wave_base == 0) A.num_tiles = P.num_tiles;
+        return;
+    }
+    const uint32_t row0 = A.base_q / (uint32_t)A.cam.width >> P.tiles.ly,
+                   row1 = A.last_pixel / (uint32_t)A.cam.width >> P.tiles.ly;
+    const uint32_t n = (row1 - row0 + 1) * P.tiles.per_row;
+    A.tile_lists = nullptr;
+    if (sizeof(TileList) * (size_t)n > 48 * (size_t)R.wave_cap * R.shadow_slots) return;
+    A.first_tile = row0 * P.tiles.per_row;
+    A.num_tiles = n;
+    A.tile_lists = reinterpret_cast<TileList*>(R.sq) - A.first_tile;
+}
+
 // The wave loop of one frame (or, with `batch`, of all jobs of a batch) on
 // scratch R (at least P.cap paths).  With `events` false no CUDA event is
 // created: no frame or kernel timing, and `stats` must be null.
@@ -1243,8 +1270,7 @@ void run_waves(SceneHost& s, RenderScratch& R, const FramePlan& P, const omv_cam
     A.num_jobs = batch ? (int32_t)batch->h_jobs->size() : 0;
     A.path_job = R.path_job;
     A.tiles = P.tiles;
-    A.num_tiles = P.num_tiles;
-    A.tile_lists = P.tile_lists;
+    A.tile_lists = nullptr;
     int occ_t = 0, occ_s = 0;
     OMV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_t, k_extend, kTraceThreads, 0));
     // threads per block of the shading-side kernels: 256, or a batch's
@@ -1297,11 +1323,6 @@ void run_waves(SceneHost& s, RenderScratch& R, const FramePlan& P, const omv_cam
         OMV_CUDA(cudaEventCreate(&e1));
         OMV_CUDA(cudaEventRecord(e0, st));
     }
-    if (A.tile_lists) {
-        const NvtxRange tile_range("omv tiles");
-        k_tiles<<<grid_for(32 * (int64_t)A.num_tiles, kTileThreads), kTileThreads, 0, st>>>(A);
-        ++launches;
-    }
     for (int64_t wb = 0; wb < total; wb += cap) {
         const NvtxRange wave_range("omv wave");
         A.wave_base = wb;
@@ -1316,6 +1337,12 @@ void run_waves(SceneHost& s, RenderScratch& R, const FramePlan& P, const omv_cam
             A.last_pixel = (uint32_t)((wb + A.wave_n - 1) / p.samples_per_pixel);
         }
         OMV_CUDA(cudaMemsetAsync(R.ctr, 0, kMaxCounters * 4, st));
+        wave_tiles(A, P, R);
+        if (A.num_tiles) {
+            const NvtxRange tile_range("omv tiles");
+            k_tiles<<<grid_for(32 * (int64_t)A.num_tiles, kTileThreads), kTileThreads, 0, st>>>(A);
+            ++launches;
+        }
         int work = 0;
         if (batch) {
             k_job_ids<<<grid_for(A.wave_n, sth), sth, 0, st>>>(A);
@@ -1478,7 +1505,7 @@ void run_waves(SceneHost& s, RenderScratch& R, const FramePlan& P, const omv_cam
 
 }  // namespace
 
-static void ensure_scratch(SceneHost& s, int64_t wave_cap, int light_slots, int shadow_slots)
+static void ensure_scratch(SceneHost& s, int64_t wave_cap, int light_slots, int shadow_slots, size_t tile_bytes = 0)
 {
     RenderScratch& R = s.scratch;
     if (R.base && R.wave_cap >= wave_cap && R.light_slots >= light_slots && R.shadow_slots >= shadow_slots) return;
@@ -1494,28 +1521,17 @@ static void ensure_scratch(SceneHost& s, int64_t wave_cap, int light_slots, int 
     }
     void* base = nullptr;
     int64_t queue_cap = queue_entries(wave_cap, s.num_lights > 0);
-    if (queue_cap > wave_cap &&
-        cudaMalloc(&base, scratch_layout(wave_cap, queue_cap, light_slots, shadow_slots).bytes) != cudaSuccess) {
-        (void)cudaGetLastError();  // the light subpaths go without queues of their own
-        base = nullptr;
-        queue_cap = wave_cap;
+    if (queue_cap > wave_cap || tile_bytes > 0) {
+        if (cudaMalloc(&base, scratch_layout(wave_cap, queue_cap, light_slots, shadow_slots, tile_bytes).bytes) !=
+            cudaSuccess) {  // the light subpaths go without queues of their own, the tile lists without their room
+            (void)cudaGetLastError();
+            base = nullptr;
+            queue_cap = wave_cap;
+            tile_bytes = 0;
+        }
     }
     if (!base) OMV_CUDA(cudaMalloc(&base, scratch_layout(wave_cap, queue_cap, light_slots, shadow_slots).bytes));
-    carve_scratch(R, base, wave_cap, queue_cap, light_slots, shadow_slots);
-}
-
-// Room for the n tile lists of a frame on `st`, in `block` or, for a captured
-// frame, its graph's.  Null (no tiles) when the memory is not there.
-static TileList* tile_room(SceneHost& s, int64_t n, cudaStream_t st, WorkBlock& block)
-{
-    const size_t bytes = sizeof(TileList) * (size_t)n;
-    try {
-        if (is_captured(st)) return static_cast<TileList*>(graph_block(s, st, bytes, GraphMemory::kTiles).p);
-        block.take(work_pool(s), bytes, bytes, st);
-        return static_cast<TileList*>(block.p);
-    } catch (const DeviceOutOfMemory&) {
-        return nullptr;
-    }
+    carve_scratch(R, base, wave_cap, queue_cap, light_slots, shadow_slots, tile_bytes);
 }
 
 // Default wave scratch: up to 32 GiB (and at most half of the free device
@@ -1538,16 +1554,13 @@ void render_frame(SceneHost& s, const omv_camera& cam, const omv_params& p, doub
         const int64_t fit = (int64_t)(budget / path_scratch_bytes(P.light_slots, P.shadow_slots));
         P.cap = std::max<int64_t>(1, std::min<int64_t>({fit, std::max<int64_t>(P.total, 1), (int64_t)0x7FFFFFFF}));
     }
-    ensure_scratch(s, P.cap, P.light_slots, P.shadow_slots);
-    WorkBlock tiles;
     if (P.total >= kTileMinPaths && p.camera_bounces > 0) {
         P.tiles = tile_grid(cam, p.samples_per_pixel);
         const int64_t n = tile_count(P.tiles, cam);
-        if (n <= kTileMaxCount) {
-            P.tile_lists = tile_room(s, n, st, tiles);
-            P.num_tiles = (uint32_t)n;
-        }
+        if (n <= kTileMaxCount) P.num_tiles = (uint32_t)n;
     }
+    ensure_scratch(s, P.cap, P.light_slots, P.shadow_slots,
+                   P.total > P.cap ? sizeof(TileList) * (size_t)P.num_tiles : 0);
     run_waves(s, s.scratch, P, cam, p, d_sum, d_sumsq, d_count, st, stats, true, true, nullptr, while_running);
 }
 

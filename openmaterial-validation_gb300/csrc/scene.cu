@@ -454,11 +454,11 @@ void free_block(const GraphMemory::Block& b)
 }
 
 // an unclaimed block of at least `bytes`, or a new one in place of all that no graph claims
-GraphMemory::Block& take_block(GraphMemory& m, size_t bytes, GraphMemory::Kind kind)
+GraphMemory::Block& take_block(GraphMemory& m, size_t bytes)
 {
     GraphMemory::Block* best = nullptr;
     for (GraphMemory::Block& b : m.blocks)
-        if (!b.used && b.kind == kind && b.bytes >= bytes && (!best || b.bytes < best->bytes)) best = &b;
+        if (!b.used && b.bytes >= bytes && (!best || b.bytes < best->bytes)) best = &b;
     if (best) return *best;
     for (auto b = m.blocks.begin(); b != m.blocks.end();) {
         if (!b->used) {
@@ -469,13 +469,10 @@ GraphMemory::Block& take_block(GraphMemory& m, size_t bytes, GraphMemory::Kind k
         }
     }
     GraphMemory::Block b;
-    b.kind = kind;
     b.bytes = bytes;
     try {
-        if (kind == GraphMemory::kRecords) {
-            OMV_CUDA(cudaEventCreateWithFlags(&b.call, cudaEventDisableTiming));
-            OMV_CUDA(cudaEventCreateWithFlags(&b.instance, cudaEventDisableTiming));
-        }
+        OMV_CUDA(cudaEventCreateWithFlags(&b.call, cudaEventDisableTiming));
+        OMV_CUDA(cudaEventCreateWithFlags(&b.instance, cudaEventDisableTiming));
         OMV_CUDA(cudaMalloc(&b.p, bytes));
         m.blocks.push_back(b);
     } catch (...) {
@@ -487,7 +484,7 @@ GraphMemory::Block& take_block(GraphMemory& m, size_t bytes, GraphMemory::Kind k
 
 }  // namespace
 
-GraphMemory::Block& graph_block(SceneHost& s, cudaStream_t st, size_t bytes, GraphMemory::Kind kind)
+GraphMemory::Block& graph_block(SceneHost& s, cudaStream_t st, size_t bytes)
 {
     const OutsideCapture outside;
     unsigned long long id = 0;
@@ -496,11 +493,11 @@ GraphMemory::Block& graph_block(SceneHost& s, cudaStream_t st, size_t bytes, Gra
     GraphMemory& m = *s.graph_memory;
     std::unique_lock<std::mutex> lock(m.mutex);
     for (GraphMemory::Block& b : m.blocks)
-        if (b.used && b.capture == id && b.kind == kind && b.bytes >= bytes) {
+        if (b.used && b.capture == id && b.bytes >= bytes) {
             b.fresh = false;
             return b;
         }
-    GraphMemory::Block& b = take_block(m, bytes, kind);
+    GraphMemory::Block& b = take_block(m, bytes);
     std::unique_ptr<GraphClaim> claim(new GraphClaim{s.graph_memory, b.p});
     cudaUserObject_t object = nullptr;
     OMV_CUDA(cudaUserObjectCreate(&object, claim.get(), end_claim, 1, cudaUserObjectNoDestructorSync));

@@ -64,6 +64,8 @@ struct RenderScratch {
     float4* sq = nullptr;        // shadow queue: 3 float4 per entry
     uint32_t* ctr = nullptr;     // per-wave queue and work counters
     unsigned long long* stats = nullptr;  // cumulative ray counters
+    void* tiles = nullptr;       // room for a frame's tile lists
+    size_t tile_bytes = 0;
 };
 
 // Tiles of a frame: 2^lx x 2^ly pixels each (beam.cuh).
@@ -146,18 +148,16 @@ struct WorkBlock {
 // captured into until the graph and its instances are gone, and then to the next
 // capture that it fits.  A replay may run beside any other call, so captured calls
 // use no buffer of the handle that another call may use or replace.  The calls of
-// one capture share a block of their kind.
+// one capture share a block, one after another, and so do the replays.
 struct GraphMemory {
-    enum Kind { kTiles, kRecords };
     struct Block {
         void* p = nullptr;
         size_t bytes = 0;
         bool used = false;
-        Kind kind = kTiles;
         unsigned long long capture = 0;
         bool fresh = false;               // no earlier call of the capture uses it
-        cudaEvent_t call = nullptr;       // kRecords: the last call of the capture
-        cudaEvent_t instance = nullptr;   // kRecords: the last replay (an external event of the graph)
+        cudaEvent_t call = nullptr;       // the last call of the capture
+        cudaEvent_t instance = nullptr;   // the last replay (an external event of the graph)
     };
     std::mutex mutex;
     std::list<Block> blocks;
@@ -244,7 +244,7 @@ WorkPool& work_pool(SceneHost& s);
 bool is_captured(cudaStream_t st);
 // a block of at least `bytes` for the call that is being captured on `st`
 // (DeviceOutOfMemory when there is none)
-GraphMemory::Block& graph_block(SceneHost& s, cudaStream_t st, size_t bytes, GraphMemory::Kind kind);
+GraphMemory::Block& graph_block(SceneHost& s, cudaStream_t st, size_t bytes);
 // orders the side stream after what `st` holds so far, and `st` after the side's
 inline void fork_side(const SceneHost::Side& x, cudaStream_t st)
 {

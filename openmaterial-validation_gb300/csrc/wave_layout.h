@@ -37,10 +37,12 @@ inline int64_t light_queue_first(int64_t wave, int64_t queue_cap)
 // Byte offsets of one wave's arrays inside a single scratch block (each array
 // starts on a 256-byte boundary).
 struct ScratchLayout {
-    size_t tp, rad, ltp, lrad, lmeta, lvp, lvr, rq0, rq1, hits, pjob, sq, ctr, stats, bytes;
+    size_t tp, rad, ltp, lrad, lmeta, lvp, lvr, rq0, rq1, hits, pjob, sq, ctr, stats, tiles, bytes;
 };
 
-inline ScratchLayout scratch_layout(int64_t wave_cap, int64_t queue_cap, int light_slots, int shadow_slots)
+// tile_bytes: room for the tile lists of a frame of several waves
+inline ScratchLayout scratch_layout(int64_t wave_cap, int64_t queue_cap, int light_slots, int shadow_slots,
+                                    size_t tile_bytes = 0)
 {
     const size_t W = (size_t)wave_cap, Q = (size_t)queue_cap;
     size_t off = 0;
@@ -64,6 +66,7 @@ inline ScratchLayout scratch_layout(int64_t wave_cap, int64_t queue_cap, int lig
     L.sq = take((size_t)shadow_slots * W * 48 + 48);
     L.ctr = take(kMaxCounters * 4);
     L.stats = take(16 * 8);
+    L.tiles = take(tile_bytes);
     L.bytes = off;
     return L;
 }

@@ -197,8 +197,8 @@ def test_captured_frame_with_more_tiles_than_any_before(gpu, scenes, torch, mode
 
 
 def test_direct_frames_of_more_tiles_between_replays(gpu, scenes, torch):
-    """A captured frame's tile lists are its graph's: direct frames with more tiles, before the capture ends and between
-    replays, change nothing."""
+    """A captured frame's tile lists are made by its replay: direct frames with more tiles, before the capture ends and
+    between replays, change nothing."""
     w = Frame(gpu, scenes, torch, *MANY_TILES[0])
     want, out = _want(torch, w), w.buffers()
     other = torch.cuda.Stream()
@@ -224,8 +224,7 @@ def test_direct_frames_of_more_tiles_between_replays(gpu, scenes, torch):
 
 
 def test_captures_one_after_another_use_the_same_memory(gpu, scenes, torch):
-    """Blocks of graphs that are gone serve the next captures: 64 graphs of frames with 36 MB of tile lists each leave
-    less than three blocks behind."""
+    """64 graphs of frames with 36 MB of tile lists each leave less than three times that behind."""
     w = Frame(gpu, scenes, torch, *MANY_TILES[2])
     out = w.buffers()
     _want(torch, w)

@@ -104,3 +104,38 @@ def test_many_instances_and_masked_materials(gpu, scenes, torch, clutter):
     rs = gpu.RenderScene(sc)
     a, b = _both(gpu, torch, rs, cam.to_c(), gpu.RendererParameters.for_scene(sc, samplesPerPixel=9, seed=2).to_c())
     assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("size", [(1537, 700, 4), (333, 41, 310), (1, 70_001, 60), (70_001, 1, 61)])
+def test_lists_of_several_waves(gpu, torch, clutter, size):
+    """Waves that begin and end inside tile rows and pixels, with all lists of the frame made at once (a handle's first
+    frame has the room for them) and with those of each wave's tiles (a handle whose scratch was made for another
+    frame, too small a wave for its tiles included)."""
+    w, h, spp = size
+    cam = gpu.PinholeCamera(w, h)
+    cam.position = np.array([0.5, 1.0, 12.0])
+    cam.adjust_to_resolution()
+    cam.set_y_fov(60.0)
+    first, used = gpu.RenderScene(clutter), gpu.RenderScene(clutter)
+    small = gpu.PinholeCamera(1100, 1000).to_c()
+    _both(gpu, torch, used, small, gpu.RendererParameters.for_scene(clutter, samplesPerPixel=1).to_c())
+    want = None
+    for wave in (0, 1_000_003, 70_001, 999):
+        if wave == 999 and w > 1:
+            continue
+        prm = gpu.RendererParameters.for_scene(clutter, samplesPerPixel=spp, seed=8, wave_paths=wave).to_c()
+        for rs in (used, first):
+            s = torch.zeros((h, w, 3), dtype=torch.float64, device="cuda")
+            c = torch.zeros((h, w), dtype=torch.int32, device="cuda")
+            if wave == 0:
+                if rs is first:
+                    continue
+                gpu.check(gpu.lib().omv_render_device_static(rs.handle, C.byref(cam.to_c()), C.byref(prm), C.c_void_p(s.data_ptr()),
+                                                             None, C.c_void_p(c.data_ptr()), None))
+                want = s
+            else:
+                gpu.check(gpu.lib().omv_render_device(rs.handle, C.byref(cam.to_c()), C.byref(prm), C.c_void_p(s.data_ptr()), None,
+                                                      C.c_void_p(c.data_ptr()), None, None))
+            torch.cuda.synchronize()
+            assert int(c.min()) == int(c.max()) == spp
+            assert float((s - want).abs().max()) <= 1e-9 * float(want.abs().max())
