@@ -841,72 +841,88 @@ void carve_wave(AdjWave& A, char* b, const AdjLayout& l, int njobs)
 constexpr size_t kAdjBudget = (size_t)8 << 30;
 constexpr int64_t kAdjMinCap = 1 << 14;  // tried at least, whatever memory is free
 
-// Where a wave's records live while its launches are in flight: the scene's own
-// block, used by one call after another (a call on another stream waits for
-// the last one's event), or, when the caller captures the stream into a graph, a
-// block of that graph, used by one call of the capture and by one replay of any
+// Where a wave's records live while its launches are in flight: a block of the
+// context's work memory, or, when the caller captures the stream into a graph, a block
+// of that graph, used by one call of the capture and by one replay of any
 // instance after another (the graph waits for and records an external event).
 struct AdjWorkspace {
-    SceneHost& s;
     cudaStream_t st;
+    WorkBlock direct;
     GraphMemory::Block* captured = nullptr;
     void* base = nullptr;
     int64_t cap = 0;
-    AdjWorkspace(SceneHost& s_, cudaStream_t st_, int64_t total, int njobs, int B, int L, bool lights)
-        : s(s_), st(st_)
+    AdjWorkspace(SceneHost& s, cudaStream_t st_, int64_t total, int njobs, int B, int L, bool lights) : st(st_)
     {
         const bool capturing = is_captured(st);
         auto need = [&](int64_t c) { return adj_layout(c, njobs, B, L, lights).bytes; };
         const size_t per = std::max<size_t>(1, (need(1 << 20) - need(0)) >> 20);
         const int64_t most = std::min<int64_t>(total, (int64_t)1 << 30);
         cap = std::max<int64_t>(1, std::min<int64_t>(most, (int64_t)(kAdjBudget / per)));
-        if (!capturing && s.adj_scratch && s.adj_bytes >= need(cap)) {
-            base = s.adj_scratch;
-        } else {
+        size_t idle = 0, largest = 0;
+        if (!capturing) idle = work_memory(s).idle(&largest);
+        if (largest < need(cap)) {
             const OutsideCapture outside;
             size_t free_b = 0, total_b = 0;
             OMV_CUDA(cudaMemGetInfo(&free_b, &total_b));
-            const size_t own = capturing ? 0 : s.adj_bytes;
-            const int64_t fit = (int64_t)(std::min(kAdjBudget, (free_b + own) / 2) / per);
+            const int64_t fit = (int64_t)(std::min(kAdjBudget, (free_b + idle) / 2) / per);
             cap = std::min(cap, std::max<int64_t>(std::min(most, kAdjMinCap), fit));
-            if (capturing) {
-                captured = &graph_block(s, st, need(cap));
-                base = captured->p;
-            } else if (s.adj_scratch && s.adj_bytes >= need(cap)) {
-                base = s.adj_scratch;
-            } else {
-                if (s.adj_scratch) {
-                    OMV_CUDA(cudaEventSynchronize(s.adj_done));
-                    cudaFree(s.adj_scratch);
-                    s.adj_scratch = nullptr;
-                    s.adj_bytes = 0;
+        }
+        for (;;) {
+            try {
+                if (capturing) {
+                    captured = &graph_block(s, st, need(cap));
+                    base = captured->p;
+                } else {
+                    base = direct.take(work_memory(s), need(cap), st);
                 }
-                OMV_CUDA(cudaMalloc(&base, need(cap)));
-                s.adj_scratch = base;
-                s.adj_bytes = need(cap);
+                break;
+            } catch (const DeviceOutOfMemory&) {  // someone else took it meanwhile
+                if (cap <= std::min(most, kAdjMinCap)) throw;
+                cap = std::max(cap / 2, std::min(most, kAdjMinCap));
             }
         }
         if (captured) {
             if (!captured->fresh) OMV_CUDA(cudaStreamWaitEvent(st, captured->call, 0));
             OMV_CUDA(cudaStreamWaitEvent(st, captured->instance, cudaEventWaitExternal));
-        } else {
-            if (!s.adj_done)
-                OMV_CUDA(cudaEventCreateWithFlags(&s.adj_done, cudaEventDisableTiming));
-            else
-                OMV_CUDA(cudaStreamWaitEvent(st, s.adj_done, 0));
         }
     }
     ~AdjWorkspace()
     {
-        if (captured) {
-            cudaEventRecord(captured->call, st);
-            cudaEventRecordWithFlags(captured->instance, st, cudaEventRecordExternal);
-        } else {
-            cudaEventRecord(s.adj_done, st);
-        }
+        if (!captured) return;
+        cudaEventRecord(captured->call, st);
+        cudaEventRecordWithFlags(captured->instance, st, cudaEventRecordExternal);
     }
     AdjWorkspace(const AdjWorkspace&) = delete;
     AdjWorkspace& operator=(const AdjWorkspace&) = delete;
+};
+
+// The side stream of an adjoint (null: its work runs in line).  It is joined
+// before the records are given back, also when a launch fails.
+struct AdjSide {
+    const SceneHost::Side* side;
+    cudaStream_t st;
+    bool forked = false;
+    AdjSide(const SceneHost::Side* s, cudaStream_t main) : side(s), st(main) {}
+    ~AdjSide()
+    {
+        if (!forked) return;
+        cudaEventRecord(side->join, side->stream);
+        cudaStreamWaitEvent(st, side->join, 0);
+    }
+    AdjSide(const AdjSide&) = delete;
+    AdjSide& operator=(const AdjSide&) = delete;
+    cudaStream_t stream() const { return side ? side->stream : st; }
+    void fork()
+    {
+        if (!side) return;
+        fork_side(*side, st);
+        forked = true;
+    }
+    void join()
+    {
+        if (forked) join_side(*side, st);
+        forked = false;
+    }
 };
 
 inline unsigned blocks_for(int64_t n, int t) { return (unsigned)std::max<int64_t>(1, (n + t - 1) / t); }
@@ -1006,14 +1022,8 @@ void run_adjoint(SceneHost& s, std::vector<AdjJob>& jobs, const omv_params& p, c
     const int lback_grid = resident_grid(k_adj_light_back, kAdjThreads, smem, s.num_sms);
     // beside the main stream: the light subpaths beside the camera rays' first
     // hits, then each bounce's connections beside the next bounce's hits
-    const SceneHost::Side* beside = lights ? side_of(s.adj_side, st) : nullptr;
-    const cudaStream_t side = beside ? beside->stream : st;
-    auto fork = [&] {
-        if (beside) fork_side(*beside, st);
-    };
-    auto join = [&] {
-        if (beside) join_side(*beside, st);
-    };
+    AdjSide beside(lights ? side_of(s.adj_side, st) : nullptr, st);
+    const cudaStream_t side = beside.stream();
     for (int64_t wb = 0; wb < total; wb += ws.cap) {
         A.wave_base = wb;
         A.wave_n = (int32_t)std::min<int64_t>(ws.cap, total - wb);
@@ -1022,7 +1032,7 @@ void run_adjoint(SceneHost& s, std::vector<AdjJob>& jobs, const omv_params& p, c
         const unsigned gen = blocks_for(A.wave_n, kShadeThreads);
         if (A.path_job) k_adj_path_jobs<<<gen, kShadeThreads, 0, st>>>(A);
         if (lights) {
-            fork();
+            beside.fork();
             k_adj_light_gen<<<gen, kShadeThreads, 0, side>>>(A);
             for (int b = 1; b <= L; ++b) {
                 const size_t off = (size_t)(b - 1) * A.cap;
@@ -1036,12 +1046,12 @@ void run_adjoint(SceneHost& s, std::vector<AdjJob>& jobs, const omv_params& p, c
             const size_t off = (size_t)(b - 1) * A.cap;
             k_adj_extend<<<trace_grid, kTraceThreads, 0, st>>>(A, A.crq + 2 * off, A.chit + off,
                                                                A.ctr + kAdjCtrCam + b - 1, work++);
-            join();
+            beside.join();
             k_adj_camera<<<camera_grid, kShadeThreads, 0, st>>>(A, b);
             if (lights) {
                 uint32_t* seen = A.ctr + kAdjCtrSeen + b - 1;
                 const uint32_t* count = A.ctr + kAdjCtrConn + b - 1;
-                fork();
+                beside.fork();
                 if (masked)
                     k_adj_shadow<true><<<trace_grid, kTraceThreads, 0, side>>>(A, count, seen, work++);
                 else
@@ -1049,7 +1059,7 @@ void run_adjoint(SceneHost& s, std::vector<AdjJob>& jobs, const omv_params& p, c
                 k_adj_connect<<<connect_grid, kAdjThreads, smem, side>>>(A, b);
             }
         }
-        join();
+        beside.join();
         for (int b = B; b >= 1; --b) k_adj_camera_back<<<back_grid, kAdjThreads, smem, st>>>(A, b);
         if (lights)
             for (int b = L; b >= 1; --b) k_adj_light_back<<<lback_grid, kAdjThreads, smem, st>>>(A, b);

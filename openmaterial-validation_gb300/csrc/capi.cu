@@ -11,7 +11,6 @@
 #include <cstring>
 #include <functional>
 #include <memory>
-#include <mutex>
 #include <new>
 #include <string>
 
@@ -25,14 +24,9 @@ struct omv_scene {
     uint32_t* count = nullptr;
     float4* image = nullptr;
     int64_t film_pixels = 0;
-    // rays and hits of omv_trace_rays, kept up to kTraceKeep bytes; one call at a time
-    std::mutex trace_mutex;
-    void* trace_space = nullptr;
-    size_t trace_bytes = 0;
     ~omv_scene()
     {
         if (h) cudaSetDevice(h->device);
-        cudaFree(trace_space);
         cudaFree(sum);
         cudaFree(sumsq);
         cudaFree(count);
@@ -367,35 +361,24 @@ omv_status omv_trace_rays(omv_scene* scene, int64_t n, const float* rays, omv_hi
         if (n < 0 || (n > 0 && (!rays || !hits))) throw omv::ArgError("invalid ray buffers");
         if (n == 0) return;
         // The pages that the hits go to are mapped while the rays are traced, and the
-        // device buffers are kept.  1M rays of a 200k-triangle scene: 1940 -> 1614 us,
-        // 100k rays 480 -> 247, 300 rays 95 -> 58.  (In chunks, hits going down on a
-        // second stream beside the next chunk: 1904 us in four, 2290 in eight; every
-        // copy of pageable memory waits on the host.)
+        // device buffers are kept up to kTraceKeep bytes.  1M rays of a 200k-triangle scene:
+        // 1940 -> 1614 us, 100k rays 480 -> 247, 300 rays 95 -> 58.  (In chunks, hits
+        // going down on a second stream beside the next chunk: 1904 us in four, 2290 in
+        // eight; every copy of pageable memory waits on the host.)
         constexpr size_t kTraceKeep = (size_t)256 << 20;
         static_assert(sizeof(omv_hit) == 32, "a hit is as large as a ray");
-        omv_scene& s = *scene;
-        const cudaStream_t st = s.h->stream;
-        const std::lock_guard<std::mutex> lock(s.trace_mutex);
+        const cudaStream_t st = scene->h->stream;
         const size_t need = 64 * (size_t)n;
-        std::unique_ptr<DevTmp> large;
-        if (need > kTraceKeep) {
-            large.reset(new DevTmp(need));
-        } else if (s.trace_bytes < need) {
-            cudaFree(s.trace_space);  // (no call is using it)
-            s.trace_space = nullptr;
-            s.trace_bytes = 0;
-            OMV_CUDA(cudaMalloc(&s.trace_space, need));
-            s.trace_bytes = need;
-        }
-        float* d_rays = large ? large->as<float>() : static_cast<float*>(s.trace_space);
+        omv::WorkBlock block;
+        float* d_rays = static_cast<float*>(block.take(omv::work_memory(*scene->h), need, st, need > kTraceKeep));
         omv_hit* d_hits = reinterpret_cast<omv_hit*>(d_rays + 8 * n);
         try {
             OMV_CUDA(cudaMemcpyAsync(d_rays, rays, sizeof(float) * 8 * n, cudaMemcpyHostToDevice, st));
-            omv::trace_rays(*s.h, n, d_rays, d_hits, st);
+            omv::trace_rays(*scene->h, n, d_rays, d_hits, st);
             map_pages(hits, sizeof(omv_hit) * (size_t)n);
             OMV_CUDA(cudaMemcpyAsync(hits, d_hits, sizeof(omv_hit) * n, cudaMemcpyDeviceToHost, st));
             OMV_CUDA(cudaStreamSynchronize(st));
-        } catch (...) {  // the buffers must not be reused under copies in flight
+        } catch (...) {  // nothing of the call is in flight once it returns
             cudaStreamSynchronize(st);
             throw;
         }

@@ -363,36 +363,100 @@ const SceneHost::Side* side_of(SceneHost::Side (&sides)[2], cudaStream_t st)
     return !capture_of(sides[1].stream, other) || other == id ? &sides[1] : nullptr;
 }
 
-WorkPool::WorkPool(int device)
+void WorkMemory::drop(std::list<Block>::iterator b) noexcept
 {
-    cudaMemPoolProps props{};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.handleTypes = cudaMemHandleTypeNone;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = device;
-    OMV_CUDA(cudaMemPoolCreate(&pool_, &props));
+    cudaFree(b->p);  // (waits for the device)
+    if (b->done) cudaEventDestroy(b->done);
+    total_ -= b->bytes;
+    blocks_.erase(b);
 }
-WorkPool::~WorkPool() { cudaMemPoolDestroy(pool_); }
 
-void* WorkPool::take(size_t bytes, size_t keep, cudaStream_t st)
+WorkMemory::Block* WorkMemory::take(size_t bytes, cudaStream_t st, bool once)
 {
-    {
-        const std::lock_guard<std::mutex> lock(mutex_);
-        if (keep > keep_) {
-            uint64_t v = keep;
-            OMV_CUDA(cudaMemPoolSetAttribute(pool_, cudaMemPoolAttrReleaseThreshold, &v));
-            keep_ = keep;
+    const OutsideCapture outside;
+    const std::lock_guard<std::mutex> lock(mutex_);
+    auto over = [](Block& b) {
+        if (b.pending && cudaEventQuery(b.done) == cudaSuccess) b.pending = false;
+        (void)cudaGetLastError();  // (not ready)
+        return !b.pending;
+    };
+    // the smallest idle block that fits, one that is free by now or on this stream before others
+    auto at = blocks_.end(), later = blocks_.end();
+    for (auto b = blocks_.begin(); b != blocks_.end(); ++b) {
+        if (b->busy || b->bytes < bytes) continue;
+        auto& best = b->st == st || over(*b) ? at : later;
+        if (best == blocks_.end() || b->bytes < best->bytes) best = b;
+    }
+    if (at == blocks_.end() && !once && total_ + bytes > kWorkKeep) {
+        if (later != blocks_.end()) {
+            at = later;
+        } else {
+            for (auto b = blocks_.begin(); b != blocks_.end() && total_ + bytes > kWorkKeep;) {
+                const auto next = std::next(b);
+                if (!b->busy) drop(b);
+                b = next;
+            }
         }
     }
-    void* p = nullptr;
-    cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, pool_, st);
-    if (e == cudaErrorMemoryAllocation) {  // idle blocks of other sizes go first
-        (void)cudaGetLastError();
-        cudaMemPoolTrimTo(pool_, 0);
-        e = cudaMallocFromPoolAsync(&p, bytes, pool_, st);
+    if (at == blocks_.end()) {
+        blocks_.push_back(Block{nullptr, bytes, true, st, nullptr, false, once});
+        const auto n = std::prev(blocks_.end());
+        total_ += bytes;
+        cudaError_t e = cudaEventCreateWithFlags(&n->done, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaMalloc(&n->p, bytes);
+        if (e == cudaErrorMemoryAllocation) {  // what no call uses goes first
+            (void)cudaGetLastError();
+            for (auto b = blocks_.begin(); b != n;) {
+                const auto next = std::next(b);
+                if (!b->busy) drop(b);
+                b = next;
+            }
+            e = cudaMalloc(&n->p, bytes);
+        }
+        if (e != cudaSuccess) drop(n);
+        OMV_CUDA(e);
+        return &*n;
     }
-    OMV_CUDA(e);
-    return p;
+    if (at->pending) OMV_CUDA(cudaStreamWaitEvent(st, at->done, 0));
+    at->busy = true;
+    at->st = st;
+    return &*at;
+}
+
+void WorkMemory::give(Block* b, cudaStream_t st) noexcept
+{
+    const std::lock_guard<std::mutex> lock(mutex_);
+    b->busy = false;
+    b->pending = true;
+    if (!b->once && cudaEventRecord(b->done, st) == cudaSuccess) return;
+    (void)cudaGetLastError();  // without the event nobody can wait for the call's work
+    drop(std::find_if(blocks_.begin(), blocks_.end(), [b](const Block& x) { return &x == b; }));
+}
+
+size_t WorkMemory::idle(size_t* largest)
+{
+    const std::lock_guard<std::mutex> lock(mutex_);
+    size_t n = 0;
+    *largest = 0;
+    for (const Block& b : blocks_)
+        if (!b.busy) {
+            n += b.bytes;
+            *largest = std::max(*largest, b.bytes);
+        }
+    return n;
+}
+
+void WorkMemory::enter()
+{
+    const std::lock_guard<std::mutex> lock(mutex_);
+    ++users_;
+}
+
+void WorkMemory::leave() noexcept
+{
+    const std::lock_guard<std::mutex> lock(mutex_);
+    if (--users_ > 0) return;
+    while (!blocks_.empty()) drop(blocks_.begin());
 }
 
 // a number of the current context (a device reset makes a new one)
@@ -409,21 +473,18 @@ static unsigned long long context_id()
     return id;
 }
 
-WorkPool& work_pool(SceneHost& s)
+WorkMemory& work_memory(SceneHost& s)
 {
-    std::call_once(s.pool_once, [&] {
-        static std::mutex mutex;
-        static auto& pools = *new std::map<std::pair<int, unsigned long long>, std::weak_ptr<WorkPool>>;
-        const OutsideCapture outside;
+    std::call_once(s.work_once, [&] {
+        // never destroyed: handles may outlive the program's static objects
+        static auto& mutex = *new std::mutex;
+        static auto& all = *new std::map<std::pair<int, unsigned long long>, WorkMemory>;
         const std::lock_guard<std::mutex> lock(mutex);
-        std::weak_ptr<WorkPool>& known = pools[{s.device, context_id()}];
-        s.pool = known.lock();
-        if (!s.pool) {
-            s.pool = std::make_shared<WorkPool>(s.device);
-            known = s.pool;
-        }
+        WorkMemory& m = all[{s.device, context_id()}];
+        m.enter();
+        s.work = &m;
     });
-    return *s.pool;
+    return *s.work;
 }
 
 namespace {
@@ -520,13 +581,11 @@ SceneHost::~SceneHost()
         if (x.stream) cudaStreamSynchronize(x.stream);
     for (void* p : allocs) cudaFree(p);
     if (scratch.base) cudaFree(scratch.base);
-    if (adj_scratch) cudaFree(adj_scratch);
     {
         const std::lock_guard<std::mutex> lock(graph_memory->mutex);
         for (const GraphMemory::Block& b : graph_memory->blocks) free_block(b);
         graph_memory->blocks.clear();
     }
-    if (adj_done) cudaEventDestroy(adj_done);
     if (mat_sets) cudaFree(mat_sets);
     if (d_jobs) cudaFree(d_jobs);
     if (batch_graph) cudaGraphExecDestroy(batch_graph);
@@ -537,6 +596,7 @@ SceneHost::~SceneHost()
     }
     if (fork_ev) cudaEventDestroy(fork_ev);
     if (join_ev) cudaEventDestroy(join_ev);
+    if (work) work->leave();
     if (stream) cudaStreamDestroy(stream);
 }
 
