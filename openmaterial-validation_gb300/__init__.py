@@ -32,7 +32,7 @@ CSRC = os.path.join(PKG_DIR, "csrc")
 BUILD_DIR = os.path.join(PKG_DIR, "_build")
 LIB_PATH = os.path.join(PKG_DIR, "libomv.so")
 SOURCES = ["bvh_build.cu", "scene.cu", "render.cu", "adjoint.cu", "fc.cu", "post.cu", "capi.cu"]
-HEADERS = ["bvh_build.h", "omv_device.cuh", "omv_types.h", "scene.h", "trace.cuh", "shade.cuh", "wave.cuh", "wave_layout.h", "beam.cuh", "dual.cuh", "crmath.cuh"]
+HEADERS = ["bvh_build.h", "omv_device.cuh", "omv_types.h", "scene.h", "trace.cuh", "shade.cuh", "wave.cuh", "wave_layout.h", "host_threads.h", "beam.cuh", "dual.cuh", "crmath.cuh"]
 ARCH = "-gencode=arch=compute_103a,code=sm_103a"
 NVCC_FLAGS = [ARCH, "-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-ffp-contract=off"]
 # translation units whose device float math must round like the reference

@@ -15,11 +15,11 @@
 #include <map>
 #include <memory>
 #include <mutex>
-#include <system_error>
 #include <thread>
 #include <vector>
 
 #include "bvh_build.h"
+#include "host_threads.h"
 #include "omv_device.cuh"
 #include "scene.h"
 
@@ -311,14 +311,7 @@ void commit_meshes(const omv_scene_desc& d, const std::vector<int>& norm_ch, con
     unsigned threads = 1;
     if (A.num_faces >= kCommitThreadFaces)
         threads = std::max(1u, std::min({16u, std::thread::hardware_concurrency(), (unsigned)todo.size()}));
-    std::vector<std::thread> pool;
-    pool.reserve(threads);
-    try {
-        for (unsigned k = 1; k < threads; ++k) pool.emplace_back(worker);
-    } catch (const std::system_error&) {  // no more threads to be had: the others do the work
-    }
-    worker();
-    for (std::thread& t : pool) t.join();
+    on_threads(threads, worker);
     for (const std::exception_ptr& e : errors)
         if (e) std::rethrow_exception(e);
 }
