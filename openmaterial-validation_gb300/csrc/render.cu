@@ -291,7 +291,6 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceMinBlocks) k_extend(const
     st.overflow = 0;
     TraceCounters tc{0u, 0u};
     const uint32_t n = *count;
-    const int lane = threadIdx.x & 31;
     auto root = [=](int k) { return path_root(jobs, path_job, k); };
     if (n <= kCoopRays) {
         const CoopCounts c = extend_rays_coop(S, items, rq, hits, n, work, sstack, root);
@@ -480,8 +479,13 @@ static __device__ __noinline__ float env_connect(const WaveArgs& A, int b, uint6
 
 // ------------------------------------------------------ camera shade ---
 // Where a camera vertex's connections to the light subpath go: the wavefront
-// queues each for k_shadow; the tail kernel tests it at once.
+// queues each for k_shadow.  The tail kernel runs in scenes without point
+// lights only and has none.
+struct NoConnections {
+    static constexpr bool kConnects = false;
+};
 struct QueueSink {
+    static constexpr bool kConnects = true;
     __device__ __forceinline__ void connect(const WaveArgs& A, int b, int k, V3 lpos, V3 pos, V3 lc)
     {
         const uint32_t sl = coalesced_append(&A.R.ctr[kCtrShadow + b]);
@@ -548,7 +552,7 @@ __device__ __forceinline__ bool camera_vertex(const WaveArgs& A, int b, int k, f
             r.z += tpn.z * e.z;
             A.R.rad[k] = r;
         }
-        if (S.num_lights > 0) {
+        if (Sink::kConnects && S.num_lights > 0) {
             const uint32_t meta = A.R.lmeta[k];
             const int lp_len = (int)(meta >> 16);
             const uint32_t li = meta & 0xFFFFu;
@@ -576,7 +580,7 @@ __device__ __forceinline__ bool camera_vertex(const WaveArgs& A, int b, int k, f
                 V3 f = material_eval(M, P, sp, LC, outV) * c;
                 lc = v3(f.x * tp.x * lRad.x, f.y * tp.y * lRad.y, f.z * tp.z * lRad.z);
                 if (intensity(lc) < A.cut) continue;
-                sink.connect(A, b, k, lPos, sp.pos, lc);
+                if constexpr (Sink::kConnects) sink.connect(A, b, k, lPos, sp.pos, lc);
             }
         }
         A.R.tp[k] = make_float4(tpn.x, tpn.y, tpn.z, mis_pdf);
@@ -759,34 +763,12 @@ __device__ __forceinline__ void tail_finish(const WaveArgs& A, uint32_t* count, 
     }
 }
 
-// A camera vertex's connections tested at once (the tail kernel's sink):
-// the path's radiance is this thread's alone while the tail runs.
-template <bool kMasked>
-struct TestSink {
-    const uint32_t* items;
-    TraceStack* st;
-    TraceCounters* tc;
-    uint32_t root;
-    uint32_t* tests;
-    __device__ __forceinline__ void connect(const WaveArgs& A, int b, int k, V3 lpos, V3 pos, V3 lc)
-    {
-        ++*tests;
-        if (is_connected<kMasked>(A.S, items, lpos, pos, *st, *tc, root)) {
-            float4 r = A.R.rad[k];
-            r.x += lc.x;
-            r.y += lc.y;
-            r.z += lc.z;
-            A.R.rad[k] = r;
-        }
-    }
-};
-
 // Camera bounces b0 .. camera bounces in one launch: each thread takes a path
 // alive at bounce b0 (queue rq_in) and runs it to its end: extension ray,
-// vertex (camera_vertex, as k_camera_shade), connections and MIS environment
-// ray tested at once, the next ray kept in registers.  The additions to the
-// path's radiance come in the wavefront's order (escape / emission, then
-// connections, then the environment ray, bounce by bounce).
+// vertex (camera_vertex, as k_camera_shade), MIS environment ray tested at once,
+// the next ray kept in registers.  The additions to the path's radiance come in
+// the wavefront's order (escape / emission, then the environment ray, bounce by
+// bounce).
 template <bool kMis, bool kMasked>
 __global__ void __launch_bounds__(kTraceThreads, 4) k_camera_tail(WaveArgs A, int b0, const float4* rq_in, uint32_t* work,
                                                                   const DevJob* jobs)
@@ -809,7 +791,7 @@ __global__ void __launch_bounds__(kTraceThreads, 4) k_camera_tail(WaveArgs A, in
             float4 ra = rq_in[2 * (size_t)i], rb = rq_in[2 * (size_t)i + 1];
             const int k = __float_as_int(rb.w);
             const uint32_t root = path_root(jobs, A.path_job, k);
-            TestSink<kMasked> sink{A.items, &st, &tc, root, &tests};
+            NoConnections sink;
             for (int b = b0; b <= A.cam_bounces; ++b) {
                 float tn = ra.w;
                 RayHit hh;
