@@ -44,3 +44,37 @@ def test_mesh_sizes_at_the_edges_of_the_classes(gpu, oracle, scenes, kind, sizes
     assert (b["inst"] != 0xFFFFFFFF).any()
     for name in ("inst", "geom", "prim", "material", "t", "u", "v"):
         assert np.array_equal(a[name].view(np.uint32), b[name].view(np.uint32)), name
+
+
+@pytest.mark.parametrize("sizes", [SHORT, LONG], ids=["short", "long"])
+@pytest.mark.parametrize("octaves", [0, 12, 40])
+def test_lines_of_growing_triangles(gpu, oracle, scenes, octaves, sizes):
+    """Triangles along a line, each larger and farther out than the one before (by a factor of 2^(octaves / number), all
+    of them finite): splits take one end off at a time, so a range goes through every class of sizes."""
+    rng = np.random.default_rng(octaves)
+    base = scenes.scene_mixed(8, 8, 1)
+    meshes, insts = [], []
+    for k, nt in enumerate(sizes):
+        one = rng.normal(size=(1, 3, 3)) + rng.normal(size=3) * 3
+        grow = 2.0 ** (octaves * (np.arange(nt) / nt - 0.5))
+        v = (one * grow[:, None, None] * 0.1).astype(np.float32) + rng.uniform(-3, 3, 3).astype(np.float32)
+        assert np.isfinite(v).all()
+        meshes.append(scenes.Mesh(positions=v.reshape(-1, 3), normals=None,
+                                  faces=np.arange(3 * nt, dtype=np.uint32).reshape(nt, 3),
+                                  material=k % len(base.materials), name=f"m{k}"))
+        t = np.eye(4, dtype=np.float32)
+        t[2, 3] = -8
+        insts.append(scenes.Instance(t, k))
+    sc = dataclasses.replace(base, meshes=meshes, instances=insts)
+    # rays past the triangles' centres, near and far, and anywhere
+    centres = np.concatenate([m.positions.reshape(-1, 3, 3).mean(axis=1) + [0, 0, -8] for m in meshes])
+    n = 40_000
+    at = centres[rng.integers(0, len(centres), n)] * (1 + 0.05 * rng.normal(size=(n, 1)))
+    o = rng.uniform([-6, -6, -14], [6, 6, -2], (n, 3))
+    d = np.where(rng.random((n, 1)) < 0.7, at - o, rng.normal(size=o.shape))
+    rays = np.zeros((n, 8), np.float32)
+    rays[:, 0:3], rays[:, 4:7], rays[:, 7] = o, d / np.linalg.norm(d, axis=1, keepdims=True), 3.4e38
+    a, b = gpu.RenderScene(sc).trace(rays), oracle.OracleScene(sc).trace(rays)
+    assert (b["inst"] != 0xFFFFFFFF).sum() > 1000
+    for name in ("inst", "geom", "prim", "material", "t", "u", "v"):
+        assert np.array_equal(a[name].view(np.uint32), b[name].view(np.uint32)), name
