@@ -27,6 +27,7 @@ struct omv_scene {
     ~omv_scene()
     {
         if (h) cudaSetDevice(h->device);
+        h.reset();  // the film after the scratch, see ~SceneHost
         cudaFree(sum);
         cudaFree(sumsq);
         cudaFree(count);

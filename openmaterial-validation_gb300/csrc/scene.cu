@@ -572,8 +572,10 @@ SceneHost::~SceneHost()
     if (stream) cudaStreamSynchronize(stream);
     for (const Side& x : {side[0], side[1], adj_side[0], adj_side[1]})
         if (x.stream) cudaStreamSynchronize(x.stream);
-    for (void* p : allocs) cudaFree(p);
+    // the scratch first: the driver puts off the work of freeing a large block until
+    // the next call, which would be the next scene's first allocation
     if (scratch.base) cudaFree(scratch.base);
+    for (void* p : allocs) cudaFree(p);
     {
         const std::lock_guard<std::mutex> lock(graph_memory->mutex);
         for (const GraphMemory::Block& b : graph_memory->blocks) free_block(b);
