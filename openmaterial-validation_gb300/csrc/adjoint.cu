@@ -28,11 +28,15 @@
 // them, never leave registers.  One gradient (forward and replay) of 512x512,
 // 32 spp, 100k triangles, 8 materials: 111 ms before, 13.1 ms so.  Jobs of a
 // batch share the waves: one step of an inverse fit of eight 128x128x16 scenes
-// 28.5 -> 5.1 ms.
+// 29 -> 5.26 ms.
 //
 // Gradients: the lanes of a warp that meet the same material reduce by
 // shuffles into the warp's sums in shared memory, the block adds its totals to
 // FP64 accumulators, and one last launch adds those to the caller's buffers.
+// The total is more exact than a thread's FP32 sums were (error against the sum
+// of 64 row bands 2.4e-8, 3.1e-7 before), but not the same from run to run: the
+// connections of a vertex are added to its G and to the light vertices' q with
+// FP32 atomics in the order in which they come, and the blocks' totals too.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -257,7 +261,8 @@ __device__ __forceinline__ V3 eval_terms(GradTerms& t, const AdjJob& J, const De
 
 // Adds the lanes' terms to the warp's sums; every lane of the warp calls it.
 // The lanes of one material pair up and halve until its first lane holds their
-// total: at most five rounds for all materials at once, where a full reduction
+// total (reduction among a warp's peers: E. Westphal, "Voting and shuffling to
+// optimize atomic operations", NVIDIA developer blog, 2015): at most five rounds for all materials at once, where a full reduction
 // per material in the warp takes up to eight times thirty shuffles (the replay
 // of 512x512x32: 9.54 ms so, 9.44 with pairs).
 __device__ __forceinline__ void add_terms(float* sums, GradTerms t)
@@ -836,19 +841,20 @@ void carve_wave(AdjWave& A, char* b, const AdjLayout& l, int njobs)
 
 // Records of one wave: up to 8 GiB, and at most half of the free memory.  Every
 // further wave pays the latency of the last, nearly empty bounces again: a
-// 512x512x32 replay with 6 bounces (14 GB of records) takes two waves, 0.34 ms
-// more than one wave of 16 GiB would (gradient step 17.05 against 16.71 ms).
+// 512x512x32 replay with 6 bounces (14 GB of records) takes two waves, 0.17 ms
+// more than one wave of 16 GiB would (gradient step 13.10 against 12.93 ms).
 constexpr size_t kAdjBudget = (size_t)8 << 30;
 constexpr int64_t kAdjMinCap = 1 << 14;  // tried at least, whatever memory is free
 
 // Where a wave's records live while its launches are in flight: a block of the
-// context's work memory, or, when the caller captures the stream into a graph, a block
-// of that graph, used by one call of the capture and by one replay of any
-// instance after another (the graph waits for and records an external event).
+// context's work memory, for the call or, when the caller captures the stream into a
+// graph, claimed for that graph, where one call of the capture and one replay of
+// any instance after another use it (the graph waits for and records an external
+// event).
 struct AdjWorkspace {
     cudaStream_t st;
     WorkBlock direct;
-    GraphMemory::Block* captured = nullptr;
+    WorkMemory::Block* captured = nullptr;
     void* base = nullptr;
     int64_t cap = 0;
     AdjWorkspace(SceneHost& s, cudaStream_t st_, int64_t total, int njobs, int B, int L, bool lights) : st(st_)
@@ -870,7 +876,7 @@ struct AdjWorkspace {
         for (;;) {
             try {
                 if (capturing) {
-                    captured = &graph_block(s, st, need(cap));
+                    captured = work_memory(s).claim(need(cap), st, &s);
                     base = captured->p;
                 } else {
                     base = direct.take(work_memory(s), need(cap), st);
@@ -882,15 +888,15 @@ struct AdjWorkspace {
             }
         }
         if (captured) {
-            if (!captured->fresh) OMV_CUDA(cudaStreamWaitEvent(st, captured->call, 0));
-            OMV_CUDA(cudaStreamWaitEvent(st, captured->instance, cudaEventWaitExternal));
+            if (captured->shared) OMV_CUDA(cudaStreamWaitEvent(st, captured->done, 0));
+            OMV_CUDA(cudaStreamWaitEvent(st, captured->replay, cudaEventWaitExternal));
         }
     }
     ~AdjWorkspace()
     {
         if (!captured) return;
-        cudaEventRecord(captured->call, st);
-        cudaEventRecordWithFlags(captured->instance, st, cudaEventRecordExternal);
+        cudaEventRecord(captured->done, st);
+        cudaEventRecordWithFlags(captured->replay, st, cudaEventRecordExternal);
     }
     AdjWorkspace(const AdjWorkspace&) = delete;
     AdjWorkspace& operator=(const AdjWorkspace&) = delete;

@@ -358,62 +358,71 @@ const SceneHost::Side* side_of(SceneHost::Side (&sides)[2], cudaStream_t st)
 
 void WorkMemory::drop(std::list<Block>::iterator b) noexcept
 {
+    const OutsideCapture outside;
     cudaFree(b->p);  // (waits for the device)
     if (b->done) cudaEventDestroy(b->done);
+    if (b->replay) cudaEventDestroy(b->replay);
     total_ -= b->bytes;
     blocks_.erase(b);
+}
+
+// idle blocks go until the others are at most `most` bytes
+void WorkMemory::drop_idle(size_t most) noexcept
+{
+    for (auto b = blocks_.begin(); b != blocks_.end() && total_ > most;) {
+        const auto next = std::next(b);
+        if (!b->busy) drop(b);
+        b = next;
+    }
+}
+
+WorkMemory::Block* WorkMemory::make(size_t bytes, cudaStream_t st, bool once)
+{
+    Block& n = blocks_.emplace_back();
+    n.bytes = bytes;
+    n.once = once;
+    n.st = st;
+    cudaError_t e = cudaEventCreateWithFlags(&n.done, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaMalloc(&n.p, bytes);
+    if (e == cudaErrorMemoryAllocation) {  // what no call uses goes first
+        (void)cudaGetLastError();
+        drop_idle(0);
+        e = cudaMalloc(&n.p, bytes);
+    }
+    total_ += bytes;
+    if (e != cudaSuccess) drop(std::prev(blocks_.end()));
+    OMV_CUDA(e);
+    return &n;
+}
+
+static bool is_over(WorkMemory::Block& b)
+{
+    if (b.pending && cudaEventQuery(b.done) == cudaSuccess) b.pending = false;
+    (void)cudaGetLastError();  // (not ready)
+    return !b.pending;
 }
 
 WorkMemory::Block* WorkMemory::take(size_t bytes, cudaStream_t st, bool once)
 {
     const OutsideCapture outside;
     const std::lock_guard<std::mutex> lock(mutex_);
-    auto over = [](Block& b) {
-        if (b.pending && cudaEventQuery(b.done) == cudaSuccess) b.pending = false;
-        (void)cudaGetLastError();  // (not ready)
-        return !b.pending;
-    };
+    end_claims();
     // the smallest idle block that fits, one that is free by now or on this stream before others
-    auto at = blocks_.end(), later = blocks_.end();
-    for (auto b = blocks_.begin(); b != blocks_.end(); ++b) {
-        if (b->busy || b->bytes < bytes) continue;
-        auto& best = b->st == st || over(*b) ? at : later;
-        if (best == blocks_.end() || b->bytes < best->bytes) best = b;
+    Block *at = nullptr, *later = nullptr;
+    for (Block& b : blocks_) {
+        if (b.busy || b.bytes < bytes) continue;
+        Block*& best = b.st == st || is_over(b) ? at : later;
+        if (!best || b.bytes < best->bytes) best = &b;
     }
-    if (at == blocks_.end() && !once && total_ + bytes > kWorkKeep) {
-        if (later != blocks_.end()) {
-            at = later;
-        } else {
-            for (auto b = blocks_.begin(); b != blocks_.end() && total_ + bytes > kWorkKeep;) {
-                const auto next = std::next(b);
-                if (!b->busy) drop(b);
-                b = next;
-            }
-        }
+    if (!at && !once && total_ + bytes > kWorkKeep) {
+        at = later;
+        if (!at) drop_idle(bytes < kWorkKeep ? kWorkKeep - bytes : 0);
     }
-    if (at == blocks_.end()) {
-        blocks_.push_back(Block{nullptr, bytes, true, st, nullptr, false, once});
-        const auto n = std::prev(blocks_.end());
-        total_ += bytes;
-        cudaError_t e = cudaEventCreateWithFlags(&n->done, cudaEventDisableTiming);
-        if (e == cudaSuccess) e = cudaMalloc(&n->p, bytes);
-        if (e == cudaErrorMemoryAllocation) {  // what no call uses goes first
-            (void)cudaGetLastError();
-            for (auto b = blocks_.begin(); b != n;) {
-                const auto next = std::next(b);
-                if (!b->busy) drop(b);
-                b = next;
-            }
-            e = cudaMalloc(&n->p, bytes);
-        }
-        if (e != cudaSuccess) drop(n);
-        OMV_CUDA(e);
-        return &*n;
-    }
+    if (!at) return make(bytes, st, once);
     if (at->pending) OMV_CUDA(cudaStreamWaitEvent(st, at->done, 0));
     at->busy = true;
     at->st = st;
-    return &*at;
+    return at;
 }
 
 void WorkMemory::give(Block* b, cudaStream_t st) noexcept
@@ -426,9 +435,67 @@ void WorkMemory::give(Block* b, cudaStream_t st) noexcept
     drop(std::find_if(blocks_.begin(), blocks_.end(), [b](const Block& x) { return &x == b; }));
 }
 
+namespace {
+
+// runs when the last of a graph and its instances is gone, on a thread that may
+// make no CUDA call and wait for none (a claimed block stays where it is)
+void CUDART_CB graph_gone(void* block) { static_cast<WorkMemory::Block*>(block)->gone.store(true); }
+
+}  // namespace
+
+WorkMemory::Block* WorkMemory::claim(size_t bytes, cudaStream_t st, const void* handle)
+{
+    const OutsideCapture outside;
+    unsigned long long id = 0;
+    cudaGraph_t graph = nullptr;
+    if (!capture_of(st, id, &graph) || !graph) throw CudaError("the stream is not being captured");
+    Block* at = nullptr;
+    {
+        const std::lock_guard<std::mutex> lock(mutex_);
+        end_claims();
+        for (Block& b : blocks_)
+            if (b.busy && b.capture == id && b.handle == handle && b.bytes >= bytes) {
+                b.shared = true;
+                return &b;
+            }
+        // an idle block that is not much too large, else a new one
+        for (Block& b : blocks_)
+            if (!b.busy && b.bytes >= bytes && b.bytes / 2 <= bytes && is_over(b) && (!at || b.bytes < at->bytes)) at = &b;
+        if (!at) at = make(bytes, st, false);
+        at->busy = true;
+        at->shared = false;
+        at->capture = id;
+        at->handle = handle;
+        total_ -= at->bytes;
+    }
+    cudaError_t e = at->replay ? cudaSuccess : cudaEventCreateWithFlags(&at->replay, cudaEventDisableTiming);
+    cudaUserObject_t object = nullptr;
+    if (e == cudaSuccess) e = cudaUserObjectCreate(&object, at, graph_gone, 1, cudaUserObjectNoDestructorSync);
+    if (e != cudaSuccess) {
+        at->gone.store(true);
+    } else if ((e = cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove)) != cudaSuccess) {
+        cudaUserObjectRelease(object, 1);  // (graph_gone)
+    }
+    OMV_CUDA(e);
+    return at;
+}
+
+// blocks whose graphs are gone
+void WorkMemory::end_claims() noexcept
+{
+    for (Block& b : blocks_)
+        if (b.capture != 0 && b.gone.exchange(false)) {
+            b.busy = b.pending = false;
+            b.capture = 0;
+            b.st = nullptr;
+            total_ += b.bytes;
+        }
+}
+
 size_t WorkMemory::idle(size_t* largest)
 {
     const std::lock_guard<std::mutex> lock(mutex_);
+    end_claims();
     size_t n = 0;
     *largest = 0;
     for (const Block& b : blocks_)
@@ -442,14 +509,15 @@ size_t WorkMemory::idle(size_t* largest)
 void WorkMemory::enter()
 {
     const std::lock_guard<std::mutex> lock(mutex_);
-    ++users_;
+    end_claims();
+    if (users_++ == 0) drop_idle(0);  // of graphs that outlived the last handle
 }
 
 void WorkMemory::leave() noexcept
 {
     const std::lock_guard<std::mutex> lock(mutex_);
-    if (--users_ > 0) return;
-    while (!blocks_.empty()) drop(blocks_.begin());
+    end_claims();
+    if (--users_ == 0) drop_idle(0);
 }
 
 // a number of the current context (a device reset makes a new one)
@@ -480,92 +548,6 @@ WorkMemory& work_memory(SceneHost& s)
     return *s.work;
 }
 
-namespace {
-
-// a graph's claim on a block; the callback runs when the last of the graph and its
-// instances is gone, on a thread that may make no CUDA call
-struct GraphClaim {
-    std::shared_ptr<GraphMemory> memory;
-    void* p;
-};
-void CUDART_CB end_claim(void* arg)
-{
-    const std::unique_ptr<GraphClaim> claim(static_cast<GraphClaim*>(arg));
-    const std::lock_guard<std::mutex> lock(claim->memory->mutex);
-    for (GraphMemory::Block& b : claim->memory->blocks)
-        if (b.p == claim->p) {
-            b.used = false;
-            b.capture = 0;
-        }
-}
-
-void free_block(const GraphMemory::Block& b)
-{
-    cudaFree(b.p);
-    if (b.used) return;  // a graph still holds the events
-    if (b.call) cudaEventDestroy(b.call);
-    if (b.instance) cudaEventDestroy(b.instance);
-}
-
-// an unclaimed block of at least `bytes`, or a new one in place of all that no graph claims
-GraphMemory::Block& take_block(GraphMemory& m, size_t bytes)
-{
-    GraphMemory::Block* best = nullptr;
-    for (GraphMemory::Block& b : m.blocks)
-        if (!b.used && b.bytes >= bytes && (!best || b.bytes < best->bytes)) best = &b;
-    if (best) return *best;
-    for (auto b = m.blocks.begin(); b != m.blocks.end();) {
-        if (!b->used) {
-            free_block(*b);
-            b = m.blocks.erase(b);
-        } else {
-            ++b;
-        }
-    }
-    GraphMemory::Block b;
-    b.bytes = bytes;
-    try {
-        OMV_CUDA(cudaEventCreateWithFlags(&b.call, cudaEventDisableTiming));
-        OMV_CUDA(cudaEventCreateWithFlags(&b.instance, cudaEventDisableTiming));
-        OMV_CUDA(cudaMalloc(&b.p, bytes));
-        m.blocks.push_back(b);
-    } catch (...) {
-        free_block(b);
-        throw;
-    }
-    return m.blocks.back();
-}
-
-}  // namespace
-
-GraphMemory::Block& graph_block(SceneHost& s, cudaStream_t st, size_t bytes)
-{
-    const OutsideCapture outside;
-    unsigned long long id = 0;
-    cudaGraph_t graph = nullptr;
-    if (!capture_of(st, id, &graph) || !graph) throw CudaError("the stream is not being captured");
-    GraphMemory& m = *s.graph_memory;
-    std::unique_lock<std::mutex> lock(m.mutex);
-    for (GraphMemory::Block& b : m.blocks)
-        if (b.used && b.capture == id && b.bytes >= bytes) {
-            b.fresh = false;
-            return b;
-        }
-    GraphMemory::Block& b = take_block(m, bytes);
-    std::unique_ptr<GraphClaim> claim(new GraphClaim{s.graph_memory, b.p});
-    cudaUserObject_t object = nullptr;
-    OMV_CUDA(cudaUserObjectCreate(&object, claim.get(), end_claim, 1, cudaUserObjectNoDestructorSync));
-    claim.release();
-    b.used = true;
-    b.capture = id;
-    b.fresh = true;
-    lock.unlock();
-    const cudaError_t e = cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove);
-    if (e != cudaSuccess) cudaUserObjectRelease(object, 1);  // ends the claim
-    OMV_CUDA(e);
-    return b;
-}
-
 SceneHost::~SceneHost()
 {
     if (device >= 0) cudaSetDevice(device);
@@ -576,11 +558,6 @@ SceneHost::~SceneHost()
     // the next call, which would be the next scene's first allocation
     if (scratch.base) cudaFree(scratch.base);
     for (void* p : allocs) cudaFree(p);
-    {
-        const std::lock_guard<std::mutex> lock(graph_memory->mutex);
-        for (const GraphMemory::Block& b : graph_memory->blocks) free_block(b);
-        graph_memory->blocks.clear();
-    }
     if (mat_sets) cudaFree(mat_sets);
     if (d_jobs) cudaFree(d_jobs);
     if (batch_graph) cudaGraphExecDestroy(batch_graph);

@@ -4,10 +4,10 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <functional>
 #include <list>
-#include <memory>
 #include <mutex>
 #include <stdexcept>
 #include <string>
@@ -106,6 +106,20 @@ struct ScenePart {
     int32_t mat_base = 0, mat_count = 0;  // without the shared missing material
 };
 
+// While it lives, this thread may make calls that an open capture forbids (they
+// take no part in it).
+struct OutsideCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    const bool set = cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess;
+    OutsideCapture() = default;
+    ~OutsideCapture()
+    {
+        if (set) cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+    OutsideCapture(const OutsideCapture&) = delete;
+    OutsideCapture& operator=(const OutsideCapture&) = delete;
+};
+
 // Device memory for what one call needs besides the wave scratch, shared by all
 // handles of a context: no handle keeps such memory of its own.  A block that a call
 // has given back is taken again by the next one that it fits, which waits on its
@@ -113,30 +127,47 @@ struct ScenePart {
 // own while all of them are at most kWorkKeep bytes.  With the context's last handle
 // everything is freed.  (A CUDA memory pool does the same by itself, but takes 6.8 ms for
 // a first block of 8 GiB and 2.5 ms for the first of a process.)
+//
+// A call that is captured claims a block for its graph, until the graph and its
+// instances are gone: replays may run beside any other call.  The calls of one
+// handle in one capture share a block, one after another, and so do the replays.
 class WorkMemory {
 public:
     struct Block {
-        void* p;
-        size_t bytes;
-        bool busy;
-        cudaStream_t st;   // of the last call
-        cudaEvent_t done;  // its end
-        bool pending;      // `done` was recorded and not seen to be over
-        bool once;         // not kept
+        void* p = nullptr;
+        size_t bytes = 0;
+        bool busy = true;
+        bool once = false;     // not kept
+        cudaStream_t st = nullptr;     // of the last call
+        cudaEvent_t done = nullptr;    // its end
+        bool pending = false;  // `done` was recorded and not seen to be over
+        // of a claimed block: its graph's capture and the handle that it is for, whether
+        // an earlier call uses it (`done` is then its end, within the capture), the end of
+        // the last replay (an external event of the graph), and whether the graph is gone
+        unsigned long long capture = 0;
+        const void* handle = nullptr;
+        bool shared = false;
+        cudaEvent_t replay = nullptr;
+        std::atomic<bool> gone{false};
     };
     // (DeviceOutOfMemory when there is no room); `once`: a block that is made for the
     // call is not kept, and the call waits for its work before it gives it back
     Block* take(size_t bytes, cudaStream_t st, bool once);
     void give(Block* b, cudaStream_t st) noexcept;
+    // for the handle's call that is being captured on `st`
+    Block* claim(size_t bytes, cudaStream_t st, const void* handle);
     size_t idle(size_t* largest);  // bytes that no call uses
     void enter();                  // a handle that uses it
     void leave() noexcept;
 
 private:
+    Block* make(size_t bytes, cudaStream_t st, bool once);
+    void end_claims() noexcept;
     void drop(std::list<Block>::iterator b) noexcept;
+    void drop_idle(size_t most) noexcept;
     std::mutex mutex_;
     std::list<Block> blocks_;
-    size_t total_ = 0;
+    size_t total_ = 0;  // without claimed blocks
     int users_ = 0;
 };
 constexpr size_t kWorkKeep = ((size_t)8 << 30) + ((size_t)256 << 20);
@@ -159,25 +190,6 @@ struct WorkBlock {
         st = stream;
         return block->p;
     }
-};
-
-// Device memory of captured calls: a block belongs to the graph that calls were
-// captured into until the graph and its instances are gone, and then to the next
-// capture that it fits.  A replay may run beside any other call, so captured calls
-// use no buffer of the handle that another call may use or replace.  The calls of
-// one capture share a block, one after another, and so do the replays.
-struct GraphMemory {
-    struct Block {
-        void* p = nullptr;
-        size_t bytes = 0;
-        bool used = false;
-        unsigned long long capture = 0;
-        bool fresh = false;               // no earlier call of the capture uses it
-        cudaEvent_t call = nullptr;       // the last call of the capture
-        cudaEvent_t instance = nullptr;   // the last replay (an external event of the graph)
-    };
-    std::mutex mutex;
-    std::list<Block> blocks;
 };
 
 struct SceneHost {
@@ -223,7 +235,6 @@ struct SceneHost {
     std::vector<ScenePart> parts;            // the scenes of a group (one for a single scene)
     std::once_flag work_once;
     WorkMemory* work = nullptr;              // work_memory
-    std::shared_ptr<GraphMemory> graph_memory = std::make_shared<GraphMemory>();
     std::mutex adj_mutex;                    // one adjoint call at a time enqueues
 
     ~SceneHost();
@@ -242,23 +253,10 @@ struct SceneHost {
 // captured ones have a side each, and a second capture that is open at the same time has
 // none (null): its work runs in line.
 const SceneHost::Side* side_of(SceneHost::Side (&sides)[2], cudaStream_t st);
-// While it lives, this thread may make calls that an open capture forbids (they
-// take no part in it).
-struct OutsideCapture {
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    OutsideCapture() { OMV_CUDA(cudaThreadExchangeStreamCaptureMode(&mode)); }
-    ~OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-    OutsideCapture(const OutsideCapture&) = delete;
-    OutsideCapture& operator=(const OutsideCapture&) = delete;
-};
-
 // that of the handle's context
 WorkMemory& work_memory(SceneHost& s);
 // whether `st` is being captured into a graph
 bool is_captured(cudaStream_t st);
-// a block of at least `bytes` for the call that is being captured on `st`
-// (DeviceOutOfMemory when there is none)
-GraphMemory::Block& graph_block(SceneHost& s, cudaStream_t st, size_t bytes);
 // orders the side stream after what `st` holds so far, and `st` after the side's
 inline void fork_side(const SceneHost::Side& x, cudaStream_t st)
 {

@@ -291,6 +291,37 @@ def test_instances_and_direct_gradients_on_their_own_streams(gpu, scenes, torch)
         w.check(direct, want, 20)
 
 
+def test_gradients_of_two_handles_in_one_capture(gpu, scenes, torch):
+    """Two handles on branches side by side, one graph after another: blocks of graphs that are gone serve the next capture
+    and the direct calls, of either handle."""
+    a, b = Gradient(gpu, scenes, torch, side=96, spp=32), Gradient(gpu, scenes, torch, side=40, spp=20)
+    wa, wb, oa, ob = _want(torch, a), _want(torch, b), a.buffers(), b.buffers()
+    branch, fork, join = torch.cuda.Stream(), torch.cuda.Event(), torch.cuda.Event()
+    torch.cuda.synchronize()
+    for _ in range(6):
+        with Graph(torch, "thread_local") as g:
+            g.begin()
+            fork.record(g.stream)
+            branch.wait_event(fork)
+            a.call(g.stream, oa)
+            b.call(branch, ob)
+            b.call(branch, ob)
+            join.record(branch)
+            a.call(g.stream, oa)
+            g.stream.wait_event(join)
+            g.end()
+            e0, e1 = g.instantiate(), g.instantiate()
+            for _ in range(3):
+                g.launch(e0)
+                g._ok(g.cu.cuGraphLaunch(e1, C.c_void_p(branch.cuda_stream)))
+            torch.cuda.synchronize()
+        a.call(g.stream, oa)
+        b.call(branch, ob)
+    torch.cuda.synchronize()
+    a.check(oa, wa, 6 * 13)
+    b.check(ob, wb, 6 * 13)
+
+
 def test_gradients_of_one_capture_share_their_records(gpu, scenes, torch):
     """Graphs of 16 gradients of 1.2 GB of records each, one graph after another, leave less than 3 GiB behind."""
     w = Gradient(gpu, scenes, torch, side=128, spp=64)
