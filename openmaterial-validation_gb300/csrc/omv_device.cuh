@@ -263,14 +263,18 @@ struct BsdfIn {
 };
 
 // BSDFModel::evaluate (BRDFModel.h:139-207): kind 0 diffuse, 1 specular, 2
-// transmitted.  Shading is bound by instruction fetch as much as by anything
-// else once a launch's lanes take different branches: every function of the
-// material model is kept to one copy per kernel (the branches of a sample meet
-// again before the azimuth, the evaluation and the Fresnel terms), which took
-// k_camera_shade from 152 to 84 KB of code and k_light_shade from 107 to 61:
-// k_camera_shade of a 641x479x17 textured frame 1720 -> 1040 us, of a
-// 1920x1080x64 point-light frame 10.6 -> 9.3 ms; the backward launches of a
-// 512x512x32 replay (168 -> 93 KB) 3.2 -> 1.55 ms.
+// transmitted.  Where a launch's lanes take different branches, shading waits
+// for instructions as much as for anything else: of a warp's stall cycles per
+// issue, "no instruction" is 6.0 of 12 on the second bounce of a 641x479x17
+// textured frame and 3.8 of 10 in the replay's k_adj_camera_back (on the sky scene,
+// whose materials are one kind, 0.5 of 11: there it waits for the gathers).  So
+// every function of the material model is kept to one copy per kernel (the
+// branches of a sample meet again before the azimuth, the evaluation and the
+// Fresnel terms), which took k_camera_shade from 152 to 84 KB of code,
+// k_light_shade from 107 to 60 and k_adj_camera_back from 168 to 83:
+// k_camera_shade of the textured frame 1720 -> 1040 us, of a 1920x1080x64
+// point-light frame 10.6 -> 9.3 ms; the backward launches of a 512x512x32 replay
+// 3.2 -> 1.55 ms.
 __device__ __forceinline__ V3 bsdf_evaluate(V3 vIn, V3 vOut, V3 norm, const float* color, float metal, float alpha,
                                             int kind, V3 Hext, float p)
 {

@@ -219,7 +219,8 @@ __device__ __forceinline__ Sorted3 sort3(float a, float b, float c)
     return Sorted3{fminf(fminf(a, b), c), med3(a, b, c), fmaxf(fmaxf(a, b), c)};
 }
 // the median of nine from three sorted triples: the middle of the largest
-// minimum, the middle median and the smallest maximum
+// minimum, the middle median and the smallest maximum (J. L. Smith,
+// "Implementing median filters in XC4000E FPGAs", XCell 23, 1996)
 __device__ __forceinline__ float median9(Sorted3 p, Sorted3 q, Sorted3 r)
 {
     return med3(fmaxf(fmaxf(p.lo, q.lo), r.lo), med3(p.mid, q.mid, r.mid), fminf(fminf(p.hi, q.hi), r.hi));
@@ -354,7 +355,9 @@ struct MedianStep<H, 3> {
     }
 };
 
-// 5x5 and 7x7 medians by forgetful selection: of the first half of the window
+// 5x5 and 7x7 medians by forgetful selection (Perrot, Domas and Couturier,
+// "Fine-tuned high-speed implementation of a GPU-based median filter", J. Signal
+// Processing Systems 75, 2014): of the first half of the window
 // and two more, neither the smallest nor the largest can be the median, so
 // both are dropped, one more element is taken in, and so on.  1920x1080, 5x5:
 // 673 us with a rank count of every element (N^2 comparisons per channel), 99

@@ -248,9 +248,10 @@ __device__ __forceinline__ void next_step(RayShares& s, uint32_t take, uint32_t 
 
 // Queues of at most this many rays are traced with eight lanes per ray
 // (coop_trace), longer ones with one ray per thread: a 256x256x16 point-light
-// frame 1121 us with the line at 2^15 (1119 at 2^16, 1142 at 2^14, 1155 at
-// 2^17; 1245 without the eight-lane path), a 64x64x1 one 532 (728), an
-// eight-scene inverse-fit step 5.78 ms (5.78, 5.91, 5.94; 5.99).
+// frame 947 us with the line at 2^15 (952 at 2^14, 959 at 2^16, 1013 at 2^17),
+// an eight-scene inverse-fit step 5.26 ms (5.25, 5.28, 5.51).  What the path
+// gave when it was added, before the second stream: the same frame 1245 -> 1121
+// us, a 64x64x1 one 728 -> 532, the step 5.99 -> 5.78 ms.
 constexpr uint32_t kCoopRays = 1u << 15;
 static_assert(kStackShared * kTraceThreads >= kStackTotal * (kTraceThreads / kCoopLanes),
               "the groups of a block share its stacks' memory");
