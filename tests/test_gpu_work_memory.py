@@ -85,3 +85,64 @@ def test_ray_queries_of_mixed_sizes_keep_little(gpu):
     r = subprocess.run([sys.executable, "-c", _SIZES, ROOT], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
     assert int(r.stdout.split("RESULT")[1]) < 640 << 20
+
+
+def test_handles_on_threads_of_their_own(gpu, scenes):
+    """Four threads, each with a handle and a stream: gradients of two sizes and ray queries of two, all at once, are those
+    of calls one after another."""
+    import ctypes as C
+    import threading
+
+    import numpy as np
+
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(2)
+    rays = np.zeros((40_000, 8), np.float32)
+    rays[:, 0:3], rays[:, 4:7], rays[:, 7] = rng.uniform(-2, 2, (len(rays), 3)) + [0, 0, 6], rng.normal(size=(len(rays), 3)), 3e38
+    work = []
+    for k in range(4):
+        sc = scenes.scene_materials(64, 64, 1, tris=4_000, n_materials=4, bounces=4, seed=k)
+        w = {"sc": sc, "rs": gpu.RenderScene(sc), "stream": torch.cuda.Stream(), "cam": gpu.PinholeCamera.from_spec(sc.camera).to_c(),
+             "adj": torch.rand((64, 64, 3), device="cuda", generator=torch.Generator(device="cuda").manual_seed(k)) - 0.3}
+        w["prm"] = [gpu.RendererParameters.for_scene(sc, seed=k, samplesPerPixel=spp).to_c() for spp in (16, 48)]
+        work.append(w)
+
+    def grad(w, i, out):
+        gpu.check(gpu.lib().omv_adjoint(w["rs"].handle, C.byref(w["cam"]), C.byref(w["prm"][i]), C.c_void_p(w["adj"].data_ptr()),
+                                        C.c_void_p(out.data_ptr()), C.c_void_p(w["stream"].cuda_stream)))
+
+    new = lambda w: torch.zeros((len(w["sc"].materials), 11), device="cuda")
+    want = [[new(w), new(w)] for w in work]
+    outs = [[new(w), new(w)] for w in work]
+    torch.cuda.synchronize()
+    hits = []
+    for w, g in zip(work, want):
+        for i in (0, 1):
+            grad(w, i, g[i])
+        torch.cuda.synchronize()
+        hits.append([w["rs"].trace(rays[:n]) for n in (3_000, 40_000)])
+    errors = []
+
+    def run(k):
+        try:
+            torch.cuda.set_device(0)
+            for step in range(12):
+                i = (step + k) % 2
+                grad(work[k], i, outs[k][i])
+                got = work[k]["rs"].trace(rays[:(3_000, 40_000)[1 - i]])
+                if not np.array_equal(got.view(np.uint32), hits[k][1 - i].view(np.uint32)):
+                    errors.append((k, step))
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    threads = [threading.Thread(target=run, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not errors, errors
+    for g, w in zip(outs, want):
+        for a, b in zip(g, w):
+            scale = float(b.abs().max())
+            assert scale > 0 and float((a - 6 * b).abs().max()) <= 1e-4 * 6 * scale
