@@ -338,3 +338,34 @@ def test_gradients_of_one_capture_share_their_records(gpu, scenes, torch):
             torch.cuda.synchronize()
     assert free0 - torch.cuda.mem_get_info()[0] < 3 * 2**30
     w.check(out, want, 128)
+
+
+def test_clone_and_child_graph_keep_the_records(gpu, scenes, torch):
+    """A clone of a captured gradient and a graph that holds it as a child outlive the captured graph, with its records:
+    direct calls and another capture in between have their own."""
+    w = Gradient(gpu, scenes, torch)
+    want, out, other = _want(torch, w), w.buffers(), w.buffers()
+    torch.cuda.synchronize()
+    with Graph(torch, "relaxed") as clone, Graph(torch, "relaxed") as parent:
+        with Graph(torch, "relaxed") as g:
+            g.begin()
+            w.call(g.stream, out)
+            g.end()
+            g._ok(g.cu.cuGraphClone(C.byref(clone.graph), g.graph))
+            g._ok(g.cu.cuGraphCreate(C.byref(parent.graph), 0))
+            node = C.c_void_p()
+            g._ok(g.cu.cuGraphAddChildGraphNode(C.byref(node), parent.graph, None, C.c_size_t(0), g.graph))
+        ec, ep = clone.instantiate(), parent.instantiate()
+        with Graph(torch, "relaxed") as later:
+            later.begin()
+            w.call(later.stream, other)
+            later.end()
+            el = later.instantiate()
+            for _ in range(5):
+                clone.launch(ec)
+                parent.launch(ep)
+                later.launch(el)
+                w.call(torch.cuda.current_stream(), other)
+            torch.cuda.synchronize()
+        w.check(out, want, 10)
+        w.check(other, want, 10)
